@@ -74,10 +74,7 @@ __global__ void __launch_bounds__(ATQ_THREADS, 2) attention_qh_kernel(const floa
                                                                    __half * __restrict__ kcache, __half * __restrict__ vcache, const uint8_t * __restrict__ mask,
                                                                    const int32_t * __restrict__ scalars, const uint16_t * __restrict__ exp_lut,
                                                                    int E, int GQA, int n_ctx, float kq_scale, float * __restrict__ out,
-                                                                   const int * __restrict__ cancel, int gdiv, int vcap, int early) {
-    // early == 0: the launch before this one may still be writing cache rows this one reads (the attention of the previous chunk
-    // of a wide prompt pass, engine.cu run_prompt_pass): nothing is fetched ahead of the wait then
-    if (!early) pib_pdl_wait();
+                                                                   const int * __restrict__ cancel, int gdiv, int vcap) {
     extern __shared__ float smem[];
     __shared__ __align__(16) float sq[HD];
     __shared__ float  s_redf[ATQ_THREADS / 32];
@@ -298,7 +295,7 @@ __global__ void __launch_bounds__(ATQ_THREADS, 2) attention_qh_kernel(const floa
 template <int HD>
 static int launch_att_qh(const float * qkv, const float * vsep, const uint8_t * desc, const float2 * rope, int rope_n_pos, int mode, __half * kc, __half * vc,
                          const uint8_t * mask, const int32_t * scalars, int E, int GQA, int n_ctx, int n_tokens, int n_head, int gdiv, float * out,
-                         const int * cancel, cudaStream_t st, int early) {
+                         const int * cancel, cudaStream_t st) {
     const int    vcap = std::min(n_ctx, ATQ_VCAP);
     const size_t smem = ((size_t) n_ctx + 32 * HD) * sizeof(float) + (size_t) vcap * HD * sizeof(__half);   // scores + 32 x HD partial sums + staged V rows
     static size_t configured = 0;
@@ -309,7 +306,7 @@ static int launch_att_qh(const float * qkv, const float * vsep, const uint8_t * 
         configured = smem;
     }
     pib_launch(attention_qh_kernel<HD>, dim3(n_head, n_tokens), dim3(ATQ_THREADS), smem, st, qkv, vsep, desc, rope, rope_n_pos, mode, kc, vc, mask, scalars,
-               pib_get_luts().exp_f16, E, GQA, n_ctx, 1.0f / sqrtf((float) HD), out, cancel, gdiv, vcap, early);
+               pib_get_luts().exp_f16, E, GQA, n_ctx, 1.0f / sqrtf((float) HD), out, cancel, gdiv, vcap);
     PIB_CHECK(cudaGetLastError());
     return PIB_OK;
 }
@@ -324,10 +321,10 @@ bool pib_attention_supported(int hd, int n_head, int n_head_kv, int n_ctx) {
 // (or [E + GQA] with V in vsep)
 int pib_attention(const float * qkv, const float * vsep, const uint8_t * desc, const float2 * rope, int rope_n_pos, int mode, __half * kc, __half * vc,
                   const uint8_t * mask, const int32_t * scalars, int n_tokens, int n_head, int n_head_kv, int hd, int n_ctx, float * out,
-                  const int * cancel, cudaStream_t st, bool cache_final) {
+                  const int * cancel, cudaStream_t st) {
     const int E = n_head * hd, GQA = n_head_kv * hd, G = n_head / n_head_kv;
-    if (hd == 128) return launch_att_qh<128>(qkv, vsep, desc, rope, rope_n_pos, mode, kc, vc, mask, scalars, E, GQA, n_ctx, n_tokens, n_head, G, out, cancel, st, cache_final ? 1 : 0);
-    if (hd == 64)  return launch_att_qh<64>(qkv, vsep, desc, rope, rope_n_pos, mode, kc, vc, mask, scalars, E, GQA, n_ctx, n_tokens, n_head, G, out, cancel, st, cache_final ? 1 : 0);
+    if (hd == 128) return launch_att_qh<128>(qkv, vsep, desc, rope, rope_n_pos, mode, kc, vc, mask, scalars, E, GQA, n_ctx, n_tokens, n_head, G, out, cancel, st);
+    if (hd == 64)  return launch_att_qh<64>(qkv, vsep, desc, rope, rope_n_pos, mode, kc, vc, mask, scalars, E, GQA, n_ctx, n_tokens, n_head, G, out, cancel, st);
     pib_set_error("attention: unsupported head_dim %d", hd);
     return PIB_ERR_UNSUPP;
 }

@@ -39,7 +39,11 @@ void rope_table_build(std::vector<float2> & tab, int n_pos, int n_dims, int mode
 bool pib_attention_supported(int hd, int n_head, int n_head_kv, int n_ctx);
 int  pib_attention(const float * qkv, const float * vsep, const uint8_t * desc, const float2 * rope, int rope_n_pos, int mode, __half * kc, __half * vc,
                    const uint8_t * mask, const int32_t * scalars, int n_tokens, int n_head, int n_head_kv, int hd, int n_ctx, float * out,
-                   const int * cancel, cudaStream_t st, bool cache_final);
+                   const int * cancel, cudaStream_t st);
+bool pib_prompt_attention_supported(int hd, int n_ctx);                       // prompt_attn.cu
+int  pib_prompt_gather(const uint8_t * desc_base, size_t stride, const pib_prompt_slots & sl, int ntok, int W, int32_t * tok, int32_t * pos, int32_t * cell, uint32_t * bits, cudaStream_t st);
+int  pib_prompt_attention(const float * qkv, const int32_t * pos, const int32_t * cell, const float2 * rope, int rope_n_pos, __half * q16, __half * kc, __half * vc, const uint8_t * mask,
+                          const int32_t * scalars, int ntok, int n_head, int n_head_kv, int hd, int n_ctx, float * out, const int * cancel, cudaStream_t st);
 int  pib_sample_topk(float * logits_dev, int n_rows, int n_vocab, const int32_t * bias_ids_dev, const float * bias_val_dev, int n_bias,
                      void * out_dev, const uint8_t * desc, const int * cancel, cudaStream_t st);
 int  pib_gemm_q4k_tc(const pib_weight * w, const void * act_dev, int b, float * y_dev, void * xhat_dev, cudaStream_t st);
@@ -518,7 +522,7 @@ void pib_context_free(pib_context * c) {
     pib_hybrid_ctx_free(c);
     pib_pipe_hop_free(c);
     for (void * b : { (void *) c->pb.x, (void *) c->pb.x2, (void *) c->pb.qkv, (void *) c->pb.att, (void *) c->pb.proj, (void *) c->pb.gu,
-                      (void *) c->pb.mask, c->pb.act, c->pb.xhat }) if (b) cudaFree(b);
+                      (void *) c->pb.mask, c->pb.act, c->pb.xhat, (void *) c->pb.ids }) if (b) cudaFree(b);
     kv_device_free(&c->kvd);
     void * bufs[] = { c->vsep, c->kcache, c->vcache, c->x, c->x2, c->qkv, c->att, c->proj, c->gu, c->mask, c->act, c->rope,
                       c->cancel_table, c->desc_dev, c->ops_dev, c->bias_ids_dev, c->bias_val_dev, c->logits_fetch_dev };
@@ -659,7 +663,7 @@ static int run_chunk_body(pib_context * c, pib_run & run, int chunk, int ntok, i
             if (L.attn_norm2) TL(9, il, pib_add_layernorm_quantize_act(wt, cur, nullptr, nullptr, nullptr, L.attn_norm, L.attn_norm_b, m->norm_eps, ntok, E, c->act, cancel, st));
             GEMV(2, il, L.wgu, c->gu);
             TL(7, il, pib_attention(c->qkv, nullptr, desc, c->rope, c->rope_n_pos, 2, c->kcache + lo, c->vcache + lo, c->mask, c->kvd.scalars, ntok, m->n_head,
-                                    m->n_head_kv, hd, (int) c->n_ctx, other, cancel, st, true));
+                                    m->n_head_kv, hd, (int) c->n_ctx, other, cancel, st));
             TL(8, il, pib_quantize_act_c(wt, other, ntok, E, c->act, cancel, st));
             GEMV(1, il, L.wo, c->proj);
             TL(10, il, pib_gelu_quantize_act(wt, c->gu, ntok, FF, c->act, cancel, st));
@@ -707,7 +711,7 @@ static int run_chunk_body(pib_context * c, pib_run & run, int chunk, int ntok, i
             if (pending_add) GEMVP(0, L.wqkv, 1, c->proj, L.attn_norm, c->x2, c->x, 0, m->rms_eps, ntok, c->qkv);
             else             GEMVP(0, L.wqkv, 1, c->x, L.attn_norm, nullptr, nullptr, 0, m->rms_eps, ntok, c->qkv);
             TL(7, il, pib_attention(c->qkv, nullptr, desc, c->rope, c->rope_n_pos, 0, c->kcache + lo, c->vcache + lo, c->mask, c->kvd.scalars, ntok,
-                                    m->n_head, m->n_head_kv, hd, (int) c->n_ctx, c->att, cancel, st, true));
+                                    m->n_head, m->n_head_kv, hd, (int) c->n_ctx, c->att, cancel, st));
             GEMVP(1, L.wo, 0, c->att, nullptr, nullptr, nullptr, 0, 0.f, ntok, c->proj);
             TL(9, il, pib_add_rmsnorm_quantize_act(wt, c->proj, c->x, c->x2, L.ffn_norm, m->rms_eps, ntok, E, c->act, cancel, st));   // x2 = ffn_inp
             GEMV(2, il, L.wgu, c->gu);
@@ -726,7 +730,7 @@ static int run_chunk_body(pib_context * c, pib_run & run, int chunk, int ntok, i
         dump_dev(c, "k", il, c->qkv + E, ntok, GQA, E + (L.wv ? 1 : 2) * GQA);
         if (!L.wv) dump_dev(c, "v", il, c->qkv + E + GQA, ntok, GQA, E + 2 * GQA);
         TL(7, il, pib_attention(c->qkv, L.wv ? c->vsep : nullptr, desc, c->rope, c->rope_n_pos, 0, c->kcache + lo, c->vcache + lo, c->mask, c->kvd.scalars, ntok,
-                                m->n_head, m->n_head_kv, hd, (int) c->n_ctx, c->att, cancel, st, true));
+                                m->n_head, m->n_head_kv, hd, (int) c->n_ctx, c->att, cancel, st));
         dump_dev(c, "att", il, c->att, ntok, E, E);
         TL(8, il, pib_quantize_act_c(wt, c->att, ntok, E, c->act, cancel, st));
         GEMV(1, il, L.wo, c->proj);
@@ -823,8 +827,8 @@ static int enqueue_decode(pib_context * c, pib_run * run, int n_tokens, int batc
 
 // ---- wide batches (prompt ingestion): the matmuls of up to PIB_PROMPT_MAX tokens at once on the tcgen05 GEMM -----------------------
 // The reference takes a prompt of up to n_batch = 512 tokens in one ggml_compute_forward_mul_mat per matrix (common.h:52, ggml.c:9388).
-// Here the per-token kernels (norm / quantise, RoPE + KV store, attention, ...) keep their 16-token descriptors, but every matmul of a
-// layer runs once for the whole pass.  Used for llama-architecture models whose matrices are all Q4_K, for decodes of more than two
+// Here every launch of a layer takes the whole pass (prompt_attn.cu for RoPE, KV store and attention; the row kernels take any number of rows);
+// the chunks' 16-token descriptors are spread into one array per field first.  Used for llama-architecture models whose matrices are all Q4_K, for decodes of more than two
 // chunks, outside exact mode (the GEMM is tolerance-checked, not bit-exact: gemm_q4k_tc.cu).
 static bool prompt_gemm_ok(const pib_context * c, int n_tokens) {
     const pib_model * m = c->model;
@@ -835,7 +839,7 @@ static bool prompt_gemm_ok(const pib_context * c, int n_tokens) {
         for (const pib_weight * w : { L.wqkv, L.wo, L.wgu, L.wdown }) if (!w || w->type != PIB_TYPE_Q4_K || !w->tiles) return false;
     }
     if (c->stage.last() && (!m->output || m->output->type != PIB_TYPE_Q4_K || !m->output->tiles)) return false;
-    return true;
+    return pib_prompt_attention_supported(m->head_dim(), (int) c->n_ctx);
 }
 
 static int prompt_bufs(pib_context * c) {
@@ -845,7 +849,7 @@ static int prompt_bufs(pib_context * c) {
     auto & b = c->pb;
     if (cudaMalloc(&b.x, P * E * 4) != cudaSuccess || cudaMalloc(&b.x2, P * E * 4) != cudaSuccess || cudaMalloc(&b.qkv, P * (E + 2 * GQA) * 4) != cudaSuccess ||
         cudaMalloc(&b.att, P * E * 4) != cudaSuccess || cudaMalloc(&b.proj, P * E * 4) != cudaSuccess || cudaMalloc(&b.gu, P * 2 * FF * 4) != cudaSuccess ||
-        cudaMalloc(&b.mask, P * c->n_ctx) != cudaSuccess ||
+        cudaMalloc(&b.mask, P * c->n_ctx) != cudaSuccess || cudaMalloc(&b.ids, P * (3 + (size_t) c->n_words) * 4) != cudaSuccess ||
         cudaMalloc(&b.act, pib_act_bytes(PIB_TYPE_Q4_K, (int64_t) KM, (int) P)) != cudaSuccess || cudaMalloc(&b.xhat, pib_gemm_xhat_bytes((int64_t) KM, (int) P)) != cudaSuccess) {
         cudaGetLastError();
         pib_set_error("decode: out of memory for the prompt path's work buffers");
@@ -866,14 +870,17 @@ static int run_prompt_pass(pib_context * c, pib_run & run, int ch0, int nch, int
 #define RC(e) do { rc = (e); if (rc != PIB_OK) return rc; c->n_kernels++; } while (0)
     auto desc_of = [&](int k) { return c->desc_dev + (size_t) dev_slot(c, slots[ch0 + k]) * c->desc_stride; };
     auto nt_of   = [&](int k) { return std::min(PIB_CHUNK, ntok - k * PIB_CHUNK); };
-    for (int k = 0; k < nch; k++) {
-        const uint8_t * desc = desc_of(k);
-        const size_t    off  = (size_t) k * PIB_CHUNK;
-        if (c->stage.first()) RC(pib_get_rows(m->tok_embd, reinterpret_cast<const int32_t *>(desc + PIB_DESC_TOK_OFF), nt_of(k), B.x + off * E, st));
-        else if (c->hop_peer) { RC(pib_hop_recv_launch(c, nt_of(k), st)); cudaMemcpyAsync(B.x + off * E, c->x, (size_t) nt_of(k) * E * 4, cudaMemcpyDeviceToDevice, st); }
+    int32_t *  ids = B.ids, * pos = ids + PIB_PROMPT_MAX, * cell = pos + PIB_PROMPT_MAX;
+    uint32_t * bits = reinterpret_cast<uint32_t *>(cell + PIB_PROMPT_MAX);
+    pib_prompt_slots sl;
+    for (int k = 0; k < PIB_PROMPT_MAX / PIB_CHUNK; k++) sl.slot[k] = dev_slot(c, slots[ch0 + std::min(k, nch - 1)]);
+    RC(pib_prompt_gather(c->desc_dev, c->desc_stride, sl, ntok, c->n_words, ids, pos, cell, bits, st));
+    RC(kv_device_mask(&c->kvd, pos, bits, ntok, B.mask, st));
+    if (c->stage.first()) RC(pib_get_rows(m->tok_embd, ids, ntok, B.x, st));
+    else for (int k = 0; k < nch; k++) {
+        const size_t off = (size_t) k * PIB_CHUNK;
+        if (c->hop_peer) { RC(pib_hop_recv_launch(c, nt_of(k), st)); cudaMemcpyAsync(B.x + off * E, c->x, (size_t) nt_of(k) * E * 4, cudaMemcpyDeviceToDevice, st); }
         else if (pib_hop_recv) RC(pib_hop_recv(c, B.x + off * E, nt_of(k), cancel));
-        RC(kv_device_mask(&c->kvd, reinterpret_cast<const int32_t *>(desc + PIB_DESC_POS_OFF), reinterpret_cast<const uint32_t *>(desc + PIB_DESC_BITS_OFF), nt_of(k),
-                          B.mask + off * c->n_ctx, st));
     }
     bool pending_add = false;
     for (int il = m->layer_begin; il < m->layer_end; il++) {
@@ -882,11 +889,10 @@ static int run_prompt_pass(pib_context * c, pib_run & run, int ch0, int nch, int
         if (pending_add) RC(pib_add_rmsnorm_quantize_act(wt, B.proj, B.x2, B.x, L.attn_norm, m->rms_eps, ntok, E, B.act, cancel, st));
         else             RC(pib_add_rmsnorm_quantize_act(wt, B.x, nullptr, nullptr, L.attn_norm, m->rms_eps, ntok, E, B.act, cancel, st));
         RC(pib_gemm_q4k_tc(L.wqkv, B.act, ntok, B.qkv, B.xhat, st));
-        for (int k = 0; k < nch; k++) {          // chunk k + 1 reads chunk k's cells from the cache: stream order
-            const size_t off = (size_t) k * PIB_CHUNK;
-            RC(pib_attention(B.qkv + off * (E + 2 * GQA), nullptr, desc_of(k), c->rope, c->rope_n_pos, 0, c->kcache + lo, c->vcache + lo, B.mask + off * c->n_ctx,
-                             c->kvd.scalars, nt_of(k), m->n_head, m->n_head_kv, hd, (int) c->n_ctx, B.att + off * E, cancel, st, k == 0));
-        }
+        // the GEMM's scratch is free between two matmuls: it holds the rotated queries
+        RC(pib_prompt_attention(B.qkv, pos, cell, c->rope, c->rope_n_pos, (__half *) B.xhat, c->kcache + lo, c->vcache + lo, B.mask, c->kvd.scalars, ntok, m->n_head, m->n_head_kv, hd,
+                                (int) c->n_ctx, B.att, cancel, st));
+        c->n_kernels++;
         RC(pib_quantize_act_c(wt, B.att, ntok, E, B.act, cancel, st));
         RC(pib_gemm_q4k_tc(L.wo, B.act, ntok, B.proj, B.xhat, st));
         RC(pib_add_rmsnorm_quantize_act(wt, B.proj, B.x, B.x2, L.ffn_norm, m->rms_eps, ntok, E, B.act, cancel, st));
