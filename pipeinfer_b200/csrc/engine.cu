@@ -1079,6 +1079,7 @@ static int enqueue_decode(pib_context * c, pib_run * run, int n_tokens, int batc
             if (run_prompt_pass(c, *run, ch0, nch, ntok, slots) != PIB_OK) run->failed = true;
         }
         for (int ch = 0; ch < n_chunks; ch++) if (c->desc_ev[slots[ch]]) cudaEventRecord(c->desc_ev[slots[ch]], c->stream);
+        pib_dense_mm_check(c->stream, 1);
     } else
     for (int ch = 0; ch < n_chunks; ch++) {
         const int nt = std::min(PIB_CHUNK, n_tokens - ch * PIB_CHUNK);
@@ -1178,7 +1179,7 @@ int pib_run_finish(pib_context * c, int run) {
     clear_cancel_flag(c, r.id);
     if (c->stage.size > 1 && c->stage.first()) pib_pipe_ship_ints(2, 0, &r.batch_id, 1);
     for (auto it = c->inflight.begin(); it != c->inflight.end(); ++it) if (*it == run) { c->inflight.erase(it); break; }
-    if (c->hy && c->model->wtype == PIB_TYPE_BF16 && pib_dense_mm_check(c->stream, 0) != PIB_OK) r.failed = true;   // a tensor-core kernel gave up on a wait
+    if (((c->hy && c->model->wtype == PIB_TYPE_BF16) || c->pb.ready) && pib_dense_mm_check(c->stream, 0) != PIB_OK) r.failed = true;   // a tensor-core kernel gave up on a wait
     r.in_use         = false;
     c->last_finished = run;     // its buffers stay reserved until the next finish (llama_get_logits_ith contract)
     c->logits_row_valid.assign((size_t) r.n_tokens, 0);

@@ -1,7 +1,7 @@
-// gemm_q4k_tc.cu -- the quantised matmul (K1) for WIDE batches (prompt ingestion, 32 .. 256 tokens at once): Q4_K weights are
-// dequantised tile by tile into fp16 shared-memory operands and multiplied on the 5th-generation tensor cores (tcgen05.mma, fp32
-// accumulators in tensor memory), the activation tile arriving by TMA.  Replaces, for these batch sizes, the reference's
-// ggml_compute_forward_mul_mat at large ne11 (ggml.c:9388) / ggml_cuda_op_mul_mat_cublas (ggml-cuda.cu:6562: dequantise + cuBLAS).
+// gemm_q4k_tc.cu -- the quantised matmul (K1) for WIDE batches (prompt ingestion, 17 .. 256 tokens at once): Q4_K weights are dequantised to fp16
+// straight into tensor memory and multiplied there on the 5th-generation tensor cores (tcgen05.mma with A in tensor memory, fp32 accumulators), the
+// activation tile arriving by TMA.  Replaces, for these batch sizes, the reference's ggml_compute_forward_mul_mat at large ne11 (ggml.c:9388) /
+// ggml_cuda_op_mul_mat_cublas (ggml-cuda.cu:6562: dequantise + cuBLAS).
 //
 // Arithmetic: y[t][r] = sum_k w(r, k) * x^(t, k) with w = d * sc * q - dmin * m (the reference's dequantize_row_q4_K formula,
 // ggml-quants.c:1917) rounded to fp16, and x^ = the token's Q8_K quantised activation q8 * d (what the reference's integer dot
@@ -9,256 +9,344 @@
 // order and not bit-exact; it is checked against the oracle to a tolerance (tests/test_gpu_gemm.py) and used for prompt chunks only
 // -- verification batches (<= 16 tokens) keep the GEMV kernels.
 //
-// One CTA per 128 output rows, 10 warps:
-//   warp 0        TMA producer: the activation tile [NB tokens x 64 k] fp16 of every k-step (cp.async.bulk.tensor.2d, 128-byte swizzle)
-//   warp 1        allocates tensor memory; one elected lane issues the MMAs (4 x K=16 per k-step) and commits them to the mbarriers
-//   warps 2..9    dequantise the weight tile [128 rows x 64 k] of every k-step from the fragment-major Q4_K records into the
-//                 128-byte-swizzled K-major operand layout (two threads per row, the next k-step's bytes already in flight);
-//                 afterwards they read the accumulators back (tcgen05.ld) and store y
-// A k-step is one 64-element chunk of a super-block (low nibbles = its first 32 elements, high nibbles = the other 32).
+// A CTA owns 128 output rows and up to 256 tokens, and one share of K when a cluster splits it:
+//   warp 0          TMA: the activation tile [NB tokens x 128 k] fp16 of every k-step (cp.async.bulk.tensor.2d, 128-byte swizzle)
+//   warp 1          allocates tensor memory, issues the MMAs (8 x K=16 per k-step) and commits them to the mbarriers
+//   warp 2          weight records: one bulk copy per 16-row tile and super-block into a ring, started before the launch wait
+//   warps 3..       G groups of 8: a warp owns one 16-row tile, turns its 16-byte fragment pieces into fp16 pairs in registers and stores them with
+//                   tcgen05.st.16x256b: the record layout (lane g, t holds rows g and g + 8, gemv_mma.cu) IS that instruction's register layout, only
+//                   the order of k inside a 64-wide chunk differs, and x^ is written in the same order (tg_kpos).  Afterwards the epilogue.
+// What bounds it: up to about 100 tokens the dequantisation, 109 warp instructions per 16 rows x 64 k issued at 0.6 per clock and scheduler (57344 x 8192
+// at 40 tokens 96 us, where the weights' bytes take 40; with the operand written to and read from shared memory, the form this replaces, 173 us); with
+// 256 tokens the tensor cores and the activation tiles' way into shared memory (203 us, before 246; 151 at the dense peak).
 #include <cuda.h>
 #include <cuda_fp16.h>
 
-#include <map>
-#include <mutex>
-#include <utility>
-#include <stdlib.h>
+#include "tc_common.cuh"
 
-#include "pib_common.cuh"
-
-#define TG_BM      128                 // output rows per CTA (UMMA M)
-#define TG_BK      64                  // k elements per step (one 128-byte swizzle row of fp16)
-#define TG_PWARPS  8                   // weight-producer warps
-#define TG_THREADS (64 + TG_PWARPS * 32)
+#define TG_BM      128                 // output rows per accumulator (UMMA M)
+#define TG_BK      128                 // k elements per step (two 128-byte swizzle rows of fp16): half a super-block
 #define TG_TILE_BYTES 2304             // Q4_K record of (16 rows, 256 k), see gemv_mma.cu
 
-// ---- PTX helpers ----------------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t tg_smem(const void * p) { return (uint32_t) __cvta_generic_to_shared(p); }
-__device__ __forceinline__ void tg_mbar_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory"); }
-__device__ __forceinline__ void tg_mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
-__device__ __forceinline__ void tg_mbar_expect_tx(uint32_t bar, uint32_t bytes) { asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory"); }
-__device__ __forceinline__ void tg_mbar_wait(uint32_t bar, uint32_t parity) {
-    asm volatile("{\n\t.reg .pred p;\n\tTG_WAIT:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1;\n\t@p bra TG_DONE;\n\tbra TG_WAIT;\n\tTG_DONE:\n\t}" ::"r"(bar), "r"(parity) : "memory");
+// G groups of 8 warps feed the accumulator (G = 2: the groups take the k-steps in turn); with G = 1 two CTAs share an SM
+template <int NB, int G> struct tg_cfg {
+    static constexpr int CTAS    = 3 - G;                                // per SM
+    static constexpr int STAGES  = G == 2 ? (NB > 128 ? 2 : 4) : NB > 64 ? 2 : 3;   // k-steps of weights in tensor memory
+    static constexpr int PIECES  = NB > 128 ? 2 : 1;                     // activations arrive in pieces of a k-step: with two stages only, whole ones are late (256 tokens:
+    static constexpr int BSTAGES = PIECES * STAGES;                      // 246 -> 193 us); with more stages a second barrier per step costs more (24 tokens: 31 -> 44)
+    static constexpr int WSTAGES = NB == 128 && G == 1 ? 2 : 3;          // super-blocks of weight records in shared memory
+    static constexpr int WARPS   = 8 * G, THREADS = 96 + 32 * WARPS;
+    static constexpr int W_BYTES = 8 * TG_TILE_BYTES, B_BYTES = NB * 256 / PIECES;
+    static constexpr int TM_COLS = 512 / CTAS;                           // tensor memory: NB accumulator columns, then STAGES x 64 columns of weights
+    static constexpr int RED     = TG_BM * NB * 4;                       // the partial sums of a K split reuse the rings
+    static constexpr int SCL_OFF = BSTAGES * B_BYTES + WSTAGES * W_BYTES; // the warps' expanded scales
+    static constexpr int RING    = SCL_OFF + WARPS * 1024;
+    static constexpr int N_BAR   = 2 * (STAGES + BSTAGES + WSTAGES) + 1;
+    static constexpr int BAR_OFF = RED > RING ? RED : RING;
+    static constexpr size_t SMEM = (size_t) BAR_OFF + N_BAR * 8 + 32 + 1024;
+    static_assert(NB + STAGES * 64 <= TM_COLS && G <= STAGES, "tensor memory");
+};
+
+// place of element e of a 64-wide chunk in both operands' rows: the record's low nibbles (e < 32) come first, a lane quarter's eight as two runs of four,
+// the middle two of each run swapped (one mask of a word of nibble bytes gives the pairs (e0, e2) and (e1, e3))
+__host__ __device__ __forceinline__ int tg_kpos(int e) { return (e & 32) + ((e >> 2) & 1) * 16 + ((e >> 3) & 3) * 4 + ((e & 1) << 1 | ((e >> 1) & 1)); }
+
+// ---- x^: quantised activations back to fp16, [b][K], k order inside a chunk as above -----------------------------------------------------------
+__global__ void __launch_bounds__(256) tg_xhat_kernel(const int8_t * __restrict__ qs, const float * __restrict__ d, int64_t n16, int K16, __half * __restrict__ xh) {
+    pib_pdl_wait();
+    pib_pdl_trigger();
+    const int64_t i = (int64_t) blockIdx.x * 256 + threadIdx.x;              // sixteen consecutive elements of one row
+    if (i >= n16) return;
+    const float dx = d[(i / K16) * (K16 / 16) + (i % K16) / 16];
+    const int4  q  = reinterpret_cast<const int4 *>(qs)[i];
+    __half *    o  = xh + (i >> 2) * 64;
+    const int   e0 = (int) (i & 3) * 16;
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const int w = u == 0 ? q.x : u == 1 ? q.y : u == 2 ? q.z : q.w;
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = __fmul_rn((float) (int8_t) (w >> (8 * j)), dx);
+        const __half2 p[2] = { __floats2half2_rn(v[0], v[2]), __floats2half2_rn(v[1], v[3]) };
+        *reinterpret_cast<uint2 *>(o + tg_kpos(e0 + 4 * u)) = *reinterpret_cast<const uint2 *>(p);
+    }
 }
-__device__ __forceinline__ void tg_fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
 __device__ __forceinline__ void tg_tma_2d(uint32_t dst, const CUtensorMap * map, uint32_t bar, int x, int y) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                  ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
 }
-// shared-memory matrix descriptor: K-major operand, 128-byte swizzle, 8-row groups 1024 bytes apart (cute::UMMA::SmemDescriptor)
-__device__ __forceinline__ uint64_t tg_desc(uint32_t smem_addr) {
-    uint64_t d = 0;
-    d |= (uint64_t) ((smem_addr >> 4) & 0x3fff);              // start address
-    d |= (uint64_t) 1 << 16;                                  // leading byte offset (unused for swizzled K-major): 1
-    d |= (uint64_t) (1024 >> 4) << 32;                        // stride byte offset between 8-row groups
-    d |= (uint64_t) 1 << 46;                                  // descriptor version (Blackwell)
-    d |= (uint64_t) 2 << 61;                                  // SWIZZLE_128B
-    return d;
+__device__ __forceinline__ void tg_bulk(uint32_t dst, const void * src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void tg_mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-                 ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+// A in tensor memory, B in shared memory; called by a converged warp
+__device__ __forceinline__ void tg_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+                 ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
 }
-__device__ __forceinline__ void tg_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+// 16 lanes x 64 columns: register 4a + j of lane (g, t) is column 8a + 2t + (j & 1) of lane g + 8 (j >> 1)
+__device__ __forceinline__ void tg_st_frag(uint32_t taddr, const uint32_t (&v)[32]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+                 "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]),
+                 "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
+                 "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]) : "memory");
 }
-
-// the order in which four consecutive k elements sit in both operands' rows: (e0, e2, e1, e3).  The weight side gets pairs
-// (e0, e2) and (e1, e3) for free from one mask of a 32-bit word of nibble bytes; the activation side is written to match.
-__host__ __device__ __forceinline__ int tg_kperm(int k) { return (k & ~3) | ((k & 1) << 1) | ((k >> 1) & 1); }
-
-// ---- x^: quantised activations back to fp16, [NB rows][K], rows >= b zero, k order permuted as above -------------------------------
-__global__ void tg_xhat_kernel(const int8_t * __restrict__ qs, const float * __restrict__ d, int b, int K, __half * __restrict__ xh, int NB) {
-    const int row = blockIdx.y;
-    const int k4  = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
-    if (k4 >= K) return;
-    __half o[4];
-    if (row < b) {
-        const float dx = d[(size_t) row * (K / 256) + k4 / 256];
-        const char4 q  = *reinterpret_cast<const char4 *>(qs + (size_t) row * K + k4);
-        const float v[4] = { __fmul_rn((float) q.x, dx), __fmul_rn((float) q.y, dx), __fmul_rn((float) q.z, dx), __fmul_rn((float) q.w, dx) };
-        o[0] = __float2half_rn(v[0]); o[1] = __float2half_rn(v[2]); o[2] = __float2half_rn(v[1]); o[3] = __float2half_rn(v[3]);
-    } else {
-        o[0] = o[1] = o[2] = o[3] = __float2half_rn(0.f);
+// Waits are bounded: TG_TRIES tries, then the block's abort flag is raised and every role gives up.  The weight producer, which is a whole
+// super-block or two ahead, sleeps in the barrier unit (up to NAP ns a try) and leaves its issue slots to the others; those poll, because a sleeper wakes late.
+#define TG_TRIES (1 << 20)
+template <uint32_t NAP> __device__ __forceinline__ uint32_t tg_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    if (NAP) asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity), "r"(NAP) : "memory");
+    else     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok;
+}
+// by a whole warp, which leaves together: what follows are .sync.aligned instructions, and lanes that left one by one would run them in parts
+template <uint32_t NAP = 0> __device__ __forceinline__ bool tg_wait(uint32_t bar, uint32_t parity, volatile int * abort_s) {
+    for (int it = 0; it < TG_TRIES; it++) {
+        if (__all_sync(0xffffffffu, tg_try<NAP>(bar, parity))) return true;
+        if ((it & 15) == 15 && __any_sync(0xffffffffu, *abort_s)) return false;
     }
-    *reinterpret_cast<uint2 *>(xh + (size_t) row * K + k4) = *reinterpret_cast<const uint2 *>(o);
-    (void) NB;
+    *abort_s = 1;
+    return false;
+}
+__device__ __forceinline__ bool tg_wait1(uint32_t bar, uint32_t parity, volatile int * abort_s) {      // by one thread
+    for (int it = 0; it < TG_TRIES; it++) {
+        if (tg_try<0>(bar, parity)) return true;
+        if ((it & 15) == 15 && *abort_s) return false;
+    }
+    *abort_s = 1;
+    return false;
+}
+
+__device__ __forceinline__ __half2 tg_h2(uint32_t v) { return *reinterpret_cast<const __half2 *>(&v); }
+__device__ __forceinline__ uint32_t tg_u(__half2 v) { return *reinterpret_cast<const uint32_t *>(&v); }
+
+// {d * sc, -dmin * m} of sub-blocks 2c, 2c + 1 of one row, each twice in a word (get_scale_min_k4, ggml-quants.c:1446): d * sc has 17 bits, so the fp16
+// product is its value rounded once
+__device__ __forceinline__ uint4 tg_scales(uint4 h, int c) {
+    const uint32_t sc = c < 2 ? h.y & 0x3f3f3f3fu : (h.w & 0x0f0f0f0fu) | (((h.y >> 6) & 0x03030303u) << 4);
+    const uint32_t mn = c < 2 ? h.z & 0x3f3f3f3fu : ((h.w >> 4) & 0x0f0f0f0fu) | (((h.z >> 6) & 0x03030303u) << 4);
+    const __half2  d = __low2half2(tg_h2(h.x)), nm = __hneg2(__high2half2(tg_h2(h.x))), k1024 = __float2half2_rn(1024.f);
+    const uint32_t s0 = c & 1 ? 0x4242 : 0x4040, s1 = s0 + 0x0101;
+    return make_uint4(tg_u(__hmul2(__hsub2(tg_h2(__byte_perm(sc, 0x64646464u, s0)), k1024), d)), tg_u(__hmul2(__hsub2(tg_h2(__byte_perm(mn, 0x64646464u, s0)), k1024), nm)),
+                      tg_u(__hmul2(__hsub2(tg_h2(__byte_perm(sc, 0x64646464u, s1)), k1024), d)), tg_u(__hmul2(__hsub2(tg_h2(__byte_perm(mn, 0x64646464u, s1)), k1024), nm)));
+}
+// (v & m) | 0x6400 in both halves, in one instruction (both constants in registers): nibbles enter fp16 as 1024 + q (low) and 1024 + 16 q (high)
+__device__ __forceinline__ __half2 tg_pick(uint32_t v, uint32_t m) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(v), "r"(m), "r"(0x64006400u));
+    return tg_h2(r);
+}
+// a word of eight nibbles -> low pairs (e0, e2), (e1, e3) and high pairs, each d1 * q + o with one rounding (q comes back exactly first)
+__device__ __forceinline__ void tg_word(uint32_t v, __half2 d_lo, __half2 o_lo, __half2 d_hi, __half2 o_hi, uint32_t & l0, uint32_t & l1, uint32_t & h0, uint32_t & h1) {
+    const __half2 k1024 = __float2half2_rn(1024.f), sixteenth = __float2half2_rn(0.0625f), k64 = __float2half2_rn(-64.f);
+    const uint32_t s = v >> 8;
+    l0 = tg_u(__hfma2(__hsub2(tg_pick(v, 0x000F000Fu), k1024), d_lo, o_lo));
+    l1 = tg_u(__hfma2(__hsub2(tg_pick(s, 0x000F000Fu), k1024), d_lo, o_lo));
+    h0 = tg_u(__hfma2(__hfma2(tg_pick(v, 0x00F000F0u), sixteenth, k64), d_hi, o_hi));
+    h1 = tg_u(__hfma2(__hfma2(tg_pick(s, 0x00F000F0u), sixteenth, k64), d_hi, o_hi));
+}
+// a chunk's two pieces of one row: registers 4a + J0 + {0, 1} of the fragment
+template <int C, int J0> __device__ __forceinline__ void tg_chunk_row(uint32_t w0, uint32_t w1, uint4 f, uint32_t (&o)[32]) {
+    const __half2 dl = tg_h2(f.x), ol = tg_h2(f.y), dh = tg_h2(f.z), oh = tg_h2(f.w);
+    tg_word(w0, dl, ol, dh, oh, o[16 * C + J0], o[16 * C + J0 + 1], o[16 * C + J0 + 8], o[16 * C + J0 + 9]);
+    tg_word(w1, dl, ol, dh, oh, o[16 * C + J0 + 4], o[16 * C + J0 + 5], o[16 * C + J0 + 12], o[16 * C + J0 + 13]);
 }
 
 // ---- the GEMM ------------------------------------------------------------------------------------------------------------------
-// NB = tokens per CTA tile (UMMA N): 32 .. 256, a multiple of 16.
-template <int NB>
-__global__ void __launch_bounds__(TG_THREADS, 2)
-gemm_q4k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, const __grid_constant__ CUtensorMap xmap, int b, float * __restrict__ y,
-                   float * __restrict__ partial) {
+// grid (row blocks, token blocks, K shares); the K shares of a tile are one cluster
+template <int NB, int G>
+__global__ void __launch_bounds__(tg_cfg<NB, G>::THREADS, tg_cfg<NB, G>::CTAS)
+gemm_q4k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int x0, const __grid_constant__ CUtensorMap xmap, int b, float * __restrict__ y, int * __restrict__ err) {
+    using C = tg_cfg<NB, G>;
     extern __shared__ __align__(1024) uint8_t tg_dsm[];
-    constexpr int A_BYTES = TG_BM * TG_BK * 2, B_BYTES = NB * TG_BK * 2;
-    constexpr int TG_STAGES = NB <= 64 ? 4 : (NB <= 128 ? 3 : 2);      // two CTAs per SM in every configuration
-    constexpr int TM_COLS = NB <= 32 ? 32 : NB <= 64 ? 64 : NB <= 128 ? 128 : 256;
-    uint8_t *  sA  = tg_dsm + ((1024u - (tg_smem(tg_dsm) & 1023u)) & 1023u);      // [TG_STAGES][128 rows][128 B], 1024-byte aligned (swizzle atom)
-    uint8_t *  sB  = sA + TG_STAGES * A_BYTES;                 // [TG_STAGES][NB rows][128 B]
-    uint64_t * bar = reinterpret_cast<uint64_t *>(sB + TG_STAGES * B_BYTES);      // full_a[S], full_b[S], empty[S], tmem_full
-    uint32_t * tmem_slot = reinterpret_cast<uint32_t *>(bar + 3 * TG_STAGES + 1);
-    const uint32_t bar_a = tg_smem(bar), bar_b = bar_a + TG_STAGES * 8, bar_e = bar_a + 2 * TG_STAGES * 8, bar_t = bar_a + 3 * TG_STAGES * 8;
+    uint8_t *  sB  = tg_dsm + ((1024u - (dt_smem(tg_dsm) & 1023u)) & 1023u);      // [BSTAGES][64 k][NB rows][128 B], 1024-byte aligned (swizzle atom)
+    uint8_t *  sW  = sB + C::BSTAGES * C::B_BYTES;                                // [WSTAGES][8 tiles][2304 B]
+    uint64_t * bar = reinterpret_cast<uint64_t *>(sB + C::BAR_OFF);
+    uint32_t * tmem_slot = reinterpret_cast<uint32_t *>(bar + C::N_BAR);
+    volatile int * abort_s = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    // weights: step full / free; activations: piece full / free; records: full / free; accumulators complete
+    const uint32_t bar_a = dt_smem(bar), bar_e = bar_a + C::STAGES * 8, bar_b = bar_e + C::STAGES * 8, bar_be = bar_b + C::BSTAGES * 8, bar_w = bar_be + C::BSTAGES * 8, bar_we = bar_w + C::WSTAGES * 8,
+                   bar_t = bar_we + C::WSTAGES * 8, bar_bf = C::PIECES == 1 ? bar_e : bar_be;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // k split (gridDim.y > 1: matrices with too few 128-row tiles to fill the machine): this CTA takes super-blocks [sb_lo, sb_hi) and
-    // writes its partial sums to partial[split][b][N]; tg_reduce_kernel adds the splits in order
-    const int sb_lo = (int) ((long long) nsb * blockIdx.y / gridDim.y), sb_hi = (int) ((long long) nsb * (blockIdx.y + 1) / gridDim.y);
-    const int n_ksteps = (sb_hi - sb_lo) * 4;
-    const int row0 = blockIdx.x * TG_BM;
-    if (gridDim.y > 1) y = partial + (size_t) blockIdx.y * b * N;
+    const int S = gridDim.z, sb_lo = (int) ((long long) nsb * blockIdx.z / S), sb_hi = (int) ((long long) nsb * (blockIdx.z + 1) / S);
+    const int n_sb = sb_hi - sb_lo, n_ksteps = n_sb * 2;
+    const int row0 = (x0 + blockIdx.x) * TG_BM;
+    const int n_tiles = min(8, (N + 15) / 16 - row0 / 16);                   // 16-row tiles this block has
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < TG_STAGES; s++) { tg_mbar_init(bar_a + s * 8, TG_PWARPS); tg_mbar_init(bar_b + s * 8, 1); tg_mbar_init(bar_e + s * 8, 1); }
-        tg_mbar_init(bar_t, 1);
+        for (int s = 0; s < C::STAGES; s++) { dt_mbar_init(bar_a + s * 8, 8); dt_mbar_init(bar_e + s * 8, 1); }
+        for (int s = 0; s < C::BSTAGES; s++) { dt_mbar_init(bar_b + s * 8, 1); dt_mbar_init(bar_be + s * 8, 1); }
+        for (int s = 0; s < C::WSTAGES; s++) { dt_mbar_init(bar_w + s * 8, 1); dt_mbar_init(bar_we + s * 8, C::WARPS); }
+        dt_mbar_init(bar_t, 1);
+        *abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tg_smem(tmem_slot)), "r"((uint32_t) TM_COLS) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dt_smem(tmem_slot)), "r"((uint32_t) C::TM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    dt_fence_before();
     __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_d = *tmem_slot;
+    dt_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    bool ok = true;
 
     if (warp == 0) {
-        // ---- TMA producer: activations ----
+        pib_pdl_wait();
+        pib_pdl_trigger();
         if (lane == 0) {
-            for (int kt = 0; kt < n_ksteps; kt++) {
-                const int s = kt % TG_STAGES;
-                if (kt >= TG_STAGES) tg_mbar_wait(bar_e + s * 8, ((kt / TG_STAGES) - 1) & 1);
-                tg_mbar_expect_tx(bar_b + s * 8, B_BYTES);
-                tg_tma_2d(tg_smem(sB + s * B_BYTES), &xmap, bar_b + s * 8, (sb_lo * 4 + kt) * TG_BK, 0);
+            for (int kp = 0; kp < C::PIECES * n_ksteps; kp++) {
+                const int s = kp % C::BSTAGES;
+                if (kp >= C::BSTAGES && !tg_wait1(bar_bf + s * 8, ((kp / C::BSTAGES) - 1) & 1, abort_s)) break;
+                dt_mbar_expect_tx(bar_b + s * 8, C::B_BYTES);
+                for (int j = 0; j < 2 / C::PIECES; j++)
+                    tg_tma_2d(dt_smem(sB + s * C::B_BYTES + j * NB * 128), &xmap, bar_b + s * 8, sb_lo * 256 + (kp * (2 / C::PIECES) + j) * 64, 0);
             }
         }
     } else if (warp == 1) {
-        // ---- MMA issuer ----
-        // instruction descriptor (cute::UMMA::InstrDescriptor): fp32 accumulate, fp16 x fp16, both K-major, N = NB, M = 128
+        // instruction descriptor: fp32 accumulate, fp16 x fp16, both K-major, N = NB, M = 128
         constexpr uint32_t idesc = (1u << 4) | ((uint32_t) (NB >> 3) << 17) | ((uint32_t) (TG_BM >> 4) << 24);
-        if (lane == 0) {
-            for (int kt = 0; kt < n_ksteps; kt++) {
-                const int s = kt % TG_STAGES;
-                const uint32_t ph = (kt / TG_STAGES) & 1;
-                tg_mbar_wait(bar_a + s * 8, ph);
-                tg_mbar_wait(bar_b + s * 8, ph);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t ad = tg_desc(tg_smem(sA + s * A_BYTES)), bd = tg_desc(tg_smem(sB + s * B_BYTES));
+        const uint64_t bd0 = dt_desc(dt_smem(sB));
+        for (int kt = 0; kt < n_ksteps && ok; kt++) {
+            const int s = kt % C::STAGES;
+            ok = tg_wait(bar_a + s * 8, (kt / C::STAGES) & 1, abort_s);
+            for (int j = 0; j < C::PIECES && ok; j++) {
+                const int kp = C::PIECES * kt + j, sp = kp % C::BSTAGES;
+                ok = tg_wait(bar_b + sp * 8, (kp / C::BSTAGES) & 1, abort_s);
+                if (!ok) break;
+                dt_fence_after();
+                const uint64_t bd = bd0 + (uint64_t) (sp * C::B_BYTES >> 4);
 #pragma unroll
-                for (int k = 0; k < TG_BK / 16; k++)            // 32 bytes further along K inside the swizzle row: + 2 in the address field
-                    tg_mma_f16(tmem_d, ad + 2 * k, bd + 2 * k, idesc, (kt | k) != 0);
-                tg_commit(bar_e + s * 8);                       // the stage is free when these MMAs have read it
+                for (int k = 0; k < 8 / C::PIECES; k++)         // 8 columns of weights and 32 bytes of activations further along K
+                    tg_mma_ts(tmem, tmem + NB + s * 64 + j * 32 + k * 8, bd + 2 * (k & 3) + (k >> 2) * (NB * 128 >> 4), idesc, (kp | k) != 0);
+                if (C::PIECES > 1) dt_commit(bar_be + sp * 8);  // the piece is free when these MMAs have read it
             }
-            tg_commit(bar_t);                                   // accumulators complete
+            if (ok) dt_commit(bar_e + s * 8);
+        }
+        if (ok) dt_commit(bar_t);
+    } else if (warp == 2) {
+        // weights are immutable: their copies do not wait for the launch before this one
+        const uint8_t * src = tiles + ((size_t) (row0 / 16 + lane) * nsb + sb_lo) * TG_TILE_BYTES;
+        for (int i = 0; i < n_sb; i++) {
+            const int s = i % C::WSTAGES;
+            if (i >= C::WSTAGES && !tg_wait<1000>(bar_we + s * 8, ((i / C::WSTAGES) - 1) & 1, abort_s)) break;
+            if (lane == 0) dt_mbar_expect_tx(bar_w + s * 8, (uint32_t) n_tiles * TG_TILE_BYTES);
+            __syncwarp();
+            if (lane < n_tiles) tg_bulk(dt_smem(sW + s * C::W_BYTES + lane * TG_TILE_BYTES), src + (size_t) i * TG_TILE_BYTES, TG_TILE_BYTES, bar_w + s * 8);
         }
     } else {
-        // ---- weight producers: warps 2..9, threads 2r and 2r + 1 <-> row r of the CTA tile (bytes 0..15 / 16..31 of its chunk) ----
-        const int p   = threadIdx.x - 64;                       // 0..255
-        const int r   = p >> 1, th = p & 1;
-        const int T   = (row0 >> 4) + (r >> 4), rr = r & 15, g = rr & 7, hf = rr >> 3;
-        const bool row_ok = row0 + r < N;
-        const uint8_t * rec0 = tiles + ((size_t) T * nsb + sb_lo) * TG_TILE_BYTES;
-        // A row's bytes of one record (4 chunks x 32 bytes, in 8-byte pieces of the fragment layout) and its header are fetched one
-        // whole record (4 k-steps) ahead into registers, and the lines of the record after that are asked into L2: the weight stream
-        // is a chain of DRAM latencies otherwise (one k-step of arithmetic hides a tenth of one).
-        uint2 cur[4][2], nxt[4][2];
-        uint4 hcur = make_uint4(0, 0, 0, 0), hnxt = make_uint4(0, 0, 0, 0);
-        auto fetch_rec = [&](int ri, uint2 (&w)[4][2], uint4 & h) {
-            const uint8_t * rec = rec0 + (size_t) ri * TG_TILE_BYTES;
-            if (row_ok) {
+        // ---- warps 3..: tensor-memory lanes 32 q .. 32 q + 31 belong to warp number q mod 4; rows q * 32 + hf * 16 ----
+        const int p = warp - 3, gs = p >> 3, q = warp & 3, hf = (p >> 2) & 1, g = lane >> 2;
+        uint4 *         scl  = reinterpret_cast<uint4 *>(sB + C::SCL_OFF) + p * 64;       // [chunks][16 rows] factors of this warp's record
+        const uint8_t * rec0 = sW + (q * 2 + hf) * TG_TILE_BYTES;
+        const uint32_t  ta0  = tmem + ((uint32_t) (q * 32 + hf * 16) << 16) + NB;
+        int      ws = 0, sl = gs, s_prev = 0;                      // ring places, counted along instead of divided
+        uint32_t wph = 0, eph = 1;                                 // phases: records full, step free (the first round passes at once)
+        constexpr int NH = 2 / G;                                  // k-steps of a record that this warp takes
+        for (int i = 0; i < n_sb && ok; i++) {
+            if (!tg_wait(bar_w + ws * 8, wph, abort_s)) { ok = false; break; }
+            const uint8_t * rec = rec0 + ws * C::W_BYTES;
+            __syncwarp();                                          // the factors of the record before have been read
+            // every lane forms the factors of one row and one (G = 2) or two chunks; the lanes of a row pair read them back per chunk
 #pragma unroll
-                for (int c = 0; c < 4; c++)
-#pragma unroll
-                    for (int t = 0; t < 2; t++) w[c][t] = __ldg(reinterpret_cast<const uint2 *>(rec + c * 512 + (g * 4 + 2 * th + t) * 16 + hf * 8));
-                h = __ldg(reinterpret_cast<const uint4 *>(rec + 2048 + rr * 16));
-            } else {
-#pragma unroll
-                for (int c = 0; c < 4; c++) w[c][0] = w[c][1] = make_uint2(0, 0);
+            for (int h = 0; h < NH; h++) {
+                const int r = lane & 15, c = (gs + h) * 2 + (lane >> 4);
+                scl[h * 32 + lane] = tg_scales(*reinterpret_cast<const uint4 *>(rec + 2048 + r * 16), c);
             }
-        };
-        const int n_rec = n_ksteps >> 2;
-        // L2 prefetch: the CTA's 8 tiles of a record step are 8 x 18 lines of 128 bytes; thread p < 144 owns line p % 18 of tile p / 18
-        const uint8_t * pf_base = (p < 144 && row0 + (p / 18) * 16 < N) ? tiles + ((size_t) ((row0 >> 4) + p / 18) * nsb + sb_lo) * TG_TILE_BYTES + (p % 18) * 128 : nullptr;
-        fetch_rec(0, cur, hcur);
-        for (int ri = 0; ri < n_rec; ri++) {
-            if (ri + 1 < n_rec) fetch_rec(ri + 1, nxt, hnxt);
-            if (pf_base && ri + 3 < n_rec) asm volatile("prefetch.global.L2 [%0];" ::"l"(pf_base + (size_t) (ri + 3) * TG_TILE_BYTES));
-            const uint4 hd = hcur;
-            // scales / mins of the record's eight sub-blocks: get_scale_min_k4 (ggml-quants.c:1446)
-            const float d = pib_h2f((uint16_t) (hd.x & 0xffff)), dmin = pib_h2f((uint16_t) (hd.x >> 16));
-            const uint32_t sc_lo = hd.y & 0x3f3f3f3fu, m_lo = hd.z & 0x3f3f3f3fu;
-            const uint32_t sc_hi = (hd.w & 0x0f0f0f0fu) | (((hd.y >> 6) & 0x03030303u) << 4), m_hi = ((hd.w >> 4) & 0x0f0f0f0fu) | (((hd.z >> 6) & 0x03030303u) << 4);
-            const __half2 k1024 = __float2half2_rn(1024.f);
+            uint4 v[2 * NH];
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const int kt = ri * 4 + c, s = kt % TG_STAGES;
-                const uint2 w[2] = { cur[c][0], cur[c][1] };
-                // sub-blocks 2c (low nibbles) and 2c + 1 (high nibbles) of the super-block
-                const int j0 = 2 * c, j1 = 2 * c + 1;
-                const float sc0 = (float) (((j0 < 4 ? sc_lo : sc_hi) >> (8 * (j0 & 3))) & 0xff), mn0 = (float) (((j0 < 4 ? m_lo : m_hi) >> (8 * (j0 & 3))) & 0xff);
-                const float sc1 = (float) (((j1 < 4 ? sc_lo : sc_hi) >> (8 * (j1 & 3))) & 0xff), mn1 = (float) (((j1 < 4 ? m_lo : m_hi) >> (8 * (j1 & 3))) & 0xff);
-                // w = d1 * q - m1: the nibbles enter fp16 as 1024 + q (bit trick), minus 1024 is exact, then one fused multiply-add per pair
-                const __half2 d1_lo = __float2half2_rn(__fmul_rn(d, sc0)), d1_hi = __float2half2_rn(__fmul_rn(d, sc1));
-                const __half2 o_lo = __float2half2_rn(-__fmul_rn(dmin, mn0)), o_hi = __float2half2_rn(-__fmul_rn(dmin, mn1));
-                if (kt >= TG_STAGES) tg_mbar_wait(bar_e + s * 8, ((kt / TG_STAGES) - 1) & 1);
-                uint8_t * arow = sA + s * A_BYTES + r * 128;
-                // output chunk j (16 bytes = 8 k) sits at chunk position j ^ (row & 7); low nibbles -> k 0..31 (chunks 0..3), high -> 32..63
+            for (int c = 0; c < 2 * NH; c++) v[c] = *reinterpret_cast<const uint4 *>(rec + (gs * 2 + c) * 512 + lane * 16);
+            __syncwarp();
 #pragma unroll
-                for (int t = 0; t < 2; t++) {
-                    // bytes 8 (2 th + t) .. + 7 of the row: two 32-bit words -> per word pairs (e0, e2), (e1, e3)
-                    uint32_t lo[4], hi[4];
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        const uint32_t v = h ? w[t].y : w[t].x;
-                        const uint32_t a0 = (v & 0x000F000Fu) | 0x64006400u, a1 = ((v >> 8) & 0x000F000Fu) | 0x64006400u;
-                        const uint32_t b0 = ((v >> 4) & 0x000F000Fu) | 0x64006400u, b1 = ((v >> 12) & 0x000F000Fu) | 0x64006400u;
-                        __half2 q;
-                        q = __hfma2(__hsub2(*reinterpret_cast<const __half2 *>(&a0), k1024), d1_lo, o_lo); lo[2 * h]     = *reinterpret_cast<uint32_t *>(&q);
-                        q = __hfma2(__hsub2(*reinterpret_cast<const __half2 *>(&a1), k1024), d1_lo, o_lo); lo[2 * h + 1] = *reinterpret_cast<uint32_t *>(&q);
-                        q = __hfma2(__hsub2(*reinterpret_cast<const __half2 *>(&b0), k1024), d1_hi, o_hi); hi[2 * h]     = *reinterpret_cast<uint32_t *>(&q);
-                        q = __hfma2(__hsub2(*reinterpret_cast<const __half2 *>(&b1), k1024), d1_hi, o_hi); hi[2 * h + 1] = *reinterpret_cast<uint32_t *>(&q);
-                    }
-                    const int ck = 2 * th + t;
-                    *reinterpret_cast<uint4 *>(arow + ((ck ^ (r & 7)) << 4))       = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-                    *reinterpret_cast<uint4 *>(arow + (((4 + ck) ^ (r & 7)) << 4)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            for (int h = 0; h < NH; h++) {                         // 128 k: chunks 2 (gs + h), + 1
+                uint32_t o[32];
+                tg_chunk_row<0, 0>(v[2 * h].x, v[2 * h].y, scl[h * 32 + g], o);
+                tg_chunk_row<0, 2>(v[2 * h].z, v[2 * h].w, scl[h * 32 + g + 8], o);
+                tg_chunk_row<1, 0>(v[2 * h + 1].x, v[2 * h + 1].y, scl[h * 32 + 16 + g], o);
+                tg_chunk_row<1, 2>(v[2 * h + 1].z, v[2 * h + 1].w, scl[h * 32 + 16 + g + 8], o);
+                if (h == NH - 1) {
+                    // The ring place is given back when every word of the record has been USED.  An arrival right behind the loads overtakes them: the next
+                    // bulk copy then overwrote words that had been asked for but not yet read (quads of rows wrong, only when calls follow one another closely).
+                    __syncwarp();
+                    if (lane == 0) dt_arrive(bar_we + ws * 8);
+                    if (++ws == C::WSTAGES) { ws = 0; wph ^= 1; }
                 }
-                tg_fence_async_smem();                              // generic-proxy writes -> visible to the tensor core's async proxy
-                __syncwarp();
-                if (lane == 0) tg_mbar_arrive(bar_a + s * 8);
+                if (i | h) {                                       // the step before: its stores had this step's arithmetic to land in
+                    dt_wait_st();
+                    dt_fence_before();
+                    if (lane == 0) dt_arrive(bar_a + s_prev * 8);
+                    __syncwarp();
+                }
+                ok = tg_wait(bar_e + sl * 8, eph, abort_s);
+                if (!ok) break;
+                dt_fence_after();
+                tg_st_frag(ta0 + sl * 64, o);
+                s_prev = sl;
+                sl += G;
+                if (sl >= C::STAGES) { sl -= C::STAGES; eph ^= 1; }
             }
-#pragma unroll
-            for (int c = 0; c < 4; c++) { cur[c][0] = nxt[c][0]; cur[c][1] = nxt[c][1]; }
-            hcur = hnxt;
         }
-        // ---- epilogue: accumulators -> y[token][row]; warp w reads tensor-memory lanes 32 (w % 4) .. + 31 ----
-        tg_mbar_wait(bar_t, 0);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int q4   = warp & 3;                               // warps 2..5 take the lower half of the columns, 6..9 the upper half
-        const int orow = row0 + q4 * 32 + lane;
-        constexpr int CH = NB / 2 >= 32 ? NB / 2 : 32;
-        const int cbeg = warp < 6 ? 0 : CH, cend = warp < 6 ? (CH < NB ? CH : NB) : NB;
+        dt_wait_st();
+        dt_fence_before();
+        if (lane == 0) dt_arrive(bar_a + s_prev * 8);
+        __syncwarp();
+        // ---- accumulators: a lane is a row; two (four) warps per 32 rows share the columns ----
+        pib_pdl_wait();
+        pib_pdl_trigger();
+        ok = ok && tg_wait(bar_t, 0, abort_s);
+        if (ok) {
+            dt_fence_after();
+            const int r = q * 32 + lane, orow = row0 + r;
+            float * part = reinterpret_cast<float *>(sB);
 #pragma unroll 1
-        for (int c0 = cbeg; c0 < cend; c0 += 32) {
-            uint32_t v[32];
-            const uint32_t taddr = tmem_d + ((uint32_t) (q4 * 32) << 16) + (uint32_t) c0;
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                         "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-                           "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
-                           "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-                           "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                         : "r"(taddr) : "memory");
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (orow < N) {
+            for (int c0 = (gs * 2 + hf) * 32; c0 < NB; c0 += 64 * G) {
+                if (S == 1 && c0 >= b) break;
+                uint32_t u[32];
+                dt_ld32(tmem + ((uint32_t) (q * 32) << 16) + c0, u);
+                dt_wait_ld();
+                if (S > 1) {                                    // this share's sums, [token][row]: the rings are free, every MMA has completed
 #pragma unroll
-                for (int j = 0; j < 32; j++) if (c0 + j < b) y[(size_t) (c0 + j) * N + orow] = __uint_as_float(v[j]);
+                    for (int j = 0; j < 32; j++) part[(c0 + j) * TG_BM + r] = __uint_as_float(u[j]);
+                } else if (orow < N) {
+#pragma unroll
+                    for (int j = 0; j < 32; j++) if (c0 + j < b) y[(size_t) (c0 + j) * N + orow] = __uint_as_float(u[j]);
+                }
             }
         }
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncwarp();
+    if (S > 1) {
+        // K shares meet through distributed shared memory: every CTA of the cluster adds its part of the tokens, in share order
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (warp >= 3 && !*abort_s) {
+            const int r = (threadIdx.x - 96) & 127, orow = row0 + r;
+            const uint32_t base = dt_smem(sB);
+            for (int j = blockIdx.z * 2 * G + ((threadIdx.x - 96) >> 7); j < b; j += 2 * G * S) {
+                float v = 0.f;
+                for (int s = 0; s < S; s++) {
+                    uint32_t a;
+                    float    o;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(base + (uint32_t) (j * TG_BM + r) * 4), "r"(s));
+                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(o) : "r"(a) : "memory");
+                    v = s ? v + o : o;
+                }
+                if (orow < N) y[(size_t) j * N + orow] = v;
+            }
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");      // nobody leaves while its sums are read
+    }
+    dt_fence_before();
     __syncthreads();
-    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"((uint32_t) TM_COLS) : "memory");
+    if (*abort_s) {
+        // a wait ran out: say so, give copies and MMAs still in flight time to land (bounded), then free the tensor memory
+        if (threadIdx.x == 0 && err) atomicExch(err, 1 + (int) blockIdx.x);
+        for (int i = 0; i < 2000; i++) __nanosleep(1000);
+        __syncthreads();
+    }
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t) C::TM_COLS) : "memory");
 }
 
 // ---- host side --------------------------------------------------------------------------------------------------------------------
@@ -274,84 +362,77 @@ static tg_encode_fn tg_encode() {
     return fn;
 }
 
-// y = sum over the k splits, in split order (deterministic)
-__global__ void tg_reduce_kernel(const float4 * __restrict__ partial, float4 * __restrict__ y, size_t n4, int nsplit) {
-    const size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n4) return;
-    float4 v = partial[i];
-    for (int sp = 1; sp < nsplit; sp++) { const float4 o = partial[(size_t) sp * n4 + i]; v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w; }
-    y[i] = v;
-}
+// tokens per CTA
+static int tg_nb_of(int b) { return b <= 32 ? 32 : b <= 64 ? 64 : b <= 96 ? 96 : b <= 128 ? 128 : b <= 192 ? 192 : 256; }
+size_t pib_gemm_xhat_bytes(int64_t K, int b) { return (size_t) (b <= 32 ? 32 : b <= 64 ? 64 : b <= 128 ? 128 : 256) * K * sizeof(__half); }
 
-// partial sums of the k split: one buffer per (device, stream), allocated on first use (prompt passes are not captured in graphs)
-#define TG_PARTIAL_BYTES ((size_t) 64 << 20)
-static float * tg_partial(cudaStream_t st) {
-    static std::map<std::pair<int, cudaStream_t>, float *> bufs;
-    static std::mutex mu;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    std::lock_guard<std::mutex> lock(mu);
-    float *& p = bufs[std::make_pair(dev, st)];
-    if (!p && cudaMalloc(&p, TG_PARTIAL_BYTES) != cudaSuccess) { cudaGetLastError(); p = nullptr; }
-    return p;
-}
-// splits for a matrix of N rows: fill the 2 x SMs CTA slots once; every split keeps at least four super-blocks
-static int tg_ksplit(int64_t N, int64_t K, int b) {
-    static const int env = getenv("PIB_GEMM_KSPLIT") ? atoi(getenv("PIB_GEMM_KSPLIT")) : 0;
-    const int ctas = (int) ((N + TG_BM - 1) / TG_BM), nsb = (int) (K / 256);
-    int s = env > 0 ? env : (2 * pib_num_sms()) / ctas;
-    if (s > 4) s = 4;
-    while (s > 1 && (nsb / s < 4 || (size_t) s * b * N * sizeof(float) > TG_PARTIAL_BYTES || (N * b) % 4)) s--;
-    return s < 1 ? 1 : s;
-}
-
-static int tg_nb_of(int b) { return b <= 32 ? 32 : b <= 64 ? 64 : b <= 128 ? 128 : 256; }
-size_t pib_gemm_xhat_bytes(int64_t K, int b) { return (size_t) tg_nb_of(b) * K * sizeof(__half); }
-
-template <int NB>
-static int tg_launch(const pib_weight * w, const __half * xh, int b, float * y, cudaStream_t st) {
+// row blocks [x0, x0 + nx), K in S shares
+template <int NB, int G>
+static int tg_launch(const pib_weight * w, const __half * xh, int b, int x0, int nx, int S, float * y, cudaStream_t st) {
+    using C = tg_cfg<NB, G>;
     tg_encode_fn enc = tg_encode();
     if (!enc) { pib_set_error("pib_gemm: cuTensorMapEncodeTiled not available"); return PIB_ERR_UNSUPP; }
     CUtensorMap map;
-    const cuuint64_t gdim[2] = { (cuuint64_t) w->K, (cuuint64_t) NB };
+    const cuuint64_t gdim[2] = { (cuuint64_t) w->K, (cuuint64_t) b };            // rows behind b are zero-filled
     const cuuint64_t gstr[1] = { (cuuint64_t) w->K * sizeof(__half) };
-    const cuuint32_t box[2]  = { TG_BK, (cuuint32_t) NB };
+    const cuuint32_t box[2]  = { 64, (cuuint32_t) NB };
     const cuuint32_t estr[2] = { 1, 1 };
     const CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void *) xh, gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { pib_set_error("pib_gemm: cuTensorMapEncodeTiled failed (%d)", (int) r); return PIB_ERR_CUDA; }
-    constexpr int    STAGES = NB <= 64 ? 4 : (NB <= 128 ? 3 : 2);
-    constexpr size_t smem = (size_t) STAGES * (TG_BM * TG_BK * 2 + NB * TG_BK * 2) + (3 * STAGES + 1) * 8 + 16 + 1024;
     static bool configured = false;
-    if (!configured) { PIB_CHECK(cudaFuncSetAttribute(gemm_q4k_tc_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)); configured = true; }
-    const int grid = (int) ((w->N + TG_BM - 1) / TG_BM);
-    int       ks   = tg_ksplit(w->N, w->K, b);
-    float *   part = ks > 1 ? tg_partial(st) : nullptr;
-    if (ks > 1 && !part) ks = 1;
-    gemm_q4k_tc_kernel<NB><<<dim3(grid, ks), TG_THREADS, smem, st>>>(w->tiles, (int) (w->K / 256), (int) w->N, map, b, y, part);
+    if (!configured) { PIB_CHECK(cudaFuncSetAttribute(gemm_q4k_tc_kernel<NB, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) C::SMEM)); configured = true; }
+    const dim3 grid((unsigned) nx, 1, (unsigned) S);
+    int * err = pib_tc_error_word(st);
+    if (S > 1) pib_launch_cluster(gemm_q4k_tc_kernel<NB, G>, grid, dim3(C::THREADS), dim3(1, 1, (unsigned) S), C::SMEM, st, w->tiles, (int) (w->K / 256), (int) w->N, x0, map, b, y, err);
+    else       pib_launch(gemm_q4k_tc_kernel<NB, G>, grid, dim3(C::THREADS), C::SMEM, st, w->tiles, (int) (w->K / 256), (int) w->N, x0, map, b, y, err);
     PIB_CHECK(cudaGetLastError());
-    if (ks > 1) {
-        const size_t n4 = (size_t) b * w->N / 4;
-        tg_reduce_kernel<<<(unsigned) ((n4 + 255) / 256), 256, 0, st>>>(reinterpret_cast<const float4 *>(part), reinterpret_cast<float4 *>(y), n4, ks);
-        PIB_CHECK(cudaGetLastError());
-    }
     return PIB_OK;
 }
 
 // y[b][N] = W x^; act_dev = the Q8_K activation planes of `b` tokens (act_quant.cu), xhat_dev = scratch of pib_gemm_xhat_bytes
 int pib_gemm_q4k_tc(const pib_weight * w, const void * act_dev, int b, float * y_dev, void * xhat_dev, cudaStream_t st) {
     if (!w || w->type != PIB_TYPE_Q4_K || !w->tiles || b < 1 || b > 256) { pib_set_error("pib_gemm: needs Q4_K tiles and 1 <= b <= 256"); return PIB_ERR_ARG; }
-    const int NB = tg_nb_of(b);
     const pib_act_layout L = pib_act_layout_of(PIB_TYPE_Q4_K, w->K, b);
     const uint8_t * act = (const uint8_t *) act_dev;
-    tg_xhat_kernel<<<dim3((unsigned) ((w->K / 4 + 255) / 256), NB), 256, 0, st>>>((const int8_t *) (act + L.qs_off), (const float *) (act + L.d_off), b, (int) w->K, (__half *) xhat_dev, NB);
+    __half * xh = (__half *) xhat_dev;
+    const int64_t n16 = (int64_t) b * (w->K / 16);
+    pib_launch(tg_xhat_kernel, dim3((unsigned) ((n16 + 255) / 256)), dim3(256), 0, st, (const int8_t *) (act + L.qs_off), (const float *) (act + L.d_off), n16, (int) (w->K / 16), xh);
     PIB_CHECK(cudaGetLastError());
-    switch (NB) {
-        case 32:  return tg_launch<32>(w, (const __half *) xhat_dev, b, y_dev, st);
-        case 64:  return tg_launch<64>(w, (const __half *) xhat_dev, b, y_dev, st);
-        case 128: return tg_launch<128>(w, (const __half *) xhat_dev, b, y_dev, st);
-        default:  return tg_launch<256>(w, (const __half *) xhat_dev, b, y_dev, st);
+    const int NB = tg_nb_of(b), nsb = (int) (w->K / 256), nx = (int) ((w->N + TG_BM - 1) / TG_BM), sms = pib_num_sms();
+    // K shares of n row blocks that fit `slots` CTAs at once; every share keeps at least two super-blocks
+    auto shares = [&](int n, int slots) { int S = 1; while (S < 8 && n * S * 2 <= slots && nsb / (S * 2) >= 2) S *= 2; return S; };
+    // One CTA with two groups, or two CTAs with one, per SM (us, one / two, 40 and 128 tokens): 12288 x 4096 (96 row blocks) 18.7 / 20.8 and 20.9 / 29.6,
+    // 10240 x 8192 (80) 31.4 / 33.4 and 33.8 / 42.7, 22016 x 4096 (172) 35.5 / 29.4 and 39.5 / 34.7, 8192 x 28672 (64, in 2 / 4 shares) 54.2 / 49.1 and 68.5 / 67.7.
+    // Above 128 tokens the accumulator takes half of the tensor memory: one.
+    const bool two = NB <= 128 && (nx > sms || (NB <= 64 && shares(nx, sms) > 1));
+    if (two) {
+        const int S = shares(nx, 2 * sms);
+        switch (NB) {
+            case 32: return tg_launch<32, 1>(w, xh, b, 0, nx, S, y_dev, st);
+            case 64: return tg_launch<64, 1>(w, xh, b, 0, nx, S, y_dev, st);
+            case 96: return tg_launch<96, 1>(w, xh, b, 0, nx, S, y_dev, st);
+            default: return tg_launch<128, 1>(w, xh, b, 0, nx, S, y_dev, st);
+        }
     }
+    // whole rounds of one CTA per SM, then what is left over in K shares (448 row blocks are three rounds and four blocks)
+    int full = nx / sms * sms, rest = nx - full;
+    if (full > 0 && shares(rest, sms) == 1) { full = nx; rest = 0; }
+    auto go = [&](int x0, int n) {
+        const int S = shares(n, sms);
+        switch (NB) {
+            case 32:  return tg_launch<32, 2>(w, xh, b, x0, n, S, y_dev, st);
+            case 64:  return tg_launch<64, 2>(w, xh, b, x0, n, S, y_dev, st);
+            case 96:  return tg_launch<96, 2>(w, xh, b, x0, n, S, y_dev, st);
+            case 128: return tg_launch<128, 2>(w, xh, b, x0, n, S, y_dev, st);
+            case 192: return tg_launch<192, 2>(w, xh, b, x0, n, S, y_dev, st);
+            default:  return tg_launch<256, 2>(w, xh, b, x0, n, S, y_dev, st);
+        }
+    };
+    int rc = PIB_OK;
+    if (full > 0) rc = go(0, full);
+    if (rc == PIB_OK && rest > 0) rc = go(full, rest);
+    return rc;
 }
 
 extern "C" size_t pib_gemm_scratch_bytes(int64_t K, int b) { return pib_gemm_xhat_bytes(K, b); }
@@ -379,8 +460,10 @@ extern "C" int pib_gemm_host(const pib_weight * w, const float * x_host, int b, 
     // the activation quantiser takes at most PIB_MAX_BATCH rows per launch; its planes are per launch, so quantise in one go
     // through the engine-internal entry point (any b)
     if (rc == PIB_OK) rc = pib_quantize_act_c(PIB_TYPE_Q4_K, x, b, w->K, act, nullptr, nullptr);
-    if (rc == PIB_OK) rc = pib_gemm_q4k_tc(w, act, b, y, xh, nullptr);
+    if (rc == PIB_OK && (rc = pib_gemm_q4k_tc(w, act, b, y, xh, nullptr)) != PIB_OK) { cudaFree(buf); return rc; }
+    if (rc == PIB_OK) rc = pib_dense_mm_check(nullptr, 1);
     if (rc == PIB_OK && cudaDeviceSynchronize() != cudaSuccess) rc = PIB_ERR_CUDA;
+    if (rc == PIB_OK && pib_dense_mm_check(nullptr, 0) != PIB_OK) { cudaFree(buf); return PIB_ERR_CUDA; }
     if (rc == PIB_OK && cudaMemcpy(y_host, y, yb, cudaMemcpyDeviceToHost) != cudaSuccess) rc = PIB_ERR_CUDA;
     if (rc == PIB_ERR_CUDA) pib_set_error("pib_gemm_host: %s", cudaGetErrorString(cudaGetLastError()));
     cudaFree(buf);
