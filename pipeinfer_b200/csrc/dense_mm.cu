@@ -8,12 +8,15 @@
 // strides; with `zrange` problem z owns a run of rows of a sorted list (tokens grouped by expert) and rows may be gathered
 // through an index list.
 //
-// Kernels: mm_tile_kernel (any shape; 64 x 64 x 16 tiles, 4 x 4 outputs per thread), for up to MV_MAXB rows mv_rows_kernel
-// (one warp per weight row, 16-byte weight loads: the weights are read once at the speed of memory), and for up to 128 float32 outputs
+// Kernels: mm_tile_kernel (any shape; 64 x 64 x 16 tiles, 4 x 4 outputs per thread), for up to MV_MAXB rows mv_mma_kernel (bfloat16 weights: 16 weight rows
+// per block against all tokens on the tensor cores) or mv_rows_kernel (float32 weights, shapes the former does not take: one warp per weight row), and for up
+// to 128 float32 outputs
 // over many rows mm_few_cols_kernel (a warp per four rows: a router's logits, where 64-wide output tiles would leave most of the machine idle).
 #include "hybrid.cuh"
 
 #include <cuda_bf16.h>
+
+#include <type_traits>
 
 #define MM_BM 64
 #define MM_BN 64
@@ -254,6 +257,109 @@ __global__ void __launch_bounds__(256) mv_pair_kernel(mm_dev a, mm_dev b, bool x
     }
 }
 
+// ---- few rows, bfloat16 weights: 16 weight rows x up to 16 tokens per block on the tensor cores (mma.sync, fp32 accumulators) ----
+// The eight warps of a block share K; a lane's 16-byte piece of a weight row (k = 32 c + 8 t .. + 7, t = lane % 4) is the A operand of two products as it
+// is: k slots 2t, 2t + 1 and 2t + 8, 2t + 9 of product j stand for elements 8t + 4j .. + 3, and the lane reads the same eight elements of "its" token for B.
+// So no value passes through shared memory, an activation is rounded once per block, and a warp's weight bytes are all in flight together -- the first ones
+// before the launch wait, because weights are immutable.
+// What bounds it: the weights' way from memory.  The form it replaces (a warp per weight row, mv_rows_kernel) rounded every activation for every weight row: at
+// four tokens 32 conversions per 16 bytes of weights.
+#define MVM_U 4                      // 32-k chunks a warp has in flight
+__device__ __forceinline__ void mvm_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t mvm_pack(float lo, float hi) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&v);
+}
+// weight rows 16 tile .. + 15 of problem z against its rows [row0, row1) (at most 8 NT).  WAIT: the launch wait comes here, behind the first weight loads
+template <int EPI, int NT, bool WAIT>
+__device__ __forceinline__ void mvm_body(const mm_dev & a, int z, int tile, int row0, int row1) {
+    __shared__ float red[8][8 * NT][16];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int nch = (a.K + 31) / 32, c0 = nch * warp / 8, c1 = nch * (warp + 1) / 8, n0 = tile * 16;
+    const __nv_bfloat16 * W = reinterpret_cast<const __nv_bfloat16 *>(a.W) + (size_t) z * a.wz + 8 * t;
+    const __nv_bfloat16 * wa = W + (size_t) min(n0 + g, a.N - 1) * a.ldw, * wb = W + (size_t) min(n0 + g + 8, a.N - 1) * a.ldw;
+    int4 ra[MVM_U], rb[MVM_U];
+    auto load = [&](int c) {
+#pragma unroll
+        for (int u = 0; u < MVM_U; u++) {
+            const bool in = c + u < c1 && (c + u) * 32 + 8 * t < a.K;
+            ra[u] = in ? ld_stream_v4(wa + (c + u) * 32) : make_int4(0, 0, 0, 0);
+            rb[u] = in ? ld_stream_v4(wb + (c + u) * 32) : make_int4(0, 0, 0, 0);
+        }
+    };
+    load(c0);
+    if (WAIT) { pib_pdl_wait(); pib_pdl_trigger(); }
+    const float * x[NT];
+    bool          has[NT];
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+        const int m = row0 + g + 8 * j;
+        has[j] = m < row1;
+        x[j]   = a.X + (size_t) z * a.xz + (int64_t) (has[j] ? (a.xrows ? a.xrows[m] / a.xdiv : m) : 0) * a.ldx + 8 * t;
+    }
+    float acc[NT][4];
+#pragma unroll
+    for (int j = 0; j < NT; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+    for (int c = c0; c < c1; c += MVM_U) {
+        if (c > c0) load(c);
+#pragma unroll
+        for (int u = 0; u < MVM_U; u++) {
+            const bool in = c + u < c1 && (c + u) * 32 + 8 * t < a.K;
+#pragma unroll
+            for (int j = 0; j < NT; j++) {
+                float4 p = make_float4(0.f, 0.f, 0.f, 0.f), q = p;
+                if (in && has[j]) { p = *reinterpret_cast<const float4 *>(x[j] + (c + u) * 32); q = *reinterpret_cast<const float4 *>(x[j] + (c + u) * 32 + 4); }
+                mvm_mma(acc[j], (uint32_t) ra[u].x, (uint32_t) rb[u].x, (uint32_t) ra[u].y, (uint32_t) rb[u].y, mvm_pack(p.x, p.y), mvm_pack(p.z, p.w));
+                mvm_mma(acc[j], (uint32_t) ra[u].z, (uint32_t) rb[u].z, (uint32_t) ra[u].w, (uint32_t) rb[u].w, mvm_pack(q.x, q.y), mvm_pack(q.z, q.w));
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+        red[warp][8 * j + 2 * t][g]     = acc[j][0]; red[warp][8 * j + 2 * t + 1][g]     = acc[j][1];
+        red[warp][8 * j + 2 * t][g + 8] = acc[j][2]; red[warp][8 * j + 2 * t + 1][g + 8] = acc[j][3];
+    }
+    __syncthreads();
+    const int m = threadIdx.x >> 4, r = threadIdx.x & 15, n = n0 + r;
+    if (m >= 8 * NT) return;                                                // whole warps: a warp holds two tokens
+    float v = red[0][m][r];
+#pragma unroll
+    for (int w = 1; w < 8; w++) v += red[w][m][r];
+    const float o = pib_epi_pairs(EPI) ? __shfl_down_sync(0xffffffffu, v, 1) : 0.f;      // paired outputs: rows 2i, 2i + 1 sit in neighbouring lanes
+    if (row0 + m >= row1) return;
+    float * Y = a.Y + (size_t) z * a.yz;
+    if (pib_epi_pairs(EPI)) { if (!(r & 1) && n + 1 < a.N) *mm_out(a, Y, row0 + m, n >> 1) = pib_glu_pair<EPI, true>(v, o, a.e0); }
+    else if (n < a.N) *mm_out(a, Y, row0 + m, n) = pib_epilogue<EPI, true>(v, a.e0, a.e1);
+}
+template <int EPI, int NT>
+__global__ void __launch_bounds__(256, 3) mv_mma_kernel(mm_dev a) {
+    if (!a.zrange && !a.zlist) { mvm_body<EPI, NT, true>(a, blockIdx.z, blockIdx.x, 0, a.M); return; }
+    pib_pdl_wait();
+    pib_pdl_trigger();
+    int z, row0, row1;
+    if (mv_problem(a, blockIdx.z, 8 * NT, z, row0, row1)) mvm_body<EPI, NT, false>(a, z, blockIdx.x, row0, row1);
+}
+// mv_experts_kernel's and mv_pair_kernel's work in this form
+template <int EPI, int NT>
+__global__ void __launch_bounds__(256, 3) mv_mma_experts_kernel(mm_dev a, mm_dev b, int tiles_a, int za) {
+    const int blk = blockIdx.x - tiles_a * za;
+    if (blk >= 0) { mvm_body<EPI, NT, true>(b, 0, blk, 0, b.M); return; }
+    pib_pdl_wait();
+    pib_pdl_trigger();
+    int z, row0, row1;
+    if (mv_problem(a, blockIdx.x / tiles_a, 8 * NT, z, row0, row1)) mvm_body<EPI, NT, false>(a, z, (int) blockIdx.x % tiles_a, row0, row1);
+}
+template <int EPI_B, int NT>
+__global__ void __launch_bounds__(256, 3) mv_mma_pair_kernel(mm_dev a, mm_dev b, int tiles_a) {
+    if ((int) blockIdx.x < tiles_a) mvm_body<PIB_EPI_NONE, NT, true>(a, 0, blockIdx.x, 0, a.M);
+    else                            mvm_body<EPI_B, NT, true>(b, 0, blockIdx.x - tiles_a, 0, b.M);
+}
+// bfloat16 weights whose 16-byte pieces and the activations' lie on 16-byte boundaries (the caller has looked at the weights)
+template <typename WT, bool ROUND> static bool mvm_fits(const mm_dev & a, bool xvec) { return std::is_same<WT, __nv_bfloat16>::value && ROUND && xvec && a.K % 8 == 0; }
+
 // ---- few outputs, many rows (a router's logits over a prompt): a warp takes FC_ROWS rows of X and NB outputs, lanes stride over k in 16-byte pieces ----
 // float32 weights and activations, no rounding.  A weight piece is used for FC_ROWS rows, so the matrix crosses L1 once per that many rows; grid.y walks the
 // outputs in runs of NB.
@@ -317,6 +423,11 @@ static int launch_mm(const pib_mm & a, const mm_dev & d, cudaStream_t st) {
     if (a.M <= MV_MAXB && vec_ok) {
         dim3 grid((unsigned) (((pib_epi_pairs(EPI) ? a.N / 2 : a.N) + 7) / 8), 1, (unsigned) (a.zlist && a.M < a.Z ? a.M : a.Z));
         const bool xvec = a.ldx % 4 == 0 && a.xz % 4 == 0 && ((uintptr_t) a.X & 15) == 0;
+        if (mvm_fits<WT, ROUND>(d, xvec)) {
+            grid.x = (unsigned) ((a.N + 15) / 16);
+            if (a.M <= 8) pib_launch(mv_mma_kernel<EPI, 1>, grid, dim3(256), (size_t) 0, st, d);
+            else          pib_launch(mv_mma_kernel<EPI, 2>, grid, dim3(256), (size_t) 0, st, d);
+        } else
         if (a.M == 1)      pib_launch(mv_rows_kernel<WT, ROUND, EPI, 1>, dim3(grid), dim3(256), (size_t) (0), st, d, xvec);
         else if (a.M == 2) pib_launch(mv_rows_kernel<WT, ROUND, EPI, 2>, dim3(grid), dim3(256), (size_t) (0), st, d, xvec);
         else if (a.M <= 4) pib_launch(mv_rows_kernel<WT, ROUND, EPI, 4>, dim3(grid), dim3(256), (size_t) (0), st, d, xvec);
@@ -370,6 +481,11 @@ template <typename WT, bool ROUND, int EPI_B>
 static void launch_pair(const mm_dev & a, const mm_dev & b, bool xva, bool xvb, cudaStream_t st) {
     const int ba = (a.N + 7) / 8, bb = ((pib_epi_pairs(EPI_B) ? b.N / 2 : b.N) + 7) / 8;
     const dim3 grid((unsigned) (ba + bb));
+    if (mvm_fits<WT, ROUND>(a, xva) && mvm_fits<WT, ROUND>(b, xvb)) {
+        const int ta = (a.N + 15) / 16, tb = (b.N + 15) / 16;
+        if (a.M <= 8) pib_launch(mv_mma_pair_kernel<EPI_B, 1>, dim3((unsigned) (ta + tb)), dim3(256), (size_t) 0, st, a, b, ta);
+        else          pib_launch(mv_mma_pair_kernel<EPI_B, 2>, dim3((unsigned) (ta + tb)), dim3(256), (size_t) 0, st, a, b, ta);
+    } else
     if (a.M == 1)      pib_launch(mv_pair_kernel<WT, ROUND, EPI_B, 1>, grid, dim3(256), (size_t) 0, st, a, b, xva, xvb, ba);
     else if (a.M == 2) pib_launch(mv_pair_kernel<WT, ROUND, EPI_B, 2>, grid, dim3(256), (size_t) 0, st, a, b, xva, xvb, ba);
     else if (a.M <= 4) pib_launch(mv_pair_kernel<WT, ROUND, EPI_B, 4>, grid, dim3(256), (size_t) 0, st, a, b, xva, xvb, ba);
@@ -400,6 +516,11 @@ template <typename WT, bool ROUND, int EPI>
 static void launch_experts(const mm_dev & a, const mm_dev & b, bool xva, bool xvb, int za, cudaStream_t st) {
     const int ba = ((pib_epi_pairs(EPI) ? a.N / 2 : a.N) + 7) / 8, bb = ((pib_epi_pairs(EPI) ? b.N / 2 : b.N) + 7) / 8, rows = a.M > b.M ? a.M : b.M;
     const dim3 grid((unsigned) (ba * za + bb));
+    if (mvm_fits<WT, ROUND>(a, xva && a.xz % 4 == 0) && mvm_fits<WT, ROUND>(b, xvb)) {
+        const int ta = (a.N + 15) / 16, tb = (b.N + 15) / 16;
+        if (rows <= 8) pib_launch(mv_mma_experts_kernel<EPI, 1>, dim3((unsigned) (ta * za + tb)), dim3(256), (size_t) 0, st, a, b, ta, za);
+        else           pib_launch(mv_mma_experts_kernel<EPI, 2>, dim3((unsigned) (ta * za + tb)), dim3(256), (size_t) 0, st, a, b, ta, za);
+    } else
     if (rows == 1)      pib_launch(mv_experts_kernel<WT, ROUND, EPI, 1>, grid, dim3(256), (size_t) 0, st, a, b, xva, xvb, ba, za);
     else if (rows == 2) pib_launch(mv_experts_kernel<WT, ROUND, EPI, 2>, grid, dim3(256), (size_t) 0, st, a, b, xva, xvb, ba, za);
     else if (rows <= 4) pib_launch(mv_experts_kernel<WT, ROUND, EPI, 4>, grid, dim3(256), (size_t) 0, st, a, b, xva, xvb, ba, za);

@@ -1,0 +1,21 @@
+"""Few rows against bfloat16 weights on the tensor cores (mv_mma_kernel, csrc/dense_mm.cu) at the edges of its tiles: weight rows that fill no tile, k that fills no
+chunk and leaves warps without any, one to sixteen tokens, strided rows, outputs in pairs.  The operands are bfloat16 (products exact in fp32), so an output is off by
+fp32 sums only: below (K + 8) 2^-23 sum |w x|."""
+import numpy as np
+import pytest
+
+from tests.rapisun_oracle import bf16_round
+from tests.test_gpu_dense_mm import mm
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,N,K,ldx", [(1, 1, 8, 8), (2, 15, 16, 20), (4, 17, 40, 40), (8, 16, 256, 260), (9, 33, 264, 264), (16, 48, 2056, 2056), (7, 100, 1280, 1284), (13, 31, 1032, 1032)])
+def test_few_rows(M, N, K, ldx):
+    rng = np.random.default_rng(M + 10 * N + K)
+    W, X = bf16_round(rng.standard_normal((N, K))), rng.standard_normal((M, ldx))
+    Xr = bf16_round(X[:, :K])
+    got, lim = mm(W, X, M, N, K, ldx=ldx).reshape(M, N), (K + 8) * 2.0 ** -23 * (np.abs(Xr) @ np.abs(W).T)
+    assert (np.abs(got - Xr @ W.T) <= lim).all()
+    one = mm(W, X[M - 1:], 1, N, K, ldx=ldx).reshape(N)              # a token's outputs do not depend on the rest of the batch
+    assert np.array_equal(one, got[M - 1])
