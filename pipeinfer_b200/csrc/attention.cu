@@ -55,8 +55,8 @@ void rope_table_build(std::vector<float2> & tab, int n_pos, int n_dims, int mode
 // (a K row in 128-bit loads, the 32 lane accumulators of the reference in registers); phase 3 gives every thread a pair of
 // output dims and a share of the 32 accumulators, each a sequential chain over its cells.  K/V of a KV head are re-read by its
 // G query heads through L2 -- a few MB per layer at these context lengths.  Masked cells are never loaded.
-#define ATQ_THREADS 256
-#define ATQ_VCAP    256          /* V rows staged in shared memory (cells 0 .. ATQ_VCAP - 1); later cells are read from global memory */
+#define ATQ_VCAP_MIN 256
+#define ATQ_VCAP    384          /* V rows staged in shared memory (cells 0 .. ATQ_VCAP - 1); later cells are read from global memory */
 // RoPE, KV store and attention in one launch.  A CTA rotates its own query head itself, rotates / converts the K and V rows of
 // ALL tokens of the batch for its KV head into shared memory (<= 16 rows: the batch's cells are the contiguous range starting at
 // the descriptor's kv head, and a token of a tree batch attends to earlier tokens of the same batch), and the first query head
@@ -66,10 +66,14 @@ void rope_table_build(std::vector<float2> & tab, int n_pos, int n_dims, int mode
 //
 // The kernel is a chain of dependent memory round trips, not of arithmetic, so everything that does not depend on the QKV
 // projection is fetched BEFORE the wait on it: the descriptor words and positions, the RoPE entries, the mask bytes and K rows of
-// the first 128 cells (registers), and the V rows of up to ATQ_VCAP cells (cp.async into shared memory).  All of it was final
+// the first 512 or 128 cells (registers), and the V rows of up to ATQ_VCAP cells (cp.async into shared memory).  All of it was final
 // before this launch's predecessor started: cache rows of earlier decodes, and the mask / scalars of the pass's first kernels.
-template <int HD>
-__global__ void __launch_bounds__(ATQ_THREADS, 2) attention_qh_kernel(const float * __restrict__ qkv, const float * __restrict__ vsep,
+//
+// 512 threads: two rounds of K rows in flight and half the rounds (22 layers of 32 heads of 64 at 300 cells, one token: 17.6 -> 10.6 us a launch; the whole step at
+// 1 / 16 tokens 966 -> 838 and 1558 -> 1414).  Heads of 128 coordinates take 512 threads while a CTA per SM serves the launch (8 layers at 300 cells, 1 / 4
+// tokens: the step 668 -> 598 and 714 -> 647) and 256 with two CTAs per SM beyond (16 tokens: 512 threads would make it 1306 instead of 1244).
+template <int HD, int ATQ_THREADS>
+__global__ void __launch_bounds__(ATQ_THREADS, HD == 64 || ATQ_THREADS == 256 ? 2 : 1) attention_qh_kernel(const float * __restrict__ qkv, const float * __restrict__ vsep,
                                                                    const uint8_t * __restrict__ desc, const float2 * __restrict__ rope, int rope_n_pos, int mode,
                                                                    __half * __restrict__ kcache, __half * __restrict__ vcache, const uint8_t * __restrict__ mask,
                                                                    const int32_t * __restrict__ scalars, const uint16_t * __restrict__ exp_lut,
@@ -105,17 +109,19 @@ __global__ void __launch_bounds__(ATQ_THREADS, 2) attention_qh_kernel(const floa
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    // phase 1 works on cell tid / 2 (+ 128 per round), two lanes per cell: round 0's mask byte and K half-row go to registers now
+    // phase 1 works on cell tid / 2 (+ ATQ_THREADS / 2 per round), two lanes per cell: the mask bytes and K half-rows of the first PRE rounds go to registers now
     const int hsel = tid & 1;
-    uint4     kreg[HD / 16];
-    bool      live0;
-    {
-        const int  i = tid >> 1, ic = max(min(i, n - 1), 0), bi = ic - cell0;
-        const bool inb = bi >= 0 && bi < ntok;
+    constexpr int PRE = ATQ_THREADS / 256;
+    uint4     kpre[PRE][HD / 16];
+    bool      lpre[PRE];
+#pragma unroll
+    for (int rd = 0; rd < PRE; rd++) {
+        const int  i = rd * (ATQ_THREADS / 2) + (tid >> 1), ic = max(min(i, n - 1), 0), bi = ic - cell0;
+        const bool use = i < n && !(bi >= 0 && bi < ntok);
         const uint4 * kr = reinterpret_cast<const uint4 *>(khead + (size_t) ic * GQA);
 #pragma unroll
-        for (int q = 0; q < HD / 16; q++) kreg[q] = inb ? make_uint4(0, 0, 0, 0) : kr[(q >> 1) * 4 + 2 * (q & 1) + hsel];
-        live0 = i < n && !mrow[ic];
+        for (int q = 0; q < HD / 16; q++) kpre[rd][q] = use ? kr[(q >> 1) * 4 + 2 * (q & 1) + hsel] : make_uint4(0, 0, 0, 0);
+        lpre[rd] = i < n && !mrow[ic];
     }
     // RoPE entries of this thread's first two rotation items (covers batches of up to 2 * 256 / half - 1 tokens)
     float2 cs_pre[2];
@@ -164,12 +170,18 @@ __global__ void __launch_bounds__(ATQ_THREADS, 2) attention_qh_kernel(const floa
     // A cell is shared by two neighbouring lanes: the even one forms vectors 0 and 2 of the four, the odd one 1 and 3, and the
     // first addition of the reduce -- (0 + 2) and (1 + 3) -- happens before the halves meet through one shuffle per lane.
     float lmax = -INFINITY;
+#pragma unroll 1
     for (int i0 = 0; i0 < n; i0 += ATQ_THREADS / 2) {
         const int  i  = i0 + (tid >> 1), ic = max(min(i, n - 1), 0), bi = ic - cell0;
         const bool inb = bi >= 0 && bi < ntok;
-        bool live = live0;
-        if (i0 > 0) {
-            // later rounds (n > 128): the row's address does not depend on the mask byte, both loads go out together
+        bool  live;
+        uint4 kreg[HD / 16];
+        if (i0 < PRE * (ATQ_THREADS / 2)) {
+#pragma unroll
+            for (int q = 0; q < HD / 16; q++) kreg[q] = i0 ? kpre[PRE - 1][q] : kpre[0][q];
+            live = i0 ? lpre[PRE - 1] : lpre[0];
+        } else {
+            // later rounds: the row's address does not depend on the mask byte, both loads go out together
             const uint4 * kr = reinterpret_cast<const uint4 *>(khead + (size_t) ic * GQA);
 #pragma unroll
             for (int q = 0; q < HD / 16; q++) kreg[q] = inb ? make_uint4(0, 0, 0, 0) : kr[(q >> 1) * 4 + 2 * (q & 1) + hsel];
@@ -250,7 +262,7 @@ __global__ void __launch_bounds__(ATQ_THREADS, 2) attention_qh_kernel(const floa
     // to accumulator c mod 32, each accumulator a sequential fma chain over its cells; then the same tree per output element;
     // the n - np cells left over are added one by one in double.  A thread owns a pair of output dims and APG of the 32
     // accumulators; the 32 x HD partial sums meet in shared memory.
-    constexpr int TPR = HD / 2, NGR = ATQ_THREADS / TPR, APG = 32 / NGR;      // hd 128: 4 groups x 8 accumulators; hd 64: 8 x 4
+    constexpr int TPR = HD / 2, NGR = ATQ_THREADS / TPR, APG = 32 / NGR;      // 512 threads, hd 128: 8 groups x 4 accumulators; hd 64: 16 x 2
     const int grp = tid / TPR, dp = tid % TPR;
     const int np  = n & ~31;
     auto vrow = [&](int c) -> const __half * {          // row of cell c for this KV head: batch rows, staged rows, or the cache
@@ -292,20 +304,23 @@ __global__ void __launch_bounds__(ATQ_THREADS, 2) attention_qh_kernel(const floa
     }
 }
 
-template <int HD>
+// V rows staged by a context: the larger number unless a long score row needs the room
+static size_t att_smem(int hd, int n_ctx, int vcap) { return ((size_t) n_ctx + 32 * hd) * sizeof(float) + (size_t) std::min(n_ctx, vcap) * hd * sizeof(__half); }
+#define ATQ_SMEM_MAX (200 * 1024)
+template <int HD, int ATQ_THREADS>
 static int launch_att_qh(const float * qkv, const float * vsep, const uint8_t * desc, const float2 * rope, int rope_n_pos, int mode, __half * kc, __half * vc,
                          const uint8_t * mask, const int32_t * scalars, int E, int GQA, int n_ctx, int n_tokens, int n_head, int gdiv, float * out,
                          const int * cancel, cudaStream_t st) {
-    const int    vcap = std::min(n_ctx, ATQ_VCAP);
-    const size_t smem = ((size_t) n_ctx + 32 * HD) * sizeof(float) + (size_t) vcap * HD * sizeof(__half);   // scores + 32 x HD partial sums + staged V rows
+    const int    vcap = std::min(n_ctx, ATQ_THREADS == 512 && att_smem(HD, n_ctx, ATQ_VCAP) <= ATQ_SMEM_MAX ? ATQ_VCAP : ATQ_VCAP_MIN);
+    const size_t smem = att_smem(HD, n_ctx, vcap);   // scores + 32 x HD partial sums + staged V rows
     static size_t configured = 0;
     if (smem > configured) {
         // several CTAs per SM (a verification batch of 3+ tokens is more CTAs than SMs): ask for the large shared-memory carve-out
-        PIB_CHECK(cudaFuncSetAttribute(attention_qh_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) std::max(smem, (size_t) 32 * 1024)));
-        PIB_CHECK(cudaFuncSetAttribute(attention_qh_kernel<HD>, cudaFuncAttributePreferredSharedMemoryCarveout, (int) cudaSharedmemCarveoutMaxShared));
+        PIB_CHECK(cudaFuncSetAttribute(attention_qh_kernel<HD, ATQ_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) std::max(smem, (size_t) 32 * 1024)));
+        PIB_CHECK(cudaFuncSetAttribute(attention_qh_kernel<HD, ATQ_THREADS>, cudaFuncAttributePreferredSharedMemoryCarveout, (int) cudaSharedmemCarveoutMaxShared));
         configured = smem;
     }
-    pib_launch(attention_qh_kernel<HD>, dim3(n_head, n_tokens), dim3(ATQ_THREADS), smem, st, qkv, vsep, desc, rope, rope_n_pos, mode, kc, vc, mask, scalars,
+    pib_launch(attention_qh_kernel<HD, ATQ_THREADS>, dim3(n_head, n_tokens), dim3(ATQ_THREADS), smem, st, qkv, vsep, desc, rope, rope_n_pos, mode, kc, vc, mask, scalars,
                pib_get_luts().exp_f16, E, GQA, n_ctx, 1.0f / sqrtf((float) HD), out, cancel, gdiv, vcap);
     PIB_CHECK(cudaGetLastError());
     return PIB_OK;
@@ -314,7 +329,7 @@ static int launch_att_qh(const float * qkv, const float * vsep, const uint8_t * 
 bool pib_attention_supported(int hd, int n_head, int n_head_kv, int n_ctx) {
     if (hd != 64 && hd != 128) return false;
     if (n_head % n_head_kv) return false;
-    return ((size_t) n_ctx + 32 * hd) * sizeof(float) + (size_t) std::min(n_ctx, ATQ_VCAP) * hd * 2 <= 200 * 1024;      // the scores of one (head, token) live in shared memory
+    return att_smem(hd, n_ctx, ATQ_VCAP_MIN) <= ATQ_SMEM_MAX;      // the scores of one (head, token) live in shared memory
 }
 
 // RoPE (mode 0: adjacent pairs, 2: NeoX) + KV store + attention of one chunk: qkv = the fused projection's output [n_tokens][E + 2 GQA]
@@ -323,8 +338,10 @@ int pib_attention(const float * qkv, const float * vsep, const uint8_t * desc, c
                   const uint8_t * mask, const int32_t * scalars, int n_tokens, int n_head, int n_head_kv, int hd, int n_ctx, float * out,
                   const int * cancel, cudaStream_t st) {
     const int E = n_head * hd, GQA = n_head_kv * hd, G = n_head / n_head_kv;
-    if (hd == 128) return launch_att_qh<128>(qkv, vsep, desc, rope, rope_n_pos, mode, kc, vc, mask, scalars, E, GQA, n_ctx, n_tokens, n_head, G, out, cancel, st);
-    if (hd == 64)  return launch_att_qh<64>(qkv, vsep, desc, rope, rope_n_pos, mode, kc, vc, mask, scalars, E, GQA, n_ctx, n_tokens, n_head, G, out, cancel, st);
+#define ATQ_GO(HD, NT) return launch_att_qh<HD, NT>(qkv, vsep, desc, rope, rope_n_pos, mode, kc, vc, mask, scalars, E, GQA, n_ctx, n_tokens, n_head, G, out, cancel, st)
+    if (hd == 128) { if (n_head * n_tokens <= pib_num_sms()) ATQ_GO(128, 512); else ATQ_GO(128, 256); }
+    if (hd == 64)  ATQ_GO(64, 512);
+#undef ATQ_GO
     pib_set_error("attention: unsupported head_dim %d", hd);
     return PIB_ERR_UNSUPP;
 }
