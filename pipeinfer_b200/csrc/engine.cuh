@@ -159,7 +159,9 @@ struct pib_context {
     std::deque<int>      inflight;        // run ids in issue order
     int                  last_finished = -1;
     float *              logits_fetch_dev = nullptr;   // head of a pipeline: staging for one row fetched from the last stage
-    std::vector<float>   logits_host;     // lazily filled rows of the last finished run
+    std::vector<float>   logits_host;     // lazily filled rows of the last finished run (prompts)
+    float *              logits_pin = nullptr;      // the same for runs of up to PIB_CHUNK tokens: page-locked, all rows in one copy
+    size_t               logits_pin_cap = 0;        // floats
     std::vector<uint8_t> logits_row_valid;
     bool                 logits_all = true;
     uint64_t             n_kernels = 0;   // launches issued by this context (bench: gpu_launches)

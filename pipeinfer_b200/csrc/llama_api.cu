@@ -416,7 +416,7 @@ float * llama_get_logits(struct llama_context * ctx) {
     if (c->last_finished < 0) return nullptr;
     const int n = c->runs[c->last_finished].n_tokens;
     for (int i = 0; i < n; i++) pib_logits_row(c, i);
-    return c->logits_host.data();
+    return const_cast<float *>(pib_logits_row(c, 0));         // rows are contiguous
 }
 
 int llama_pib_get_top8(struct llama_context * ctx, int32_t i, llama_token_data * out8) {
