@@ -233,6 +233,130 @@ gemv_blk32_kernel(const uint8_t * __restrict__ tiles, int ngr, int N, const int8
     if (threadIdx.x == 0) counters[T] = 0;
 }
 
+// The same for matrices whose row tiles are there all at once (few, and long): WARPS warps per tile, no k split, every warp streams its records through a private
+// ring in shared memory filled by cp.async, STAGES - 1 of them in flight (as gemv_q4k_ring_kernel).
+// What bounds it: a warp's chain of memory latencies, which more warps and a deeper prefetch shorten.  4096 x 4096 Q4_0 at 8 / 16 tokens 6.2 / 12.0 -> 4.4 / 7.7 us,
+// 4096 x 11008 9.8 / 20.8 -> 8.5 / 15.5, 11264 x 2048 (four warps) 7.3 -> 5.3.  With several rounds of tiles new CTAs keep arriving with their first records in flight, the
+// ring's extra pass through shared memory is what counts (22016 x 4096 at 7 tokens 16.0 -> 16.5, Q8_0 18.9 -> 24.5), and gemv_blk32_kernel stays.
+template <int WT, int NT, int WARPS, int STAGES>
+__global__ void __launch_bounds__(WARPS * 32, NT == 1 ? (WARPS == 4 ? 5 : 2) : (WARPS == 4 ? 3 : 1))
+gemv_blk32_ring_kernel(const uint8_t * __restrict__ tiles, int ngr, int N, const int8_t * __restrict__ aqs, const __half * __restrict__ adx, int b, float * __restrict__ y, const int * __restrict__ cancel) {
+    if (PIB_CANCELLED(cancel)) { pib_pdl_wait(); return; }
+    constexpr int REC = WT == PIB_TYPE_Q4_0 ? 2304 : 4352, PIECES = (REC + 511) / 512;        // 512 bytes per warp-wide copy, the last one half
+    constexpr int NQ  = WT == PIB_TYPE_Q4_0 ? 4 : 8;            // 16-byte quant pieces per lane and record
+    extern __shared__ __align__(16) uint8_t bk_smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int T = blockIdx.x;
+    const uint8_t * tbase  = tiles + (size_t) T * ngr * REC + lane * 16;
+    uint8_t *       ring   = bk_smem + warp * (STAGES * REC);
+    const uint32_t  ring_a = (uint32_t) __cvta_generic_to_shared(ring) + lane * 16;
+    int ps = warp;                                         // prefetch cursor
+    auto issue = [&](int stage) {
+        if (ps < ngr) {
+            const uint8_t * src = tbase + (size_t) ps * REC;
+            const uint32_t  dst = ring_a + stage * REC;
+#pragma unroll
+            for (int c = 0; c < PIECES; c++)
+                if (c < PIECES - 1 || lane < 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + c * 512), "l"(src + c * 512) : "memory");
+            ps += WARPS;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // the weights are immutable: their copies start before the wait on the kernel that produces the activations
+#pragma unroll
+    for (int i = 0; i < STAGES - 1; i++) issue(i);
+
+    float acc[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; n++) { acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f; }
+    const int8_t * a_q[NT];
+    const __half * a_d[NT][2];
+#pragma unroll
+    for (int n = 0; n < NT; n++) {
+        a_q[n] = aqs + (size_t) min(n * 8 + g, b - 1) * ngr * 256 + t * 64;
+#pragma unroll
+        for (int e = 0; e < 2; e++) a_d[n][e] = adx + (size_t) min(n * 8 + 2 * t + e, b - 1) * ngr * 8;
+    }
+    pib_pdl_wait();
+    pib_pdl_trigger();
+    int stage = 0;
+    for (int s = warp; s < ngr; s += WARPS) {
+        int4 aq[NT][4];
+        int4 ax[NT][2];
+#pragma unroll
+        for (int n = 0; n < NT; n++) {
+            const int4 * ap = reinterpret_cast<const int4 *>(a_q[n] + (size_t) s * 256);
+#pragma unroll
+            for (int c = 0; c < 4; c++) aq[n][c] = __ldg(ap + c);
+#pragma unroll
+            for (int e = 0; e < 2; e++) ax[n][e] = __ldg(reinterpret_cast<const int4 *>(a_d[n][e] + (size_t) s * 8));
+        }
+        __syncwarp();                                           // every lane has used the stage about to be refilled
+        issue((stage + STAGES - 1) % STAGES);
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
+        __syncwarp();
+        const uint8_t * rs = ring + stage * REC;
+        int4 wq[NQ], dq[2];
+#pragma unroll
+        for (int c = 0; c < NQ; c++) wq[c] = *reinterpret_cast<const int4 *>(rs + c * 512 + lane * 16);
+        dq[0] = *reinterpret_cast<const int4 *>(rs + (REC - 256) + g * 16);
+        dq[1] = *reinterpret_cast<const int4 *>(rs + (REC - 256) + (g + 8) * 16);
+        const uint32_t dw0[4] = { (uint32_t) dq[0].x, (uint32_t) dq[0].y, (uint32_t) dq[0].z, (uint32_t) dq[0].w };   // row g:   d of blocks 2i | 2i+1
+        const uint32_t dw1[4] = { (uint32_t) dq[1].x, (uint32_t) dq[1].y, (uint32_t) dq[1].z, (uint32_t) dq[1].w };   // row g+8
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            int a0, a1, a2, a3;
+            if (WT == PIB_TYPE_Q4_0) {
+                const int4     w  = wq[j >> 1];
+                const uint32_t w0 = (uint32_t) ((j & 1) ? w.z : w.x), w1 = (uint32_t) ((j & 1) ? w.w : w.y);
+                a0 = bk_sub8(w0 & 0x0F0F0F0Fu); a2 = bk_sub8((w0 >> 4) & 0x0F0F0F0Fu);
+                a1 = bk_sub8(w1 & 0x0F0F0F0Fu); a3 = bk_sub8((w1 >> 4) & 0x0F0F0F0Fu);
+            } else {
+                const int4 w = wq[j & (NQ - 1)];
+                a0 = w.x; a1 = w.y; a2 = w.z; a3 = w.w;
+            }
+            const float d0 = __half2float(__ushort_as_half((unsigned short) ((j & 1) ? dw0[j >> 1] >> 16 : dw0[j >> 1] & 0xffffu)));
+            const float d1 = __half2float(__ushort_as_half((unsigned short) ((j & 1) ? dw1[j >> 1] >> 16 : dw1[j >> 1] & 0xffffu)));
+#pragma unroll
+            for (int n = 0; n < NT; n++) {
+                const int4 bq = aq[n][j >> 1];
+                int c[4] = { 0, 0, 0, 0 };
+                bk_mma_s8(c, a0, a1, a2, a3, (j & 1) ? bq.z : bq.x, (j & 1) ? bq.w : bq.y);
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const int4     xv = ax[n][e];
+                    const uint32_t xw = (uint32_t) ((j >> 1) == 0 ? xv.x : (j >> 1) == 1 ? xv.y : (j >> 1) == 2 ? xv.z : xv.w);
+                    const float    dx = __half2float(__ushort_as_half((unsigned short) ((j & 1) ? xw >> 16 : xw & 0xffffu)));
+                    acc[n][e]     = fmaf(__fmul_rn(d0, dx), (float) c[e], acc[n][e]);
+                    acc[n][2 + e] = fmaf(__fmul_rn(d1, dx), (float) c[2 + e], acc[n][2 + e]);
+                }
+            }
+        }
+        stage = stage + 1 == STAGES ? 0 : stage + 1;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                            // the rings are done with: their memory becomes the reduction buffer
+
+    float (*red)[NT * 8][16] = reinterpret_cast<float (*)[NT * 8][16]>(bk_smem);
+#pragma unroll
+    for (int n = 0; n < NT; n++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            red[warp][n * 8 + 2 * t + e][g]     = acc[n][e];
+            red[warp][n * 8 + 2 * t + e][g + 8] = acc[n][2 + e];
+        }
+    __syncthreads();
+    for (int i = threadIdx.x; i < NT * 8 * 16; i += WARPS * 32) {
+        const int tok = i / 16, r = i % 16, row = T * 16 + r;
+        if (tok < b && row < N) {
+            float v = red[0][tok][r];
+#pragma unroll
+            for (int w2 = 1; w2 < WARPS; w2++) v += red[w2][tok][r];
+            y[(size_t) tok * N + row] = v;
+        }
+    }
+}
+
 // ---- launcher -----------------------------------------------------------------------------------------------------------
 struct bk_scratch { float * partial = nullptr; unsigned int * counters = nullptr; };
 static std::map<std::pair<int, cudaStream_t>, bk_scratch> g_bk_scratch;
@@ -261,11 +385,28 @@ bool pib_gemv_blk32_supported(const pib_weight * w, int b) {
     return w && (w->type == PIB_TYPE_Q4_0 || w->type == PIB_TYPE_Q8_0) && w->tiles != nullptr && b >= 1 && b <= PIB_MAX_BATCH;
 }
 
+template <int WT, int NT, int WARPS, int STAGES>
+static int bk_ring_launch(const pib_weight * w, int ngr, const int8_t * aqs, const __half * adx, int b, float * y_dev, const int * cancel, cudaStream_t st) {
+    const size_t smem = (size_t) WARPS * STAGES * bk_rec_bytes(WT);
+    static bool configured = false;
+    if (!configured) { PIB_CHECK(cudaFuncSetAttribute(gemv_blk32_ring_kernel<WT, NT, WARPS, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)); configured = true; }
+    PIB_CHECK(pib_launch(gemv_blk32_ring_kernel<WT, NT, WARPS, STAGES>, dim3((unsigned) ((w->N + 15) / 16)), dim3(WARPS * 32), smem, st, w->tiles, ngr, (int) w->N, aqs, adx, b, y_dev, cancel));
+    return PIB_OK;
+}
+
 int pib_gemv_blk32(const pib_weight * w, const void * act_dev, int b, float * y_dev, const int * cancel, cudaStream_t st) {
     if (!pib_gemv_blk32_supported(w, b)) { pib_set_error("pib_gemv: the tensor-core variant needs Q4_0 / Q8_0 weights with tiles"); return PIB_ERR_UNSUPP; }
     const pib_act_layout L   = pib_act_layout_of(w->type, w->K, b);
     const uint8_t *      act = (const uint8_t *) act_dev;
     const int            ngr = (int) ((w->K + 255) / 256), n_tiles = (int) ((w->N + 15) / 16);
+    const int8_t *       aqs = (const int8_t *) (act + L.qsp_off);
+    const __half *       adx = (const __half *) (act + L.bs8_off);    // dxp plane of the 32-element block formats
+    // the ring: eight warps per tile while two such CTAs per SM hold every tile, four (Q4_0, one token group) while five do
+    if (n_tiles <= 4 * pib_num_sms() && ngr >= 16) {
+        if (w->type == PIB_TYPE_Q4_0) return b <= 8 ? bk_ring_launch<PIB_TYPE_Q4_0, 1, 8, 4>(w, ngr, aqs, adx, b, y_dev, cancel, st) : bk_ring_launch<PIB_TYPE_Q4_0, 2, 8, 4>(w, ngr, aqs, adx, b, y_dev, cancel, st);
+        return b <= 8 ? bk_ring_launch<PIB_TYPE_Q8_0, 1, 8, 3>(w, ngr, aqs, adx, b, y_dev, cancel, st) : bk_ring_launch<PIB_TYPE_Q8_0, 2, 8, 3>(w, ngr, aqs, adx, b, y_dev, cancel, st);
+    }
+    if (w->type == PIB_TYPE_Q4_0 && b <= 8 && n_tiles <= 5 * pib_num_sms() && n_tiles > 2 * pib_num_sms()) return bk_ring_launch<PIB_TYPE_Q4_0, 1, 4, 4>(w, ngr, aqs, adx, b, y_dev, cancel, st);
     // k splits: enough CTAs to fill the machine when there are few row tiles; at least two records per warp
     int split = 1;
     while (n_tiles * split < pib_split_fill_target() && split * 2 * BK_WARPS <= ngr && split < 16) split *= 2;     // see gemv_mma.cu
@@ -273,8 +414,6 @@ int pib_gemv_blk32(const pib_weight * w, const void * act_dev, int b, float * y_
     bk_scratch * s = nullptr;
     if (split > 1 && bk_ensure_scratch(st, &s) != PIB_OK) { pib_set_error("pib_gemv: scratch allocation failed"); return PIB_ERR_NOMEM; }
     const dim3     grid(n_tiles, split);
-    const int8_t * aqs = (const int8_t *) (act + L.qsp_off);
-    const __half * adx = (const __half *) (act + L.bs8_off);          // dxp plane of the 32-element block formats
     float *        pp  = s ? s->partial : nullptr;
     unsigned int * cc  = s ? s->counters : nullptr;
     cudaError_t    e;
