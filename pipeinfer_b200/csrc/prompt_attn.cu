@@ -10,14 +10,15 @@
 // difference (there: a table over fp16 differences), weights are rounded to fp16 before they are divided by their sum (there: after), the sum is held
 // in double.  So nothing is rounded more often than there, and only the order of the fp32 sums differs.
 //
-// What bounds it: the launch has 4 MFLOP per (head, 64 tokens, 64 cells) and at most a few hundred CTAs, so it is latency: one warp group per
-// scheduler walks its tiles one after the other.  mma.sync on register operands is taken rather than tcgen05: a tile's scores go straight from the
-// accumulator registers through exp into the next product's A operand, and at 0.1 of a prompt's time the trip through tensor memory has nothing to win.
+// What bounds it: the launch has 4 MFLOP per (head, 64 tokens, 64 cells) and at most a few hundred CTAs, so it is latency: warps walk their tiles one after the
+// other (256 tokens, 32 heads of 128, up to 700 cells: 33 us with one group of four warps per CTA, 25 with two that take the tiles in turn, the rotation 7; the sixteen
+// launches before: 913).  mma.sync on register operands is taken rather than tcgen05: a tile's scores go straight from the accumulator registers through exp into the
+// next product's A operand, and at 0.1 of a prompt's time the trip through tensor memory has nothing to win.
 #include "pib_common.cuh"
 #include "desc.cuh"
 #include "engine.cuh"
 
-#define PA_ROWS   64                 // tokens per CTA: 4 warps x 16
+#define PA_ROWS   64                 // tokens per CTA: 4 warps x 16, twice
 #define PA_CELLS  64                 // cells per tile
 #define PA_TILES  1024               // tiles of the visibility bitmap: contexts of up to 65536 cells
 
@@ -92,29 +93,39 @@ __device__ __forceinline__ uint32_t pa_seen16(const uint8_t * __restrict__ mrow,
     return ~hid & in;
 }
 
+// two groups of four warps take the tiles in turn, each with its own stages and running state, and meet at the end
+__device__ __forceinline__ void pa_group_sync(int grp) { asm volatile("bar.sync %0, 128;" ::"r"(grp + 1) : "memory"); }
+__device__ __forceinline__ bool pa_group_any(int grp, bool v) {
+    int r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %2, 0;\n\tbar.red.or.pred q, %1, 128, p;\n\tselp.b32 %0, 1, 0, q;\n\t}" : "=r"(r) : "r"(grp + 1), "r"((int) v) : "memory");
+    return r != 0;
+}
+
 template <int HD>
-__global__ void __launch_bounds__(128, HD == 64 ? 3 : 2)
+__global__ void __launch_bounds__(256, HD == 64 ? 2 : 1)
 prompt_attn_kernel(const __half * __restrict__ q16, const __half * __restrict__ kc, const __half * __restrict__ vc, const uint8_t * __restrict__ mask, const int32_t * __restrict__ scalars,
                    int ntok, int E, int GQA, int gdiv, int n_ctx, float kq_scale, float * __restrict__ out, const int * __restrict__ cancel) {
     constexpr int CH = HD / 8, ROWB = HD * 2, TILEB = PA_CELLS * ROWB;            // 16-byte pieces and bytes of a cache row, bytes of a tile
-    extern __shared__ __align__(128) uint8_t pa_sm[];                            // K[2 stages] | V[2 stages]
+    extern __shared__ __align__(128) uint8_t pa_sm[];                            // per group K[2 stages] | V[2 stages]; at the end group 1's state
     __shared__ uint32_t seen_tiles[PA_TILES / 32];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
+    const int grp = threadIdx.x >> 7, tid = threadIdx.x & 127, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
     const int head = blockIdx.x, row0 = (gridDim.y - 1 - blockIdx.y) * PA_ROWS;   // the last rows see most cells: they start first
-    const uint32_t sm = (uint32_t) __cvta_generic_to_shared(pa_sm);
+    const uint8_t * own = pa_sm + grp * 4 * TILEB;
+    const uint32_t  sm = (uint32_t) __cvta_generic_to_shared(own);
     const bool vec = (n_ctx & 15) == 0;
     pib_pdl_wait();
     pib_pdl_trigger();
-    if (PIB_CANCELLED(cancel)) return;
+    // one decision for the block: the flag can change while its warps read it, and the groups' barriers count on every thread
+    if (__syncthreads_or(PIB_CANCELLED(cancel))) return;
     const int n = min(scalars[2], n_ctx), n_tiles = (n + PA_CELLS - 1) / PA_CELLS;
     const __half * kh = kc + (size_t) (head / gdiv) * HD, * vh = vc + (size_t) (head / gdiv) * HD;
 
     // tiles that some row of the block sees (a prompt's later cells, other sequences' cells: none)
-    if (tid < PA_TILES / 32) seen_tiles[tid] = 0;
+    if (threadIdx.x < PA_TILES / 32) seen_tiles[threadIdx.x] = 0;
     __syncthreads();
     {
         const int rows = min(PA_ROWS, ntok - row0), per = (n + 15) / 16;
-        for (int i = tid; i < rows * per; i += 128) {
+        for (int i = threadIdx.x; i < rows * per; i += 256) {
             const int r = i / per, c = (i - r * per) * 16;
             if (pa_seen16(mask + (size_t) (row0 + r) * n_ctx, c, n, vec)) atomicOr(&seen_tiles[c / PA_CELLS / 32], 1u << (c / PA_CELLS % 32));
         }
@@ -155,27 +166,28 @@ prompt_attn_kernel(const __half * __restrict__ q16, const __half * __restrict__ 
     constexpr float LOG2E = 1.44269504088896340736f;
 
     int tile = next_tile(0), stage = 0;
+    if (grp) tile = next_tile(tile + 1);
     if (tile < n_tiles) load_tile(tile, 0);
     while (tile < n_tiles) {
-        const int nxt = next_tile(tile + 1);
+        const int nxt = next_tile(next_tile(tile + 1) + 1);
         if (nxt < n_tiles) load_tile(nxt, stage ^ 1);
         const uint32_t bits_a = pa_seen16(mask + (size_t) rac * n_ctx, tile * PA_CELLS + 16 * t4, n, vec);
         const uint32_t bits_b = pa_seen16(mask + (size_t) rbc * n_ctx, tile * PA_CELLS + 16 * t4, n, vec);
         if (nxt < n_tiles) asm volatile("cp.async.wait_group 1;" ::: "memory");
         else               asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
+        pa_group_sync(grp);
         const uint32_t sk = sm + (uint32_t) (stage * TILEB), sv = sk + 2 * TILEB;
         // a value that is no number (or infinite) must not reach rows that do not see its cell: 0 x inf.  Rare, so the tile then takes its products one by one
         int odd = 0;
         for (int i = tid; i < PA_CELLS * CH; i += 128) {
-            const uint4 v = *reinterpret_cast<const uint4 *>(pa_sm + stage * TILEB + 2 * TILEB + i * 16);
+            const uint4 v = *reinterpret_cast<const uint4 *>(own + stage * TILEB + 2 * TILEB + i * 16);
 #pragma unroll
             for (int q = 0; q < 4; q++) {
                 const uint32_t w = q == 0 ? v.x : q == 1 ? v.y : q == 2 ? v.z : v.w;
                 odd |= ((w & 0x7c00u) == 0x7c00u) | ((w & 0x7c000000u) == 0x7c000000u);
             }
         }
-        odd = __syncthreads_or(odd);
+        odd = pa_group_any(grp, odd);
 
         float s[8][4];
 #pragma unroll
@@ -244,19 +256,42 @@ prompt_attn_kernel(const __half * __restrict__ q16, const __half * __restrict__ 
                     const int      r = j * 8 + e;
 #pragma unroll
                     for (int i = 0; i < HD / 8; i++) {
-                        const uint32_t v = *reinterpret_cast<const uint32_t *>(pa_sm + stage * TILEB + 2 * TILEB + r * ROWB + ((i ^ (r & 7)) << 4) + t4 * 4);
+                        const uint32_t v = *reinterpret_cast<const uint32_t *>(own + stage * TILEB + 2 * TILEB + r * ROWB + ((i ^ (r & 7)) << 4) + t4 * 4);
                         const float    v0 = pib_h2f((uint16_t) v), v1 = pib_h2f((uint16_t) (v >> 16));
                         if (fa != 0.f) { o[i][0] = fmaf(fa, v0, o[i][0]); o[i][1] = fmaf(fa, v1, o[i][1]); }
                         if (fb != 0.f) { o[i][2] = fmaf(fb, v0, o[i][2]); o[i][3] = fmaf(fb, v1, o[i][3]); }
                     }
                 }
         }
-        __syncthreads();                                                          // the stage is free for the tile after next
+        pa_group_sync(grp);                                                       // the stage is free for the tile after next
         tile = nxt;
         stage ^= 1;
     }
 #pragma unroll
     for (int d = 1; d < 4; d <<= 1) { l_a += __shfl_xor_sync(0xffffffffu, l_a, d); l_b += __shfl_xor_sync(0xffffffffu, l_b, d); }
+    // group 1 leaves its state per row and its sums; group 0 adds them, both brought to the common maximum
+    __syncthreads();
+    float *  po = reinterpret_cast<float *>(pa_sm) + tid;                         // [HD / 2][128 threads]
+    float *  pm = reinterpret_cast<float *>(pa_sm) + HD / 2 * 128 + tid * 2;
+    double * pl = reinterpret_cast<double *>(pa_sm + HD / 2 * 512 + 1024) + tid * 2;
+    if (grp) {
+#pragma unroll
+        for (int i = 0; i < HD / 8; i++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) po[(i * 4 + e) * 128] = o[i][e];
+        pm[0] = m_a; pm[1] = m_b; pl[0] = l_a; pl[1] = l_b;
+    }
+    __syncthreads();
+    if (grp) return;
+    const float x_a = fmaxf(m_a, pm[0]), x_b = fmaxf(m_b, pm[1]), u_a = x_a == -INFINITY ? 0.f : x_a, u_b = x_b == -INFINITY ? 0.f : x_b;
+    const float f_a = exp2f((m_a - u_a) * LOG2E), f_b = exp2f((m_b - u_b) * LOG2E), h_a = exp2f((pm[0] - u_a) * LOG2E), h_b = exp2f((pm[1] - u_b) * LOG2E);
+    l_a = l_a * (double) f_a + pl[0] * (double) h_a;
+    l_b = l_b * (double) f_b + pl[1] * (double) h_b;
+#pragma unroll
+    for (int i = 0; i < HD / 8; i++) {
+        o[i][0] = fmaf(po[(i * 4) * 128], h_a, o[i][0] * f_a);     o[i][1] = fmaf(po[(i * 4 + 1) * 128], h_a, o[i][1] * f_a);
+        o[i][2] = fmaf(po[(i * 4 + 2) * 128], h_b, o[i][2] * f_b); o[i][3] = fmaf(po[(i * 4 + 3) * 128], h_b, o[i][3] * f_b);
+    }
     const float i_a = (float) (1.0 / l_a), i_b = (float) (1.0 / l_b);
 #pragma unroll
     for (int i = 0; i < HD / 8; i++) {
@@ -272,9 +307,9 @@ bool pib_prompt_attention_supported(int hd, int n_ctx) { return (hd == 64 || hd 
 template <int HD>
 static int pa_launch(const __half * q16, const __half * kc, const __half * vc, const uint8_t * mask, const int32_t * scalars, int ntok, int n_head, int n_head_kv, int n_ctx, float * out,
                      const int * cancel, cudaStream_t st) {
-    constexpr size_t smem = (size_t) 4 * PA_CELLS * HD * sizeof(__half);
+    constexpr size_t smem = (size_t) 8 * PA_CELLS * HD * sizeof(__half);
     PIB_CHECK(cudaFuncSetAttribute(prompt_attn_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-    pib_launch(prompt_attn_kernel<HD>, dim3(n_head, (ntok + PA_ROWS - 1) / PA_ROWS), dim3(128), smem, st, q16, kc, vc, mask, scalars, ntok, n_head * HD, n_head_kv * HD, n_head / n_head_kv,
+    pib_launch(prompt_attn_kernel<HD>, dim3(n_head, (ntok + PA_ROWS - 1) / PA_ROWS), dim3(256), smem, st, q16, kc, vc, mask, scalars, ntok, n_head * HD, n_head_kv * HD, n_head / n_head_kv,
                n_ctx, 1.0f / sqrtf((float) HD), out, cancel);
     PIB_CHECK(cudaGetLastError());
     return PIB_OK;
