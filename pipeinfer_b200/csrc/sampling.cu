@@ -15,15 +15,24 @@
 
 // A row is divided over P blocks of a thread-block cluster (contiguous slices of the vocabulary); each finds the best eight and, once the cluster knows the maximum,
 // the exponentials' sum of its slice, and the first block merges the P sorted lists and sums through distributed shared memory.
-// What bounds it: chains of block-wide rounds.  One block of 1024 threads per row took 27 us for a row of 32 000 (16 for 8 000), whatever the number of rows.
+// What bounds it: chains of block-wide rounds, so a round is two warp reductions in hardware (redux on order-preserving keys) and one barrier, and a thread looks for its
+// best two only.  One row of 32 000: 27 -> 14 us, 256 rows: 40, 1 512 rows of 8 000: 42 (with eight-place lists sorted per thread and shuffles 99).
 #define SMP_THREADS 256
 #define SMP_TOPK    8
 #define SMP_PARTS   8
-#define SMP_REG     32
 #define SMP_NONE    0x7fffffff
 
-// b is ahead of a: larger, or equal and earlier (std::max_element semantics); places without an element come last
-__device__ __forceinline__ bool smp_ahead(float bv, int bi, float av, int ai) { return bi != SMP_NONE && (ai == SMP_NONE || bv > av || (bv == av && bi < ai)); }
+// order-preserving keys: larger value, larger key; what is no number comes last, but in front of places without an element (0)
+__device__ __forceinline__ uint32_t smp_key(float v) {
+    const uint32_t u = __float_as_uint(v);
+    return v != v ? 1u : (u & 0x80000000u) ? ~u : u | 0x80000000u;
+}
+// the warp's best (key, index): the largest key, the smallest index among equals
+__device__ __forceinline__ void smp_warp_best(uint32_t & key, int & idx) {
+    const uint32_t k = __reduce_max_sync(0xffffffffu, key);
+    idx = __reduce_min_sync(0xffffffffu, key == k ? idx : SMP_NONE);
+    key = k;
+}
 
 __global__ void __launch_bounds__(SMP_THREADS) sample_topk_kernel(float * __restrict__ logits, int n_vocab,
                                                                   const int32_t * __restrict__ bias_ids, const float * __restrict__ bias_val,
@@ -31,9 +40,10 @@ __global__ void __launch_bounds__(SMP_THREADS) sample_topk_kernel(float * __rest
     pib_pdl_wait();
     pib_pdl_trigger();
     constexpr int NW = SMP_THREADS / 32;
-    __shared__ float  s_val[2][NW], s_top[SMP_TOPK];
-    __shared__ int    s_idx[2][NW], s_topi[SMP_TOPK];
-    __shared__ double s_sum[NW], s_total;
+    __shared__ uint32_t s_key[2][NW], s_topk[SMP_TOPK];
+    __shared__ int      s_idx[2][NW], s_topi[SMP_TOPK];
+    __shared__ float    s_topv[SMP_TOPK];
+    __shared__ double   s_sum[NW], s_total;
     cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
     const int P = gridDim.y, part = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float *   l = logits + (size_t) blockIdx.x * n_vocab;
@@ -42,96 +52,55 @@ __global__ void __launch_bounds__(SMP_THREADS) sample_topk_kernel(float * __rest
     const int  lo = (int) ((long long) n_vocab * part / P), hi = off ? lo : (int) ((long long) n_vocab * (part + 1) / P);
     for (int k = tid; k < n_bias; k += SMP_THREADS) if (bias_ids[k] >= lo && bias_ids[k] < hi) l[bias_ids[k]] += bias_val[k];
     __syncthreads();
-    // A thread keeps its elements in registers when they are at most SMP_REG (all loads in flight together) and looks for its best one only; otherwise one pass keeps
-    // the 8 largest of its strided elements, sorted (value descending, index ascending: the indices a thread sees only grow, so strict comparisons keep the
-    // earlier one of two equal values in front)
-    const bool few = hi - lo <= SMP_REG * SMP_THREADS;
-    float tv[SMP_REG];
-    int   ti[SMP_TOPK];
-    auto best_of = [&](float & bv, int & bi) {                    // few: the best element left; taken ones are marked in `gone`
-        bv = -INFINITY; bi = SMP_NONE;
-#pragma unroll
-        for (int j = 0; j < SMP_REG; j++) {
-            const int i = lo + tid + j * SMP_THREADS;
-            if (i < hi && !((uint32_t) ti[0] >> j & 1u) && (bi == SMP_NONE || tv[j] > bv)) { bv = tv[j]; bi = i; }
-        }
-    };
-    float hv;
-    int   hidx;
-    if (few) {
-#pragma unroll
-        for (int j = 0; j < SMP_REG; j++) { const int i = lo + tid + j * SMP_THREADS; tv[j] = i < hi ? l[i] : -INFINITY; }
-        ti[0] = 0;                                                // bit j: element j has been taken
-        best_of(hv, hidx);
-    } else {
-#pragma unroll
-        for (int j = 0; j < SMP_TOPK; j++) { tv[j] = -INFINITY; ti[j] = SMP_NONE; }
-#pragma unroll 4
-        for (int i = lo + tid; i < hi; i += SMP_THREADS) {
-            const float v = l[i];
-            if (v > tv[SMP_TOPK - 1] || ti[SMP_TOPK - 1] == SMP_NONE) {
-                tv[SMP_TOPK - 1] = v; ti[SMP_TOPK - 1] = i;
-#pragma unroll
-                for (int j = SMP_TOPK - 1; j > 0; j--) {
-                    if (tv[j] > tv[j - 1] || ti[j - 1] == SMP_NONE) {
-                        const float fv = tv[j]; tv[j] = tv[j - 1]; tv[j - 1] = fv;
-                        const int   fi = ti[j]; ti[j] = ti[j - 1]; ti[j - 1] = fi;
-                    }
-                }
-            }
-        }
-        hv = tv[0]; hidx = ti[0];
+    // A thread walks its strided elements for the best two (key descending, index ascending: indices only grow, so strict comparisons keep the earlier one of equals in
+    // front).  One that gives away both looks for its next among the elements behind the last one it gave: after it in (key descending, index ascending) order.
+    uint32_t k0 = 0, k1 = 0;
+    int      i0 = SMP_NONE, i1 = SMP_NONE;
+#pragma unroll 8
+    for (int i = lo + tid; i < hi; i += SMP_THREADS) {
+        const uint32_t k = smp_key(l[i]);
+        if (k > k0) { k1 = k0; i1 = i0; k0 = k; i0 = i; }
+        else if (k > k1) { k1 = k; i1 = i; }
     }
-    // eight rounds over the heads of the per-thread lists; every warp finds the block's best from the warps' (two sets of places: one barrier per round)
-    for (int k = 0; k < SMP_TOPK; k++) {
-        float bv = hv;
-        int   bi = hidx;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-            const int   oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (smp_ahead(ov, oi, bv, bi)) { bv = ov; bi = oi; }
-        }
-        if (lane == 0) { s_val[k & 1][warp] = bv; s_idx[k & 1][warp] = bi; }
+    // eight rounds; every warp finds the block's best from the warps' (two sets of places: one barrier per round)
+    for (int r = 0; r < SMP_TOPK; r++) {
+        uint32_t bk = k0;
+        int      bi = i0;
+        smp_warp_best(bk, bi);
+        if (lane == 0) { s_key[r & 1][warp] = bk; s_idx[r & 1][warp] = bi; }
         __syncthreads();
-        bv = s_val[k & 1][lane % NW]; bi = s_idx[k & 1][lane % NW];
-#pragma unroll
-        for (int o = NW / 2; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-            const int   oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (smp_ahead(ov, oi, bv, bi)) { bv = ov; bi = oi; }
-        }
-        if (tid == 0) { s_top[k] = bv; s_topi[k] = bi; }
-        if (hidx == bi && bi != SMP_NONE) {                       // the winner pops its head
-            if (few) {
-                ti[0] |= 1u << ((bi - lo - tid) / SMP_THREADS);
-                best_of(hv, hidx);
-            } else {
-#pragma unroll
-                for (int j = 0; j < SMP_TOPK - 1; j++) { tv[j] = tv[j + 1]; ti[j] = ti[j + 1]; }
-                tv[SMP_TOPK - 1] = -INFINITY; ti[SMP_TOPK - 1] = SMP_NONE;
-                hv = tv[0]; hidx = ti[0];
+        bk = s_key[r & 1][lane % NW]; bi = s_idx[r & 1][lane % NW];
+        smp_warp_best(bk, bi);
+        if (tid == 0) { s_topk[r] = bk; s_topi[r] = bi; s_topv[r] = bi == SMP_NONE ? -INFINITY : l[bi]; }
+        if (bi != SMP_NONE && i0 == bi) {                         // the winner gives its best away
+            const uint32_t gk = k0;
+            const int      gi = i0;
+            k0 = k1; i0 = i1; k1 = 0; i1 = SMP_NONE;
+            if (i0 == SMP_NONE) {
+                for (int i = lo + tid; i < hi; i += SMP_THREADS) {
+                    const uint32_t k = smp_key(l[i]);
+                    if ((k < gk || (k == gk && i > gi)) && k > k0) { k0 = k; i0 = i; }
+                }
             }
         }
     }
     if (P > 1) cl.sync(); else __syncthreads();
     // the row's maximum: lane p looks at part p's best (one remote load each, not P in a row)
-    float max_l = lane >= P ? -INFINITY : P > 1 ? *cl.map_shared_rank(s_top, lane) : s_top[0];
+    float max_l;
     {
-        int mi = lane >= P ? SMP_NONE : P > 1 ? *cl.map_shared_rank(s_topi, lane) : s_topi[0];
-#pragma unroll
-        for (int o = SMP_PARTS / 2; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, max_l, o);
-            const int   oi = __shfl_xor_sync(0xffffffffu, mi, o);
-            if (smp_ahead(ov, oi, max_l, mi)) { max_l = ov; mi = oi; }
-        }
-        max_l = __shfl_sync(0xffffffffu, max_l, 0);
+        const int p = lane < P ? lane : 0;
+        uint32_t  bk = lane >= P ? 0u : P > 1 ? *cl.map_shared_rank(s_topk, p) : s_topk[0];
+        int       bi = lane >= P ? SMP_NONE : P > 1 ? *cl.map_shared_rank(s_topi, p) : s_topi[0];
+        const float v = P > 1 ? *cl.map_shared_rank(s_topv, p) : s_topv[0];
+        const uint32_t mine = bk;
+        const int      idx = bi;
+        smp_warp_best(bk, bi);
+        const unsigned who = __ballot_sync(0xffffffffu, mine == bk && idx == bi);
+        max_l = __shfl_sync(0xffffffffu, v, __ffs((int) who) - 1);
     }
     double sum = 0.0;
-    if (few) {
-#pragma unroll
-        for (int j = 0; j < SMP_REG; j++) if (lo + tid + j * SMP_THREADS < hi) sum += (double) expf(tv[j] - max_l);
-    } else for (int i = lo + tid; i < hi; i += SMP_THREADS) sum += (double) expf(l[i] - max_l);
+#pragma unroll 8
+    for (int i = lo + tid; i < hi; i += SMP_THREADS) sum += (double) expf(l[i] - max_l);
     sum = warp_sum_d(sum);
     if (lane == 0) s_sum[warp] = sum;
     __syncthreads();
@@ -142,35 +111,35 @@ __global__ void __launch_bounds__(SMP_THREADS) sample_topk_kernel(float * __rest
     }
     if (P > 1) cl.sync(); else __syncthreads();
     if (part == 0 && warp == 0) {
-        // lane p < P walks part p's sorted list
-        const float * pv = P > 1 ? cl.map_shared_rank(s_top, lane < P ? lane : 0) : s_top;
-        const int *   pi = P > 1 ? cl.map_shared_rank(s_topi, lane < P ? lane : 0) : s_topi;
-        float mv[SMP_TOPK];
-        int   mi[SMP_TOPK];
+        // lane p < P holds part p's sorted list
+        const int        p = lane < P ? lane : 0;
+        const uint32_t * pk = P > 1 ? cl.map_shared_rank(s_topk, p) : s_topk;
+        const int *      pi = P > 1 ? cl.map_shared_rank(s_topi, p) : s_topi;
+        const float *    pv = P > 1 ? cl.map_shared_rank(s_topv, p) : s_topv;
+        uint32_t mk[SMP_TOPK];
+        int      mi[SMP_TOPK];
+        float    mv[SMP_TOPK];
 #pragma unroll
-        for (int j = 0; j < SMP_TOPK; j++) { mv[j] = lane < P ? pv[j] : -INFINITY; mi[j] = lane < P ? pi[j] : SMP_NONE; }
-        const double mine = lane >= P ? 0.0 : P > 1 ? *cl.map_shared_rank(&s_total, lane) : s_total;
+        for (int j = 0; j < SMP_TOPK; j++) { mk[j] = lane < P ? pk[j] : 0u; mi[j] = lane < P ? pi[j] : SMP_NONE; mv[j] = pv[j]; }
+        const double mine = lane >= P ? 0.0 : P > 1 ? *cl.map_shared_rank(&s_total, p) : s_total;
         double t = 0.0;
 #pragma unroll
-        for (int p = 0; p < SMP_PARTS; p++) t += __shfl_sync(0xffffffffu, mine, p);
-        for (int k = 0; k < SMP_TOPK; k++) {
-            float bv = mv[0];
-            int   bi = mi[0];
-#pragma unroll
-            for (int o = SMP_PARTS / 2; o > 0; o >>= 1) {
-                const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-                const int   oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (smp_ahead(ov, oi, bv, bi)) { bv = ov; bi = oi; }
-            }
+        for (int q = 0; q < SMP_PARTS; q++) t += __shfl_sync(0xffffffffu, mine, q);
+        for (int r = 0; r < SMP_TOPK; r++) {
+            uint32_t bk = mk[0];
+            int      bi = mi[0];
+            smp_warp_best(bk, bi);
+            const unsigned who = __ballot_sync(0xffffffffu, mk[0] == bk && mi[0] == bi);
+            const float    bv = __shfl_sync(0xffffffffu, mv[0], __ffs((int) who) - 1);
             if (lane == 0 && !off) {
-                out[blockIdx.x].id[k]    = bi == SMP_NONE ? 0 : bi;
-                out[blockIdx.x].logit[k] = bv;
-                out[blockIdx.x].p[k]     = (float) ((double) expf(bv - max_l) / t);
+                out[blockIdx.x].id[r]    = bi == SMP_NONE ? 0 : bi;
+                out[blockIdx.x].logit[r] = bi == SMP_NONE ? -INFINITY : bv;
+                out[blockIdx.x].p[r]     = (float) ((double) expf((bi == SMP_NONE ? -INFINITY : bv) - max_l) / t);
             }
             if (mi[0] == bi && bi != SMP_NONE) {
 #pragma unroll
-                for (int j = 0; j < SMP_TOPK - 1; j++) { mv[j] = mv[j + 1]; mi[j] = mi[j + 1]; }
-                mv[SMP_TOPK - 1] = -INFINITY; mi[SMP_TOPK - 1] = SMP_NONE;
+                for (int j = 0; j < SMP_TOPK - 1; j++) { mk[j] = mk[j + 1]; mi[j] = mi[j + 1]; mv[j] = mv[j + 1]; }
+                mk[SMP_TOPK - 1] = 0u; mi[SMP_TOPK - 1] = SMP_NONE;
             }
         }
     }
@@ -180,9 +149,9 @@ __global__ void __launch_bounds__(SMP_THREADS) sample_topk_kernel(float * __rest
 int pib_sample_topk(float * logits_dev, int n_rows, int n_vocab, const int32_t * bias_ids_dev, const float * bias_val_dev,
                     int n_bias, void * out_dev, const uint8_t * desc, const int * cancel, cudaStream_t st) {
     (void) desc;
-    // as many parts as the register form needs (8192 elements each), more while the machine has room for the blocks and a thread would have more than four elements
+    // parts while the machine has room for the blocks and a thread has more than four elements
     int P = 1;
-    while (P < SMP_PARTS && (n_vocab > P * SMP_REG * SMP_THREADS || ((long long) n_rows * P * 2 <= 4LL * pib_num_sms() && n_vocab >= P * 8 * SMP_THREADS))) P <<= 1;
+    while (P < SMP_PARTS && (long long) n_rows * P * 2 <= 8LL * pib_num_sms() && n_vocab >= P * 8 * SMP_THREADS) P <<= 1;
     if (P > 1) pib_launch_cluster(sample_topk_kernel, dim3((unsigned) n_rows, (unsigned) P), dim3(SMP_THREADS), dim3(1, (unsigned) P, 1), 0, st, logits_dev, n_vocab, bias_ids_dev, bias_val_dev, n_bias,
                                   (pib_row_result *) out_dev, cancel);
     else       pib_launch(sample_topk_kernel, dim3((unsigned) n_rows), dim3(SMP_THREADS), 0, st, logits_dev, n_vocab, bias_ids_dev, bias_val_dev, n_bias, (pib_row_result *) out_dev, cancel);
