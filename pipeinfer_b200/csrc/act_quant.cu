@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(AQ_THREADS) act_quant_kernel(const float * x, 
                                                                const uint16_t * __restrict__ lut,
                                                                const float * __restrict__ addend, float * sum_out,
                                                                const int * __restrict__ cancel, int64_t xstride,
-                                                               const float * __restrict__ bias, const float * __restrict__ addend2) {
+                                                               const float * __restrict__ bias, const float * __restrict__ addend2, __half * __restrict__ xh) {
     const int     row  = blockIdx.x;
     const float * xr   = x + (size_t) row * xstride;
     const float * x2r  = x2 ? (x2_per_row ? x2 + (size_t) row * xstride : x2) : nullptr;
@@ -245,7 +245,9 @@ __global__ void __launch_bounds__(AQ_THREADS) act_quant_kernel(const float * x, 
                 vo[1] = make_float4(v[4], v[5], v[6], v[7]);
             }
             const size_t rs = (size_t) row * nsb + sb;
-            q8k_quantise_sb(v, lane, qs + (size_t) row * K + sb * PIB_QK_K, qsp + (size_t) row * K + sb * PIB_QK_K, (int16_t *) bsplane + rs * 16, bs8plane + rs * 16,
+            // a prompt pass: the fp16 rows of the tensor-core GEMM are all that its matmuls read
+            if (xh) q8k_quantise_sb(v, lane, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, xh + (size_t) row * K + sb * PIB_QK_K);
+            else q8k_quantise_sb(v, lane, qs + (size_t) row * K + sb * PIB_QK_K, qsp + (size_t) row * K + sb * PIB_QK_K, (int16_t *) bsplane + rs * 16, bs8plane + rs * 16,
                             sbs + rs * 8, qsl + rs * 64, dplane + rs, q6p + (size_t) row * K + sb * PIB_QK_K, b16 + rs * 32);
         }
     }
@@ -255,7 +257,7 @@ template <int PRO>
 static int launch_aq(int wtype, const float * x, const float * x2, int x2_per_row, float eps, int b, int64_t K, void * act,
                      float * vout, const uint16_t * lut, cudaStream_t st, const float * addend = nullptr,
                      float * sum_out = nullptr, const int * cancel = nullptr, int64_t xstride = 0, const float * bias = nullptr,
-                     const float * addend2 = nullptr) {
+                     const float * addend2 = nullptr, void * xhat = nullptr) {
     if (xstride == 0) xstride = K;
     const pib_act_layout L = pib_act_layout_of(wtype, K, b);
     int8_t * qs = (int8_t *) act + L.qs_off;
@@ -272,8 +274,8 @@ static int launch_aq(int wtype, const float * x, const float * x2, int x2_per_ro
     const int64_t units = wtype == PIB_TYPE_Q4_K ? K / PIB_QK_K : K / PIB_QK;
     const int     parts = (int) max((int64_t) 1, min((int64_t) 32, (units + AQ_THREADS / 32 - 1) / (AQ_THREADS / 32)));
     const dim3    grid(b, parts);
-    if (wtype == PIB_TYPE_Q4_K) pib_launch(act_quant_kernel<true, PRO>, grid, dim3(AQ_THREADS), 0, st, x, x2, x2_per_row, eps, K, qs, d, bs, b8, qp, ql, sb, q6, b6, vout, lut, addend, sum_out, cancel, xstride, bias, addend2);
-    else                        pib_launch(act_quant_kernel<false, PRO>, grid, dim3(AQ_THREADS), 0, st, x, x2, x2_per_row, eps, K, qs, d, bs, b8, qp, ql, sb, q6, b6, vout, lut, addend, sum_out, cancel, xstride, bias, addend2);
+    if (wtype == PIB_TYPE_Q4_K) pib_launch(act_quant_kernel<true, PRO>, grid, dim3(AQ_THREADS), 0, st, x, x2, x2_per_row, eps, K, qs, d, bs, b8, qp, ql, sb, q6, b6, vout, lut, addend, sum_out, cancel, xstride, bias, addend2, (__half *) xhat);
+    else                        pib_launch(act_quant_kernel<false, PRO>, grid, dim3(AQ_THREADS), 0, st, x, x2, x2_per_row, eps, K, qs, d, bs, b8, qp, ql, sb, q6, b6, vout, lut, addend, sum_out, cancel, xstride, bias, addend2, (__half *) xhat);
     PIB_CHECK(cudaGetLastError());
     return PIB_OK;
 }
@@ -302,26 +304,27 @@ extern "C" int pib_norm_quantize_act(int wtype, int norm_kind, const float * x_d
 }
 
 // ---- internal (engine) entry points ---------------------------------------------------------------------------------
+// xhat (Q8_K only): the rows go there as the tensor-core GEMM's fp16 operand instead of into the planes of act_dev
 // silu(gate) * up -> quantised activations for the down projection; gate_up: [b][2*K] rows = {gate[K], up[K]}
 int pib_silu_mul_quantize_act(int wtype, const float * gate_dev, const float * up_dev, int64_t row_stride, int b, int64_t K,
-                              void * act_dev, const int * cancel, cudaStream_t st) {
+                              void * act_dev, const int * cancel, cudaStream_t st, void * xhat) {
     if (check_args(wtype, b, K) != PIB_OK) return PIB_ERR_ARG;
     return launch_aq<PRO_SILU_MUL>(wtype, gate_dev, up_dev, 1, 0.f, b, K, act_dev, nullptr, pib_get_luts().silu_f16, st,
-                                   nullptr, nullptr, cancel, row_stride);
+                                   nullptr, nullptr, cancel, row_stride, nullptr, nullptr, xhat);
 }
 
-int pib_quantize_act_c(int wtype, const float * x_dev, int b, int64_t K, void * act_dev, const int * cancel, cudaStream_t st) {
+int pib_quantize_act_c(int wtype, const float * x_dev, int b, int64_t K, void * act_dev, const int * cancel, cudaStream_t st, void * xhat) {
     if (check_args(wtype, b, K) != PIB_OK) return PIB_ERR_ARG;
-    return launch_aq<PRO_PLAIN>(wtype, x_dev, nullptr, 0, 0.f, b, K, act_dev, nullptr, nullptr, st, nullptr, nullptr, cancel);
+    return launch_aq<PRO_PLAIN>(wtype, x_dev, nullptr, 0, 0.f, b, K, act_dev, nullptr, nullptr, st, nullptr, nullptr, cancel, 0, nullptr, nullptr, xhat);
 }
 
 // [sum_out = x + addend;] act = quantise(rmsnorm(sum or x) * w)
 int pib_add_rmsnorm_quantize_act(int wtype, const float * x_dev, const float * addend_dev, float * sum_out_dev,
                                  const float * norm_w_dev, float eps, int b, int64_t K, void * act_dev, const int * cancel,
-                                 cudaStream_t st) {
+                                 cudaStream_t st, void * xhat) {
     if (check_args(wtype, b, K) != PIB_OK) return PIB_ERR_ARG;
     return launch_aq<PRO_RMSNORM>(wtype, x_dev, norm_w_dev, 0, eps, b, K, act_dev, nullptr, nullptr, st, addend_dev, sum_out_dev,
-                                  cancel);
+                                  cancel, 0, nullptr, nullptr, xhat);
 }
 
 // falcon: [sum_out = (x + addend) + addend2;] act = quantise(layernorm(sum or x) * w + bias)

@@ -27,10 +27,10 @@ bool pib_gemv_pro_supported(const pib_weight * w, int b);
 int  pib_gemv_pro(const pib_weight * w, int pro, const float * x, const float * x2, const float * addend, float * sum_out, int64_t xstride, float eps,
                   int b, float * y, const int * cancel, cudaStream_t st);
 int  pib_silu_mul_quantize_act(int wtype, const float * gate_dev, const float * up_dev, int64_t row_stride, int b, int64_t K,
-                               void * act_dev, const int * cancel, cudaStream_t st);
-int  pib_quantize_act_c(int wtype, const float * x_dev, int b, int64_t K, void * act_dev, const int * cancel, cudaStream_t st);
+                               void * act_dev, const int * cancel, cudaStream_t st, void * xhat = nullptr);
+int  pib_quantize_act_c(int wtype, const float * x_dev, int b, int64_t K, void * act_dev, const int * cancel, cudaStream_t st, void * xhat = nullptr);
 int  pib_add_rmsnorm_quantize_act(int wtype, const float * x_dev, const float * addend_dev, float * sum_out_dev,
-                                  const float * norm_w_dev, float eps, int b, int64_t K, void * act_dev, const int * cancel, cudaStream_t st);
+                                  const float * norm_w_dev, float eps, int b, int64_t K, void * act_dev, const int * cancel, cudaStream_t st, void * xhat = nullptr);
 int  pib_add_layernorm_quantize_act(int wtype, const float * x_dev, const float * addend_dev, const float * addend2_dev,
                                     float * sum_out_dev, const float * norm_w_dev, const float * norm_b_dev, float eps, int b,
                                     int64_t K, void * act_dev, const int * cancel, cudaStream_t st);
@@ -522,7 +522,7 @@ void pib_context_free(pib_context * c) {
     pib_hybrid_ctx_free(c);
     pib_pipe_hop_free(c);
     for (void * b : { (void *) c->pb.x, (void *) c->pb.x2, (void *) c->pb.qkv, (void *) c->pb.att, (void *) c->pb.proj, (void *) c->pb.gu,
-                      (void *) c->pb.mask, c->pb.act, c->pb.xhat, (void *) c->pb.ids }) if (b) cudaFree(b);
+                      (void *) c->pb.mask, c->pb.xhat, (void *) c->pb.ids }) if (b) cudaFree(b);
     kv_device_free(&c->kvd);
     void * bufs[] = { c->vsep, c->kcache, c->vcache, c->x, c->x2, c->qkv, c->att, c->proj, c->gu, c->mask, c->act, c->rope,
                       c->cancel_table, c->desc_dev, c->ops_dev, c->bias_ids_dev, c->bias_val_dev, c->logits_fetch_dev };
@@ -851,7 +851,7 @@ static int prompt_bufs(pib_context * c) {
     if (cudaMalloc(&b.x, P * E * 4) != cudaSuccess || cudaMalloc(&b.x2, P * E * 4) != cudaSuccess || cudaMalloc(&b.qkv, P * (E + 2 * GQA) * 4) != cudaSuccess ||
         cudaMalloc(&b.att, P * E * 4) != cudaSuccess || cudaMalloc(&b.proj, P * E * 4) != cudaSuccess || cudaMalloc(&b.gu, P * 2 * FF * 4) != cudaSuccess ||
         cudaMalloc(&b.mask, P * c->n_ctx) != cudaSuccess || cudaMalloc(&b.ids, P * (3 + (size_t) c->n_words) * 4) != cudaSuccess ||
-        cudaMalloc(&b.act, pib_act_bytes(PIB_TYPE_Q4_K, (int64_t) KM, (int) P)) != cudaSuccess || cudaMalloc(&b.xhat, pib_gemm_xhat_bytes((int64_t) KM, (int) P)) != cudaSuccess) {
+        cudaMalloc(&b.xhat, pib_gemm_xhat_bytes((int64_t) KM, (int) P)) != cudaSuccess) {
         cudaGetLastError();
         pib_set_error("decode: out of memory for the prompt path's work buffers");
         return PIB_ERR_NOMEM;
@@ -887,26 +887,26 @@ static int run_prompt_pass(pib_context * c, pib_run & run, int ch0, int nch, int
     for (int il = m->layer_begin; il < m->layer_end; il++) {
         const pib_layer & L  = m->layers[il];
         const size_t      lo = (size_t) (il - m->layer_begin) * c->n_ctx * GQA;
-        if (pending_add) RC(pib_add_rmsnorm_quantize_act(wt, B.proj, B.x2, B.x, L.attn_norm, m->rms_eps, ntok, E, B.act, cancel, st));
-        else             RC(pib_add_rmsnorm_quantize_act(wt, B.x, nullptr, nullptr, L.attn_norm, m->rms_eps, ntok, E, B.act, cancel, st));
-        RC(pib_gemm_q4k_tc(L.wqkv, B.act, ntok, B.qkv, B.xhat, st));
-        // the GEMM's scratch is free between two matmuls: it holds the rotated queries
+        if (pending_add) RC(pib_add_rmsnorm_quantize_act(wt, B.proj, B.x2, B.x, L.attn_norm, m->rms_eps, ntok, E, nullptr, cancel, st, B.xhat));
+        else             RC(pib_add_rmsnorm_quantize_act(wt, B.x, nullptr, nullptr, L.attn_norm, m->rms_eps, ntok, E, nullptr, cancel, st, B.xhat));
+        RC(pib_gemm_q4k_tc(L.wqkv, nullptr, ntok, B.qkv, B.xhat, st));
+        // the GEMM's operand rows are free between a matmul and the next quantiser: they hold the rotated queries
         RC(pib_prompt_attention(B.qkv, pos, cell, c->rope, c->rope_n_pos, (__half *) B.xhat, c->kcache + lo, c->vcache + lo, B.mask, c->kvd.scalars, ntok, m->n_head, m->n_head_kv, hd,
                                 (int) c->n_ctx, B.att, cancel, st));
         c->n_kernels++;
-        RC(pib_quantize_act_c(wt, B.att, ntok, E, B.act, cancel, st));
-        RC(pib_gemm_q4k_tc(L.wo, B.act, ntok, B.proj, B.xhat, st));
-        RC(pib_add_rmsnorm_quantize_act(wt, B.proj, B.x, B.x2, L.ffn_norm, m->rms_eps, ntok, E, B.act, cancel, st));
-        RC(pib_gemm_q4k_tc(L.wgu, B.act, ntok, B.gu, B.xhat, st));
-        RC(pib_silu_mul_quantize_act(wt, B.gu, B.gu + FF, 2 * (int64_t) FF, ntok, FF, B.act, cancel, st));
-        RC(pib_gemm_q4k_tc(L.wdown, B.act, ntok, B.proj, B.xhat, st));
+        RC(pib_quantize_act_c(wt, B.att, ntok, E, nullptr, cancel, st, B.xhat));
+        RC(pib_gemm_q4k_tc(L.wo, nullptr, ntok, B.proj, B.xhat, st));
+        RC(pib_add_rmsnorm_quantize_act(wt, B.proj, B.x, B.x2, L.ffn_norm, m->rms_eps, ntok, E, nullptr, cancel, st, B.xhat));
+        RC(pib_gemm_q4k_tc(L.wgu, nullptr, ntok, B.gu, B.xhat, st));
+        RC(pib_silu_mul_quantize_act(wt, B.gu, B.gu + FF, 2 * (int64_t) FF, ntok, FF, nullptr, cancel, st, B.xhat));
+        RC(pib_gemm_q4k_tc(L.wdown, nullptr, ntok, B.proj, B.xhat, st));
         pending_add = true;
     }
     if (c->stage.last()) {
-        if (pending_add) RC(pib_add_rmsnorm_quantize_act(wt, B.proj, B.x2, B.x, m->output_norm, m->rms_eps, ntok, E, B.act, cancel, st));
-        else             RC(pib_add_rmsnorm_quantize_act(wt, B.x, nullptr, nullptr, m->output_norm, m->rms_eps, ntok, E, B.act, cancel, st));
+        if (pending_add) RC(pib_add_rmsnorm_quantize_act(wt, B.proj, B.x2, B.x, m->output_norm, m->rms_eps, ntok, E, nullptr, cancel, st, B.xhat));
+        else             RC(pib_add_rmsnorm_quantize_act(wt, B.x, nullptr, nullptr, m->output_norm, m->rms_eps, ntok, E, nullptr, cancel, st, B.xhat));
         float * lg = run.logits + (size_t) ch0 * PIB_CHUNK * m->n_vocab;
-        RC(pib_gemm_q4k_tc(m->output, B.act, ntok, lg, B.xhat, st));
+        RC(pib_gemm_q4k_tc(m->output, nullptr, ntok, lg, B.xhat, st));
         RC(pib_sample_topk(lg, ntok, m->n_vocab, c->bias_ids_dev, c->bias_val_dev, c->n_bias, run.res_dev + (size_t) ch0 * PIB_CHUNK, desc_of(0), cancel, st));
     } else {
         // the stage's output, chunk by chunk, to the next stage (its hop slots hold one 16-token chunk each)

@@ -130,7 +130,7 @@ struct pib_context {
 
     // wide-batch (prompt) path: work buffers for up to PIB_PROMPT_MAX tokens at once, allocated on the first prompt that uses them
     struct PromptBufs { float * x = nullptr, * x2 = nullptr, * qkv = nullptr, * att = nullptr, * proj = nullptr, * gu = nullptr;
-                        uint8_t * mask = nullptr; void * act = nullptr, * xhat = nullptr;
+                        uint8_t * mask = nullptr; void * xhat = nullptr;      // xhat: the matmuls' fp16 operand rows
                         int32_t * ids = nullptr;      // a pass's token ids | positions | cells [3][PIB_PROMPT_MAX], then sequence bitsets [PIB_PROMPT_MAX][n_words]
                         bool ready = false; } pb;
     int      fuse_pro = 0;                 // 1: small llama-arch Q4_K models run norm / quantise / silu inside the consuming GEMV (PIB_FUSE_PRO, engine.cu)

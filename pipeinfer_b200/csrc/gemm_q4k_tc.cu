@@ -22,6 +22,7 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include "q8k_quant.cuh"
 #include "tc_common.cuh"
 
 #define TG_BM      128                 // output rows per accumulator (UMMA M)
@@ -46,10 +47,6 @@ template <int NB, int G> struct tg_cfg {
     static constexpr size_t SMEM = (size_t) BAR_OFF + N_BAR * 8 + 32 + 1024;
     static_assert(NB + STAGES * 64 <= TM_COLS && G <= STAGES, "tensor memory");
 };
-
-// place of element e of a 64-wide chunk in both operands' rows: the record's low nibbles (e < 32) come first, a lane quarter's eight as two runs of four,
-// the middle two of each run swapped (one mask of a word of nibble bytes gives the pairs (e0, e2) and (e1, e3))
-__host__ __device__ __forceinline__ int tg_kpos(int e) { return (e & 32) + ((e >> 2) & 1) * 16 + ((e >> 3) & 3) * 4 + ((e & 1) << 1 | ((e >> 1) & 1)); }
 
 // ---- x^: quantised activations back to fp16, [b][K], k order inside a chunk as above -----------------------------------------------------------
 __global__ void __launch_bounds__(256) tg_xhat_kernel(const int8_t * __restrict__ qs, const float * __restrict__ d, int64_t n16, int K16, __half * __restrict__ xh) {
@@ -390,14 +387,15 @@ static int tg_launch(const pib_weight * w, const __half * xh, int b, int x0, int
     return PIB_OK;
 }
 
-// y[b][N] = W x^; act_dev = the Q8_K activation planes of `b` tokens (act_quant.cu), xhat_dev = scratch of pib_gemm_xhat_bytes
+// y[b][N] = W x^; act_dev = the Q8_K activation planes of `b` tokens (act_quant.cu), xhat_dev = scratch of pib_gemm_xhat_bytes; or act_dev = null and xhat_dev already
+// written by the quantiser (51 launches of 4 us in a 700-token prompt through four layers)
 int pib_gemm_q4k_tc(const pib_weight * w, const void * act_dev, int b, float * y_dev, void * xhat_dev, cudaStream_t st) {
     if (!w || w->type != PIB_TYPE_Q4_K || !w->tiles || b < 1 || b > 256) { pib_set_error("pib_gemm: needs Q4_K tiles and 1 <= b <= 256"); return PIB_ERR_ARG; }
     const pib_act_layout L = pib_act_layout_of(PIB_TYPE_Q4_K, w->K, b);
     const uint8_t * act = (const uint8_t *) act_dev;
     __half * xh = (__half *) xhat_dev;
     const int64_t n16 = (int64_t) b * (w->K / 16);
-    pib_launch(tg_xhat_kernel, dim3((unsigned) ((n16 + 255) / 256)), dim3(256), 0, st, (const int8_t *) (act + L.qs_off), (const float *) (act + L.d_off), n16, (int) (w->K / 16), xh);
+    if (act) pib_launch(tg_xhat_kernel, dim3((unsigned) ((n16 + 255) / 256)), dim3(256), 0, st, (const int8_t *) (act + L.qs_off), (const float *) (act + L.d_off), n16, (int) (w->K / 16), xh);
     PIB_CHECK(cudaGetLastError());
     const int NB = tg_nb_of(b), nsb = (int) (w->K / 256), nx = (int) ((w->N + TG_BM - 1) / TG_BM), sms = pib_num_sms();
     // K shares of n row blocks that fit `slots` CTAs at once; every share keeps at least two super-blocks
@@ -437,12 +435,13 @@ int pib_gemm_q4k_tc(const pib_weight * w, const void * act_dev, int b, float * y
 
 extern "C" size_t pib_gemm_scratch_bytes(int64_t K, int b) { return pib_gemm_xhat_bytes(K, b); }
 extern "C" int pib_gemm(const pib_weight * w, const void * act_dev, int b, float * y_dev, void * scratch_dev, pib_stream s) {
+    if (!act_dev || !y_dev || !scratch_dev) { pib_set_error("pib_gemm: bad arguments"); return PIB_ERR_ARG; }
     return pib_gemm_q4k_tc(w, act_dev, b, y_dev, scratch_dev, (cudaStream_t) s);
 }
 // activation quantiser for any number of rows (pib_quantize_act is limited to verification batches)
 extern "C" int pib_quantize_act_rows(int wtype, const float * x_dev, int b, int64_t K, void * act_dev, pib_stream s);
 
-int pib_quantize_act_c(int wtype, const float * x_dev, int b, int64_t K, void * act_dev, const int * cancel, cudaStream_t st);
+int pib_quantize_act_c(int wtype, const float * x_dev, int b, int64_t K, void * act_dev, const int * cancel, cudaStream_t st, void * xhat = nullptr);
 
 // host-buffer convenience for the parity tests (like pib_mul_mat_host): x_host [b][K] fp32 -> y_host [b][N]
 extern "C" int pib_gemm_host(const pib_weight * w, const float * x_host, int b, float * y_host) {

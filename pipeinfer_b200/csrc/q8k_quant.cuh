@@ -5,13 +5,18 @@
 #pragma once
 #include "pib_common.cuh"
 
+// place of element e of a 64-wide chunk in the fp16 rows that the tensor-core GEMM multiplies (gemm_q4k_tc.cu): the weight record's low nibbles (e < 32) come first,
+// a lane quarter's eight as two runs of four, the middle two of each run swapped (one mask of a word of nibble bytes gives the pairs (e0, e2) and (e1, e3))
+__host__ __device__ __forceinline__ int tg_kpos(int e) { return (e & 32) + ((e >> 2) & 1) * 16 + ((e >> 3) & 3) * 4 + ((e & 1) << 1 | ((e >> 1) & 1)); }
+
 // Every pointer addresses this super-block's part of its plane (see pib_act_layout) and may be null:
 //   qs   [256] int8   quants in element order           qsp [256] int8   the same in B-fragment order of mma.m16n8k32
 //   bs   [16]  int16  sums of 16                         bs8 [16]  int8   sub-block (32) sums split as 64 hi + lo: hi[8], lo[8]
 //   sbs  [8]   int16  sub-block sums                     qsl [64]  int2   B registers of the lane-exact kernel     d [1] float
+//   xh   [256] fp16   quants times d in the GEMM's order (tg_kpos)
 //   q6p  [256] int8   quants in the k16 B-fragment order of the Q6_K kernel      b16 [32] int8   sums of 16 split as 64 hi + lo: hi[16], lo[16]
 __device__ __forceinline__ void q8k_quantise_sb(const float (&v)[8], int lane, int8_t * qs, int8_t * qsp, int16_t * bs, int8_t * bs8,
-                                                int16_t * sbs, int2 * qsl, float * d, int8_t * q6p = nullptr, int8_t * b16 = nullptr) {
+                                                int16_t * sbs, int2 * qsl, float * d, int8_t * q6p = nullptr, int8_t * b16 = nullptr, __half * xh = nullptr) {
     // first element (in index order) with the largest |x|: strict '>' scan, ties keep the lower index
     float amax = 0.0f, mx = 0.0f;
     int   idx  = 1 << 30;
@@ -37,6 +42,16 @@ __device__ __forceinline__ void q8k_quantise_sb(const float (&v)[8], int lane, i
 #pragma unroll
         for (int j = 0; j < 8; j++) q[j] = min(127, __float2int_rn(__fmul_rn(iscale, v[j])));
         dval = 1.0f / iscale;
+    }
+    if (xh) {                                                              // this lane's eight elements are two runs of one 64-wide chunk
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            float w[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) w[j] = __fmul_rn((float) q[4 * u + j], dval);
+            const __half2 p[2] = { __floats2half2_rn(w[0], w[2]), __floats2half2_rn(w[1], w[3]) };
+            *reinterpret_cast<uint2 *>(xh + (lane >> 3) * 64 + tg_kpos((lane & 7) * 8 + 4 * u)) = *reinterpret_cast<const uint2 *>(p);
+        }
     }
     int2 packed;
     packed.x = (q[0] & 0xff) | ((q[1] & 0xff) << 8) | ((q[2] & 0xff) << 16) | ((q[3] & 0xff) << 24);
