@@ -38,15 +38,17 @@ __global__ void __launch_bounds__(256) embed_scale_kernel(const WT * __restrict_
     pib_pdl_wait();
     pib_pdl_trigger();
     const WT * r = embd + (size_t) tok[blockIdx.x] * W;
-    for (int i = threadIdx.x; i < W; i += blockDim.x) {
+    const int i = blockIdx.y * blockDim.x + threadIdx.x;          // a thread per channel: one block per token walked its row in a chain of loads (7.5 us of a decode step)
+    if (i < W) {
         const float v = (float) r[i] * scale;
         for (int s = 0; s < copies; s++) x[((size_t) blockIdx.x * copies + s) * W + i] = v;
     }
 }
 // copies: every token's row is written that many times, one after the other (the residual streams of hyper-connections start equal)
 int pib_embed_scale(const pib_weight * embd, const int32_t * tok, float scale, int T, int W, float * x, cudaStream_t st, int copies) {
-    if (embd->type == PIB_TYPE_BF16) pib_launch(embed_scale_kernel<__nv_bfloat16>, dim3(T), dim3(256), (size_t) 0, st, (const __nv_bfloat16 *) embd->base, tok, scale, W, x, copies);
-    else                             pib_launch(embed_scale_kernel<float>, dim3(T), dim3(256), (size_t) 0, st, (const float *) embd->base, tok, scale, W, x, copies);
+    const dim3 grid((unsigned) T, (unsigned) ((W + 255) / 256));
+    if (embd->type == PIB_TYPE_BF16) pib_launch(embed_scale_kernel<__nv_bfloat16>, grid, dim3(256), (size_t) 0, st, (const __nv_bfloat16 *) embd->base, tok, scale, W, x, copies);
+    else                             pib_launch(embed_scale_kernel<float>, grid, dim3(256), (size_t) 0, st, (const float *) embd->base, tok, scale, W, x, copies);
     CKL();
     return PIB_OK;
 }
