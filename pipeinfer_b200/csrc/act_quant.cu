@@ -54,7 +54,8 @@ __device__ __forceinline__ void aq_value8(const float * xr, const float * __rest
     }
 }
 
-template <bool Q8K, int PRO>
+// XH: a prompt pass, the rows go to xh as the tensor-core GEMM's fp16 operand and nowhere else
+template <bool Q8K, int PRO, bool XH>
 __global__ void __launch_bounds__(AQ_THREADS) act_quant_kernel(const float * x, const float * __restrict__ x2,
                                                                int x2_per_row, float eps, int64_t K,
                                                                int8_t * __restrict__ qs, float * __restrict__ dplane,
@@ -245,8 +246,7 @@ __global__ void __launch_bounds__(AQ_THREADS) act_quant_kernel(const float * x, 
                 vo[1] = make_float4(v[4], v[5], v[6], v[7]);
             }
             const size_t rs = (size_t) row * nsb + sb;
-            // a prompt pass: the fp16 rows of the tensor-core GEMM are all that its matmuls read
-            if (xh) q8k_quantise_sb(v, lane, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, xh + (size_t) row * K + sb * PIB_QK_K);
+            if (XH) q8k_quantise_sb(v, lane, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, xh + (size_t) row * K + sb * PIB_QK_K);
             else q8k_quantise_sb(v, lane, qs + (size_t) row * K + sb * PIB_QK_K, qsp + (size_t) row * K + sb * PIB_QK_K, (int16_t *) bsplane + rs * 16, bs8plane + rs * 16,
                             sbs + rs * 8, qsl + rs * 64, dplane + rs, q6p + (size_t) row * K + sb * PIB_QK_K, b16 + rs * 32);
         }
@@ -274,8 +274,13 @@ static int launch_aq(int wtype, const float * x, const float * x2, int x2_per_ro
     const int64_t units = wtype == PIB_TYPE_Q4_K ? K / PIB_QK_K : K / PIB_QK;
     const int     parts = (int) max((int64_t) 1, min((int64_t) 32, (units + AQ_THREADS / 32 - 1) / (AQ_THREADS / 32)));
     const dim3    grid(b, parts);
-    if (wtype == PIB_TYPE_Q4_K) pib_launch(act_quant_kernel<true, PRO>, grid, dim3(AQ_THREADS), 0, st, x, x2, x2_per_row, eps, K, qs, d, bs, b8, qp, ql, sb, q6, b6, vout, lut, addend, sum_out, cancel, xstride, bias, addend2, (__half *) xhat);
-    else                        pib_launch(act_quant_kernel<false, PRO>, grid, dim3(AQ_THREADS), 0, st, x, x2, x2_per_row, eps, K, qs, d, bs, b8, qp, ql, sb, q6, b6, vout, lut, addend, sum_out, cancel, xstride, bias, addend2, (__half *) xhat);
+#define AQ_GO(Q8K, XH) pib_launch(act_quant_kernel<Q8K, PRO, XH>, grid, dim3(AQ_THREADS), 0, st, x, x2, x2_per_row, eps, K, qs, d, bs, b8, qp, ql, sb, q6, b6, vout, lut, addend, sum_out, cancel, \
+                               xstride, bias, addend2, (__half *) xhat)
+    constexpr bool PROMPT = PRO == PRO_PLAIN || PRO == PRO_RMSNORM || PRO == PRO_SILU_MUL;
+    if (wtype != PIB_TYPE_Q4_K) AQ_GO(false, false);
+    else if (PROMPT && xhat)    AQ_GO(true, PROMPT);
+    else                        AQ_GO(true, false);
+#undef AQ_GO
     PIB_CHECK(cudaGetLastError());
     return PIB_OK;
 }
