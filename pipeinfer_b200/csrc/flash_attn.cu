@@ -254,7 +254,7 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap qh, const __grid_constant_
                 *reinterpret_cast<uint4 *>(prow + C::P_TILE + off) = make_uint4(lo4[0], lo4[1], lo4[2], lo4[3]);
             }
             l += l2;
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            dt_fence_async();
             dt_fence_before();
             dt_arrive(bar_p + 8 * w);
         }

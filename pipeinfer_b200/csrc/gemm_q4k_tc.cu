@@ -265,8 +265,10 @@ gemm_q4k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int x0, c
                 tg_chunk_row<1, 0>(v[2 * h + 1].x, v[2 * h + 1].y, scl[h * 32 + 16 + g], o);
                 tg_chunk_row<1, 2>(v[2 * h + 1].z, v[2 * h + 1].w, scl[h * 32 + 16 + g + 8], o);
                 if (h == NH - 1) {
-                    // The ring place is given back when every word of the record has been USED.  An arrival right behind the loads overtakes them: the next
-                    // bulk copy then overwrote words that had been asked for but not yet read (quads of rows wrong, only when calls follow one another closely).
+                    // The ring place is given back to a bulk copy, a write of the async proxy, which nothing orders behind this lane's generic reads of the record but a
+                    // proxy fence: every lane's reads, its fence, the warp's meeting, one arrival.  (Without the fence and with the arrival right behind the loads
+                    // quads of rows came out wrong where calls follow one another closely, 69 of 200 calls.)
+                    dt_fence_async();
                     __syncwarp();
                     if (lane == 0) dt_arrive(bar_we + ws * 8);
                     if (++ws == C::WSTAGES) { ws = 0; wph ^= 1; }

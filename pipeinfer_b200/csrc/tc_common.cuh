@@ -48,6 +48,8 @@ __device__ __forceinline__ void dt_commit(uint32_t bar) {
     asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void dt_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+// orders this thread's accesses to shared memory before and after it across proxies: loads and stores on one side, TMA, bulk copies and MMA operands on the other
+__device__ __forceinline__ void dt_fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 // 32 columns of this warp's 32 tensor-memory lanes, to and from registers (a lane's row each); the caller waits
 __device__ __forceinline__ void dt_ld32(uint32_t taddr, uint32_t * v) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
