@@ -126,6 +126,9 @@ int pib_gemm_host(const pib_weight * w, const float * x_host, int b, float * y_h
  * (the fp16 copy of the activations the TMA loads from). */
 size_t pib_gemm_scratch_bytes(int64_t K, int b);
 int    pib_gemm(const pib_weight * w, const void * act_dev, int b, float * y_dev, void * scratch_dev, pib_stream s);
+/* pib_gemm returns when the launch is made.  Every wait inside the kernel is bounded; one that runs out leaves y_dev unwritten in places and the stream's error
+ * word set.  This call waits for the stream and returns 0, or PIB_ERR_CUDA when that has happened to any pib_gemm on it since the last check. */
+int    pib_gemm_check(pib_stream s);
 int    pib_quantize_act_rows(int wtype, const float * x_dev, int b, int64_t K, void * act_dev, pib_stream s);
 
 /* ---- K3: embedding rows ---------------------------------------------------------------------------------------- */

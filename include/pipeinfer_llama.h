@@ -283,6 +283,7 @@ int  llama_pib_profile_read(struct llama_context * ctx, int32_t * kind, int32_t 
 int  llama_pib_matrix_shape(const struct llama_model * model, int layer, int kind, int64_t * N, int64_t * K, uint64_t * bytes);
 /* debugging aids for parity work: a work buffer of the last chunk; the handle of a resident weight matrix */
 int  llama_pib_debug_read(struct llama_context * ctx, int which, float * out, int n_floats);
+int  llama_pib_debug_tc_error(struct llama_context * ctx, int word);
 const struct pib_weight * llama_pib_debug_weight(const struct llama_model * model, int layer, int which);
 
 #ifdef __cplusplus

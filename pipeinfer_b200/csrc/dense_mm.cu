@@ -589,9 +589,8 @@ extern "C" int pib_dense_mm_host(int wtype, const void * W, int64_t w_elems, int
         a.W = dW; a.wtype = wtype; a.ldw = ldw; a.wz = wz; a.X = dX; a.ldx = ldx; a.xz = xz; a.xrows = xrows ? dR : nullptr; a.xdiv = xdiv;
         a.Y = dY; a.ldy = ldy; a.yz = yz; a.M = M; a.N = N; a.K = K; a.Z = Z; a.zrange = zrange ? dZ : nullptr; a.epi = epi; a.exact = exact; a.e0 = e0; a.e1 = e1;
         rc = pib_dense_mm(a, nullptr);
-        if (rc == PIB_OK && wtype == PIB_TYPE_BF16 && !exact) { pib_dense_mm_check(nullptr, 1); }
         if (rc == PIB_OK && cudaDeviceSynchronize() != cudaSuccess) { pib_set_error("dense matmul: %s", cudaGetErrorString(cudaGetLastError())); rc = PIB_ERR_CUDA; }
-        if (rc == PIB_OK && wtype == PIB_TYPE_BF16 && !exact) rc = pib_dense_mm_check(nullptr, 0);
+        if (rc == PIB_OK && wtype == PIB_TYPE_BF16 && !exact) rc = pib_tc_check(nullptr);
         if (rc == PIB_OK) cudaMemcpy(Y, dY, (size_t) y_elems * 4, cudaMemcpyDeviceToHost);
     } else pib_set_error("dense matmul: out of memory for the test buffers");
     for (void * p : { dW, (void *) dX, (void *) dY, (void *) dR, (void *) dZ }) if (p) cudaFree(p);

@@ -270,12 +270,24 @@ int pib_dense_mm_tc(const pib_mm & a, cudaStream_t st) {
     }
 }
 
-// the error word of this stream's tensor-core matmuls.  enqueue = 1: copy it to pinned memory in stream order (no wait);
-// enqueue = 0: read that copy (the caller has waited for the stream, or for an event behind the copy); 0 = no kernel gave up on a wait
-int pib_dense_mm_check(cudaStream_t st, int enqueue) {
+// what a kernel leaves in its stream's error word when a bounded wait runs out (0: nothing happened)
+int pib_tc_error(int word) {
+    if (word) pib_set_error("a tensor-core kernel gave up on a barrier wait (block %d)", word - 1);
+    return word ? PIB_ERR_CUDA : PIB_OK;
+}
+int pib_tc_error_copy(cudaStream_t st, int * host) {
     dt_scratch * sc = dt_scratch_of(st, 0);
-    if (!sc) return PIB_OK;
-    if (enqueue) return cudaMemcpyAsync(sc->err_host, sc->err, 4, cudaMemcpyDeviceToHost, st) == cudaSuccess ? PIB_OK : PIB_ERR_CUDA;
-    if (*sc->err_host) { pib_set_error("dense matmul: a tensor-core kernel gave up on a barrier wait (CTA %d)", *sc->err_host - 1); return PIB_ERR_CUDA; }
-    return PIB_OK;
+    return sc && cudaMemcpyAsync(host, sc->err, 4, cudaMemcpyDeviceToHost, st) == cudaSuccess ? PIB_OK : PIB_ERR_CUDA;
+}
+int pib_tc_error_clear(cudaStream_t st) {
+    dt_scratch * sc = dt_scratch_of(st, 0);
+    return sc && cudaMemsetAsync(sc->err, 0, 4, st) == cudaSuccess ? PIB_OK : PIB_ERR_CUDA;
+}
+int pib_tc_check(cudaStream_t st) {
+    dt_scratch * sc = dt_scratch_of(st, 0);
+    if (!sc || pib_tc_error_copy(st, sc->err_host) != PIB_OK || pib_tc_error_clear(st) != PIB_OK || cudaStreamSynchronize(st) != cudaSuccess) {
+        pib_set_error("tensor-core kernels: %s", cudaGetErrorString(cudaGetLastError()));
+        return PIB_ERR_CUDA;
+    }
+    return pib_tc_error(*sc->err_host);
 }

@@ -538,6 +538,7 @@ void pib_context_free(pib_context * c) {
         if (r.res_host) cudaFreeHost(r.res_host);
         if (r.acc_dev) cudaFree(r.acc_dev);
         if (r.acc_host) cudaFreeHost(r.acc_host);
+        if (r.tc_err) cudaFreeHost(r.tc_err);
     }
     for (auto e : c->desc_ev) if (e) cudaEventDestroy(e);
     if (c->cancel_ev) cudaEventDestroy(c->cancel_ev);
@@ -871,6 +872,15 @@ static int run_prompt_pass(pib_context * c, pib_run & run, int ch0, int nch, int
 #define RC(e) do { rc = (e); if (rc != PIB_OK) return rc; c->n_kernels++; } while (0)
     auto desc_of = [&](int k) { return c->desc_dev + (size_t) dev_slot(c, slots[ch0 + k]) * c->desc_stride; };
     auto nt_of   = [&](int k) { return std::min(PIB_CHUNK, ntok - k * PIB_CHUNK); };
+    // The stream's error word as it is behind this pass's kernels and in front of whatever takes their output to another stage.  It is cleared when the run's last pass
+    // is enqueued: a later copy includes the earlier passes.
+    auto error_word = [&]() -> int {
+        run.tc_used = true;
+        if (pib_tc_error_copy(st, run.tc_err) != PIB_OK) return PIB_ERR_CUDA;
+        if (c->stage.size > 1 && !c->stage.first())
+            PIB_CHECK(cudaLaunchHostFunc(st, [](void * p) { const pib_run * r = (const pib_run *) p; if (*r->tc_err) pib_pipe_post_failure(r->batch_id); }, &run));
+        return PIB_OK;
+    };
     int32_t *  ids = B.ids, * pos = ids + PIB_PROMPT_MAX, * cell = pos + PIB_PROMPT_MAX;
     uint32_t * bits = reinterpret_cast<uint32_t *>(cell + PIB_PROMPT_MAX);
     pib_prompt_slots sl;
@@ -908,7 +918,9 @@ static int run_prompt_pass(pib_context * c, pib_run & run, int ch0, int nch, int
         float * lg = run.logits + (size_t) ch0 * PIB_CHUNK * m->n_vocab;
         RC(pib_gemm_q4k_tc(m->output, nullptr, ntok, lg, B.xhat, st));
         RC(pib_sample_topk(lg, ntok, m->n_vocab, c->bias_ids_dev, c->bias_val_dev, c->n_bias, run.res_dev + (size_t) ch0 * PIB_CHUNK, desc_of(0), cancel, st));
+        if ((rc = error_word()) != PIB_OK) return rc;
     } else {
+        if ((rc = error_word()) != PIB_OK) return rc;
         // the stage's output, chunk by chunk, to the next stage (its hop slots hold one 16-token chunk each)
         for (int k = 0; k < nch; k++) {
             const size_t off = (size_t) k * PIB_CHUNK * E;
@@ -934,7 +946,8 @@ pib_run * pib_take_run(pib_context * c, int n_tokens) {
     for (auto & r : c->runs) {
         if (r.in_use || r.id == c->last_finished) continue;
         if (!r.done) cudaEventCreateWithFlags(&r.done, cudaEventDisableTiming);
-        if (!r.acc_dev && (cudaMalloc(&r.acc_dev, sizeof(pib_accept_result)) != cudaSuccess || cudaMallocHost(&r.acc_host, sizeof(pib_accept_result)) != cudaSuccess)) {
+        if ((!r.acc_dev && (cudaMalloc(&r.acc_dev, sizeof(pib_accept_result)) != cudaSuccess || cudaMallocHost(&r.acc_host, sizeof(pib_accept_result)) != cudaSuccess)) ||
+            (!r.tc_err && cudaMallocHost(&r.tc_err, sizeof(int)) != cudaSuccess)) {
             pib_set_error("decode: out of memory for a run slot");
             cudaGetLastError();
             return nullptr;
@@ -1071,7 +1084,7 @@ static int enqueue_decode(pib_context * c, pib_run * run, int n_tokens, int batc
     int64_t t_mark = slow_trace() ? now_us() : 0;
     if (pib_apply_devops(c) != PIB_OK) return -1;
     SLOW_MARK("  apply ops");
-    run->in_use = true; run->batch_id = batch_id; run->n_tokens = n_tokens; run->failed = false;
+    run->in_use = true; run->batch_id = batch_id; run->n_tokens = n_tokens; run->failed = false; run->tc_used = false;
     cudaMemcpyAsync(c->cancel_table, c->run_id_host + run->id, sizeof(int), cudaMemcpyHostToDevice, c->stream);   // "this run executes now"
     if (prompt_gemm_ok(c, n_tokens) && prompt_bufs(c) == PIB_OK) {
         const int per = PIB_PROMPT_MAX / PIB_CHUNK;
@@ -1080,7 +1093,7 @@ static int enqueue_decode(pib_context * c, pib_run * run, int n_tokens, int batc
             if (run_prompt_pass(c, *run, ch0, nch, ntok, slots) != PIB_OK) run->failed = true;
         }
         for (int ch = 0; ch < n_chunks; ch++) if (c->desc_ev[slots[ch]]) cudaEventRecord(c->desc_ev[slots[ch]], c->stream);
-        pib_dense_mm_check(c->stream, 1);
+        if (pib_tc_error_clear(c->stream) != PIB_OK) run->failed = true;
     } else
     for (int ch = 0; ch < n_chunks; ch++) {
         const int nt = std::min(PIB_CHUNK, n_tokens - ch * PIB_CHUNK);
@@ -1180,7 +1193,8 @@ int pib_run_finish(pib_context * c, int run) {
     clear_cancel_flag(c, r.id);
     if (c->stage.size > 1 && c->stage.first()) pib_pipe_ship_ints(2, 0, &r.batch_id, 1);
     for (auto it = c->inflight.begin(); it != c->inflight.end(); ++it) if (*it == run) { c->inflight.erase(it); break; }
-    if (((c->hy && c->model->wtype == PIB_TYPE_BF16) || c->pb.ready) && pib_dense_mm_check(c->stream, 0) != PIB_OK) r.failed = true;   // a tensor-core kernel gave up on a wait
+    if (r.tc_used && pib_tc_error(*r.tc_err) != PIB_OK) r.failed = true;
+    if (c->stage.size > 1 && c->stage.first() && pib_pipe_take_failure(r.batch_id)) { pib_set_error("finish: a kernel of another stage gave up on a barrier wait (batch %d)", r.batch_id); r.failed = true; }
     r.in_use         = false;
     c->last_finished = run;     // its buffers stay reserved until the next finish (llama_get_logits_ith contract)
     c->logits_row_valid.assign((size_t) r.n_tokens, 0);

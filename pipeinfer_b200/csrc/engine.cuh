@@ -90,6 +90,8 @@ struct pib_run {                   // one (possibly still executing) decode: the
     bool         has_walk  = false;       // the batch came with an acceptance table: only the walk's result crosses to the host
     bool         rows_on_host = false;
     pib_accept_result * acc_dev = nullptr, * acc_host = nullptr;
+    int *        tc_err    = nullptr;     // pinned: the stream's error word behind this run's kernels (pib_tc_error_copy)
+    bool         tc_used   = false;       // the run launched kernels that set it
 };
 
 struct pib_stage {                 // pipeline position of this process (1-GPU: first && last)
@@ -211,6 +213,9 @@ int  pib_kv_sync_replicas(pib_context * c);
 bool pib_pipe_ring_active();
 bool pib_pipe_nccl_active();
 void pib_pipe_install_hooks();
+// a stage whose kernels gave up on a wait says so for its batch before its output leaves; the head asks when the batch's results are there
+extern "C" void pib_pipe_post_failure(int32_t batch_id);
+extern "C" int  pib_pipe_take_failure(int32_t batch_id);     // 1: some stage posted it (and forgets it)
 int  pib_pipe_ship_decode(int batch_id, int n_tokens, int n_chunks, const uint8_t * const * descs, size_t desc_stride,
                           const int * slots, const KvOp * ops, int n_ops);
 int  pib_pipe_ship_ints(int kind, int tag, const int32_t * vals, int n);      // kind: 2 finish, 3 cancel, 5 return, 6 shutdown

@@ -341,7 +341,7 @@ gemm_q4k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int x0, c
     __syncthreads();
     if (*abort_s) {
         // a wait ran out: say so, give copies and MMAs still in flight time to land (bounded), then free the tensor memory
-        if (threadIdx.x == 0 && err) atomicExch(err, 1 + (int) blockIdx.x);
+        if (threadIdx.x == 0) atomicExch(err, 1 + (int) blockIdx.x);
         for (int i = 0; i < 2000; i++) __nanosleep(1000);
         __syncthreads();
     }
@@ -383,6 +383,7 @@ static int tg_launch(const pib_weight * w, const __half * xh, int b, int x0, int
     if (!configured) { PIB_CHECK(cudaFuncSetAttribute(gemm_q4k_tc_kernel<NB, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) C::SMEM)); configured = true; }
     const dim3 grid((unsigned) nx, 1, (unsigned) S);
     int * err = pib_tc_error_word(st);
+    if (!err) { pib_set_error("pib_gemm: no memory for the stream's error word"); return PIB_ERR_NOMEM; }
     if (S > 1) pib_launch_cluster(gemm_q4k_tc_kernel<NB, G>, grid, dim3(C::THREADS), dim3(1, 1, (unsigned) S), C::SMEM, st, w->tiles, (int) (w->K / 256), (int) w->N, x0, map, b, y, err);
     else       pib_launch(gemm_q4k_tc_kernel<NB, G>, grid, dim3(C::THREADS), C::SMEM, st, w->tiles, (int) (w->K / 256), (int) w->N, x0, map, b, y, err);
     PIB_CHECK(cudaGetLastError());
@@ -440,6 +441,7 @@ extern "C" int pib_gemm(const pib_weight * w, const void * act_dev, int b, float
     if (!act_dev || !y_dev || !scratch_dev) { pib_set_error("pib_gemm: bad arguments"); return PIB_ERR_ARG; }
     return pib_gemm_q4k_tc(w, act_dev, b, y_dev, scratch_dev, (cudaStream_t) s);
 }
+extern "C" int pib_gemm_check(pib_stream s) { return pib_tc_check((cudaStream_t) s); }
 // activation quantiser for any number of rows (pib_quantize_act is limited to verification batches)
 extern "C" int pib_quantize_act_rows(int wtype, const float * x_dev, int b, int64_t K, void * act_dev, pib_stream s);
 
@@ -462,9 +464,7 @@ extern "C" int pib_gemm_host(const pib_weight * w, const float * x_host, int b, 
     // through the engine-internal entry point (any b)
     if (rc == PIB_OK) rc = pib_quantize_act_c(PIB_TYPE_Q4_K, x, b, w->K, act, nullptr, nullptr);
     if (rc == PIB_OK && (rc = pib_gemm_q4k_tc(w, act, b, y, xh, nullptr)) != PIB_OK) { cudaFree(buf); return rc; }
-    if (rc == PIB_OK) rc = pib_dense_mm_check(nullptr, 1);
-    if (rc == PIB_OK && cudaDeviceSynchronize() != cudaSuccess) rc = PIB_ERR_CUDA;
-    if (rc == PIB_OK && pib_dense_mm_check(nullptr, 0) != PIB_OK) { cudaFree(buf); return PIB_ERR_CUDA; }
+    if (rc == PIB_OK && (rc = pib_tc_check(nullptr)) != PIB_OK) { cudaFree(buf); return rc; }
     if (rc == PIB_OK && cudaMemcpy(y_host, y, yb, cudaMemcpyDeviceToHost) != cudaSuccess) rc = PIB_ERR_CUDA;
     if (rc == PIB_ERR_CUDA) pib_set_error("pib_gemm_host: %s", cudaGetErrorString(cudaGetLastError()));
     cudaFree(buf);

@@ -602,6 +602,13 @@ extern "C" int llama_pib_debug_read(struct llama_context * ctx, int which, float
 }
 
 // debugging aid: handle of a resident weight matrix (layer < 0: 0 = token_embd, 1 = output; else 0 qkv, 1 o, 2 gate|up, 3 down)
+// the error word of the context's stream, as a tensor-core kernel whose wait ran out would leave it (tests)
+extern "C" int llama_pib_debug_tc_error(struct llama_context * ctx, int word) {
+    int * err = pib_tc_error_word(ctx->c->stream);
+    PIB_CHECK(cudaStreamSynchronize(ctx->c->stream));
+    if (!err || cudaMemcpy(err, &word, 4, cudaMemcpyHostToDevice) != cudaSuccess) return PIB_ERR_CUDA;
+    return PIB_OK;
+}
 extern "C" const pib_weight * llama_pib_debug_weight(const struct llama_model * model, int layer, int which) {
     const pib_model * m = model->m;
     if (layer < 0) return which == 0 ? m->tok_embd : m->output;

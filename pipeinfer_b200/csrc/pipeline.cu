@@ -40,6 +40,8 @@
 // control ring
 #define PIPE_MAX_RANKS 16
 #define PIPE_MAGIC     0x31424950u
+#define PIPE_FAILED    32
+#define PIPE_NO_BATCH  INT32_MIN
 enum { REC_PAD = 0, REC_DECODE = 1, REC_FINISH = 2, REC_CANCEL = 3, REC_BIAS = 4, REC_RETURN = 5, REC_SHUTDOWN = 6, REC_INTS = 7, REC_LOGITS = 8 };
 
 struct alignas(64) ring_word { std::atomic<uint64_t> v; char pad[56]; };
@@ -58,6 +60,8 @@ struct ring_hdr {
     cudaIpcMemHandle_t    hop_ipc[PIPE_MAX_RANKS];
     std::atomic<uint32_t> hop_gen[PIPE_MAX_RANKS];
     uint32_t              hop_embd[PIPE_MAX_RANKS];
+    // batches that some stage failed (pib_pipe_post_failure); free places hold PIPE_NO_BATCH
+    std::atomic<int32_t>  failed[PIPE_FAILED];
 };
 struct rec_hdr { uint32_t bytes, kind; };
 struct rec_decode { int32_t batch_id, n_tokens, n_chunks, n_ops; uint32_t desc_stride, pad; };
@@ -131,6 +135,7 @@ extern "C" int pib_pipe_ring_open(const char * name, int rank, int n_ranks, size
         P.h->head.v.store(0); P.h->bar_count.v.store(0); P.h->bar_gen.v.store(0); P.h->ids_ready.store(0);
         P.h->created_us = (uint64_t) (now_s() * 1e6);
         for (int i = 0; i < PIPE_MAX_RANKS; i++) { P.h->tail[i].v.store(0); P.h->hop_gen[i].store(0); }
+        for (auto & f : P.h->failed) f.store(PIPE_NO_BATCH);
         P.h->magic.store(PIPE_MAGIC, std::memory_order_release);
     } else {
         spinner sp;
@@ -229,6 +234,22 @@ static const rec_hdr * rec_peek(bool nowait) {
 static void rec_pop(const rec_hdr * h) {
     const uint64_t t = P.h->tail[P.rank].v.load(std::memory_order_relaxed);
     P.h->tail[P.rank].v.store(t + h->bytes, std::memory_order_release);
+}
+
+// ---- failures, the one message that goes from a stage's host to the head's: the place is written before the stage's output leaves, so the head sees it no later than
+// the batch's results
+extern "C" void pib_pipe_post_failure(int32_t batch_id) {
+    if (!P.h) return;
+    for (auto & f : P.h->failed) {
+        int32_t none = PIPE_NO_BATCH;
+        if (f.compare_exchange_strong(none, batch_id) || none == batch_id) return;
+    }
+    P.h->failed[0].store(batch_id);          // more failed batches than any head has in flight: the oldest were never asked for
+}
+extern "C" int pib_pipe_take_failure(int32_t batch_id) {
+    int found = 0;
+    if (P.h) for (auto & f : P.h->failed) { int32_t id = batch_id; if (f.compare_exchange_strong(id, PIPE_NO_BATCH)) found = 1; }
+    return found;
 }
 
 // ---- records written by the head (called from engine.cu) -------------------------------------------------------------

@@ -75,6 +75,5 @@ __device__ __forceinline__ void dt_fence_after() { asm volatile("tcgen05.fence::
 // instruction descriptor: fp32 accumulators, bfloat16 x bfloat16, both operands K-major, M x N outputs
 __host__ __device__ constexpr uint32_t dt_idesc(int M, int N) { return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t) (N >> 3) << 17) | ((uint32_t) (M >> 4) << 24); }
 
-// dense_mma.cu: a 3-D bfloat16 tensor map {d0, d1, d2} with boxes of 64 x box1 x 1 and 128-byte swizzle (strides in bytes); the stream's error word
+// dense_mma.cu: a 3-D bfloat16 tensor map {d0, d1, d2} with boxes of 64 x box1 x 1 and 128-byte swizzle (strides in bytes)
 int   pib_tma_map3(CUtensorMap * map, const void * base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s1_bytes, uint64_t s2_bytes, uint32_t box1);
-int * pib_tc_error_word(cudaStream_t st);

@@ -146,6 +146,22 @@ def main():
     assert all(torch.equal(a, alls[0]) for a in alls), "random trace: replicas differ"
     assert int(alls[0][1]) > 0
 
+    # ---- a stage's failure reaches the head for its batch, once; more failures than there are places do no harm --------------
+    if rank > 0:
+        for bid in (5, 9, 5, -3):
+            L.pib_pipe_post_failure(bid)
+    dist.barrier()
+    if rank == 0:
+        assert [L.pib_pipe_take_failure(b) for b in (4, 5, 5, -3, 9, 9, 0)] == [0, 1, 0, 1, 1, 0, 0]
+    dist.barrier()
+    for bid in range(100, 200):
+        L.pib_pipe_post_failure(bid)
+    dist.barrier()
+    if rank == 0:
+        assert sum(L.pib_pipe_take_failure(b) for b in range(100, 200)) == 32
+        assert not any(L.pib_pipe_take_failure(b) for b in range(100, 200))
+    dist.barrier()
+
     L.pib_pipe_ring_close()
     dist.barrier()
     dist.destroy_process_group()
