@@ -22,9 +22,9 @@
 #define SMP_PARTS   8
 #define SMP_NONE    0x7fffffff
 
-// order-preserving keys: larger value, larger key; what is no number comes last, but in front of places without an element (0)
+// order-preserving keys: larger value, larger key, the two zeros one key (the sum is +0 for both); what is no number comes last, but in front of places without an element (0)
 __device__ __forceinline__ uint32_t smp_key(float v) {
-    const uint32_t u = __float_as_uint(v);
+    const uint32_t u = __float_as_uint(v + 0.0f);
     return v != v ? 1u : (u & 0x80000000u) ? ~u : u | 0x80000000u;
 }
 // the warp's best (key, index): the largest key, the smallest index among equals
