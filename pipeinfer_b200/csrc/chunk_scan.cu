@@ -252,7 +252,7 @@ int pib_chunk_scan_run(const pib_chunk_scan & a, void * buf, cudaStream_t st) {
     CKL();
     auto mm = [&](const bf16 * X, int M, const bf16 * Wt, int N, int K, float * Y) {
         pib_mm m;
-        m.W = Wt; m.wtype = PIB_TYPE_BF16; m.ldw = K; m.wz = (int64_t) N * K; m.X = (const float *) X; m.ldx = K; m.xz = (int64_t) M * K; m.x_bf16 = 1;
+        m.W = Wt; m.w_made = 1; m.wtype = PIB_TYPE_BF16; m.ldw = K; m.wz = (int64_t) N * K; m.X = (const float *) X; m.ldx = K; m.xz = (int64_t) M * K; m.x_bf16 = 1;
         m.Y = Y; m.ldy = N; m.yz = (int64_t) M * N; m.M = M; m.N = N; m.K = K; m.Z = Z;
         return pib_dense_mm(m, st);
     };

@@ -36,6 +36,7 @@ struct mm_dev {
     float e0, e1;
     const int32_t * zlist;
     float * Y2; int64_t ld2; int n2; const int32_t * rows2;      // outputs n >= n2: Y2[rows2[m] * ld2 + n - n2]
+    int w_made;                                                  // W comes from an earlier launch (pib_mm)
 };
 __device__ __forceinline__ float * mm_out(const mm_dev & a, float * Y, int m, int n) { return n >= a.n2 ? a.Y2 + (size_t) a.rows2[m] * a.ld2 + (n - a.n2) : Y + (size_t) m * a.ldy + n; }
 
@@ -261,7 +262,7 @@ __global__ void __launch_bounds__(256) mv_pair_kernel(mm_dev a, mm_dev b, bool x
 // The eight warps of a block share K; a lane's 16-byte piece of a weight row (k = 32 c + 8 t .. + 7, t = lane % 4) is the A operand of two products as it
 // is: k slots 2t, 2t + 1 and 2t + 8, 2t + 9 of product j stand for elements 8t + 4j .. + 3, and the lane reads the same eight elements of "its" token for B.
 // So no value passes through shared memory, an activation is rounded once per block, and a warp's weight bytes are all in flight together -- the first ones
-// before the launch wait, because weights are immutable.
+// before the launch wait where W is a weight, which nothing writes (not for the key and value rows that an attention gathers and passes as W: pib_mm.w_made).
 // What bounds it: the weights' way from memory.  The form it replaces (a warp per weight row, mv_rows_kernel) rounded every activation for every weight row: at
 // four tokens 32 conversions per 16 bytes of weights.
 #define MVM_U 4                      // 32-k chunks a warp has in flight
@@ -273,7 +274,7 @@ __device__ __forceinline__ uint32_t mvm_pack(float lo, float hi) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t *>(&v);
 }
-// weight rows 16 tile .. + 15 of problem z against its rows [row0, row1) (at most 8 NT).  WAIT: the launch wait comes here, behind the first weight loads
+// weight rows 16 tile .. + 15 of problem z against its rows [row0, row1) (at most 8 NT).  WAIT: the launch wait comes here, behind the first loads of immutable weights
 template <int EPI, int NT, bool WAIT>
 __device__ __forceinline__ void mvm_body(const mm_dev & a, int z, int tile, int row0, int row1) {
     __shared__ float red[8][8 * NT][16];
@@ -290,8 +291,9 @@ __device__ __forceinline__ void mvm_body(const mm_dev & a, int z, int tile, int 
             rb[u] = in ? ld_stream_v4(wb + (c + u) * 32) : make_int4(0, 0, 0, 0);
         }
     };
+    if (WAIT && a.w_made) pib_pdl_wait();
     load(c0);
-    if (WAIT) { pib_pdl_wait(); pib_pdl_trigger(); }
+    if (WAIT) { pib_pdl_wait(); pib_pdl_trigger(); }      // a second wait returns at once
     const float * x[NT];
     bool          has[NT];
 #pragma unroll
@@ -452,7 +454,7 @@ int pib_dense_mm(const pib_mm & a, cudaStream_t st) {
         if (rc != PIB_ERR_UNSUPP) return rc;
     }
     if (a.x_bf16) { pib_set_error("dense matmul: bfloat16 activations need the tensor-core path (more than 16 rows, strides multiples of 8)"); return PIB_ERR_UNSUPP; }
-    mm_dev d = { a.W, a.ldw, a.wz, a.X, a.ldx, a.xz, a.xrows, a.xdiv < 1 ? 1 : a.xdiv, a.Y, a.ldy, a.yz, a.M, a.N, a.K, a.zrange, a.e0, a.e1, a.zlist, a.Y2, a.ld2, a.Y2 ? a.n2 : 0x7fffffff, a.rows2 };
+    mm_dev d = { a.W, a.ldw, a.wz, a.X, a.ldx, a.xz, a.xrows, a.xdiv < 1 ? 1 : a.xdiv, a.Y, a.ldy, a.yz, a.M, a.N, a.K, a.zrange, a.e0, a.e1, a.zlist, a.Y2, a.ld2, a.Y2 ? a.n2 : 0x7fffffff, a.rows2, a.w_made };
     if (a.wtype == PIB_TYPE_F32 && a.exact && !a.Y2 && a.N <= 128 && a.M > MV_MAXB && a.Z == 1 && !a.xrows && !a.zrange && a.epi == PIB_EPI_NONE) {
         const int  NB = a.N <= 8 ? 8 : a.N <= 16 ? 16 : 24;
         const bool vec = a.K % 4 == 0 && a.ldw % 4 == 0 && a.ldx % 4 == 0 && (((uintptr_t) a.W | (uintptr_t) a.X) & 15) == 0;
@@ -500,7 +502,7 @@ int pib_dense_mm_pair(const pib_mm & a, const pib_mm & b, cudaStream_t st) {
         const int rc = pib_dense_mm(a, st);
         return rc != PIB_OK ? rc : pib_dense_mm(b, st);
     }
-    auto dev = [](const pib_mm & m) { return mm_dev{ m.W, m.ldw, m.wz, m.X, m.ldx, m.xz, nullptr, 1, m.Y, m.ldy, m.yz, m.M, m.N, m.K, nullptr, m.e0, m.e1, nullptr, nullptr, 0, 0x7fffffff, nullptr }; };
+    auto dev = [](const pib_mm & m) { return mm_dev{ m.W, m.ldw, m.wz, m.X, m.ldx, m.xz, nullptr, 1, m.Y, m.ldy, m.yz, m.M, m.N, m.K, nullptr, m.e0, m.e1, nullptr, nullptr, 0, 0x7fffffff, nullptr, m.w_made }; };
     auto xvec = [](const pib_mm & m) { return m.ldx % 4 == 0 && ((uintptr_t) m.X & 15) == 0; };
 #define PAIR_GO(WT, ROUND) do { if (b.epi == PIB_EPI_NONE) launch_pair<WT, ROUND, PIB_EPI_NONE>(dev(a), dev(b), xvec(a), xvec(b), st); \
                                 else launch_pair<WT, ROUND, PIB_EPI_GEGLU_PAIR>(dev(a), dev(b), xvec(a), xvec(b), st); } while (0)
@@ -536,7 +538,7 @@ int pib_dense_mm_experts(const pib_mm & a, const pib_mm & b, cudaStream_t st) {
         return rc != PIB_OK ? rc : pib_dense_mm(b, st);
     }
     auto dev = [](const pib_mm & m) {
-        return mm_dev{ m.W, m.ldw, m.wz, m.X, m.ldx, m.xz, m.xrows, m.xdiv < 1 ? 1 : m.xdiv, m.Y, m.ldy, m.yz, m.M, m.N, m.K, m.zrange, m.e0, m.e1, m.zlist, nullptr, 0, 0x7fffffff, nullptr };
+        return mm_dev{ m.W, m.ldw, m.wz, m.X, m.ldx, m.xz, m.xrows, m.xdiv < 1 ? 1 : m.xdiv, m.Y, m.ldy, m.yz, m.M, m.N, m.K, m.zrange, m.e0, m.e1, m.zlist, nullptr, 0, 0x7fffffff, nullptr, m.w_made };
     };
     auto xvec = [](const pib_mm & m) { return m.ldx % 4 == 0 && ((uintptr_t) m.X & 15) == 0; };
     const int za = a.zlist && a.M < a.Z ? a.M : a.Z;
@@ -567,6 +569,36 @@ pib_weight * pib_dense_upload(int type, const void * host, int64_t N, int64_t K)
         return nullptr;
     }
     return w;
+}
+
+// a producer of W that lets the launch behind it start at once and is late itself
+__global__ void mm_late_copy_kernel(const uint4 * __restrict__ src, uint4 * __restrict__ dst, int n16) {
+    pib_pdl_wait();
+    pib_pdl_trigger();
+    for (int i = 0; i < 200; i++) __nanosleep(1000);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n16; i += gridDim.x * blockDim.x) dst[i] = src[i];
+}
+// for the tests: Y[M][N] = X[M][K] W^T with W [N][K] (bfloat16 bits) written by the launch right in front of the matmul; K a multiple of 8
+extern "C" int pib_dense_mm_made_host(const void * W, const float * X, float * Y, int M, int N, int K) {
+    if (M < 1 || N < 1 || K < 8 || K % 8) { pib_set_error("dense matmul: bad arguments"); return PIB_ERR_ARG; }
+    const size_t wb = (size_t) N * K * 2, xb = (size_t) M * K * 4, yb = (size_t) M * N * 4;
+    uint8_t * src = nullptr, * dst = nullptr; float * dX = nullptr, * dY = nullptr;
+    int rc = PIB_OK;
+    if (cudaMalloc(&src, wb) != cudaSuccess || cudaMalloc(&dst, wb) != cudaSuccess || cudaMalloc(&dX, xb) != cudaSuccess || cudaMalloc(&dY, yb) != cudaSuccess) rc = PIB_ERR_NOMEM;
+    if (rc == PIB_OK) {
+        cudaMemcpy(src, W, wb, cudaMemcpyHostToDevice);
+        cudaMemcpy(dX, X, xb, cudaMemcpyHostToDevice);
+        cudaMemset(dst, 0, wb);
+        pib_mm a;
+        a.W = dst; a.ldw = K; a.X = dX; a.ldx = K; a.Y = dY; a.ldy = N; a.M = M; a.N = N; a.K = K; a.w_made = 1;
+        // one block: the matmul's blocks find room beside it
+        pib_launch(mm_late_copy_kernel, dim3(1), dim3(256), (size_t) 0, (cudaStream_t) nullptr, (const uint4 *) src, (uint4 *) dst, (int) (wb / 16));
+        rc = pib_dense_mm(a, nullptr);
+        if (rc == PIB_OK && cudaMemcpy(Y, dY, yb, cudaMemcpyDeviceToHost) != cudaSuccess) rc = PIB_ERR_CUDA;
+    }
+    for (void * p : { (void *) src, (void *) dst, (void *) dX, (void *) dY }) if (p) cudaFree(p);
+    if (rc != PIB_OK) pib_set_error("dense matmul: %s", cudaGetErrorString(cudaGetLastError()));
+    return rc;
 }
 
 // host-buffer convenience for the parity tests: every operand in host memory, shapes and strides as in pib_mm (elements).

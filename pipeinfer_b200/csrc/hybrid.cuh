@@ -245,6 +245,7 @@ struct pib_mm {
     // outputs n >= n2 of row m go to Y2[rows2[m] * ld2 + n - n2] (keys and values straight into their cache cells); Z 1, no paired epilogue
     float *         Y2 = nullptr; int64_t ld2 = 0; int n2 = 0x7fffffff; const int32_t * rows2 = nullptr;
     int             x_bf16 = 0;                          // 1: X already holds bfloat16 rows (ldx in elements, a multiple of 8): tensor-core path only, no staging copy
+    int             w_made = 0;                          // 1: W is not a weight but the work of an earlier launch on this stream: nothing of it is read ahead of the launch wait
 };
 #ifdef __CUDACC__
 // FAST (served mode, where the result is rounded to bfloat16 as the next matmul's operand): the exponential through ex2.approx, no branch

@@ -527,12 +527,12 @@ int pib_latent_attention_mm(const float * q, int ldq, const float * qlat, const 
     pib_launch(lat_qcat_kernel, dim3(dim3((unsigned) nq, (unsigned) H)), dim3(128), (size_t) (0), st, q, ldq, qlat, H, L.dim, L.rot_dim, L.rot_dims, L.rot_pairs, R, L.scale, b.pos, rope, t0, Qc);
     CKL();
     pib_mm a;
-    a.W = Kb; a.wtype = PIB_TYPE_BF16; a.ldw = RK; a.X = Qc; a.ldx = RK; a.Y = S; a.ldy = NKp; a.M = nq * H; a.N = NK; a.K = RK;
+    a.W = Kb; a.w_made = 1; a.wtype = PIB_TYPE_BF16; a.ldw = RK; a.X = Qc; a.ldx = RK; a.Y = S; a.ldy = NKp; a.M = nq * H; a.N = NK; a.K = RK;
     int rc = pib_dense_mm(a, st);
     if (rc != PIB_OK) return rc;
     if ((rc = pib_window_softmax(S, P, NKp, NK, j0, L.window, b.pos, t0, nq * H, nq * H, H, L.sink, st)) != PIB_OK) return rc;
     pib_mm v;
-    v.W = Vt; v.wtype = PIB_TYPE_BF16; v.ldw = 2 * NKp; v.Y = ctx + (size_t) t0 * H * R; v.ldy = R; v.M = nq * H; v.N = R; v.K = 2 * NKp;
+    v.W = Vt; v.w_made = 1; v.wtype = PIB_TYPE_BF16; v.ldw = 2 * NKp; v.Y = ctx + (size_t) t0 * H * R; v.ldy = R; v.M = nq * H; v.N = R; v.K = 2 * NKp;
     if (nq * H > 16) { v.X = (const float *) P; v.ldx = 2 * NKp; v.x_bf16 = 1; return pib_dense_mm(v, st); }
     // a last block of very few rows goes to the row kernel, which reads fp32: widen the weights again
     pib_launch(lat_widen_kernel, dim3((unsigned) (nq * H)), dim3(256), (size_t) 0, st, (const __nv_bfloat16 *) P, 2 * NKp, S);

@@ -373,13 +373,13 @@ int pib_kv_attention_mm(const pib_kv_query & q, const pib_hlayer & L, const pib_
     CKL();
     if (pib_flash_attention_fits(L)) return pib_flash_attention(q, L, t0, nq, p0, j0, n_front, NK, Kb, Vt, Qc, out, st);
     pib_mm a;
-    a.W = Kb; a.wtype = PIB_TYPE_BF16; a.ldw = 3 * D; a.wz = (int64_t) NKp * 3 * D; a.X = Qc; a.ldx = 3 * D; a.xz = (int64_t) M * 3 * D; a.x_bf16 = 1;
+    a.W = Kb; a.w_made = 1; a.wtype = PIB_TYPE_BF16; a.ldw = 3 * D; a.wz = (int64_t) NKp * 3 * D; a.X = Qc; a.ldx = 3 * D; a.xz = (int64_t) M * 3 * D; a.x_bf16 = 1;
     a.Y = S; a.ldy = NKp; a.yz = (int64_t) M * NKp; a.M = M; a.N = NK; a.K = 3 * D; a.Z = GK;
     int rc = pib_dense_mm(a, st);
     if (rc != PIB_OK) return rc;
     if ((rc = pib_window_softmax(S, P, NKp, NK, j0, L.window, b.pos, t0, GK * M, M, rep, L.sink, st, L.mask, L.keep, n_front, L.softcap, L.slopes, L.rel, L.n_rel)) != PIB_OK) return rc;
     pib_mm v;
-    v.W = Vt; v.wtype = PIB_TYPE_BF16; v.ldw = 2 * NKp; v.wz = (int64_t) V * 2 * NKp; v.X = (const float *) P; v.ldx = 2 * NKp; v.xz = (int64_t) M * 2 * NKp; v.x_bf16 = 1;
+    v.W = Vt; v.w_made = 1; v.wtype = PIB_TYPE_BF16; v.ldw = 2 * NKp; v.wz = (int64_t) V * 2 * NKp; v.X = (const float *) P; v.ldx = 2 * NKp; v.xz = (int64_t) M * 2 * NKp; v.x_bf16 = 1;
     v.Y = Qc; v.ldy = V; v.yz = (int64_t) M * V; v.M = M; v.N = V; v.K = 2 * NKp; v.Z = GK;              // the query rows are used up: the outputs take their place
     if ((rc = pib_dense_mm(v, st)) != PIB_OK) return rc;
     pib_launch(kv_token_order_kernel, dim3((unsigned) nq), dim3(256), (size_t) 0, st, (const float *) Qc, out, q.gate, q.ldg, H, maps, rep, nq, V, t0);

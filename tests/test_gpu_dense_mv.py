@@ -1,9 +1,12 @@
 """Few rows against bfloat16 weights on the tensor cores (mv_mma_kernel, csrc/dense_mm.cu) at the edges of its tiles: weight rows that fill no tile, k that fills no
 chunk and leaves warps without any, one to sixteen tokens, strided rows, outputs in pairs.  The operands are bfloat16 (products exact in fp32), so an output is off by
 fp32 sums only: below (K + 8) 2^-23 sum |w x|."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
+from pipeinfer_b200 import load
 from tests.rapisun_oracle import bf16_round
 from tests.test_gpu_dense_mm import mm
 
@@ -19,3 +22,18 @@ def test_few_rows(M, N, K, ldx):
     assert (np.abs(got - Xr @ W.T) <= lim).all()
     one = mm(W, X[M - 1:], 1, N, K, ldx=ldx).reshape(N)              # a token's outputs do not depend on the rest of the batch
     assert np.array_equal(one, got[M - 1])
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 24, 64), (16, 40, 2048)])
+def test_weight_rows_of_the_launch_in_front(M, N, K):
+    """W that an earlier launch makes (an attention's gathered keys): none of it is read before that launch is through, however late it is"""
+    lib = load()
+    lib.init(0)
+    L = lib.L
+    L.pib_dense_mm_made_host.argtypes = [C.c_void_p] * 3 + [C.c_int] * 3
+    rng = np.random.default_rng(M + N + K)
+    W, X = bf16_round(rng.standard_normal((N, K))), bf16_round(rng.standard_normal((M, K)))
+    bits, x, y = (W.astype(np.float32).view(np.uint32) >> 16).astype(np.uint16), X.astype(np.float32), np.full((M, N), np.nan, np.float32)
+    for _ in range(3):
+        lib.check(L.pib_dense_mm_made_host(bits.ctypes.data, x.ctypes.data, y.ctypes.data, M, N, K))
+        assert (np.abs(y - X @ W.T) <= (K + 8) * 2.0 ** -23 * (np.abs(X) @ np.abs(W).T)).all()
