@@ -945,6 +945,7 @@ static int run_prompt_pass(pib_context * c, pib_run & run, int ch0, int nch, int
 pib_run * pib_take_run(pib_context * c, int n_tokens) {
     for (auto & r : c->runs) {
         if (r.in_use || r.id == c->last_finished) continue;
+        r.want_lo = r.want_hi = 0;
         if (!r.done) cudaEventCreateWithFlags(&r.done, cudaEventDisableTiming);
         if ((!r.acc_dev && (cudaMalloc(&r.acc_dev, sizeof(pib_accept_result)) != cudaSuccess || cudaMallocHost(&r.acc_host, sizeof(pib_accept_result)) != cudaSuccess)) ||
             (!r.tc_err && cudaMallocHost(&r.tc_err, sizeof(int)) != cudaSuccess)) {
@@ -1227,8 +1228,8 @@ const float * pib_logits_row(pib_context * c, int i) {
     if (i < 0 || i >= r.n_tokens || (!r.logits && !remote)) return nullptr;
     const size_t V = (size_t) c->model->n_vocab;
     if (!remote && r.n_tokens <= PIB_CHUNK) {
-        // A decode or verification batch: all rows cross together into page-locked memory on the first one asked for.  A copy of one row into pageable memory takes
-        // 23 us at 8 000 values and 50 at 32 000, nearly all of it latency, and a sampler wants every row.
+        // A decode or verification batch: the rows marked in it cross together into page-locked memory on the first one asked for.  A copy of one row into pageable
+        // memory takes 23 us at 8 000 values and 50 at 32 000, nearly all of it latency, and a sampler wants every row it marked.  Any other row crosses alone.
         const size_t n = (size_t) r.n_tokens * V;
         if (c->logits_pin_cap < n) {
             if (c->logits_pin) cudaFreeHost(c->logits_pin);
@@ -1238,10 +1239,12 @@ const float * pib_logits_row(pib_context * c, int i) {
         }
         if (c->logits_pin_cap >= n) {
             if (!c->logits_row_valid[i]) {
-                cudaMemcpyAsync(c->logits_pin, r.logits, n * 4, cudaMemcpyDeviceToHost, c->stream);
+                const bool   marked = i >= r.want_lo && i < r.want_hi;
+                const size_t lo = marked ? r.want_lo : i, k = marked ? r.want_hi - r.want_lo : 1;
+                cudaMemcpyAsync(c->logits_pin + lo * V, r.logits + lo * V, k * V * 4, cudaMemcpyDeviceToHost, c->stream);
                 cudaStreamSynchronize(c->stream);
-                c->d2h_bytes += n * 4;
-                c->logits_row_valid.assign((size_t) r.n_tokens, 1);
+                c->d2h_bytes += k * V * 4;
+                std::fill_n(c->logits_row_valid.begin() + lo, k, 1);
             }
             return c->logits_pin + (size_t) i * V;
         }

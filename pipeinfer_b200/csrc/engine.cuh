@@ -89,6 +89,7 @@ struct pib_run {                   // one (possibly still executing) decode: the
     int          cap_tokens = 0;
     bool         has_walk  = false;       // the batch came with an acceptance table: only the walk's result crosses to the host
     bool         rows_on_host = false;
+    int          want_lo = 0, want_hi = 0;   // logits rows that the caller marked in its batch: [want_lo, want_hi) holds all of them
     pib_accept_result * acc_dev = nullptr, * acc_host = nullptr;
     int *        tc_err    = nullptr;     // pinned: the stream's error word behind this run's kernels (pib_tc_error_copy)
     bool         tc_used   = false;       // the run launched kernels that set it
@@ -162,7 +163,7 @@ struct pib_context {
     int                  last_finished = -1;
     float *              logits_fetch_dev = nullptr;   // head of a pipeline: staging for one row fetched from the last stage
     std::vector<float>   logits_host;     // lazily filled rows of the last finished run (prompts)
-    float *              logits_pin = nullptr;      // the same for runs of up to PIB_CHUNK tokens: page-locked, all rows in one copy
+    float *              logits_pin = nullptr;      // the same for runs of up to PIB_CHUNK tokens: page-locked, the marked rows in one copy
     size_t               logits_pin_cap = 0;        // floats
     std::vector<uint8_t> logits_row_valid;
     bool                 logits_all = true;

@@ -383,7 +383,17 @@ static int start_from_batch(llama_context * ctx, const llama_batch & batch) {
         for (int i = 0; i < n; i++) seqp[i] = &seq1[i];
         ns = nseq.data(); sp = seqp.data();
     }
-    return pib_decode_start(ctx->c, n, batch.token, p, ns, sp, batch.batch_id);
+    const int run = pib_decode_start(ctx->c, n, batch.token, p, ns, sp, batch.batch_id);
+    if (run < 0) return run;
+    // rows that the caller will read (llama.cpp:5798): those it marked, else all or the last one
+    pib_run & r = ctx->c->runs[run];
+    r.want_lo = batch.logits || ctx->c->logits_all ? 0 : n - 1;
+    r.want_hi = n;
+    if (batch.logits) {
+        while (r.want_lo < n && !batch.logits[r.want_lo]) r.want_lo++;
+        while (r.want_hi > r.want_lo && !batch.logits[r.want_hi - 1]) r.want_hi--;
+    }
+    return run;
 }
 
 int llama_decode(struct llama_context * ctx, struct llama_batch batch) {
@@ -414,7 +424,9 @@ float * llama_get_logits_ith(struct llama_context * ctx, int32_t i) { return con
 float * llama_get_logits(struct llama_context * ctx) {
     pib_context * c = ctx->c;
     if (c->last_finished < 0) return nullptr;
-    const int n = c->runs[c->last_finished].n_tokens;
+    pib_run & r = c->runs[c->last_finished];
+    const int n = r.n_tokens;
+    r.want_lo = 0; r.want_hi = n;                             // every row, marked or not
     for (int i = 0; i < n; i++) pib_logits_row(c, i);
     return const_cast<float *>(pib_logits_row(c, 0));         // rows are contiguous
 }
@@ -601,7 +613,6 @@ extern "C" int llama_pib_debug_read(struct llama_context * ctx, int which, float
     return cudaMemcpy(out, src, sizeof(float) * (size_t) n_floats, cudaMemcpyDeviceToHost) == cudaSuccess ? 0 : -1;
 }
 
-// debugging aid: handle of a resident weight matrix (layer < 0: 0 = token_embd, 1 = output; else 0 qkv, 1 o, 2 gate|up, 3 down)
 // the error word of the context's stream, as a tensor-core kernel whose wait ran out would leave it (tests)
 extern "C" int llama_pib_debug_tc_error(struct llama_context * ctx, int word) {
     int * err = pib_tc_error_word(ctx->c->stream);
@@ -609,6 +620,7 @@ extern "C" int llama_pib_debug_tc_error(struct llama_context * ctx, int word) {
     if (!err || cudaMemcpy(err, &word, 4, cudaMemcpyHostToDevice) != cudaSuccess) return PIB_ERR_CUDA;
     return PIB_OK;
 }
+// debugging aid: handle of a resident weight matrix (layer < 0: 0 = token_embd, 1 = output; else 0 qkv, 1 o, 2 gate|up, 3 down)
 extern "C" const pib_weight * llama_pib_debug_weight(const struct llama_model * model, int layer, int which) {
     const pib_model * m = model->m;
     if (layer < 0) return which == 0 ? m->tok_embd : m->output;
