@@ -22,6 +22,8 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include <atomic>
+
 #include "q8k_quant.cuh"
 #include "tc_common.cuh"
 
@@ -365,6 +367,39 @@ static tg_encode_fn tg_encode() {
 static int tg_nb_of(int b) { return b <= 32 ? 32 : b <= 64 ? 64 : b <= 96 ? 96 : b <= 128 ? 128 : b <= 192 ? 192 : 256; }
 size_t pib_gemm_xhat_bytes(int64_t K, int b) { return (size_t) (b <= 32 ? 32 : b <= 64 ? 64 : b <= 128 ? 128 : 256) * K * sizeof(__half); }
 
+// Clusters of S CTAs, one CTA per SM, that the machine holds at once: not every GPC's SMs divide by S, so it is fewer than the SMs do (148 SMs: 148, 74, 33, 15 of
+// 1, 2, 4, 8 CTAs, which the launches bear out: 34 clusters of 4 take two rounds).
+template <int NB>
+static int tg_fit(int S) {
+    using C = tg_cfg<NB, 2>;
+    static std::atomic<int> known[4];                                            // of 1, 2, 4, 8; + 1
+    std::atomic<int> & k = known[S == 1 ? 0 : S == 2 ? 1 : S == 4 ? 2 : 3];
+    if (const int v = k.load()) return v - 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(gemm_q4k_tc_kernel<NB, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) C::SMEM) == cudaSuccess) {
+        cudaLaunchAttribute at;
+        memset(&at, 0, sizeof(at));
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = 1; at.val.clusterDim.y = 1; at.val.clusterDim.z = (unsigned) S;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1, 1, (unsigned) S); cfg.blockDim = dim3(C::THREADS); cfg.dynamicSmemBytes = C::SMEM; cfg.attrs = &at; cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, gemm_q4k_tc_kernel<NB, 2>, &cfg) != cudaSuccess) n = 0;
+    }
+    cudaGetLastError();
+    k.store(n + 1);
+    return n;
+}
+static int tg_fit_nb(int NB, int S) {
+    switch (NB) {
+        case 32:  return tg_fit<32>(S);
+        case 64:  return tg_fit<64>(S);
+        case 96:  return tg_fit<96>(S);
+        case 128: return tg_fit<128>(S);
+        case 192: return tg_fit<192>(S);
+        default:  return tg_fit<256>(S);
+    }
+}
+
 // row blocks [x0, x0 + nx), K in S shares
 template <int NB, int G>
 static int tg_launch(const pib_weight * w, const __half * xh, int b, int x0, int nx, int S, float * y, cudaStream_t st) {
@@ -401,14 +436,20 @@ int pib_gemm_q4k_tc(const pib_weight * w, const void * act_dev, int b, float * y
     if (act) pib_launch(tg_xhat_kernel, dim3((unsigned) ((n16 + 255) / 256)), dim3(256), 0, st, (const int8_t *) (act + L.qs_off), (const float *) (act + L.d_off), n16, (int) (w->K / 16), xh);
     PIB_CHECK(cudaGetLastError());
     const int NB = tg_nb_of(b), nsb = (int) (w->K / 256), nx = (int) ((w->N + TG_BM - 1) / TG_BM), sms = pib_num_sms();
-    // K shares of n row blocks that fit `slots` CTAs at once; every share keeps at least two super-blocks
-    auto shares = [&](int n, int slots) { int S = 1; while (S < 8 && n * S * 2 <= slots && nsb / (S * 2) >= 2) S *= 2; return S; };
+    // K shares of n row blocks, with G groups, whose clusters all find room at once; every share keeps at least two super-blocks.  With two CTAs per SM, S of them need
+    // the room of S / 2, less a sixteenth that packing loses (occupancy queries count one CTA of this kernel per SM; of 4 CTAs 70 clusters ran at once, 72 did not).
+    // us at 34 and 37 blocks of K = 4096 / 100 tokens and 17 of 8192 / 256, shares by room / by SMs alone: 16.9 / 22.5, 16.8 / 22.8, 22.6 / 31.6.
+    auto shares = [&](int n, int G) {
+        int S = 1;
+        while (S < 8 && nsb / (S * 2) >= 2 && n <= (G == 2 ? tg_fit_nb(NB, S * 2) : tg_fit_nb(NB, S) * 15 / 16)) S *= 2;
+        return S;
+    };
     // One CTA with two groups, or two CTAs with one, per SM (us, one / two, 40 and 128 tokens): 12288 x 4096 (96 row blocks) 18.7 / 20.8 and 20.9 / 29.6,
     // 10240 x 8192 (80) 31.4 / 33.4 and 33.8 / 42.7, 22016 x 4096 (172) 35.5 / 29.4 and 39.5 / 34.7, 8192 x 28672 (64, in 2 / 4 shares) 54.2 / 49.1 and 68.5 / 67.7.
     // Above 128 tokens the accumulator takes half of the tensor memory: one.
-    const bool two = NB <= 128 && (nx > sms || (NB <= 64 && shares(nx, sms) > 1));
+    const bool two = NB <= 128 && (nx > sms || (NB <= 64 && shares(nx, 2) > 1));
     if (two) {
-        const int S = shares(nx, 2 * sms);
+        const int S = shares(nx, 1);
         switch (NB) {
             case 32: return tg_launch<32, 1>(w, xh, b, 0, nx, S, y_dev, st);
             case 64: return tg_launch<64, 1>(w, xh, b, 0, nx, S, y_dev, st);
@@ -418,9 +459,9 @@ int pib_gemm_q4k_tc(const pib_weight * w, const void * act_dev, int b, float * y
     }
     // whole rounds of one CTA per SM, then what is left over in K shares (448 row blocks are three rounds and four blocks)
     int full = nx / sms * sms, rest = nx - full;
-    if (full > 0 && shares(rest, sms) == 1) { full = nx; rest = 0; }
+    if (full > 0 && shares(rest, 2) == 1) { full = nx; rest = 0; }
     auto go = [&](int x0, int n) {
-        const int S = shares(n, sms);
+        const int S = shares(n, 2);
         switch (NB) {
             case 32:  return tg_launch<32, 2>(w, xh, b, x0, n, S, y_dev, st);
             case 64:  return tg_launch<64, 2>(w, xh, b, x0, n, S, y_dev, st);
