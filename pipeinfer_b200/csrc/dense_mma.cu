@@ -275,17 +275,20 @@ int pib_tc_error(int word) {
     if (word) pib_set_error("a tensor-core kernel gave up on a barrier wait (block %d)", word - 1);
     return word ? PIB_ERR_CUDA : PIB_OK;
 }
-int pib_tc_error_copy(cudaStream_t st, int * host) {
-    dt_scratch * sc = dt_scratch_of(st, 0);
-    return sc && cudaMemcpyAsync(host, sc->err, 4, cudaMemcpyDeviceToHost, st) == cudaSuccess ? PIB_OK : PIB_ERR_CUDA;
+// one launch for both: a copy and a memset are two commands of the host, in every decode step of a layer-list model
+__global__ void tc_error_take_kernel(int * err, int * host, int clear) {
+    *host = *err;
+    if (clear) *err = 0;
 }
-int pib_tc_error_clear(cudaStream_t st) {
+int pib_tc_error_take(cudaStream_t st, int * host, bool clear) {
     dt_scratch * sc = dt_scratch_of(st, 0);
-    return sc && cudaMemsetAsync(sc->err, 0, 4, st) == cudaSuccess ? PIB_OK : PIB_ERR_CUDA;
+    if (!sc) return PIB_ERR_NOMEM;
+    tc_error_take_kernel<<<1, 1, 0, st>>>(sc->err, host, clear ? 1 : 0);
+    return cudaGetLastError() == cudaSuccess ? PIB_OK : PIB_ERR_CUDA;
 }
 int pib_tc_check(cudaStream_t st) {
     dt_scratch * sc = dt_scratch_of(st, 0);
-    if (!sc || pib_tc_error_copy(st, sc->err_host) != PIB_OK || pib_tc_error_clear(st) != PIB_OK || cudaStreamSynchronize(st) != cudaSuccess) {
+    if (!sc || pib_tc_error_take(st, sc->err_host, true) != PIB_OK || cudaStreamSynchronize(st) != cudaSuccess) {
         pib_set_error("tensor-core kernels: %s", cudaGetErrorString(cudaGetLastError()));
         return PIB_ERR_CUDA;
     }

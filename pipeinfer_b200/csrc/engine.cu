@@ -538,7 +538,6 @@ void pib_context_free(pib_context * c) {
         if (r.res_host) cudaFreeHost(r.res_host);
         if (r.acc_dev) cudaFree(r.acc_dev);
         if (r.acc_host) cudaFreeHost(r.acc_host);
-        if (r.tc_err) cudaFreeHost(r.tc_err);
     }
     for (auto e : c->desc_ev) if (e) cudaEventDestroy(e);
     if (c->cancel_ev) cudaEventDestroy(c->cancel_ev);
@@ -872,11 +871,11 @@ static int run_prompt_pass(pib_context * c, pib_run & run, int ch0, int nch, int
 #define RC(e) do { rc = (e); if (rc != PIB_OK) return rc; c->n_kernels++; } while (0)
     auto desc_of = [&](int k) { return c->desc_dev + (size_t) dev_slot(c, slots[ch0 + k]) * c->desc_stride; };
     auto nt_of   = [&](int k) { return std::min(PIB_CHUNK, ntok - k * PIB_CHUNK); };
-    // The stream's error word as it is behind this pass's kernels and in front of whatever takes their output to another stage.  It is cleared when the run's last pass
-    // is enqueued: a later copy includes the earlier passes.
+    // The stream's error word as it is behind this pass's kernels and in front of whatever takes their output to another stage.  The run's last pass
+    // clears it: a later copy includes the earlier passes.
     auto error_word = [&]() -> int {
         run.tc_used = true;
-        if (pib_tc_error_copy(st, run.tc_err) != PIB_OK) return PIB_ERR_CUDA;
+        if ((rc = pib_tc_error_take(st, run.tc_err, ch0 + nch == (int) slots.size())) != PIB_OK) return rc;
         if (c->stage.size > 1 && !c->stage.first())
             PIB_CHECK(cudaLaunchHostFunc(st, [](void * p) { const pib_run * r = (const pib_run *) p; if (*r->tc_err) pib_pipe_post_failure(r->batch_id); }, &run));
         return PIB_OK;
@@ -947,12 +946,13 @@ pib_run * pib_take_run(pib_context * c, int n_tokens) {
         if (r.in_use || r.id == c->last_finished) continue;
         r.want_lo = r.want_hi = 0;
         if (!r.done) cudaEventCreateWithFlags(&r.done, cudaEventDisableTiming);
-        if ((!r.acc_dev && (cudaMalloc(&r.acc_dev, sizeof(pib_accept_result)) != cudaSuccess || cudaMallocHost(&r.acc_host, sizeof(pib_accept_result)) != cudaSuccess)) ||
-            (!r.tc_err && cudaMallocHost(&r.tc_err, sizeof(int)) != cudaSuccess)) {
+        if (!r.acc_host && ((!r.acc_dev && cudaMalloc(&r.acc_dev, sizeof(pib_accept_result)) != cudaSuccess) ||
+                            cudaMallocHost(&r.acc_host, sizeof(pib_accept_result) + sizeof(int)) != cudaSuccess)) {
             pib_set_error("decode: out of memory for a run slot");
             cudaGetLastError();
             return nullptr;
         }
+        r.tc_err = reinterpret_cast<int *>(r.acc_host + 1);
         const int cap = ((n_tokens + PIB_CHUNK - 1) / PIB_CHUNK) * PIB_CHUNK;
         if ((c->stage.last() || c->stage.first()) && r.cap_tokens < cap) {
             if (r.res_dev) { cudaStreamSynchronize(c->stream); cudaFree(r.logits); cudaFree(r.res_dev); cudaFreeHost(r.res_host); }
@@ -1094,7 +1094,7 @@ static int enqueue_decode(pib_context * c, pib_run * run, int n_tokens, int batc
             if (run_prompt_pass(c, *run, ch0, nch, ntok, slots) != PIB_OK) run->failed = true;
         }
         for (int ch = 0; ch < n_chunks; ch++) if (c->desc_ev[slots[ch]]) cudaEventRecord(c->desc_ev[slots[ch]], c->stream);
-        if (pib_tc_error_clear(c->stream) != PIB_OK) run->failed = true;
+        if (run->failed) pib_tc_error_take(c->stream, run->tc_err, true);      // the passes that were not enqueued did not clear it
     } else
     for (int ch = 0; ch < n_chunks; ch++) {
         const int nt = std::min(PIB_CHUNK, n_tokens - ch * PIB_CHUNK);

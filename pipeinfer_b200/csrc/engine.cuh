@@ -91,7 +91,7 @@ struct pib_run {                   // one (possibly still executing) decode: the
     bool         rows_on_host = false;
     int          want_lo = 0, want_hi = 0;   // logits rows that the caller marked in its batch: [want_lo, want_hi) holds all of them
     pib_accept_result * acc_dev = nullptr, * acc_host = nullptr;
-    int *        tc_err    = nullptr;     // pinned: the stream's error word behind this run's kernels (pib_tc_error_copy)
+    int *        tc_err    = nullptr;     // pinned, behind acc_host: the stream's error word behind this run's kernels (pib_tc_error_take)
     bool         tc_used   = false;       // the run launched kernels that set it
 };
 

@@ -910,7 +910,7 @@ int pib_hybrid_decode_start(pib_context * c, int n_tokens, const int32_t * token
         c->d2h_bytes += sizeof(pib_row_result) * (size_t) T;
         run->rows_on_host = true;
     }
-    if ((run->tc_used = hy->dtype == PIB_TYPE_BF16) && (pib_tc_error_copy(st, run->tc_err) != PIB_OK || pib_tc_error_clear(st) != PIB_OK)) run->failed = true;
+    if ((run->tc_used = hy->dtype == PIB_TYPE_BF16) && pib_tc_error_take(st, run->tc_err, true) != PIB_OK) run->failed = true;
     cudaEventRecord(run->done, st);
     c->inflight.push_back(run->id);
     c->n_decode++;

@@ -273,8 +273,7 @@ int pib_dense_mm_pair(const pib_mm & a, const pib_mm & b, cudaStream_t st);   //
 int pib_dense_mm_experts(const pib_mm & routed, const pib_mm & shared, cudaStream_t st);   // a grouped matmul and a plain one with the same epilogue; in decode steps one launch
 // dense_mma.cu: the error word of a stream, which a tensor-core kernel sets when one of its bounded waits runs out
 int * pib_tc_error_word(cudaStream_t st);                 // device word; null: no memory for it
-int pib_tc_error_copy(cudaStream_t st, int * host);       // in stream order, to page-locked memory
-int pib_tc_error_clear(cudaStream_t st);                  // in stream order
+int pib_tc_error_take(cudaStream_t st, int * host, bool clear);      // copies it to page-locked memory, and clears it, in stream order
 int pib_tc_error(int word);                               // a copied word as a status
 int pib_tc_check(cudaStream_t st);                        // waits for the stream; the status since the last check
 pib_weight * pib_dense_upload(int type, const void * host, int64_t N, int64_t K);   // type: PIB_TYPE_BF16 / PIB_TYPE_F32, row-major [N][K]
