@@ -54,7 +54,8 @@ def test_gemm_edges(oracle, N, K, b):
                                    (2048, 4096, 40), (19200, 1024, 64),                        # <64, 1>
                                    (19200, 1024, 90), (19200, 1024, 128),                      # <96, 1>, <128, 1>
                                    (10240, 2048, 17), (10240, 2048, 50),                       # <32, 2>, <64, 2>
-                                   (10240, 2048, 96), (2048, 4096, 80),                        # <96, 2>, one share and eight
+                                   (10240, 2048, 96), (2048, 4096, 80), (1910, 4096, 80),      # <96, 2>, one share, four and eight (15 row blocks)
+                                   (4220, 4096, 90), (4230, 4096, 90), (9460, 2048, 70), (9480, 2048, 70),      # 33 / 34 and 74 / 75 row blocks: four shares, two; two, one
                                    (10240, 2048, 128), (4096, 4096, 100),                      # <128, 2>, one share and four
                                    (10240, 2048, 188), (4096, 4096, 129), (19200, 1024, 180),  # <192, 2>, one share, four, a round and two blocks
                                    (10240, 2048, 250), (4096, 4096, 256)])                     # <256, 2>, one share and four
