@@ -3,7 +3,7 @@
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference] [--config 70b|7b|tiny]
 
-Workload (BASELINE.json configs[2], the one the metric is quoted on): Dolphin/Llama-2-70B-architecture target in Q4_K
+Workload (the one the metric is quoted on): Dolphin/Llama-2-70B-architecture target in Q4_K
 (38.8 GB, fits one B200) + TinyLlama-1.1B-architecture draft, random-init weights generated in HBM ("bigram" flavour:
 both models predict a fixed permutation of the last token, the draft agreeing with the target on --agree of the tokens),
 synthetic 64-token prompt, flags of the authors' launch script (examples/speculative/scripts/dolphin_tinyllama_8_nodes.sh:
@@ -122,7 +122,7 @@ class ClockSampler:
 
 
 # --------------------------------------------------------------------------------------------------------------------
-# reference arm / cpu_baseline: the UNMODIFIED reference `speculative` (oracle/_ref, built from /root/reference by
+# reference arm / cpu_baseline: the UNMODIFIED reference `speculative` (oracle/_ref, built from the reference's sources by
 # oracle/Makefile) under the mini-MPI shim on this box's host cores.  A 70B-width model cannot be run at full depth on the
 # host in bounded time, so the sample is depth-reduced (same width, same draft) at two depths and the per-token time is
 # extrapolated linearly in the number of target layers.
@@ -226,7 +226,7 @@ def main():
                     help="plain = non-speculative greedy decoding through the same pipeline (the reference's `main`): the second denominator")
     ap.add_argument("--sched-policy", default="chain2", choices=["reference", "chain1", "chain2", "chain3"],
                     help="scheduler policy: chain2 (the library's default: text-identical to the reference's policy, checked in the first "
-                         "warm-up step), the reference's own, or the other chain-continuation policies (PIB_SCHED_CHAIN, DESIGN.md §9)")
+                         "warm-up step), the reference's own, or the other chain-continuation policies (PIB_SCHED_CHAIN)")
     ap.add_argument("--no-draft-priority", action="store_true")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-plain", action="store_true", help="skip the non-speculative generation after the timed steps (plain_tok_s, plain_tokens_sha)")
@@ -266,7 +266,7 @@ def main():
         t0 = time.time()
         r = run_reference_sample(args.config, args, budget="large")
         if r is None:
-            print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/speculative not built (needs /root/reference at build time)"}))
+            print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/speculative not built (needs the reference's sources at build time)"}))
             return 0
         line = {"impl": "reference", "metric": "accepted tokens/sec", "value": r["value"], "unit": "tokens/s", "n_gpus": args.gpus,
                 "steps": args.steps, "warmup": args.warmup, "ms_per_step": 1000.0 * args.n_predict / r["value"] if r["value"] else None,
@@ -358,7 +358,7 @@ def main():
             config["sched_policy"] = "reference (fallback: %s changed the text)" % args.sched_policy
     os.environ["PIB_SCHED_CHAIN"] = policy_env
     if policy_env != "0":
-        config["workload"] += ", scheduler policy %s (additive, text-identical; DESIGN.md §9)" % args.sched_policy
+        config["workload"] += ", scheduler policy %s (additive, text-identical)" % args.sched_policy
     b0, e0l = ranges[rank] if world > 1 else (0, L)
     prof_layer = (b0 + e0l) // 2
     lib.llama_pib_profile_layer(tgt.ctx, prof_layer)
@@ -387,7 +387,7 @@ def main():
     lib.llama_pib_profile_layer(tgt.ctx, -1)
     k1 = launches()
     # outside the timed region: one NON-SPECULATIVE greedy generation through the same pipeline (the reference's `main`): the second
-    # denominator of north_star, measured in the same run, and the text every speculative step must reproduce
+    # denominator of the speed-up, measured in the same run, and the text every speculative step must reproduce
     plain = None
     if args.mode == "speculative" and not args.no_plain:
         if rank != 0:
@@ -447,7 +447,7 @@ def main():
         lib.llama_pib_matrix_shape(tgt.model, prof_layer, k, C.byref(N_), C.byref(K_), C.byref(by))
         mean_b = sum(x[0] for x in lst) / len(lst)
         mean_ms = sum(x[1] for x in lst) / len(lst)
-        alg = by.value + mean_b * K_.value * 4 + mean_b * N_.value * 4        # SURVEY §8d: weights + F32 activations in + F32 out
+        alg = by.value + mean_b * K_.value * 4 + mean_b * N_.value * 4        # weights + F32 activations in + F32 out
         kernels[KIND[k]] = {"launches": len(lst), "N": N_.value, "K": K_.value, "mean_batch": round(mean_b, 2), "mean_ms": mean_ms,
                             "algorithmic_bytes": alg, "achieved_gbs": alg / mean_ms / 1e6, "frac": alg / mean_ms / 1e6 / peak}
     dom = kernels.get("gate_up")
@@ -511,7 +511,7 @@ def main():
                                "formula": "n_tokens * n_embd * 4 B of fp32 activations per hop (%d B per token), stored by the sending stage's last kernel into the "
                                           "next stage's memory; 80 B per verification batch (device-side acceptance walk) back to the head" % (E * 4),
                                "nvlink_tx_bytes_counter": "not exposed on this driver: NVML_FI_DEV_NVLINK_THROUGHPUT_DATA_TX returns NVML_ERROR_NOT_SUPPORTED and "
-                                                          "`nvidia-smi nvlink -gt d` prints N/A (tools/nvlink_probe.py); the byte counts above are counted at the "
+                                                          "`nvidia-smi nvlink -gt d` prints N/A; the byte counts above are counted at the "
                                                           "point where each transfer is enqueued" if all(h["nvlink_tx_bytes_counter"] is None for h in hops) else "KiB counters read around the timed steps"}
     print(json.dumps(line))
     return 0

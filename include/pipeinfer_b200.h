@@ -37,7 +37,7 @@ extern "C" {
 #define PIB_TYPE_BF16 30   /* dense bfloat16 rows (models loaded from a folder: config.json + model.safetensors); PIB_TYPE_F32 rows in a float32 context */
 #define PIB_TYPE_Q6_K 14   /* matmul + embedding rows (output.weight / attn_v / ffn_down of Q4_K_M files, Q6_K files); activations as for Q4_K (Q8_K) */
 
-#define PIB_MAX_BATCH 16          /* verification batch handled by the dequant-GEMV path (north_star: batch 1-16) */
+#define PIB_MAX_BATCH 16          /* verification batch handled by the dequant-GEMV path (batch 1-16) */
 
 typedef struct pib_weight pib_weight;   /* a weight matrix repacked into HBM (layout private to the library) */
 typedef void * pib_stream;              /* cudaStream_t, or NULL for the legacy default stream */

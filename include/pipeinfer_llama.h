@@ -213,7 +213,7 @@ void         llama_reset_timings(struct llama_context * ctx);
 const char * llama_print_system_info(void);
 void         llama_log_set(void (*log_callback)(int level, const char * text, void * user_data), void * user_data);
 
-/* ---- additive extensions (no counterpart in llama.h; needed for device-side acceptance, SURVEY.md §8b) ---- */
+/* ---- additive extensions (no counterpart in llama.h; needed for device-side acceptance) ---- */
 /* sorted top-8 {id, logit, p} of logits row i of the last finished run: 96 bytes instead of n_vocab floats */
 int  llama_pib_get_top8(struct llama_context * ctx, int32_t i, llama_token_data * out8);
 /* Draft-vs-target acceptance on the device (the walk of examples/speculative/speculative.cpp:439-560 under greedy sampling).

@@ -1,12 +1,12 @@
 /*
  * mpi.h -- mini-MPI shim (TEST INFRASTRUCTURE, not product code).
  *
- * The reference's pipeline transport (/root/reference/ggml-mpi.c:5) includes <mpi.h>, but this
+ * The reference's pipeline transport (ggml-mpi.c:5) includes <mpi.h>, but this
  * image ships no MPI and nothing can be installed.  This header + mpi_shim.c provide exactly the
- * 18 entry points and the constants ggml-mpi.c uses (enumerated in SURVEY.md §8c), implemented as
+ * 18 entry points and the constants ggml-mpi.c uses, implemented as
  * a single-host, multi-process message queue in POSIX shared memory.  Semantics honoured:
  *   - per-(sender, communicator) non-overtaking order (what the worker loop relies on,
- *     /root/reference/llama.cpp:9941-9977),
+ *     llama.cpp:9941-9977),
  *   - MPI_Bsend never blocks (the reference attaches a 128 MiB buffer, ggml-mpi.c:77-79),
  *   - MPI_Probe / MPI_Iprobe with ANY_SOURCE / ANY_TAG and MPI_Get_count.
  * It is only ever linked into binaries built under oracle/_ref/.

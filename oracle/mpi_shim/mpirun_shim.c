@@ -4,7 +4,7 @@
  *   mpirun_shim -np N [--arena-mb M] [--timeout S] [--out-prefix P] prog [args...]
  *
  * Stands in for `mpirun -np N prog args` (how the reference launches `speculative`,
- * /root/reference/examples/speculative/scripts/dolphin_tinyllama_8_nodes.sh) on a box that has no MPI.
+ * examples/speculative/scripts/dolphin_tinyllama_8_nodes.sh) on a box that has no MPI.
  * Creates the shared segment, starts N copies of prog with MPISHIM_{SHM,RANK,SIZE} set, and returns
  * the worst exit status.  If one rank dies abnormally, or the timeout expires, the others are killed.
  * With --out-prefix P every rank's stdout goes to P.<rank>.out (stderr to P.<rank>.err).

@@ -22,7 +22,7 @@ ACT_BLOCK = {TYPE_Q4_0: (32, 34), TYPE_Q8_0: (32, 34), TYPE_Q4_K: (256, 292), TY
 
 
 def build(ref=True):
-    """make liboracle.so (and oracle/_ref/* when /root/reference exists and ref=True)."""
+    """make liboracle.so (and oracle/_ref/* when the reference's sources are there and ref=True)."""
     target = [] if ref else ["oracle"]
     subprocess.run(["make", "-s", "-j8", "-C", HERE] + target, check=True)
 

@@ -6,7 +6,7 @@
  * that branch's *association order* (8 lanes, lane-wise fused multiply-add, then the same horizontal reduction), so
  * that results are bit-identical to the compiled reference and not merely close.  Compiled with -ffp-contract=off;
  * every fused multiply-add the reference performs is written as an explicit fmaf().
- * All paths below are relative to /root/reference.
+ * All paths below are relative to the reference project.
  */
 #define _GNU_SOURCE
 #include "pib_oracle.h"

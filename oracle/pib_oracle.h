@@ -4,7 +4,7 @@
  * TEST INFRASTRUCTURE.  Only tests/, __graft_entry__.smoke() and bench.py's cpu_baseline / reference legs may
  * load this library; the product (libpipeinfer_b200.so) never links, loads or calls it.
  *
- * Every function cites the reference lines it restates (paths relative to /root/reference).  The restatement is
+ * Every function cites the reference lines it restates (paths relative to the reference project).  The restatement is
  * pinned two ways (tests/test_oracle_*.py): against the *compiled reference itself* (oracle/_ref/libggml_ref.so,
  * oracle/_ref/ref_decode_dump, built by oracle/Makefile from the sources where they lie) on seeded inputs, and
  * against the fixtures those produced, committed under tests/golden/.

@@ -5,7 +5,7 @@
 // batches and llama_kv_cache_seq_rm/cp/keep -- and dumps what the reference produced:
 //   <out>.logits.bin   float32 [n_tokens][n_vocab] for every decode, concatenated   (llama_get_logits_ith)
 //   <out>.kv.txt       one line per "KV" command: used_cells, then "cell:pos:seq,seq,..." for every non-empty cell
-//                      (llama_kv_cache_view_update, /root/reference/llama.cpp:9160-9222), plus "D rc" lines.
+//                      (llama_kv_cache_view_update, llama.cpp:9160-9222), plus "D rc" lines.
 //
 // usage: ref_decode_dump model.gguf n_ctx max_seq script.txt out_prefix [n_threads]
 // script:   D <n>            followed by n lines:  <token> <pos> <n_seq> <seq>...

@@ -1,7 +1,7 @@
 // oracle/ref_unicode_probe.cpp -- TEST INFRASTRUCTURE.  Exposes the reference's own codepoint classifier (unicode.h:360-403,
 // the tables the BPE pre-tokenizer consults) through a C symbol, so tests/test_tokenizer_cpu.py can compare the generated
 // table in pipeinfer_b200/csrc/unicode_classes.inc with it over all of Unicode.  Compiled against the header where it lies
-// under /root/reference (oracle/Makefile -> oracle/_ref/libunicode_probe.so); nothing of it is copied.
+// in the reference project (oracle/Makefile -> oracle/_ref/libunicode_probe.so); nothing of it is copied.
 #include <cstdint>
 #include <string>
 

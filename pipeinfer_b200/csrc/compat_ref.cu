@@ -88,7 +88,7 @@ bool llama_save_session_file(struct llama_context * ctx, const char * path_sessi
 
 // ---- samplers (llama.cpp:7019-7500) ----
 // The three truncation samplers below exist so that the reference's unmodified common/sampling.cpp links against this library;
-// greedy decoding (the path of SURVEY.md section 8) never calls them.  Behaviour as llama.cpp:7048-7130, own formulation.
+// greedy decoding never calls them.  Behaviour as llama.cpp:7048-7130, own formulation.
 static inline bool by_logit_desc(const llama_token_data & a, const llama_token_data & b) { return a.logit > b.logit; }
 
 void llama_sample_top_k(struct llama_context *, llama_token_data_array * cand, int k, size_t min_keep) {

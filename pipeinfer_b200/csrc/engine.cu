@@ -227,7 +227,7 @@ pib_model * pib_model_load_gguf(const char * path, int layer_begin, int layer_en
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// model: synthetic (random init generated directly as quantised blocks on the device; SURVEY.md §8d)
+// model: synthetic (random init generated directly as quantised blocks on the device)
 __device__ __forceinline__ uint32_t hash32(uint32_t x) {
     x ^= x >> 16; x *= 0x7feb352dU; x ^= x >> 15; x *= 0x846ca68bU; x ^= x >> 16;
     return x;

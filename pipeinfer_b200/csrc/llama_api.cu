@@ -40,7 +40,7 @@ static void ensure_init() {
     if (lr) dev = atoi(lr);
     if (pib_init(dev) != PIB_OK) {
         fprintf(stderr, "libpipeinfer_b200: %s\n", pib_last_error());
-        abort();      // the reference's hard failures are GGML_ASSERT -> abort (SURVEY §8b); there is no CPU path
+        abort();      // the reference's hard failures are GGML_ASSERT -> abort; there is no CPU path
     }
     done = true;
 }
@@ -197,7 +197,7 @@ int llama_pib_set_priority(struct llama_context * ctx, int high) {
     cudaStreamDestroy(c->stream);
     c->stream = ns;
     // A/B switch for the draft's matmul kernel only (the context the scheduler marks high-priority): its matrices are small
-    // enough that the fixed cost of a launch, not bandwidth, sets the time (DESIGN.md §8); e.g. PIB_KEEP_PLANES=1 PIB_DRAFT_GEMV_VARIANT=1
+    // enough that the fixed cost of a launch, not bandwidth, sets the time; e.g. PIB_KEEP_PLANES=1 PIB_DRAFT_GEMV_VARIANT=1
     const char * dv = high ? getenv("PIB_DRAFT_GEMV_VARIANT") : nullptr;
     if (dv) c->gemv_variant = atoi(dv);
     return 0;
@@ -439,7 +439,7 @@ int llama_pib_get_top8(struct llama_context * ctx, int32_t i, llama_token_data *
     return 0;
 }
 
-// acceptance on the device (north_star item 4): the table of the NEXT decode started on this context
+// acceptance on the device: the table of the NEXT decode started on this context
 void llama_pib_set_accept_table(struct llama_context * ctx, int32_t n_branches, int32_t keep, int32_t speculative, const int32_t * len,
                                 const int32_t * rows, const int32_t * toks, int32_t depth_stride) {
     pib_accept_table & T = ctx->c->tree_pending;

@@ -1,7 +1,7 @@
 // scheduler.cu -- PipeInfer's continuous asynchronous speculation scheduler (host, integer logic) on top of the
 // llama.h-compatible ABI of this library.
 //
-// Behavioural restatement of the reference's examples/speculative/speculative.cpp (S1-S6 of SURVEY.md §8a), re-organised as
+// Behavioural restatement of the reference's examples/speculative/speculative.cpp, re-organised as
 // one class; every step cites the reference lines whose behaviour it reproduces.  What differs by design:
 //   * both pipeline heads live in this process, so the MPI_Bcast lock-step of the two head ranks (llama_sync_token /
 //     llama_sync_token_data / llama_swap_comm, speculative.cpp:323-326, 454, 973-983) disappears;
@@ -93,7 +93,7 @@ class Scheduler {
     // PIB_REFERENCE_HAZARDS=1 restores the two behaviours of the reference that can make the text differ from the greedy
     // text (see check_for_cancel and speculation_loop); for A/B runs only
     bool            reference_hazards = getenv("PIB_REFERENCE_HAZARDS") != nullptr && atoi(getenv("PIB_REFERENCE_HAZARDS")) != 0;
-    // Scheduler policy (PIB_SCHED_CHAIN; default 2 since round 2: measured on the GPU, 98 -> 146 accepted tokens/s on one B200 with
+    // Scheduler policy (PIB_SCHED_CHAIN; default 2: measured on the GPU, 98 -> 146 accepted tokens/s on one B200 with
     // the 70B / 1.1B pair, text identical; PIB_SCHED_CHAIN=0 is the reference's policy, event for event -- tests/test_scheduler_sim.py).
     // 1: keep the chain of speculative runs alive across a verification.  The
     // reference restarts drafting from the last verified token after EVERY run it verifies (speculative.cpp:392-394), so when

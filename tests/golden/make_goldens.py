@@ -1,6 +1,6 @@
 #!/usr/bin/env python
 """Generate the committed golden fixtures by RUNNING THE COMPILED REFERENCE (oracle/_ref, built by oracle/Makefile
-from /root/reference).  Run in the build container only (the GPU box has no /root/reference); the outputs are
+from its sources).  Run only where those are; the outputs are
 committed so that every test can check the oracle -- and the CUDA path -- against what the reference produced.
 
   python tests/golden/make_goldens.py
@@ -313,7 +313,7 @@ def wide_goldens():
     run_ref(os.path.join(HERE, "wide_q4_k.gguf"), script, os.path.join(HERE, "decode_wide_long"), n_ctx=6144, max_seq=8, threads=4)
 
 
-# ---- BASELINE.json configs[0] at its real shape: TinyLlama-1.1B architecture, Q8_0 (1.17 GB: not committed; tools/make_gguf.py
+# ---- the one-GPU 1.1B model at its real shape: TinyLlama-1.1B architecture, Q8_0 (1.17 GB: not committed; tools/make_gguf.py
 # --direct regenerates it bit for bit from the seed, the sha256 of the file is part of the fixture) ----
 C1 = dict(n_layer=22, n_embd=2048, n_head=32, n_head_kv=4, n_ff=5632, n_vocab=32000, quant="q8_0", seed=11,
           emb_scale=0.05)     # embedding / output rows of std 0.05: logits of a realistic size (std ~2), every layer matters

@@ -54,7 +54,7 @@ struct sim_config {
     int32_t n_vocab;
     uint64_t seed;
     double  spec_issue_extra_us;     // extra host time to issue a speculative target run / a non-speculative one (the state of the
-    double  nonspec_issue_extra_us;  // library BEFORE the host KV-mirror fix: ~900 and ~500 us, see DESIGN.md §5)
+    double  nonspec_issue_extra_us;  // library BEFORE the host KV-mirror fix: ~900 and ~500 us)
     double  head_frac, tail_frac;    // share of the target's layers on the first / last stage (0 = all stages equal); stage_us is the MEAN
 };
 // defaults: fitted to the 8-GPU runs of the 70B / 1.1B pair in profiles/ (plain 89, classic 182, PipeInfer 206 / 204 / 184 / 163

@@ -1,5 +1,5 @@
 // tests/sched_sim/sim_ref_surface.cpp -- TEST INFRASTRUCTURE: the rest of the llama.h surface, so that the REFERENCE's own
-// examples/speculative/speculative.cpp + common/*.cpp (compiled from /root/reference, unmodified) link against the
+// examples/speculative/speculative.cpp + common/*.cpp (compiled from the reference, unmodified) link against the
 // virtual-clock engine model of sim_llama.cpp instead of llama.o / ggml*.o.  oracle/Makefile builds it as
 // oracle/_ref/speculative_sim.  Purpose: drive the reference's scheduler and this repository's scheduler with the same
 // clock, model and KV bookkeeping and compare what they ask of the target (tests/test_scheduler_sim.py).

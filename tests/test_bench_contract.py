@@ -11,7 +11,7 @@ ROOT = os.path.abspath(os.path.join(os.path.dirname(__file__), ".."))
 
 
 @pytest.mark.skipif(not os.path.exists(os.path.join(ROOT, "oracle", "_ref", "speculative")),
-                    reason="oracle/_ref is built only where /root/reference exists")
+                    reason="oracle/_ref is built only where the reference's sources are")
 def test_reference_arm_prints_the_contract_line():
     r = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference", "--config", "tiny", "--steps", "1",
                         "--warmup", "0"], cwd=ROOT, capture_output=True, text=True, timeout=600)

@@ -1,5 +1,5 @@
 """bench.py's layer split: the head GPU (which also runs the draft) takes the share of the target's layers that balances the work per
-run; checked here against the splits the round-2 measurements ran with."""
+run; checked here against the splits that earlier measurements ran with."""
 import os
 import sys
 

@@ -69,9 +69,9 @@ def test_cli_two_stages_matches_reference_text(golden_dir, tmp_path):
 REF_ON_OURS = os.path.join(ROOT, "oracle", "_ref", "speculative_b200")
 
 
-@pytest.mark.skipif(not os.path.exists(REF_ON_OURS), reason="oracle/_ref/speculative_b200 is built only where /root/reference exists")
+@pytest.mark.skipif(not os.path.exists(REF_ON_OURS), reason="oracle/_ref/speculative_b200 is built only where the reference's sources are")
 def test_unmodified_reference_speculative_runs_on_this_library(golden_dir, tmp_path):
-    # the reference's own examples/speculative/speculative.cpp + common/*.cpp, compiled from /root/reference and linked against
+    # the reference's own examples/speculative/speculative.cpp + common/*.cpp, compiled from the reference and linked against
     # libpipeinfer_b200.so instead of llama.o / ggml*.o (oracle/Makefile): their scheduler and sampling code drive this engine
     # through llama.h alone, and must print what they print on top of their own CPU engine
     gold = json.load(open(os.path.join(golden_dir, "speculative_q8_0.json")))
@@ -87,7 +87,7 @@ def test_unmodified_reference_speculative_runs_on_this_library(golden_dir, tmp_p
 MAIN_ON_OURS = os.path.join(ROOT, "oracle", "_ref", "main_b200")
 
 
-@pytest.mark.skipif(not os.path.exists(MAIN_ON_OURS), reason="oracle/_ref/main_b200 is built only where /root/reference exists")
+@pytest.mark.skipif(not os.path.exists(MAIN_ON_OURS), reason="oracle/_ref/main_b200 is built only where the reference's sources are")
 def test_unmodified_reference_main_runs_on_this_library(golden_dir, tmp_path):
     # examples/main/main.cpp (plain greedy decoding, the paper's "sequential" baseline), same treatment
     gold = json.load(open(os.path.join(golden_dir, "speculative_q8_0.json")))

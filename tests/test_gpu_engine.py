@@ -163,9 +163,9 @@ def test_decode_trace_at_benchmark_attention_shapes(llama, golden_dir, stem, mod
 
 @pytest.mark.parametrize("exact", [True, False])
 def test_config1_real_shape_trace(llama, golden_dir, tmp_path, exact):
-    """BASELINE.json configs[0] at its real shape (TinyLlama-1.1B architecture, 22 layers, Q8_0, 32000-token vocabulary):
+    """The one-GPU 1.1B model at its real shape (TinyLlama-1.1B architecture, 22 layers, Q8_0, 32000-token vocabulary):
     eight decodes -- prompt, single tokens, tree batches -- against the reference's CPU build.  Exact mode: the same bits (so
-    north_star's 1e-2 holds with room to spare).  Fast mode: a few rounding flips per row over 22 layers, ~5e-4 of the logit
+    a bound of 1e-2 holds with room to spare).  Fast mode: a few rounding flips per row over 22 layers, ~5e-4 of the logit
     scale (top logit ~100 here): the measured figure is printed and held to 2e-1."""
     meta = json.load(open(os.path.join(golden_dir, "c1_tinyllama_q8_0.json")))
     sh = meta["shape"]
@@ -272,7 +272,7 @@ def test_cancel_mid_flight_on_k_split_shapes_leaves_the_next_decode_intact(llama
 
 
 def test_prompt_through_the_tensor_core_gemm_matches_the_chunked_path(llama):
-    """north_star item 2: prompts (> 32 tokens) run their matmuls on the tcgen05 GEMM, 256 tokens per pass; verification batches keep the
+    """Prompts (> 32 tokens) run their matmuls on the tcgen05 GEMM, 256 tokens per pass; verification batches keep the
     GEMV.  Same model, same 300-token prompt, both ways: logits within 2e-2 of each other (fp16 operands against int8 x int4 integer
     arithmetic, on a model whose top logits are ~10), same argmax on every row that is not a near tie; and the KV cache the GEMM pass
     leaves behind serves a following single-token decode equally well."""
@@ -300,7 +300,7 @@ def test_prompt_through_the_tensor_core_gemm_matches_the_chunked_path(llama):
 
 
 def test_device_acceptance_walk_matches_the_host_walk(llama, golden_dir):
-    """north_star item 4: the draft-vs-target comparison of speculative.cpp:439-560 runs on the device right after sampling.  A
+    """The draft-vs-target comparison of speculative.cpp:439-560 runs on the device right after sampling.  A
     5-row tree batch (trunk + two branches) is decoded twice: once plainly (rows read back, walked in Python as the reference's
     loop does), once with the acceptance table (only the walk's result comes back).  Drafted tokens are chosen from the first
     pass so that the walk follows branch 1 for two steps and then fails -- and, second case, fails at once."""

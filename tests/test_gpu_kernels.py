@@ -1,6 +1,6 @@
 """Parity of the CUDA operators (through the C ABI of libpipeinfer_b200.so) against the oracle and the golden fixtures.
 Integer work (activation blocks, weight round trip, embedding rows) must be bit-exact; fp32 dot products may differ
-from the reference only by the order of fp32 additions (tolerance below; north_star: logits within 1e-2 max-abs)."""
+from the reference only by the order of fp32 additions (tolerance below)."""
 import os
 
 import numpy as np

@@ -1,5 +1,5 @@
 """Multi-GPU: the target split over 2 (and 4) pipeline stages, one process per GPU over NCCL, must generate exactly what
-one GPU generates, with identical KV bookkeeping on every stage.  Needs >= 2 GPUs on the box (gpurun --gpus 2)."""
+one GPU generates, with identical KV bookkeeping on every stage.  Needs >= 2 GPUs on the machine."""
 import os
 import subprocess
 import sys

@@ -110,7 +110,7 @@ def test_decode_trace_at_benchmark_shapes_matches_reference_bit_exact(oracle, go
 
 
 def test_config1_real_shape_trace_matches_reference_bit_exact(oracle, golden_dir, tmp_path):
-    # BASELINE.json configs[0] at its real shape (22 layers, 2048 wide, 32000 tokens, Q8_0): the model file is regenerated from
+    # the one-GPU 1.1B model at its real shape (22 layers, 2048 wide, 32000 tokens, Q8_0): the model file is regenerated from
     # its seed (1.17 GB, not committed) and must hash to what the reference was given
     import hashlib, json, subprocess, sys
     meta = json.load(open(os.path.join(golden_dir, "c1_tinyllama_q8_0.json")))

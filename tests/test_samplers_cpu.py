@@ -9,7 +9,7 @@ import pytest
 
 ROOT = os.path.abspath(os.path.join(os.path.dirname(__file__), ".."))
 REF = os.path.join(ROOT, "oracle", "_ref", "libllama_ref.so")
-pytestmark = pytest.mark.skipif(not os.path.exists(REF), reason="oracle/_ref is built only where /root/reference exists")
+pytestmark = pytest.mark.skipif(not os.path.exists(REF), reason="oracle/_ref is built only where the reference's sources are")
 
 
 class TokenData(C.Structure):

@@ -127,7 +127,7 @@ def test_chain_policy_resumes_and_pays_with_a_good_draft(monkeypatch):
 # ---- differential: the reference's own scheduler (speculative.cpp, unmodified) on the same model --------------------------
 import os
 
-needs_ref = pytest.mark.skipif(not os.path.exists(sim.REF_BIN), reason="oracle/_ref/speculative_sim is built only where /root/reference exists")
+needs_ref = pytest.mark.skipif(not os.path.exists(sim.REF_BIN), reason="oracle/_ref/speculative_sim is built only where the reference's sources are")
 
 DIFF_CASES = [
     # (model fields, flags)
@@ -145,7 +145,7 @@ DIFF_CASES = [
 def test_schedule_is_the_reference_schedule(case, monkeypatch, tmp_path):
     """Same clock, same model, same flags: every target decode (batch id, tokens, positions, sequence sets, KV cell), every
     finish and every cancel this scheduler issues is the one examples/speculative/speculative.cpp issues, at the same virtual
-    time -- rows S1-S6 of SURVEY.md §8a.  (PIB_REFERENCE_HAZARDS=1: the two deliberate deviations are switched off.)"""
+    time.  (PIB_REFERENCE_HAZARDS=1: the two deliberate deviations are switched off.)"""
     fields, flags = DIFF_CASES[case]
     fields = dict(fields, n_vocab=4096, call_us=0)
     text = "".join(chr(33 + (i * (7 + case)) % 90) for i in range(47))
@@ -201,7 +201,7 @@ CLASSIC_CASES = [
 ]
 
 
-@pytest.mark.skipif(not os.path.exists(sim.REF_BIN_CLASSIC), reason="oracle/_ref/speculative_orig_sim is built only where /root/reference exists")
+@pytest.mark.skipif(not os.path.exists(sim.REF_BIN_CLASSIC), reason="oracle/_ref/speculative_orig_sim is built only where the reference's sources are")
 @pytest.mark.parametrize("case", range(len(CLASSIC_CASES)))
 def test_classic_speculation_is_the_reference_schedule(case, monkeypatch, tmp_path):
     """pib_speculative_orig_generate against examples/speculative_orig/speculative.cpp (unmodified) on the same model: same
@@ -254,7 +254,7 @@ def test_random_configurations_give_the_reference_schedule(block, monkeypatch, t
 
 def test_on_one_gpu_the_redundant_runs_are_what_costs(monkeypatch):
     """one stage (no pipeline): the reference policy spends every other pass of the target on a one-token run; policies 2 and 3
-    drop most of them.  The model is within 5 % of the measured one-GPU numbers for the reference policy (DESIGN.md §9)."""
+    drop most of them.  The model is within 5 % of the measured one-GPU numbers for the reference policy."""
     cfg = sim.default_config(n_stages=1, stage_us=10320.0, stage_tok_us=480.0, seed=3)
     kw = dict(n_draft=3, max_spec_runs=2, n_prompt=64, n_predict=192, n_ctx=2048)
     tps = {}

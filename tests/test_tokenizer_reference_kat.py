@@ -1,10 +1,10 @@
 """CPU-only: the reference's own tokenizer tests, run against this library.
 
-/root/reference/tests/test-tokenizer-0-{llama,falcon}.cpp hold known-answer vectors (text -> ids, made with the original
-SentencePiece / HF tokenizers) for the vocabularies shipped in /root/reference/models/ggml-vocab-{llama,falcon}.gguf;
+tests/test-tokenizer-0-{llama,falcon}.cpp hold known-answer vectors (text -> ids, made with the original
+SentencePiece / HF tokenizers) for the vocabularies shipped in models/ggml-vocab-{llama,falcon}.gguf;
 test-tokenizer-1-{llama,bpe}.cpp check round trips over every token and every codepoint.  The vectors are parsed out of
-the .cpp files where they lie and the vocabularies are opened in place (vocab_only: no GPU), so these tests run only in
-the container that has /root/reference.
+the .cpp files where they lie and the vocabularies are opened in place (vocab_only: no GPU), so these tests run only on
+a machine that has the reference's sources.
 """
 import ctypes as C
 import os
@@ -16,7 +16,7 @@ from tests.test_tokenizer_cpu import ROOT, open_vocab
 
 REFDIR = "/root/reference"
 pytestmark = pytest.mark.skipif(not os.path.exists(os.path.join(REFDIR, "models", "ggml-vocab-falcon.gguf")),
-                                reason="needs the vocabulary files under /root/reference/models")
+                                reason="needs the vocabulary files under the reference's models/")
 LIB = os.path.join(ROOT, "pipeinfer_b200", "libpipeinfer_b200.so")
 REF_LIB = os.path.join(ROOT, "oracle", "_ref", "libllama_ref.so")
 

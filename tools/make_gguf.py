@@ -1,13 +1,13 @@
 #!/usr/bin/env python
 """Write a random-init GGUF v3 file of a llama-arch model (TEST TOOLING, not product code).
 
-There is no network for checkpoints, so every model in BASELINE.json's configs is a seeded random
+There is no network for checkpoints, so every model of the benchmark is a seeded random
 initialisation of the named architecture.  Tensor names and hyper-parameter keys are the ones the
-reference loader reads (/root/reference/llama.cpp:2227-2276 hparams, :351-403 tensor tables,
+reference loader reads (llama.cpp:2227-2276 hparams, :351-403 tensor tables,
 :2756-2812 llama tensors).  The vocabulary is synthetic and character-level (see `synth_vocab`), so
 neither this script nor the tests need the reference's models/ggml-vocab-*.gguf.
 
-Two weight flavours (SURVEY.md §8d):
+Two weight flavours:
   iid     every 2-D weight ~ N(0, 0.02^2): target and draft disagree, acceptance ~ 0 (exercises cancel).
   bigram  token_embd[t] = g_t, output[pi(t)] = g_t for a fixed permutation pi, block weights scaled by
           --eps so the residual stream stays ~ g_t: both models predict pi(last token), so drafts get
@@ -32,7 +32,7 @@ CHAR0 = N_SPECIAL + N_BYTE   # first printable-character token (space == U+2581)
 
 def synth_vocab(n_vocab):
     """3 specials, 256 byte tokens, 95 single printable ASCII characters, then filler pieces that no
-    text can produce.  With it the reference SPM tokenizer (/root/reference/llama.cpp:5970-6110) maps a
+    text can produce.  With it the reference SPM tokenizer (llama.cpp:5970-6110) maps a
     prompt one character -> one token, so tests know the ids without running a tokenizer."""
     toks, scores, types = [], [], []
     for t, ty in (("<unk>", 2), ("<s>", 3), ("</s>", 3)):
