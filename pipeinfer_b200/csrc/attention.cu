@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(ATQ_THREADS, HD == 64 || ATQ_THREADS == 256 ? 
         for (int q = 0; q < HD / 16; q++) kpre[rd][q] = use ? kr[(q >> 1) * 4 + 2 * (q & 1) + hsel] : make_uint4(0, 0, 0, 0);
         lpre[rd] = i < n && !mrow[ic];
     }
-    // RoPE entries of this thread's first two rotation items (covers batches of up to 2 * 256 / half - 1 tokens)
+    // RoPE entries of this thread's first two rotation items (covers batches of up to 2 * ATQ_THREADS / half - 1 tokens)
     float2 cs_pre[2];
 #pragma unroll
     for (int it = 0; it < 2; it++) {
