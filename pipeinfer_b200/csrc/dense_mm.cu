@@ -263,11 +263,13 @@ __global__ void __launch_bounds__(256) mv_pair_kernel(mm_dev a, mm_dev b, bool x
 // is: k slots 2t, 2t + 1 and 2t + 8, 2t + 9 of product j stand for elements 8t + 4j .. + 3, and the lane reads the same eight elements of "its" token for B.
 // So no value passes through shared memory, an activation is rounded once per block, and a warp's weight bytes are all in flight together -- the first ones
 // before the launch wait where W is a weight, which nothing writes (not for the key and value rows that an attention gathers and passes as W: pib_mm.w_made).
+// The tensor core cuts what falls off its accumulator, always towards zero, so every product of 16 k starts from none and is added up here, rounded to nearest: one
+// accumulator for all of a warp's k drifted (error against 64 bits 2.4e-7 at K = 2048, 2.1e-6 at 16384; now 8.5e-8 and 1.7e-7, fused multiply-adds 8.0e-8 and 1.7e-7).
 // What bounds it: the weights' way from memory.  The form it replaces (a warp per weight row, mv_rows_kernel) rounded every activation for every weight row: at
-// four tokens 32 conversions per 16 bytes of weights.
+// four tokens 32 conversions per 16 bytes of weights (5632 x 2048, 1 / 4 / 16 tokens: 5.8 / 6.1 / 9.1 us, at four 21.7 before).
 #define MVM_U 4                      // 32-k chunks a warp has in flight
 __device__ __forceinline__ void mvm_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ uint32_t mvm_pack(float lo, float hi) {
@@ -314,8 +316,11 @@ __device__ __forceinline__ void mvm_body(const mm_dev & a, int z, int tile, int 
             for (int j = 0; j < NT; j++) {
                 float4 p = make_float4(0.f, 0.f, 0.f, 0.f), q = p;
                 if (in && has[j]) { p = *reinterpret_cast<const float4 *>(x[j] + (c + u) * 32); q = *reinterpret_cast<const float4 *>(x[j] + (c + u) * 32 + 4); }
-                mvm_mma(acc[j], (uint32_t) ra[u].x, (uint32_t) rb[u].x, (uint32_t) ra[u].y, (uint32_t) rb[u].y, mvm_pack(p.x, p.y), mvm_pack(p.z, p.w));
-                mvm_mma(acc[j], (uint32_t) ra[u].z, (uint32_t) rb[u].z, (uint32_t) ra[u].w, (uint32_t) rb[u].w, mvm_pack(q.x, q.y), mvm_pack(q.z, q.w));
+                float c4[4] = { 0.f, 0.f, 0.f, 0.f }, d4[4] = { 0.f, 0.f, 0.f, 0.f };
+                mvm_mma(c4, (uint32_t) ra[u].x, (uint32_t) rb[u].x, (uint32_t) ra[u].y, (uint32_t) rb[u].y, mvm_pack(p.x, p.y), mvm_pack(p.z, p.w));
+                mvm_mma(d4, (uint32_t) ra[u].z, (uint32_t) rb[u].z, (uint32_t) ra[u].w, (uint32_t) rb[u].w, mvm_pack(q.x, q.y), mvm_pack(q.z, q.w));
+#pragma unroll
+                for (int e = 0; e < 4; e++) acc[j][e] += c4[e] + d4[e];
             }
         }
     }

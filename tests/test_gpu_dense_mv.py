@@ -37,3 +37,15 @@ def test_weight_rows_of_the_launch_in_front(M, N, K):
     for _ in range(3):
         lib.check(L.pib_dense_mm_made_host(bits.ctypes.data, x.ctypes.data, y.ctypes.data, M, N, K))
         assert (np.abs(y - X @ W.T) <= (K + 8) * 2.0 ** -23 * (np.abs(X) @ np.abs(W).T)).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(3, 32, 8192), (12, 48, 16384)])
+def test_sums_do_not_drift(M, N, K):
+    """long sums of one sign: the tensor core cuts towards zero, per 16 k and by less than an ulp of their sum, 2^-23; what is added up outside is rounded to nearest.
+    So the error's mean stays within 2^-23 for any K (one accumulator for all of a warp's k was off by 2e-6 at 16384)"""
+    rng = np.random.default_rng(M + K)
+    W, X = bf16_round(rng.uniform(0.5, 1, (N, K))), bf16_round(rng.uniform(0.5, 1, (M, K)))
+    got = mm(W, X, M, N, K).reshape(M, N).astype(np.float64)
+    rel = got / (X.astype(np.float64) @ W.astype(np.float64).T) - 1
+    print("K %d: mean relative error %.2g, mean size %.2g" % (K, rel.mean(), np.abs(rel).mean()))
+    assert abs(rel.mean()) < 2.0 ** -23
