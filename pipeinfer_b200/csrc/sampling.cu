@@ -16,7 +16,7 @@
 // A row is divided over P blocks of a thread-block cluster (contiguous slices of the vocabulary); each finds the best eight and, once the cluster knows the maximum,
 // the exponentials' sum of its slice, and the first block merges the P sorted lists and sums through distributed shared memory.
 // What bounds it: chains of block-wide rounds, so a round is two warp reductions in hardware (redux on order-preserving keys) and one barrier, and a thread looks for its
-// best two only.  One row of 32 000: 27 -> 14 us, 256 rows: 40, 1 512 rows of 8 000: 42 (with eight-place lists sorted per thread and shuffles 99).
+// best two only.  One row of 32 000: 27 -> 14 us, 256 rows: 44 -> 32, 1 512 rows of 8 000: 106 -> 39 (before: a block per row, eight-place lists sorted per thread).
 #define SMP_THREADS 256
 #define SMP_TOPK    8
 #define SMP_PARTS   8
@@ -149,9 +149,11 @@ __global__ void __launch_bounds__(SMP_THREADS) sample_topk_kernel(float * __rest
 int pib_sample_topk(float * logits_dev, int n_rows, int n_vocab, const int32_t * bias_ids_dev, const float * bias_val_dev,
                     int n_bias, void * out_dev, const uint8_t * desc, const int * cancel, cudaStream_t st) {
     (void) desc;
-    // parts while the machine has room for the blocks and a thread has more than four elements
-    int P = 1;
-    while (P < SMP_PARTS && (long long) n_rows * P * 2 <= 8LL * pib_num_sms() && n_vocab >= P * 8 * SMP_THREADS) P <<= 1;
+    // Parts while a thread has more than four elements and all blocks run at once: three per SM, less a sixteenth that packing clusters loses (us of 2 / 4 / 8 parts of 32 000
+    // values: 48 rows 15.5 / 13.1 / 13.3, 56 15.5 / 15.5 / 22.7, 100 20.7 / 15.7 / 33.5, 148 22.9 / 27.5 / 45.2).  However many rows there are, long ones need several
+    // blocks to have enough loads in flight (256 rows of 128 000, 1 / 2 / 4 parts: 203 / 115 / 100; of 65 000 57 / 52 / 56; of 32 000 32 / 35 / 40).
+    int P = n_vocab > 96000 ? 4 : n_vocab > 48000 ? 2 : 1;
+    while (P < SMP_PARTS && 16LL * n_rows * P * 2 <= 45LL * pib_num_sms() && n_vocab >= P * 8 * SMP_THREADS) P <<= 1;
     if (P > 1) pib_launch_cluster(sample_topk_kernel, dim3((unsigned) n_rows, (unsigned) P), dim3(SMP_THREADS), dim3(1, (unsigned) P, 1), 0, st, logits_dev, n_vocab, bias_ids_dev, bias_val_dev, n_bias,
                                   (pib_row_result *) out_dev, cancel);
     else       pib_launch(sample_topk_kernel, dim3((unsigned) n_rows), dim3(SMP_THREADS), 0, st, logits_dev, n_vocab, bias_ids_dev, bias_val_dev, n_bias, (pib_row_result *) out_dev, cancel);

@@ -33,7 +33,8 @@ def top8(L, f, x, ids, val):
 
 
 @pytest.mark.parametrize("rows,V,kind", [(1, 5, "plain"), (2, 8, "plain"), (3, 255, "ties"), (1, 4095, "plain"), (1, 4096, "ties"), (4, 4097, "plain"), (1, 8192, "inf"), (16, 32000, "ties"), (1, 32768, "plain"),
-                                         (1, 32769, "plain"), (2, 65000, "inf"), (1, 151000, "ties"), (300, 1000, "ties"), (700, 9000, "plain")])
+                                         (1, 32769, "plain"), (2, 65000, "inf"), (1, 151000, "ties"), (300, 1000, "ties"), (700, 9000, "plain"), (26, 32000, "ties"),
+                                         (27, 32000, "plain"), (52, 20000, "plain"), (53, 20000, "ties"), (104, 9000, "plain"), (209, 5000, "plain"), (120, 49000, "ties"), (110, 97000, "plain")])
 def test_topk(fn, rows, V, kind):
     L, f = fn
     rng = np.random.default_rng(rows + V)
