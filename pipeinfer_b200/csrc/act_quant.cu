@@ -272,8 +272,12 @@ static int launch_aq(int wtype, const float * x, const float * x2, int x2_per_ro
     // a warp per super-block or 32-element block: a warp that takes several takes them one after the other, and each is a chain of a load, a reduction and stores
     // (K = 5632, silu: 5.1 us with floor(22 / 8) CTAs per row; Q8_0 blocks of K = 4096, norm: 6.4 us with four blocks per warp)
     const int64_t units = wtype == PIB_TYPE_Q4_K ? K / PIB_QK_K : K / PIB_QK;
-    const int     parts = (int) max((int64_t) 1, min((int64_t) 32, (units + AQ_THREADS / 32 - 1) / (AQ_THREADS / 32)));
-    const dim3    grid(b, parts);
+    int64_t parts = (units + AQ_THREADS / 32 - 1) / (AQ_THREADS / 32);
+    // every CTA forms the row's norm for itself: no more of them than run at once, three per SM (16 rows, norm, Q8_0 blocks: K = 8192 with 24 / 32 CTAs per row 3.9 / 5.1 us,
+    // 14848 5.4 / 7.6), down to one per 32 blocks
+    if (wtype != PIB_TYPE_Q4_K) parts = min(parts, max((int64_t) (3 * pib_num_sms() / b), units / 32));
+    parts = max((int64_t) 1, min((int64_t) 32, parts));
+    const dim3    grid(b, (unsigned) parts);
 #define AQ_GO(Q8K, XH) pib_launch(act_quant_kernel<Q8K, PRO, XH>, grid, dim3(AQ_THREADS), 0, st, x, x2, x2_per_row, eps, K, qs, d, bs, b8, qp, ql, sb, q6, b6, vout, lut, addend, sum_out, cancel, \
                                xstride, bias, addend2, (__half *) xhat)
     constexpr bool PROMPT = PRO == PRO_PLAIN || PRO == PRO_RMSNORM || PRO == PRO_SILU_MUL;
