@@ -16,7 +16,7 @@
 // A row is divided over P blocks of a thread-block cluster (contiguous slices of the vocabulary); each finds the best eight and, once the cluster knows the maximum,
 // the exponentials' sum of its slice, and the first block merges the P sorted lists and sums through distributed shared memory.
 // What bounds it: chains of block-wide rounds, so a round is two warp reductions in hardware (redux on order-preserving keys) and one barrier, and a thread looks for its
-// best two only.  One row of 32 000: 27 -> 14 us, 256 rows: 44 -> 32, 1 512 rows of 8 000: 106 -> 39 (before: a block per row, eight-place lists sorted per thread).
+// best two only.  One row of 32 000: 25 -> 10 us, 256 rows: 44 -> 32, 1 512 rows of 8 000: 106 -> 39 (before: a block per row, eight-place lists sorted per thread).
 #define SMP_THREADS 256
 #define SMP_TOPK    8
 #define SMP_PARTS   8
