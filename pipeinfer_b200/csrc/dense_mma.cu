@@ -1,6 +1,7 @@
 // dense_mma.cu -- the dense matmul on the tensor cores: Y[m][n] = sum_k bf16(X[m][k]) * W[n][k], W bfloat16 rows, fp32 accumulation.
 //
-// More than DT_ROWS_MAX rows (prompt portions): dense_tc_kernel, tcgen05.  A CTA owns 128 weight rows x NB tokens of one problem z:
+// More than DT_ROWS_MAX rows (prompt portions), tcgen05.  One problem: pairs of SMs (dense_pair.cu).  Several problems or rows grouped by expert: dense_tc_kernel, whose CTA owns
+// 128 weight rows x NB tokens of one problem z:
 //   warp 0       one lane streams both operands by TMA (cp.async.bulk.tensor.3d, 128-byte swizzle): the weight tile [128 n][64 k] and
 //                the activation tile [NB m][64 k] of every k-step land in one stage and complete one mbarrier
 //   warp 1       allocates tensor memory; an elected lane issues tcgen05.mma.cta_group::1.kind::f16 (bf16 x bf16 -> fp32, M 128, N NB, 4 x K 16 per
@@ -258,11 +259,15 @@ int pib_dense_mm_tc(const pib_mm & a, cudaStream_t st) {
     // the token tile: as wide as the rows of one problem allow (grouped problems: the average share of an expert)
     const int per = grouped ? (a.M + a.Z - 1) / a.Z : a.M;
     const int NB = per <= 32 ? 32 : per <= 64 ? 64 : 128;
+    int pair = 0, shares = 1;
+    if (!grouped && a.Z == 1) pib_dense_pair_plan(a.M, a.N, a.K, &pair, &shares);
     CUtensorMap wmap, xmap;
+    const uint32_t xbox = (uint32_t) (pair ? pair / 2 : NB);
     int rc = pib_tma_map3(&wmap, a.W, (uint64_t) a.K, (uint64_t) a.N, (uint64_t) a.Z, (uint64_t) a.ldw * 2, (uint64_t) (a.Z > 1 ? a.wz : (int64_t) a.N * a.ldw) * 2, DT_BM);
-    if (rc == PIB_OK && a.x_bf16) rc = pib_tma_map3(&xmap, a.X, (uint64_t) a.K, (uint64_t) a.M, (uint64_t) a.Z, (uint64_t) a.ldx * 2, (uint64_t) (a.Z > 1 ? a.xz : (int64_t) a.M * a.ldx) * 2, (uint32_t) NB);
-    else if (rc == PIB_OK) rc = pib_tma_map3(&xmap, sc->xs, (uint64_t) Kp, (uint64_t) a.M, (uint64_t) Zs, (uint64_t) Kp * 2, (uint64_t) a.M * Kp * 2, (uint32_t) NB);
+    if (rc == PIB_OK && a.x_bf16) rc = pib_tma_map3(&xmap, a.X, (uint64_t) a.K, (uint64_t) a.M, (uint64_t) a.Z, (uint64_t) a.ldx * 2, (uint64_t) (a.Z > 1 ? a.xz : (int64_t) a.M * a.ldx) * 2, xbox);
+    else if (rc == PIB_OK) rc = pib_tma_map3(&xmap, sc->xs, (uint64_t) Kp, (uint64_t) a.M, (uint64_t) Zs, (uint64_t) Kp * 2, (uint64_t) a.M * Kp * 2, xbox);
     if (rc != PIB_OK) return rc;
+    if (pair) return pib_dense_pair(a, wmap, xmap, pair, shares, sc->err, st);
     switch (NB) {
         case 32:  return dt_launch<32>(a, wmap, xmap, grouped ? 0 : 1, sc->err, st);
         case 64:  return dt_launch<64>(a, wmap, xmap, grouped ? 0 : 1, sc->err, st);

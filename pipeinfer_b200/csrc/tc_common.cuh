@@ -77,3 +77,6 @@ __host__ __device__ constexpr uint32_t dt_idesc(int M, int N) { return (1u << 4)
 
 // dense_mma.cu: a 3-D bfloat16 tensor map {d0, d1, d2} with boxes of 64 x box1 x 1 and 128-byte swizzle (strides in bytes)
 int   pib_tma_map3(CUtensorMap * map, const void * base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s1_bytes, uint64_t s2_bytes, uint32_t box1);
+// dense_pair.cu: the dense matmul on pairs of SMs; tile width and shares of K for M rows and N outputs, and the launch for maps with boxes of 128 weight rows and half a tile of X rows
+void  pib_dense_pair_plan(int M, int N, int K, int * nb, int * shares);
+int   pib_dense_pair(const pib_mm & a, const CUtensorMap & wmap, const CUtensorMap & xmap, int NB, int shares, int * err, cudaStream_t st);

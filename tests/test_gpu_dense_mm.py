@@ -51,6 +51,24 @@ def test_plain(M, N, K):
     np.testing.assert_allclose(got32, ref32, rtol=1e-5, atol=3e-6 * np.sqrt(K))
 
 
+@pytest.mark.parametrize("M,N,K,epi", [(17, 1, 16, 0), (31, 255, 128, 0), (32, 257, 136, 1), (33, 256, 1024, 0), (65, 300, 2056, 1), (255, 256, 120, 0), (257, 512, 5632, 0), (700, 255, 264, 1),
+                                       (40, 5000, 512, 0), (1000, 8448, 256, 0), (2050, 4100, 64, 0), (4096, 5121, 40, 1)])
+def test_tiles_of_sm_pairs(M, N, K, epi):
+    """edges of the pairs' tiles (256 weight rows, 32 .. 256 tokens, k-steps of 128), K in shares, and more tiles than two per pair (accumulators in turn);
+    fp32 accumulation of bfloat16 products: |error| <= K * 2^-23 * sum |x w|, here against the largest row"""
+    rng = np.random.default_rng(M + N + K)
+    W = bf16_round(rng.standard_normal((N, K)))
+    X = bf16_round(rng.standard_normal((M, K)))
+    ref = X @ W.T
+    bound = np.abs(X) @ np.abs(W).T * 2.0 ** -23 * K + 1e-30
+    if epi:
+        z = np.maximum(ref, 0.0)
+        bound = (2 * z + bound) * bound + 2.0 ** -23 * z * z
+        ref = z * z
+    got = mm(W, X, M, N, K, epi=epi).reshape(M, N)
+    assert (np.abs(got - ref) <= bound).all()
+
+
 @pytest.mark.parametrize("M,F,K", [(1, 225, 200), (2, 65, 72), (7, 128, 1024), (16, 100, 104), (17, 196, 184), (100, 65, 200), (300, 500, 520), (1100, 228, 200)])
 def test_paired_gated_epilogue(M, F, K):
     """weight rows interleaved (gate i, linear part i): output i = a sigmoid(1.702 a) (b + 1), a = min(g, limit), b = clamp(u, -limit, limit) -- in the row
