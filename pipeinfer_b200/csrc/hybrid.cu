@@ -152,6 +152,22 @@ static int grow_attn_mm(pib_context * c, size_t kw, size_t kx, int q_rows, int s
     return PIB_OK;
 }
 
+// the operands of the attention on chip: keys, values, queries (in the same buffers)
+static int grow_flash(pib_context * c, size_t kb, size_t vb, size_t qb) {
+    pib_hybrid_ctx * x = c->hy;
+    auto grow = [&](void ** p, size_t * cap, size_t need) {
+        if (need <= *cap) return true;
+        cudaStreamSynchronize(c->stream);
+        if (*p) cudaFree(*p);
+        *cap = need + need / 4;
+        if (cudaMalloc(p, *cap) != cudaSuccess) { cudaGetLastError(); *p = nullptr; *cap = 0; return false; }
+        return true;
+    };
+    if (grow(&x->am_kb, &x->am_kb_cap, kb) && grow(&x->am_vt, &x->am_vt_cap, vb) && grow((void **) &x->am_q, &x->am_q_cap, qb)) return PIB_OK;
+    pib_set_error("decode: out of memory for the attention's operands");
+    return PIB_ERR_NOMEM;
+}
+
 static int grow_chunk(pib_context * c, size_t need) {
     pib_hybrid_ctx * x = c->hy;
     if (need <= x->chunk_cap) return PIB_OK;
@@ -224,6 +240,10 @@ static int grow_scratch(pib_context * c, int T) {
 #define MM_ATTN_MIN_ROW 192
 #define MM_ATTN_BLOCK   512
 #define FLASH_ATTN_BLOCK 4096     // the form that keeps its scores on chip
+#define FLASH_ATTN_COLS  16384    // key columns laid out for one launch of it
+// Shorter portions go to the per-token kernel (two 2048-wide layers, us a prompt call, this form / per token: one sequence of 32 tokens 260 / 251, 48 274 / 282, 100 299 / 325;
+// three 340 / 325, 359 / 375, 406 / 542; eight 506 / 540, 540 / 630, 696 / 1075).  More than the 16 tokens of a captured step, whose portions may change.
+#define FLASH_ATTN_MIN_LEN 48
 // a recurrence's matmul form works through a segment in blocks of at most MM_SCAN_BLOCK tokens (its operands take a few hundred MB per block)
 #define MM_SCAN_BLOCK   2048
 struct pib_hseg { int start, len, seq, slot; bool fresh; };
@@ -334,29 +354,54 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
         const int H = L.heads * L.maps, G = L.kv_heads * L.maps, D = L.dim, V = L.vdim;      // query rows and key heads: one per map
         const double keys = key_pairs(L.window, L.mask, L.keep);
         const bool mm_ok = !exact && D % 8 == 0 && D >= 16 && V >= 16 && attn_mm_enabled();
+        const bool flash = mm_ok && pib_flash_attention_fits(L);                                           // no score rows in memory: shorter portions, longer blocks
+        const int  min_len = flash ? FLASH_ATTN_MIN_LEN : MM_ATTN_MIN_LEN;
         bool any_mm = false, any_simt = false;
-        for (const pib_hseg & g : segs) { if (mm_ok && g.len >= MM_ATTN_MIN_LEN) any_mm = true; else any_simt = true; }
+        for (const pib_hseg & g : segs) { if (mm_ok && g.len >= min_len) any_mm = true; else any_simt = true; }
         if (any_simt)
             RC(HK_KVATTN, 2.0 * keys * H * (D + V), 4.0 * keys * G * (D + V) + 4.0 * Td * H * (D + V),
-               pib_kv_attention(q, L, B, cache, row, x->cellmap, (int) c->n_ctx, out, any_mm ? B.mmflag : nullptr, st));
+               pib_kv_attention(q, L, B, cache, row, x->cellmap, (int) c->n_ctx, out, any_mm ? (flash ? B.faflag : B.mmflag) : nullptr, st));
+        // portions of all segments gathered into launches of up to FLASH_ATTN_COLS key columns
+        std::vector<pib_attn_block> blocks;
+        double bl_pairs = 0, bl_keys = 0, bl_tok = 0;
+        auto launch = [&]() -> int {
+            if (blocks.empty()) return PIB_OK;
+            long long cols = 0, rows = 0;
+            size_t kb = 0, vb = 0;
+            pib_flash_attention_place(blocks, L.heads / L.kv_heads, &cols, &rows);
+            const size_t qb = pib_flash_attention_bytes(L, cols, rows, &kb, &vb);
+            if ((rc = grow_flash(c, kb, vb, qb)) != PIB_OK) return rc;
+            RC(HK_FLASH, 2.0 * H * bl_pairs * (D + V), 4.0 * bl_keys * G * (D + V) + 4.0 * bl_tok * H * (D + V),
+               pib_flash_attention(q, L, blocks, (int) cols, (int) rows, cache, row, x->cellmap, (int) c->n_ctx, x->am_kb, x->am_vt, x->am_q, out, st));
+            nk++;
+            blocks.clear();
+            bl_pairs = bl_keys = bl_tok = 0;
+            return PIB_OK;
+        };
         for (const pib_hseg & g : segs) {
-            if (!mm_ok || g.len < MM_ATTN_MIN_LEN) continue;
-            const bool flash = pib_flash_attention_fits(L);                                                 // no score rows in memory: longer blocks
+            if (!mm_ok || g.len < min_len) continue;
             const int block = flash ? FLASH_ATTN_BLOCK : MM_ATTN_BLOCK, nb = (g.len + block - 1) / block, per = (g.len + nb - 1) / nb;      // blocks of equal size: none is left with a handful of rows
             for (int o = 0; o < g.len; o += per) {
                 const int nq = std::min(per, g.len - o), p0 = B_pos_host[g.start + o];
                 int j0 = L.mask == PIB_MASK_CHUNK ? p0 - p0 % L.window : std::max(0, p0 - L.window + 1), n_front = 0;
                 if (L.keep > 0) { if (j0 <= L.keep) j0 = 0; else n_front = L.keep; }        // kept first positions: columns of their own in front of the window's
                 const int NK = n_front + p0 + nq - j0;
-                if ((rc = grow_attn_mm(c, (size_t) G * std::max(D, V), (size_t) 3 * G * D, nq * H, flash ? 0 : nq * H, NK, (size_t) std::max(6 * D, 4 * V))) != PIB_OK) return rc;
                 double pairs = 0;                                            // (token, key) pairs of the block, for the profile: the two products the attention is
                 for (int i = 0; i < nq; i++) pairs += L.mask == PIB_MASK_CHUNK ? (p0 + i) % L.window + 1 : std::min<int64_t>(p0 + i + 1, (int64_t) L.window + L.keep);
-                RC(flash ? HK_FLASH : HK_KVATTN_MM, 2.0 * H * pairs * (D + V), 4.0 * NK * G * (D + V) + 4.0 * nq * H * (D + V),
+                if (flash) {
+                    if (!blocks.empty() && ((int) blocks.size() == pib_flash_attention_max() || bl_keys + NK > FLASH_ATTN_COLS) && (rc = launch()) != PIB_OK) return rc;
+                    blocks.push_back({ nq, g.start + o, p0, j0, n_front, NK, g.slot, g.len < MM_ATTN_MIN_LEN ? 2 : 1, 0, 0, 0, 0 });
+                    bl_pairs += pairs; bl_keys += NK; bl_tok += nq;
+                    continue;
+                }
+                if ((rc = grow_attn_mm(c, (size_t) G * std::max(D, V), (size_t) 3 * G * D, nq * H, nq * H, NK, (size_t) std::max(6 * D, 4 * V))) != PIB_OK) return rc;
+                RC(HK_KVATTN_MM, 2.0 * H * pairs * (D + V), 4.0 * NK * G * (D + V) + 4.0 * nq * H * (D + V),
                    pib_kv_attention_mm(q, L, B, cache, row, x->cellmap + (size_t) g.slot * c->n_ctx, g.start + o, nq, p0, j0, n_front, NK, x->am_kb, x->am_vt, x->am_q, x->am_s,
                                        x->am_p, out, st));
-                nk += flash ? 2 : 5;
+                nk += 5;
             }
         }
+        if ((rc = launch()) != PIB_OK) return rc;
         return PIB_OK;
     };
     // windowed attention over cached key / value heads: projections, convolution, norms + value mixing + cache write, attention, output
@@ -835,8 +880,8 @@ int pib_hybrid_decode_start(pib_context * c, int n_tokens, const int32_t * token
         }
         x->slots.len[(size_t) g.slot] += g.len;
     }
-    // bookkeeping: [tok | pos | cell | slot | seg] x T, then [seg_start | seg_len | seg_slot] x S
-    const int S = (int) segs.size(), words = 6 * T + 3 * S;
+    // bookkeeping: [tok | pos | cell | slot | seg | mmflag | faflag] x T, then [seg_start | seg_len | seg_slot] x S
+    const int S = (int) segs.size(), words = 7 * T + 3 * S;
     if (words > x->meta_cap) {
         cudaStreamSynchronize(st);
         for (auto & g : c->graphs) if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
@@ -857,8 +902,8 @@ int pib_hybrid_decode_start(pib_context * c, int n_tokens, const int32_t * token
     int32_t * mh = x->meta_host[ring];
     for (int sgi = 0; sgi < S; sgi++) {
         const pib_hseg & g = segs[(size_t) sgi];
-        for (int i = g.start; i < g.start + g.len; i++) { mh[3 * T + i] = g.slot; mh[4 * T + i] = sgi; mh[5 * T + i] = g.len >= MM_ATTN_MIN_LEN ? 1 : 0; }
-        mh[6 * T + sgi] = g.start; mh[6 * T + S + sgi] = g.len; mh[6 * T + 2 * S + sgi] = g.slot;
+        for (int i = g.start; i < g.start + g.len; i++) { mh[3 * T + i] = g.slot; mh[4 * T + i] = sgi; mh[5 * T + i] = g.len >= MM_ATTN_MIN_LEN ? 1 : 0; mh[6 * T + i] = g.len >= FLASH_ATTN_MIN_LEN ? 1 : 0; }
+        mh[7 * T + sgi] = g.start; mh[7 * T + S + sgi] = g.len; mh[7 * T + 2 * S + sgi] = g.slot;
     }
     memcpy(mh, token, (size_t) T * 4);
     memcpy(mh + T, pos, (size_t) T * 4);
@@ -867,7 +912,7 @@ int pib_hybrid_decode_start(pib_context * c, int n_tokens, const int32_t * token
     cudaEventRecord(x->meta_ev[ring], st);
     c->h2d_bytes += (size_t) words * 4;
     const int32_t * md = x->meta_dev;
-    pib_hbatch B = { md, md + T, md + 2 * T, md + 3 * T, md + 4 * T, md + 5 * T, md + 6 * T, md + 6 * T + S, md + 6 * T + 2 * S, T, S };
+    pib_hbatch B = { md, md + T, md + 2 * T, md + 3 * T, md + 4 * T, md + 5 * T, md + 6 * T, md + 7 * T, md + 7 * T + S, md + 7 * T + 2 * S, T, S };
     run->in_use = true; run->batch_id = batch_id; run->n_tokens = T; run->failed = false; run->has_walk = false;
     c->tree_pending.n_branches = 0;
     cudaMemcpyAsync(c->cancel_table, c->run_id_host + run->id, sizeof(int), cudaMemcpyHostToDevice, st);

@@ -282,6 +282,7 @@ pib_weight * pib_dense_upload(int type, const void * host, int64_t N, int64_t K)
 struct pib_hbatch {                  // device view of one batch's bookkeeping
     const int32_t * tok, * pos, * cell, * slot, * seg;       // [T]
     const int32_t * mmflag;                                   // [T] 1: the token's attention runs in the matmul form (long portions, served mode)
+    const int32_t * faflag;                                   // [T] 1: ... on the form that keeps its scores on chip (flash_attn.cu), where the layer has heads for it
     const int32_t * seg_start, * seg_len, * seg_slot;         // [S]
     int T, S;
 };
@@ -330,7 +331,15 @@ int pib_kv_attention_mm(const pib_kv_query & q, const pib_hlayer & L, const pib_
                         void * Kb, void * Vt, float * Qc, float * S, void * P, float * out, cudaStream_t st);
 // flash_attn.cu: the same for heads of up to 128 coordinates, scores and weights in tensor memory
 bool pib_flash_attention_fits(const pib_hlayer & L);
-int pib_flash_attention(const pib_kv_query & q, const pib_hlayer & L, int t0, int nq, int p0, int j0, int n_front, int NK, const void * Kb, const void * Vt, const void * Qc, float * out, cudaStream_t st);
+struct pib_attn_block {              // consecutive tokens of one segment: batch rows t0 .., positions p0 ..; NK key columns: n_front kept first positions, then j0, j0 + 1, ...
+    int nq, t0, p0, j0, n_front, NK, slot, v_parts;           // v_parts 2: values enter with the remainder of their rounding
+    int cols, row_blocks, col0, row0;                         // where its operands lie (pib_flash_attention_place)
+};
+void pib_flash_attention_place(std::vector<pib_attn_block> & blocks, int rep, long long * cols, long long * rows);
+size_t pib_flash_attention_bytes(const pib_hlayer & L, long long cols, long long rows, size_t * k_bytes, size_t * v_bytes);      // operand buffers; the queries' is returned
+int pib_flash_attention_max();                                // portions in a launch
+int pib_flash_attention(const pib_kv_query & q, const pib_hlayer & L, const std::vector<pib_attn_block> & blocks, int C, int R, const float * cache, int cache_row, const int32_t * cellmap, int n_ctx,
+                        void * Kb, void * Vt, void * Qc, float * out, cudaStream_t st);
 int pib_token_shift(const float * h, const float * mu, int n_mix, const pib_hbatch & b, float * state, size_t state_stride, size_t shift_off, int W, float * mixes, cudaStream_t st);
 int pib_rows_act(float * z, int ld, int n, int T, int op, const float * bias, cudaStream_t st);           // op 0: tanh; 1: exp(-exp(z + bias))
 int pib_delta_prep(float * cv, int ldc, const pib_hlayer & L, const float * proj, int ldp, int b_off, int a_off, float * bg, int T, cudaStream_t st);

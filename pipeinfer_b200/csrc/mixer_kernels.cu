@@ -281,8 +281,7 @@ int pib_kv_attention(const pib_kv_query & q, const pib_hlayer & L, const pib_hba
 // scores [nq * rep][NK] = (scale * queries of the rep heads that share g) x keys^T, the masked softmax over each row, outputs = weights x
 // values.  Scores keep fp32 accuracy on bfloat16 tensor cores: a number enters as its bfloat16 part and the remainder of that rounding,
 // queries as rows [hi | lo | hi], keys as rows [hi | hi | lo] (3 D wide: hi.hi + lo.hi + hi.lo), and a weight enters the value matmul as
-// [hi | lo] against the values twice side by side.  Heads of up to 128 coordinates take these operands to flash_attn.cu, which keeps scores and weights on chip; others
-// go through score rows in memory.  These kernels prepare the operands -- keys [G][NKp][3 D], values transposed
+// [hi | lo] against the values twice side by side, through score rows in memory.  (Heads of up to 128 coordinates: flash_attn.cu, which keeps scores and weights on chip.)  These kernels prepare the operands -- keys [G][NKp][3 D], values transposed
 // [G][V][2 NKp], query rows [G][nq * rep][3 D], all bfloat16 -- and put the outputs [G][nq * rep][V] back in token order.
 __device__ __forceinline__ void mk_split(float x, __nv_bfloat16 & hi, __nv_bfloat16 & lo) { hi = __float2bfloat16_rn(x); lo = __float2bfloat16_rn(x - __bfloat162float(hi)); }
 // columns [0, n_front) are positions 0 .. n_front - 1, the columns behind them positions j0, j0 + 1, ...
@@ -371,7 +370,6 @@ int pib_kv_attention_mm(const pib_kv_query & q, const pib_hlayer & L, const pib_
     CKL();
     pib_launch(kv_query_rows_kernel, dim3((unsigned) nq), dim3(256), (size_t) 0, st, q.q, q.ldq, (__nv_bfloat16 *) Qc, H, maps, rep, nq, D, t0, L.scale);
     CKL();
-    if (pib_flash_attention_fits(L)) return pib_flash_attention(q, L, t0, nq, p0, j0, n_front, NK, Kb, Vt, Qc, out, st);
     pib_mm a;
     a.W = Kb; a.w_made = 1; a.wtype = PIB_TYPE_BF16; a.ldw = 3 * D; a.wz = (int64_t) NKp * 3 * D; a.X = Qc; a.ldx = 3 * D; a.xz = (int64_t) M * 3 * D; a.x_bf16 = 1;
     a.Y = S; a.ldy = NKp; a.yz = (int64_t) M * NKp; a.M = M; a.N = NK; a.K = 3 * D; a.Z = GK;

@@ -415,6 +415,29 @@ def test_long_portions_take_the_matmul_forms(tmp_path, name):
     s.close()
 
 
+@pytest.mark.parametrize("name", ["wide_heads", "far_keys"])
+def test_portions_of_many_lengths_in_one_batch(tmp_path, name):
+    """served mode: one launch takes the portions of all sequences, around the shortest it takes, where values stop entering in two parts, at the edges of its key tiles and of its
+    row blocks; continued portions (keys of earlier batches in front), beside decoded tokens; and as many portions as fit a launch"""
+    cfg = CONFIGS[name]()
+    W = O.random_weights(cfg, 29)
+    lens = [47, 48, 49, 63, 64, 65, 127, 128, 129, 1, 200]
+    seqs = [tokens(cfg, 2 * n + 2, 40 + i) for i, n in enumerate(lens)]
+    refs = [oracle_logits(cfg, W, t) for t in seqs]
+    s = Served(tmp_path, cfg, W, float32=False, n_ctx=2048, slots=16)
+    a = s.step([(i, t[:n]) for i, (t, n) in enumerate(zip(seqs, lens))])
+    b = s.step([(i, t[n:]) for i, (t, n) in reversed(list(enumerate(zip(seqs, lens))))])
+    s.close()
+    for i, ref in enumerate(refs):
+        assert close16(row_err(np.concatenate([a[i], b[i]]), ref)), lens[i]
+    many = [tokens(cfg, 47 + i % 3, 80 + i) for i in range(32)]
+    s = Served(tmp_path, cfg, W, float32=False, n_ctx=1792, slots=32)
+    got = s.step(list(enumerate(many)))
+    s.close()
+    for i, t in enumerate(many):
+        assert close16(row_err(got[i], oracle_logits(cfg, W, t))), i
+
+
 @pytest.mark.parametrize("float32", [True, False])
 def test_medium_model_long_prompt_cuts_and_batches(tmp_path, float32):
     cfg = CONFIGS["medium"]()
