@@ -458,7 +458,7 @@ int pib_dense_mm(const pib_mm & a, cudaStream_t st) {
         const int rc = pib_dense_mm_tc(a, st);
         if (rc != PIB_ERR_UNSUPP) return rc;
     }
-    if (a.x_bf16) { pib_set_error("dense matmul: bfloat16 activations need the tensor-core path (more than 16 rows, strides multiples of 8)"); return PIB_ERR_UNSUPP; }
+    if (a.x_bf16 || a.y_bf16) { pib_set_error("dense matmul: bfloat16 activations need the tensor-core path (more than 16 rows, strides multiples of 8)"); return PIB_ERR_UNSUPP; }
     mm_dev d = { a.W, a.ldw, a.wz, a.X, a.ldx, a.xz, a.xrows, a.xdiv < 1 ? 1 : a.xdiv, a.Y, a.ldy, a.yz, a.M, a.N, a.K, a.zrange, a.e0, a.e1, a.zlist, a.Y2, a.ld2, a.Y2 ? a.n2 : 0x7fffffff, a.rows2, a.w_made };
     if (a.wtype == PIB_TYPE_F32 && a.exact && !a.Y2 && a.N <= 128 && a.M > MV_MAXB && a.Z == 1 && !a.xrows && !a.zrange && a.epi == PIB_EPI_NONE) {
         const int  NB = a.N <= 8 ? 8 : a.N <= 16 ? 16 : 24;

@@ -243,7 +243,12 @@ static int dt_launch(const pib_mm & a, const CUtensorMap & wmap, const CUtensorM
 
 static bool dt_enabled() { static const int on = getenv("PIB_DENSE_TC") ? atoi(getenv("PIB_DENSE_TC")) : 1; return on != 0; }
 
+bool pib_dense_takes_rows(const pib_weight * w, int M) {
+    return dt_enabled() && w && w->type == PIB_TYPE_BF16 && M > DT_ROWS_MAX && !((uintptr_t) w->base & 15) && w->K % 8 == 0 && w->K >= 16;
+}
+
 int pib_dense_mm_tc(const pib_mm & a, cudaStream_t st) {
+    if (a.y_bf16 && (a.Z != 1 || a.zrange || a.Y2)) return PIB_ERR_UNSUPP;
     if (!dt_enabled() || a.wtype != PIB_TYPE_BF16) return PIB_ERR_UNSUPP;
     if (a.M <= DT_ROWS_MAX) return PIB_ERR_UNSUPP;                       // few rows: the memory-bound kernels of dense_mm.cu
     // TMA wants 16-byte aligned bases and strides

@@ -68,7 +68,7 @@ __device__ __forceinline__ void dp_commit(uint32_t bar, uint16_t mask) {
 
 struct dp_args {
     int M, N, K, NB, tiles_m, tiles, shares, w_made;
-    float * Y; int64_t ldy;
+    float * Y; int64_t ldy; int y_bf16;                          // y_bf16: Y holds bfloat16 rows
     float e0, e1;
     float * Y2; int64_t ld2; int n2; const int32_t * rows2;      // outputs n >= n2 go to Y2[rows2[m] * ld2 + n - n2]
     int * err;
@@ -81,10 +81,19 @@ template <int EPI, int COLS> __device__ __forceinline__ void dp_out(const dp_arg
 #pragma unroll
         for (int j = 0; j < COLS; j++) {
             const float mine = __uint_as_float(v[j]), other = __shfl_xor_sync(0xffffffffu, mine, 1);
-            if (!(orow & 1) && orow + 1 < A.N && j < left) A.Y[(size_t) (m0 + j) * A.ldy + (orow >> 1)] = pib_glu_pair<EPI, true>(mine, other, A.e0);
+            if (!(orow & 1) && orow + 1 < A.N && j < left) {
+                const size_t at = (size_t) (m0 + j) * A.ldy + (orow >> 1);
+                const float  o  = pib_glu_pair<EPI, true>(mine, other, A.e0);
+                if (A.y_bf16) reinterpret_cast<__nv_bfloat16 *>(A.Y)[at] = __float2bfloat16_rn(o);
+                else          A.Y[at] = o;
+            }
         }
     } else if (orow < A.N) {
-        if (w0 + 31 < A.n2) {                        // none of the warp's rows goes to Y2
+        if (A.y_bf16) {
+            __nv_bfloat16 * p = reinterpret_cast<__nv_bfloat16 *>(A.Y) + (size_t) m0 * A.ldy + orow;
+#pragma unroll
+            for (int j = 0; j < COLS; j++, p += A.ldy) if (j < left) *p = __float2bfloat16_rn(pib_epilogue<EPI, true>(__uint_as_float(v[j]), A.e0, A.e1));
+        } else if (w0 + 31 < A.n2) {                 // none of the warp's rows goes to Y2
             float * p = A.Y + (size_t) m0 * A.ldy + orow;
 #pragma unroll
             for (int j = 0; j < COLS; j++, p += A.ldy) if (j < left) *p = pib_epilogue<EPI, true>(__uint_as_float(v[j]), A.e0, A.e1);
@@ -262,7 +271,7 @@ void pib_dense_pair_plan(int M, int N, int K, int * nb, int * shares) {
 
 int pib_dense_pair(const pib_mm & a, const CUtensorMap & wmap, const CUtensorMap & xmap, int NB, int shares, int * err, cudaStream_t st) {
     const int tiles_m = (a.M + NB - 1) / NB, tiles = tiles_m * ((a.N + 255) / 256), pairs = pib_num_sms() / 2;
-    const dp_args A = { a.M, a.N, a.K, NB, tiles_m, tiles, shares, a.w_made, a.Y, a.ldy, a.e0, a.e1, a.Y2, a.ld2, a.Y2 ? a.n2 : 0x7fffffff, a.rows2, err };
+    const dp_args A = { a.M, a.N, a.K, NB, tiles_m, tiles, shares, a.w_made, a.Y, a.ldy, a.y_bf16, a.e0, a.e1, a.Y2, a.ld2, a.Y2 ? a.n2 : 0x7fffffff, a.rows2, err };
     const dim3 grid((unsigned) (2 * shares * (shares > 1 || tiles < pairs ? tiles : pairs)));
 #define DP_GO(EPI) do {                                                                                                                            \
         static bool configured = false;                                                                                                            \

@@ -39,7 +39,7 @@ struct fa_args {
     float softcap;
     const float * sink, * slopes, * rel; int n_rel;
     const float * gate; int ldg;
-    float * out;
+    float * out; int out_bf16;                       // out_bf16: out holds bfloat16 rows
     int * err;
     pib_attn_block seg[FA_SEGS];                     // portions, those with the most row blocks first
 };
@@ -357,7 +357,11 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap qh, const __grid_constant_
                             const float4 g = *reinterpret_cast<const float4 *>(gbuf + r * 36 + (lane & 7) * 4);
                             x.x *= 1.0f / (1.0f + __expf(-g.x)); x.y *= 1.0f / (1.0f + __expf(-g.y)); x.z *= 1.0f / (1.0f + __expf(-g.z)); x.w *= 1.0f / (1.0f + __expf(-g.w));
                         }
-                        if (r < rows && col) *reinterpret_cast<float4 *>(A.out + (size_t) rr * A.V + cl) = x;
+                        if (r >= rows || !col) continue;
+                        if (A.out_bf16) {
+                            const __nv_bfloat162 a = __floats2bfloat162_rn(x.x, x.y), b = __floats2bfloat162_rn(x.z, x.w);
+                            *reinterpret_cast<uint2 *>(reinterpret_cast<__nv_bfloat16 *>(A.out) + (size_t) rr * A.V + cl) = make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+                        } else *reinterpret_cast<float4 *>(A.out + (size_t) rr * A.V + cl) = x;
                     }
                 } else {
                     for (int r = 0; r < rows; r++) {
@@ -365,7 +369,8 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap qh, const __grid_constant_
                         if (c + lane >= A.V) continue;
                         float x = buf[r * 36 + lane];
                         if (A.gate) x *= 1.0f / (1.0f + __expf(-A.gate[(size_t) (rr / A.H) * A.ldg + (size_t) (rr % A.H) * A.V + c + lane]));
-                        A.out[(size_t) rr * A.V + c + lane] = x;
+                        if (A.out_bf16) reinterpret_cast<__nv_bfloat16 *>(A.out)[(size_t) rr * A.V + c + lane] = __float2bfloat16_rn(x);
+                        else A.out[(size_t) rr * A.V + c + lane] = x;
                     }
                 }
             }
@@ -511,7 +516,7 @@ void pib_flash_attention_place(std::vector<pib_attn_block> & blocks, int rep, lo
 int pib_flash_attention_max() { return FA_SEGS; }
 
 int pib_flash_attention(const pib_kv_query & q, const pib_hlayer & L, const std::vector<pib_attn_block> & blocks, int C, int R, const float * cache, int cache_row, const int32_t * cellmap, int n_ctx,
-                        void * Kb, void * Vt, void * Qc, float * out, cudaStream_t st) {
+                        void * Kb, void * Vt, void * Qc, float * out, cudaStream_t st, bool out_bf16) {
     const int D = L.dim, V = L.vdim, maps = L.maps, rep = L.heads / L.kv_heads, Z = L.kv_heads * maps, n = (int) blocks.size();
     if (n < 1 || n > FA_SEGS) { pib_set_error("attention: %d portions in a launch", n); return PIB_ERR_ARG; }
     fa_gather_args g = { cache, cache_row, cellmap, n_ctx, q.q, q.ldq, cache_row % 4 == 0 && ((uintptr_t) cache & 15) == 0, q.ldq % 4 == 0 && ((uintptr_t) q.q & 15) == 0,
@@ -536,7 +541,7 @@ int pib_flash_attention(const pib_kv_query & q, const pib_hlayer & L, const std:
     int t_end = 0;
     for (const pib_attn_block & b : blocks) t_end = std::max(t_end, b.t0 + b.nq);
     const int vec_out = V % 4 == 0 && ((uintptr_t) out & 15) == 0 && (!q.gate || (q.ldg % 4 == 0 && ((uintptr_t) q.gate & 15) == 0 && (size_t) q.ldg * ((size_t) t_end + 1) / 4 < (1ull << 32)));
-    fa_args A = { rep, maps, L.heads * maps, V, VN, Z, n, L.window, L.mask, L.keep, vec_out, rel_smem, L.softcap, L.sink, L.slopes, L.rel, L.n_rel, q.gate, q.ldg, out, err, {} };
+    fa_args A = { rep, maps, L.heads * maps, V, VN, Z, n, L.window, L.mask, L.keep, vec_out, rel_smem, L.softcap, L.sink, L.slopes, L.rel, L.n_rel, q.gate, q.ldg, out, out_bf16 ? 1 : 0, err, {} };
     std::copy(blocks.begin(), blocks.end(), A.seg);
     int row_blocks = 0;
     for (const pib_attn_block & b : blocks) row_blocks += b.row_blocks;

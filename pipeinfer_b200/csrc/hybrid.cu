@@ -285,6 +285,15 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
         return a;
     };
     auto mm = [&](const pib_weight * w, const float * X, int ldx, float * Y, int ldy, int epi, float e0 = 0.f, float e1 = 0.f) { return pib_dense_mm(mm_of(w, X, ldx, Y, ldy, epi, e0, e1), st); };
+    // rows that only a tensor-core matmul reads are written as its bfloat16 operand by the kernel that makes them (the values that the matmul's own rounding would give)
+    const bool dump = getenv("PIB_HYBRID_DUMP") != nullptr;
+    auto takes = [&](const pib_weight * w) { return !exact && !dump && pib_dense_takes_rows(w, T); };
+    bool h_bf16 = false;                              // x->h holds such rows
+    auto mm16 = [&](const pib_weight * w, const float * X, float * Y, int ldy, int epi, float e0, float e1, bool x16, bool y16) {
+        pib_mm a = mm_of(w, X, (int) w->K, Y, ldy, epi, e0, e1);
+        a.x_bf16 = x16; a.y_bf16 = y16;
+        return pib_dense_mm(a, st);
+    };
     // gated frame: the residual gate's matmul x->rg = R x->h shares a launch with the sublayer's first one in decode steps
     const bool pairs = T <= 16;
     const pib_weight * gate_w = nullptr;              // a gate whose matmul is still to be launched
@@ -349,8 +358,8 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
         RC(HK_HO, mmfl(L.wo), mmby(L.wo), mm(L.wo, x->att, H * L.vdim, x->y, W, PIB_EPI_NONE));
         return PIB_OK;
     };
-    // the attention of cached key / value heads over `q`: per-token kernel, or the matmul form for long portions in served mode
-    auto kv_attend = [&](const pib_hlayer & L, const pib_kv_query & q, float * cache, int row, float * out) -> int {
+    // the attention of cached key / value heads over `q` (out16: asks for bfloat16 rows, and is told): per-token kernel, or the matmul form for long portions in served mode
+    auto kv_attend = [&](const pib_hlayer & L, const pib_kv_query & q, float * cache, int row, float * out, bool * out16 = nullptr) -> int {
         const int H = L.heads * L.maps, G = L.kv_heads * L.maps, D = L.dim, V = L.vdim;      // query rows and key heads: one per map
         const double keys = key_pairs(L.window, L.mask, L.keep);
         const bool mm_ok = !exact && D % 8 == 0 && D >= 16 && V >= 16 && attn_mm_enabled();
@@ -358,6 +367,8 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
         const int  min_len = flash ? FLASH_ATTN_MIN_LEN : MM_ATTN_MIN_LEN;
         bool any_mm = false, any_simt = false;
         for (const pib_hseg & g : segs) { if (mm_ok && g.len >= min_len) any_mm = true; else any_simt = true; }
+        const bool o16 = out16 && flash && any_mm && !any_simt;          // bfloat16 rows out, where the caller asks and one form makes them all
+        if (out16) *out16 = o16;
         if (any_simt)
             RC(HK_KVATTN, 2.0 * keys * H * (D + V), 4.0 * keys * G * (D + V) + 4.0 * Td * H * (D + V),
                pib_kv_attention(q, L, B, cache, row, x->cellmap, (int) c->n_ctx, out, any_mm ? (flash ? B.faflag : B.mmflag) : nullptr, st));
@@ -372,7 +383,7 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
             const size_t qb = pib_flash_attention_bytes(L, cols, rows, &kb, &vb);
             if ((rc = grow_flash(c, kb, vb, qb)) != PIB_OK) return rc;
             RC(HK_FLASH, 2.0 * H * bl_pairs * (D + V), 4.0 * bl_keys * G * (D + V) + 4.0 * bl_tok * H * (D + V),
-               pib_flash_attention(q, L, blocks, (int) cols, (int) rows, cache, row, x->cellmap, (int) c->n_ctx, x->am_kb, x->am_vt, x->am_q, out, st));
+               pib_flash_attention(q, L, blocks, (int) cols, (int) rows, cache, row, x->cellmap, (int) c->n_ctx, x->am_kb, x->am_vt, x->am_q, out, st, o16));
             nk++;
             blocks.clear();
             bl_pairs = bl_keys = bl_tok = 0;
@@ -425,10 +436,12 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
         const int H = L.heads, D = L.dim, V = L.vdim, nq = H * D, ng = L.out_gate ? H * V : 0, ldp = (nq + ng + 3) & ~3, row = hy->cache_row[L.cache_id];
         float * cache = x->cache[L.cache_id];
         pib_mm a = mm_of(L.qkv, hin, W, x->proj, ldp, PIB_EPI_NONE);
+        a.x_bf16 = h_bf16;
         if (L.kv_from < 0) { a.Y2 = cache; a.ld2 = row; a.n2 = nq + ng; a.rows2 = B.cell; }
         RC(HK_QKV, mmfl(L.qkv), mmby(L.qkv), pib_dense_mm(a, st));
-        if ((rc = kv_attend(L, { x->proj, ldp, L.out_gate ? x->proj + nq : nullptr, ldp }, cache, row, x->att)) != PIB_OK) return rc;
-        RC(HK_AO, mmfl(L.wo), mmby(L.wo), mm(L.wo, x->att, H * V, x->y, W, PIB_EPI_NONE));
+        bool att16 = false;
+        if ((rc = kv_attend(L, { x->proj, ldp, L.out_gate ? x->proj + nq : nullptr, ldp }, cache, row, x->att, takes(L.wo) ? &att16 : nullptr)) != PIB_OK) return rc;
+        RC(HK_AO, mmfl(L.wo), mmby(L.wo), mm16(L.wo, x->att, x->y, W, PIB_EPI_NONE, 0.f, 0.f, att16, false));
         return PIB_OK;
     };
     // RWKV-style time mixing: the five token-shift mixes, r | k | v | g as four problems of one launch, the decay's two small matmuls, the recurrence
@@ -694,10 +707,11 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
     };
     // sandwich frame: what the sublayer before left is normed, scaled and added by the kernel that norms the stream for the next one
     pib_sublayer_y leftn;
-    auto sandwich = [&](const float * w, const float * b, const pib_hlayer * moe = nullptr) -> int {
+    auto sandwich = [&](const float * w, const float * b, const pib_hlayer * moe = nullptr, bool h16 = false) -> int {
+        h_bf16 = w && h16;
         pib_norm_route nr;
         if (moe) { nr.rows = (const float *) moe->router->base; nr.R = router_of(*moe); nr.ids = x->ids; nr.wts = x->wts; nr.offs = x->offs; nr.perm = x->perm; nr.inv = x->inv; nr.act = x->act; nr.done = x->done; }
-        RC(moe ? HK_NORM_ROUTE : HK_SANDWICH, moe ? mmfl(moe->router) : 0, (moe ? wbytes(moe->router) : 0.0) + 4.0 * Td * Wd * ((leftn.y ? 3.0 : leftn.top ? 2.0 : 1.0) + leftn.top + (w ? 1.0 : 0.0)), pib_sandwich_norm(x->x, leftn, w, b, eps, T, W, w ? x->h : nullptr, st, moe ? &nr : nullptr));
+        RC(moe ? HK_NORM_ROUTE : HK_SANDWICH, moe ? mmfl(moe->router) : 0, (moe ? wbytes(moe->router) : 0.0) + 4.0 * Td * Wd * ((leftn.y ? 3.0 : leftn.top ? 2.0 : 1.0) + leftn.top + (w ? 1.0 : 0.0)), pib_sandwich_norm(x->x, leftn, w, b, eps, T, W, w ? x->h : nullptr, st, moe ? &nr : nullptr, h_bf16));
         leftn = pib_sublayer_y();
         return PIB_OK;
     };
@@ -705,14 +719,15 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
         const pib_hlayer & L = hy->layers[il];
         int lds = 0;
         if (hy->form == PIB_FORM_SANDWICH) {
-            if ((rc = sandwich(L.norm1, L.norm1_b)) != PIB_OK) return rc;
+            if ((rc = sandwich(L.norm1, L.norm1_b, nullptr, L.mixer == PIB_MIXER_KV && takes(L.qkv))) != PIB_OK) return rc;
             if ((rc = run_mixer(L, x->h)) != PIB_OK) return rc;
             leftn.y = x->y; leftn.w = L.post1; leftn.b = L.post1_b;
             const bool routed = L.mlp == PIB_MLP_MOE && pib_norm_route_fits(T, W, router_of(L));      // small batches: the router rides on the norm
-            if (L.mlp != PIB_MLP_NONE && (rc = sandwich(L.norm2, L.norm2_b, routed ? &L : nullptr)) != PIB_OK) return rc;
+            if (L.mlp != PIB_MLP_NONE && (rc = sandwich(L.norm2, L.norm2_b, routed ? &L : nullptr, L.mlp == PIB_MLP_RELU2 && takes(L.up))) != PIB_OK) return rc;
             if (L.mlp == PIB_MLP_RELU2) {
-                RC(HK_UP, mmfl(L.up), mmby(L.up), mm(L.up, x->h, W, x->proj, L.ff, PIB_EPI_RELU2));
-                RC(HK_DOWN, mmfl(L.down), mmby(L.down), mm(L.down, x->proj, L.ff, x->y, W, PIB_EPI_NONE));
+                const bool z16 = takes(L.up) && takes(L.down);
+                RC(HK_UP, mmfl(L.up), mmby(L.up), mm16(L.up, x->h, x->proj, L.ff, PIB_EPI_RELU2, 0.f, 0.f, h_bf16, z16));
+                RC(HK_DOWN, mmfl(L.down), mmby(L.down), mm16(L.down, x->proj, x->y, W, PIB_EPI_NONE, 0.f, 0.f, z16, false));
                 leftn.y = x->y;
             } else if (L.mlp == PIB_MLP_MOE && L.expert == PIB_EXPERT_SWIGLU) {
                 if ((rc = run_experts(L, x->h, &lds, routed)) != PIB_OK) return rc;
@@ -743,8 +758,9 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
             if (L.mlp == PIB_MLP_GLU) {
                 RC(HK_HYPER, 0, hby, pib_hyper_norm(x->x, Sn, pend_y, pend_b, L.hc2, L.norm2, L.norm2_b, eps, T, W, x->h, st));
                 // gate and up rows are interleaved: the clamps, the gate's sigmoid and the product ride on the matmul's way out
-                RC(HK_GATEUP, mmfl(L.up), wbytes(L.up) + 4.0 * Td * (Wd + L.ff), mm(L.up, x->h, W, x->proj, L.ff, PIB_EPI_GLU_PAIR, L.limit_s));
-                RC(HK_DOWN, mmfl(L.down), mmby(L.down), mm(L.down, x->proj, L.ff, x->y, W, PIB_EPI_NONE));
+                const bool z16 = takes(L.up) && takes(L.down);
+                RC(HK_GATEUP, mmfl(L.up), wbytes(L.up) + 4.0 * Td * (Wd + L.ff), mm16(L.up, x->h, x->proj, L.ff, PIB_EPI_GLU_PAIR, L.limit_s, 0.f, false, z16));
+                RC(HK_DOWN, mmfl(L.down), mmby(L.down), mm16(L.down, x->proj, x->y, W, PIB_EPI_NONE, 0.f, 0.f, z16, false));
                 pend_y = x->y; pend_b = L.hc2;
             } else if (L.mlp != PIB_MLP_NONE) { pib_set_error("decode: feed-forward %d in a layer with hyper-connections", L.mlp); return PIB_ERR_UNSUPP; }
         } else if (hy->form == PIB_FORM_PRENORM) {
@@ -758,8 +774,9 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
             pend_y = x->y; pend_b = L.o_bias;
             if (L.mlp == PIB_MLP_XIELU) {
                 if ((rc = prenorm(L.g2, nullptr, 0, true)) != PIB_OK) return rc;
-                RC(HK_UP, mmfl(L.up), mmby(L.up), mm(L.up, x->h, W, x->proj, L.ff, PIB_EPI_XIELU, L.act[2], L.act[3]));      // the activation rides on the matmul's way out
-                RC(HK_DOWN, mmfl(L.down), mmby(L.down), mm(L.down, x->proj, L.ff, x->y, W, PIB_EPI_NONE));
+                const bool z16 = takes(L.up) && takes(L.down);
+                RC(HK_UP, mmfl(L.up), mmby(L.up), mm16(L.up, x->h, x->proj, L.ff, PIB_EPI_XIELU, L.act[2], L.act[3], false, z16));      // the activation rides on the matmul's way out
+                RC(HK_DOWN, mmfl(L.down), mmby(L.down), mm16(L.down, x->proj, x->y, W, PIB_EPI_NONE, 0.f, 0.f, z16, false));
                 pend_y = x->y; pend_b = nullptr;
             } else if (L.mlp != PIB_MLP_NONE) { pib_set_error("decode: feed-forward %d in a pre-norm layer", L.mlp); return PIB_ERR_UNSUPP; }
         } else if (hy->form == PIB_FORM_PARALLEL) {
@@ -813,13 +830,13 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
             if (FILE * f = fopen(path, "wb")) { fwrite(hb.data(), 4, hb.size(), f); fclose(f); }
         }
     }
-    if (hy->form == PIB_FORM_SANDWICH)      { if ((rc = sandwich(m->output_norm, hy->final_b)) != PIB_OK) return rc; }
+    if (hy->form == PIB_FORM_SANDWICH)      { if ((rc = sandwich(m->output_norm, hy->final_b, nullptr, takes(m->output))) != PIB_OK) return rc; }
     else if (hy->form == PIB_FORM_GATED)    { if ((rc = gated(m->output_norm, nullptr, 0)) != PIB_OK) return rc; }
     else if (hy->form == PIB_FORM_HYPER)    RC(HK_FINAL, 0, (4.0 * hy->streams + 8.0) * Td * Wd, pib_hyper_norm(x->x, hy->streams, pend_y, pend_b, nullptr, m->output_norm, hy->final_b, eps, T, W, x->h, st));
     else if (hy->form == PIB_FORM_PRENORM)  { if ((rc = prenorm(hy->final_g, nullptr, 0, false)) != PIB_OK) return rc; }
     else if (hy->form == PIB_FORM_PARALLEL) RC(HK_FINAL, 0, 8.0 * Td * Wd, pib_rms_norm2(x->x, m->output_norm, nullptr, eps, hy->logit_scale, T, W, x->h, nullptr, st));
     else                                    RC(HK_FINAL, 0, 8.0 * Td * Wd, pib_layer_norm(x->x, m->output_norm, eps, T, W, x->h, 0, st));
-    RC(HK_HEAD, mmfl(m->output), mmby(m->output), mm(m->output, x->h, W, run.logits, m->n_vocab, PIB_EPI_NONE));
+    RC(HK_HEAD, mmfl(m->output), mmby(m->output), mm16(m->output, x->h, run.logits, m->n_vocab, PIB_EPI_NONE, 0.f, 0.f, h_bf16, false));
     RC(HK_SAMPLE, 0, 4.0 * Td * m->n_vocab, pib_sample_topk(run.logits, T, m->n_vocab, c->bias_ids_dev, c->bias_val_dev, c->n_bias, run.res_dev, c->desc_dev, c->cancel_table, st));
 #undef RC
     return PIB_OK;

@@ -245,6 +245,7 @@ struct pib_mm {
     // outputs n >= n2 of row m go to Y2[rows2[m] * ld2 + n - n2] (keys and values straight into their cache cells); Z 1, no paired epilogue
     float *         Y2 = nullptr; int64_t ld2 = 0; int n2 = 0x7fffffff; const int32_t * rows2 = nullptr;
     int             x_bf16 = 0;                          // 1: X already holds bfloat16 rows (ldx in elements, a multiple of 8): tensor-core path only, no staging copy
+    int             y_bf16 = 0;                          // 1: Y gets bfloat16 rows (ldy in elements): where pib_dense_takes_rows
     int             w_made = 0;                          // 1: W is not a weight but the work of an earlier launch on this stream: nothing of it is read ahead of the launch wait
 };
 #ifdef __CUDACC__
@@ -269,6 +270,7 @@ template <int EPI, bool FAST> __device__ __forceinline__ float pib_glu_pair(floa
 }
 #endif
 int pib_dense_mm(const pib_mm & a, cudaStream_t st);
+bool pib_dense_takes_rows(const pib_weight * w, int M);   // a matmul of M rows with w alone runs on the tensor cores of SM pairs: bfloat16 rows in (x_bf16) and out (y_bf16)
 int pib_dense_mm_pair(const pib_mm & a, const pib_mm & b, cudaStream_t st);   // two independent matmuls; in decode steps one launch
 int pib_dense_mm_experts(const pib_mm & routed, const pib_mm & shared, cudaStream_t st);   // a grouped matmul and a plain one with the same epilogue; in decode steps one launch
 // dense_mma.cu: the error word of a stream, which a tensor-core kernel sets when one of its bounded waits runs out
@@ -339,7 +341,7 @@ void pib_flash_attention_place(std::vector<pib_attn_block> & blocks, int rep, lo
 size_t pib_flash_attention_bytes(const pib_hlayer & L, long long cols, long long rows, size_t * k_bytes, size_t * v_bytes);      // operand buffers; the queries' is returned
 int pib_flash_attention_max();                                // portions in a launch
 int pib_flash_attention(const pib_kv_query & q, const pib_hlayer & L, const std::vector<pib_attn_block> & blocks, int C, int R, const float * cache, int cache_row, const int32_t * cellmap, int n_ctx,
-                        void * Kb, void * Vt, void * Qc, float * out, cudaStream_t st);
+                        void * Kb, void * Vt, void * Qc, float * out, cudaStream_t st, bool out_bf16 = false);
 int pib_token_shift(const float * h, const float * mu, int n_mix, const pib_hbatch & b, float * state, size_t state_stride, size_t shift_off, int W, float * mixes, cudaStream_t st);
 int pib_rows_act(float * z, int ld, int n, int T, int op, const float * bias, cudaStream_t st);           // op 0: tanh; 1: exp(-exp(z + bias))
 int pib_delta_prep(float * cv, int ldc, const pib_hlayer & L, const float * proj, int ldp, int b_off, int a_off, float * bg, int T, cudaStream_t st);
@@ -396,7 +398,7 @@ struct pib_norm_route {              // the router of the mixture that reads h, 
     float * wts = nullptr;
 };
 bool pib_norm_route_fits(int T, int W, const pib_router & R);
-int pib_sandwich_norm(float * x, const pib_sublayer_y & o, const float * w, const float * b, float eps, int T, int W, float * h, cudaStream_t st, const pib_norm_route * route = nullptr);
+int pib_sandwich_norm(float * x, const pib_sublayer_y & o, const float * w, const float * b, float eps, int T, int W, float * h, cudaStream_t st, const pib_norm_route * route = nullptr, bool h_bf16 = false);
 // chunk_scan.cu: n tokens of one segment (batch rows t0 ..) of a recurrence with one decay per head and token, as matmuls (served mode)
 struct pib_chunk_scan {
     const float * q = nullptr, * k = nullptr, * v = nullptr; int ldq = 0, ldk = 0, ldv = 0;   // rows [G][D], [G][D], [H][V] per token

@@ -33,22 +33,39 @@ __device__ __forceinline__ float mk_sigmoid(float z) { return 1.0f / (1.0f + exp
 __device__ __forceinline__ float mk_silu(float z) { return z / (1.0f + expf(-z)); }
 
 // ---- embedding, norms ------------------------------------------------------------------------------------------------------------
-template <typename WT>
+// a thread per VEC channels: one block per token walked its row in a chain of loads (7.5 us of a decode step); a channel per thread took 16 us for 1512 tokens of 2048
+template <typename WT, int VEC>
 __global__ void __launch_bounds__(256) embed_scale_kernel(const WT * __restrict__ embd, const int32_t * __restrict__ tok, float scale, int W, float * __restrict__ x, int copies) {
     pib_pdl_wait();
     pib_pdl_trigger();
-    const WT * r = embd + (size_t) tok[blockIdx.x] * W;
-    const int i = blockIdx.y * blockDim.x + threadIdx.x;          // a thread per channel: one block per token walked its row in a chain of loads (7.5 us of a decode step)
-    if (i < W) {
-        const float v = (float) r[i] * scale;
-        for (int s = 0; s < copies; s++) x[((size_t) blockIdx.x * copies + s) * W + i] = v;
+    const int i = (blockIdx.y * blockDim.x + threadIdx.x) * VEC;
+    if (i >= W) return;
+    const WT * r = embd + (size_t) tok[blockIdx.x] * W + i;
+    float v[VEC];
+    if (VEC == 4 && sizeof(WT) == 2) {
+        const uint2 w = *reinterpret_cast<const uint2 *>(r);
+        v[0] = __uint_as_float(w.x << 16) * scale; v[1 % VEC] = __uint_as_float(w.x & 0xffff0000u) * scale; v[2 % VEC] = __uint_as_float(w.y << 16) * scale; v[3 % VEC] = __uint_as_float(w.y & 0xffff0000u) * scale;
+    } else if (VEC == 4) {
+        const float4 w = *reinterpret_cast<const float4 *>(r);
+        v[0] = w.x * scale; v[1 % VEC] = w.y * scale; v[2 % VEC] = w.z * scale; v[3 % VEC] = w.w * scale;
+    } else v[0] = (float) r[0] * scale;
+    for (int s = 0; s < copies; s++) {
+        float * o = x + ((size_t) blockIdx.x * copies + s) * W + i;
+        if (VEC == 4) *reinterpret_cast<float4 *>(o) = make_float4(v[0], v[1 % VEC], v[2 % VEC], v[3 % VEC]);
+        else *o = v[0];
     }
 }
 // copies: every token's row is written that many times, one after the other (the residual streams of hyper-connections start equal)
 int pib_embed_scale(const pib_weight * embd, const int32_t * tok, float scale, int T, int W, float * x, cudaStream_t st, int copies) {
-    const dim3 grid((unsigned) T, (unsigned) ((W + 255) / 256));
-    if (embd->type == PIB_TYPE_BF16) pib_launch(embed_scale_kernel<__nv_bfloat16>, grid, dim3(256), (size_t) 0, st, (const __nv_bfloat16 *) embd->base, tok, scale, W, x, copies);
-    else                             pib_launch(embed_scale_kernel<float>, grid, dim3(256), (size_t) 0, st, (const float *) embd->base, tok, scale, W, x, copies);
+    const bool vec = W % 4 == 0 && (((uintptr_t) embd->base | (uintptr_t) x) & 15) == 0;
+    const int  threads = vec && T <= 32 ? 128 : 256, per = threads * (vec ? 4 : 1);      // few tokens: more blocks
+    const dim3 grid((unsigned) T, (unsigned) ((W + per - 1) / per));
+#define EMB_GO(WT) do {                                                                                                                            \
+        if (vec) pib_launch(embed_scale_kernel<WT, 4>, grid, dim3(threads), (size_t) 0, st, (const WT *) embd->base, tok, scale, W, x, copies);    \
+        else     pib_launch(embed_scale_kernel<WT, 1>, grid, dim3(threads), (size_t) 0, st, (const WT *) embd->base, tok, scale, W, x, copies);    \
+    } while (0)
+    if (embd->type == PIB_TYPE_BF16) EMB_GO(__nv_bfloat16); else EMB_GO(float);
+#undef EMB_GO
     CKL();
     return PIB_OK;
 }

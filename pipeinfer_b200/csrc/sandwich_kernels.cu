@@ -4,6 +4,8 @@
 //           mixture is summed here, it never exists in memory), LN' the norm behind it with layer scale and residual multiplier in its weight and bias
 //   h[t]  = LN(x[t]), the norm in front of the sublayer that follows (or the model's last one)
 //   small batches in front of a mixture: the router's logits of h[t] and the token's choice on the same launch; the last block to finish sorts the pairs
+#include <cuda_bf16.h>
+
 #include "hybrid.cuh"
 #include "moe_route.cuh"
 
@@ -22,6 +24,12 @@ template <int VEC> __device__ __forceinline__ void sw_store(float * p, const sw_
     if (VEC == 4) *reinterpret_cast<float4 *>(p) = make_float4(r.v[0], r.v[1 % VEC], r.v[2 % VEC], r.v[3 % VEC]);
     else *p = r.v[0];
 }
+template <int VEC> __device__ __forceinline__ void sw_store16(__nv_bfloat16 * p, const sw_vec<VEC> & r) {
+    if (VEC == 4) {
+        const __nv_bfloat162 a = __floats2bfloat162_rn(r.v[0], r.v[1 % VEC]), b = __floats2bfloat162_rn(r.v[2 % VEC], r.v[3 % VEC]);
+        *reinterpret_cast<uint2 *>(p) = make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+    } else *p = __float2bfloat16_rn(r.v[0]);
+}
 __device__ __forceinline__ float sw_block_sum(float v, float * red) {
     v = warp_sum(v);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -37,7 +45,7 @@ struct sw_args {
     float * x;
     pib_sublayer_y o;
     const float * w, * b; float eps; int W;
-    float * h;
+    float * h; int h_bf16;                        // h_bf16: h holds bfloat16 rows
     pib_norm_route route;
 };
 // mean and 1 / sqrt(variance + eps) of the block's row, held in registers as NV pieces of VEC channels per thread
@@ -160,7 +168,8 @@ __global__ void __launch_bounds__(NV >= 4 ? 512 : 1024) sandwich_norm_kernel(sw_
             sw_vec<VEC> h;
 #pragma unroll
             for (int i = 0; i < VEC; i++) h.v[i] = fmaf((x[n].v[i] - mx.x) * mx.y, w.v[i], b.v[i]);
-            sw_store<VEC>(A.h + row + c, h);             // a thread wrote and read only its own channels of this token: hin may be h
+            if (A.h_bf16) sw_store16<VEC>(reinterpret_cast<__nv_bfloat16 *>(A.h) + row + c, h);
+            else          sw_store<VEC>(A.h + row + c, h);             // a thread wrote and read only its own channels of this token: hin may be h
             if (ROUTE) sw_store<VEC>(sw_dyn + c, h);
         }
     }
@@ -170,9 +179,10 @@ static size_t sw_route_smem(int T, int W, const pib_router & R) { return (size_t
 bool pib_norm_route_fits(int T, int W, const pib_router & R) {
     return W % 4 == 0 && T <= MOE_SMALL_T && T * R.top <= MOE_SMALL_PAIRS && R.E <= MOE_SMALL_E && sw_route_smem(T, W, R) <= 46 * 1024;
 }
-// o empty: only the norm of x; h null: only the sum; route: see pib_norm_route (the caller has asked pib_norm_route_fits)
-int pib_sandwich_norm(float * x, const pib_sublayer_y & o, const float * w, const float * b, float eps, int T, int W, float * h, cudaStream_t st, const pib_norm_route * route) {
-    sw_args A = { x, o, w, b, eps, W, h, pib_norm_route() };
+// o empty: only the norm of x; h null: only the sum; h_bf16: h gets bfloat16 rows (what the tensor-core matmul behind it reads); route: see pib_norm_route (the caller has asked pib_norm_route_fits)
+int pib_sandwich_norm(float * x, const pib_sublayer_y & o, const float * w, const float * b, float eps, int T, int W, float * h, cudaStream_t st, const pib_norm_route * route, bool h_bf16) {
+    sw_args A = { x, o, w, b, eps, W, h, h_bf16 ? 1 : 0, pib_norm_route() };
+    if (route && h_bf16) { pib_set_error("sandwich norm: the router reads float rows"); return PIB_ERR_ARG; }
     if (route) {
         const int rc = pib_moe_router_check(route->R);
         if (rc != PIB_OK) return rc;
