@@ -622,7 +622,13 @@ gemv_q4k_ring_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, 
         if (tok < b && row < N) {
             float v = red[0][tok][r];
 #pragma unroll
-            for (int w2 = 1; w2 < WARPS; w2++) v += red[w2][tok][r];
+            for (int w2 = 1; w2 < 4; w2++) v += red[w2][tok][r];
+            if (WARPS == 8) {                                   // two halves, as two K shares would add up
+                float u = red[4 % WARPS][tok][r];
+#pragma unroll
+                for (int w2 = 5; w2 < 8; w2++) u += red[w2 % WARPS][tok][r];
+                v += u;
+            }
             if (nsplit == 1) y[(size_t) tok * N + row] = v;
             else partial[((size_t) split * b + tok) * N + row] = v;
         }
@@ -1074,9 +1080,11 @@ int pib_gemv_ring(const pib_weight * w, const void * act_dev, int b, float * y_d
         int runs = 0, pmax = 0;
         if (b > 8 && (long long) n_tiles * nsb >= 16384 && stream_plan(n_tiles, nsb, b, &runs, &pmax)) return pib_gemv_stream(w, act_dev, b, y_dev, cancel, st);
     }
-    // one wave of CTAs or less (4 CTAs of 4 warps per SM): eight warps per tile halve every warp's chain of records
+    // one wave of CTAs or less (4 CTAs of 4 warps per SM): eight warps per tile halve every warp's chain of records.  With 8 to 15 super-blocks they take the place of
+    // K shares, which meet through memory (K = 2048, shares / eight warps, us: 2560 rows at 1 token 3.5 / 2.0, at 12 5.2 / 4.1; 4096 at 1 4.0 / 2.2); tiles enough to go
+    // without shares keep four warps (8192 rows: 3.1 / 4.2)
     static const int wide_on = getenv("PIB_RING_WIDE") ? atoi(getenv("PIB_RING_WIDE")) : 1;
-    const bool wide = wide_on && n_tiles <= 2 * pib_num_sms() * 2 && nsb >= 16;          // <= 2 CTAs of 8 warps per SM
+    const bool wide = wide_on && n_tiles <= 2 * pib_num_sms() * 2 && (nsb >= 16 || (nsb >= 8 && n_tiles < pib_split_fill_target()));          // <= 2 CTAs of 8 warps per SM
     static const int split_env = getenv("PIB_RING_SPLIT") ? atoi(getenv("PIB_RING_SPLIT")) : 0;
     const int  split = fit_split(split_env > 0 ? split_env : wide ? 1 : choose_split_direct(n_tiles, nsb), b, w->N, n_tiles);
     mm_scratch * s = nullptr;
