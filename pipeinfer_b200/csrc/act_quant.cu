@@ -66,8 +66,9 @@ __global__ void __launch_bounds__(AQ_THREADS) act_quant_kernel(const float * x, 
                                                                const uint16_t * __restrict__ lut,
                                                                const float * __restrict__ addend, float * sum_out,
                                                                const int * __restrict__ cancel, int64_t xstride,
-                                                               const float * __restrict__ bias, const float * __restrict__ addend2, __half * __restrict__ xh) {
+                                                               const float * __restrict__ bias, const float * __restrict__ addend2, __half * __restrict__ xh, float * __restrict__ dxo) {
     const int     row  = blockIdx.x;
+    const pib_oct oct  = pib_oct_of(row, (int) gridDim.x);
     const float * xr   = x + (size_t) row * xstride;
     const float * x2r  = x2 ? (x2_per_row ? x2 + (size_t) row * xstride : x2) : nullptr;
     const int     lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -224,9 +225,10 @@ __global__ void __launch_bounds__(AQ_THREADS) act_quant_kernel(const float * x, 
                 }
             }
             // fragment-order copy for the tensor-core GEMV (gemv_blk32.cu): element e = 16 h + 4 t + i of block j of a group
-            // of eight goes to 64 t + 8 j + 4 h + i, so that a lane's B operands of a whole group are 64 contiguous bytes
-            qsp[(size_t) row * nbp * 32 + (blk >> 3) * 256 + ((lane & 15) >> 2) * 64 + (blk & 7) * 8 + (lane >> 4) * 4 + (lane & 3)] = (int8_t) q;
-            if (lane == 0) dxp[(size_t) row * nbp + blk] = __float2half_rn(d);
+            // of eight is byte 8 (j & 1) + 4 h + i of quarter t of piece j >> 1
+            const int j = (int) (blk & 7);
+            qsp[(size_t) oct.before * nbp * 32 + (((size_t) (blk >> 3) * 4 + (j >> 1)) * oct.gs + oct.g) * 64 + ((lane & 15) >> 2) * 16 + (j & 1) * 8 + (lane >> 4) * 4 + (lane & 3)] = (int8_t) q;
+            if (lane == 0) dxp[(size_t) oct.before * nbp + ((size_t) (blk >> 3) * oct.gs + oct.g) * 8 + j] = __float2half_rn(d);
         }
     } else {
         // one warp per 256-element super-block, lane owns 8 consecutive elements
@@ -247,8 +249,11 @@ __global__ void __launch_bounds__(AQ_THREADS) act_quant_kernel(const float * x, 
             }
             const size_t rs = (size_t) row * nsb + sb;
             if (XH) q8k_quantise_sb(v, lane, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, xh + (size_t) row * K + sb * PIB_QK_K);
-            else q8k_quantise_sb(v, lane, qs + (size_t) row * K + sb * PIB_QK_K, qsp + (size_t) row * K + sb * PIB_QK_K, (int16_t *) bsplane + rs * 16, bs8plane + rs * 16,
-                            sbs + rs * 8, qsl + rs * 64, dplane + rs, q6p + (size_t) row * K + sb * PIB_QK_K, b16 + rs * 32);
+            else {
+                const size_t os = (size_t) oct.before * nsb + (size_t) sb * oct.gs + oct.g, of = (size_t) oct.before * K + (size_t) sb * oct.gs * PIB_QK_K + oct.g * 64;
+                q8k_quantise_sb(v, lane, qs + (size_t) row * K + sb * PIB_QK_K, qsp + of, (int16_t *) bsplane + rs * 16, bs8plane + os * 16, sbs + rs * 8, qsl + rs * 64, dplane + rs,
+                                q6p + of, b16 + os * 32, nullptr, 64 * oct.gs, dxo + os);
+            }
         }
     }
 }
@@ -269,6 +274,7 @@ static int launch_aq(int wtype, const float * x, const float * x2, int x2_per_ro
     int16_t * sb = (int16_t *) ((uint8_t *) act + L.sbs_off);
     int8_t *  q6 = (int8_t *) act + L.q6p_off;
     int8_t *  b6 = (int8_t *) act + L.b16_off;
+    float *   dx = (float *) ((uint8_t *) act + L.dxo_off);
     // a warp per super-block or 32-element block: a warp that takes several takes them one after the other, and each is a chain of a load, a reduction and stores
     // (K = 5632, silu: 5.1 us with floor(22 / 8) CTAs per row; Q8_0 blocks of K = 4096, norm: 6.4 us with four blocks per warp)
     const int64_t units = wtype == PIB_TYPE_Q4_K ? K / PIB_QK_K : K / PIB_QK;
@@ -279,7 +285,7 @@ static int launch_aq(int wtype, const float * x, const float * x2, int x2_per_ro
     parts = max((int64_t) 1, min((int64_t) 32, parts));
     const dim3    grid(b, (unsigned) parts);
 #define AQ_GO(Q8K, XH) pib_launch(act_quant_kernel<Q8K, PRO, XH>, grid, dim3(AQ_THREADS), 0, st, x, x2, x2_per_row, eps, K, qs, d, bs, b8, qp, ql, sb, q6, b6, vout, lut, addend, sum_out, cancel, \
-                               xstride, bias, addend2, (__half *) xhat)
+                               xstride, bias, addend2, (__half *) xhat, dx)
     constexpr bool PROMPT = PRO == PRO_PLAIN || PRO == PRO_RMSNORM || PRO == PRO_SILU_MUL;
     if (wtype != PIB_TYPE_Q4_K) AQ_GO(false, false);
     else if (PROMPT && xhat)    AQ_GO(true, PROMPT);

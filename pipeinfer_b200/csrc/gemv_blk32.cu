@@ -122,11 +122,13 @@ gemv_blk32_kernel(const uint8_t * __restrict__ tiles, int ngr, int N, const int8
     for (int n = 0; n < NT; n++) { acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f; }
     const int8_t * a_q[NT];
     const __half * a_d[NT][2];
+    int            gs[NT];                                      // tokens of the octet (pib_oct)
 #pragma unroll
     for (int n = 0; n < NT; n++) {
-        a_q[n] = aqs + (size_t) min(n * 8 + g, b - 1) * ngr * 256 + t * 64;
+        gs[n] = min(8, b - 8 * n);
+        a_q[n] = aqs + (size_t) n * 8 * ngr * 256 + min(g, gs[n] - 1) * 64 + t * 16;
 #pragma unroll
-        for (int e = 0; e < 2; e++) a_d[n][e] = adx + (size_t) min(n * 8 + 2 * t + e, b - 1) * ngr * 8;
+        for (int e = 0; e < 2; e++) a_d[n][e] = adx + ((size_t) n * 8 * ngr + min(2 * t + e, gs[n] - 1)) * 8;
     }
 
     int4 wq[NQ], dq[2];
@@ -153,11 +155,12 @@ gemv_blk32_kernel(const uint8_t * __restrict__ tiles, int ngr, int N, const int8
         int4 ax[NT][2];
 #pragma unroll
         for (int n = 0; n < NT; n++) {
-            const int4 * ap = reinterpret_cast<const int4 *>(a_q[n] + (size_t) s * 256);
+            const int sg = s * gs[n];
+            const int4 * ap = reinterpret_cast<const int4 *>(a_q[n] + (size_t) sg * 256);
 #pragma unroll
-            for (int c = 0; c < 4; c++) aq[n][c] = __ldg(ap + c);
+            for (int c = 0; c < 4; c++) aq[n][c] = __ldg(ap + c * 4 * gs[n]);
 #pragma unroll
-            for (int e = 0; e < 2; e++) ax[n][e] = __ldg(reinterpret_cast<const int4 *>(a_d[n][e] + (size_t) s * 8));
+            for (int e = 0; e < 2; e++) ax[n][e] = __ldg(reinterpret_cast<const int4 *>(a_d[n][e] + (size_t) sg * 8));
         }
         const uint32_t dw0[4] = { (uint32_t) dq[0].x, (uint32_t) dq[0].y, (uint32_t) dq[0].z, (uint32_t) dq[0].w };   // row g:   d of blocks 2i | 2i+1
         const uint32_t dw1[4] = { (uint32_t) dq[1].x, (uint32_t) dq[1].y, (uint32_t) dq[1].z, (uint32_t) dq[1].w };   // row g+8
@@ -271,11 +274,13 @@ gemv_blk32_ring_kernel(const uint8_t * __restrict__ tiles, int ngr, int N, const
     for (int n = 0; n < NT; n++) { acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f; }
     const int8_t * a_q[NT];
     const __half * a_d[NT][2];
+    int            gs[NT];                                      // tokens of the octet (pib_oct)
 #pragma unroll
     for (int n = 0; n < NT; n++) {
-        a_q[n] = aqs + (size_t) min(n * 8 + g, b - 1) * ngr * 256 + t * 64;
+        gs[n] = min(8, b - 8 * n);
+        a_q[n] = aqs + (size_t) n * 8 * ngr * 256 + min(g, gs[n] - 1) * 64 + t * 16;
 #pragma unroll
-        for (int e = 0; e < 2; e++) a_d[n][e] = adx + (size_t) min(n * 8 + 2 * t + e, b - 1) * ngr * 8;
+        for (int e = 0; e < 2; e++) a_d[n][e] = adx + ((size_t) n * 8 * ngr + min(2 * t + e, gs[n] - 1)) * 8;
     }
     pib_pdl_wait();
     pib_pdl_trigger();
@@ -285,11 +290,12 @@ gemv_blk32_ring_kernel(const uint8_t * __restrict__ tiles, int ngr, int N, const
         int4 ax[NT][2];
 #pragma unroll
         for (int n = 0; n < NT; n++) {
-            const int4 * ap = reinterpret_cast<const int4 *>(a_q[n] + (size_t) s * 256);
+            const int sg = s * gs[n];
+            const int4 * ap = reinterpret_cast<const int4 *>(a_q[n] + (size_t) sg * 256);
 #pragma unroll
-            for (int c = 0; c < 4; c++) aq[n][c] = __ldg(ap + c);
+            for (int c = 0; c < 4; c++) aq[n][c] = __ldg(ap + c * 4 * gs[n]);
 #pragma unroll
-            for (int e = 0; e < 2; e++) ax[n][e] = __ldg(reinterpret_cast<const int4 *>(a_d[n][e] + (size_t) s * 8));
+            for (int e = 0; e < 2; e++) ax[n][e] = __ldg(reinterpret_cast<const int4 *>(a_d[n][e] + (size_t) sg * 8));
         }
         __syncwarp();                                           // every lane has used the stage about to be refilled
         issue((stage + STAGES - 1) % STAGES);

@@ -209,25 +209,27 @@ gemv_q4k_mma_kernel(const uint8_t * __restrict__ tiles, int nsb, int n_tiles, in
     const int8_t * a_qs[NT];
     const int8_t * a_b8[NT];
     const float *  a_dx[NT][2];
+    int            gs[NT];                                      // tokens of the octet (pib_oct)
 #pragma unroll
     for (int n = 0; n < NT; n++) {
-        const int tok = min(n * 8 + g, b - 1);
-        a_qs[n] = aqs + (size_t) tok * K + t * 64;
-        a_b8[n] = abs8 + (size_t) tok * nsb * 16 + (t & 1) * 4;
+        gs[n] = min(8, b - 8 * n);
+        a_qs[n] = aqs + (size_t) n * 8 * K + min(g, gs[n] - 1) * 64 + t * 16;
+        a_b8[n] = abs8 + ((size_t) n * 8 * nsb + min(g, gs[n] - 1)) * 16 + (t & 1) * 4;
 #pragma unroll
-        for (int e = 0; e < 2; e++) a_dx[n][e] = ad + (size_t) min(n * 8 + 2 * t + e, b - 1) * nsb;
+        for (int e = 0; e < 2; e++) a_dx[n][e] = ad + (size_t) n * 8 * nsb + min(2 * t + e, gs[n] - 1);
     }
     auto load_act = [&](act_frag<NT> & f, int s) {
 #pragma unroll
         for (int n = 0; n < NT; n++) {
-            const int4 * ap = reinterpret_cast<const int4 *>(a_qs[n] + (size_t) s * 256);
+            const int sg = s * gs[n];
+            const int4 * ap = reinterpret_cast<const int4 *>(a_qs[n] + (size_t) sg * 256);
 #pragma unroll
-            for (int c = 0; c < 4; c++) f.q[n][c] = __ldg(ap + c);
-            const int * bp = reinterpret_cast<const int *>(a_b8[n] + (size_t) s * 16);
+            for (int c = 0; c < 4; c++) f.q[n][c] = __ldg(ap + c * 4 * gs[n]);
+            const int * bp = reinterpret_cast<const int *>(a_b8[n] + (size_t) sg * 16);
             f.mh[n] = __ldg(bp);
             f.ml[n] = __ldg(bp + 2);
 #pragma unroll
-            for (int e = 0; e < 2; e++) f.dx[n][e] = __ldg(a_dx[n][e] + s);
+            for (int e = 0; e < 2; e++) f.dx[n][e] = __ldg(a_dx[n][e] + sg);
         }
     };
     act_frag<NT> A0;
@@ -356,7 +358,7 @@ gemv_q4k_mma_kernel(const uint8_t * __restrict__ tiles, int nsb, int n_tiles, in
 // (ACT_SMEM: the activation planes live in shared memory -- the prologue-fused kernel -- and are read with ordinary loads)
 template <int NT, bool ACT_SMEM = false>
 __device__ __forceinline__ void q4k_record(const int4 (&wq)[4], const int4 (&hq)[2], int s, int t, const int8_t * const (&a_qs)[NT],
-                                           const int8_t * const (&a_b8)[NT], const float * const (&a_dx)[NT][2], float (&acc)[NT][4]) {
+                                           const int8_t * const (&a_b8)[NT], const float * const (&a_dx)[NT][2], const int (&gs)[NT], float (&acc)[NT][4]) {
     const q4k_hdr H0 = decode_hdr(make_uint4((uint32_t) hq[0].x, (uint32_t) hq[0].y, (uint32_t) hq[0].z, (uint32_t) hq[0].w));
     const q4k_hdr H1 = decode_hdr(make_uint4((uint32_t) hq[1].x, (uint32_t) hq[1].y, (uint32_t) hq[1].z, (uint32_t) hq[1].w));
     int4  aq[NT][4];
@@ -364,14 +366,15 @@ __device__ __forceinline__ void q4k_record(const int4 (&wq)[4], const int4 (&hq)
     float adx[NT][2];
 #pragma unroll
     for (int n = 0; n < NT; n++) {
-        const int4 * ap = reinterpret_cast<const int4 *>(a_qs[n] + (size_t) s * 256);
+        const int sg = s * gs[n];
+        const int4 * ap = reinterpret_cast<const int4 *>(a_qs[n] + (size_t) sg * 256);
 #pragma unroll
-        for (int c = 0; c < 4; c++) aq[n][c] = ACT_SMEM ? ap[c] : __ldg(ap + c);
-        const int * bp = reinterpret_cast<const int *>(a_b8[n] + (size_t) s * 16);
+        for (int c = 0; c < 4; c++) aq[n][c] = ACT_SMEM ? ap[c * 4 * gs[n]] : __ldg(ap + c * 4 * gs[n]);
+        const int * bp = reinterpret_cast<const int *>(a_b8[n] + (size_t) sg * 16);
         amh[n] = ACT_SMEM ? bp[0] : __ldg(bp);
         aml[n] = ACT_SMEM ? bp[2] : __ldg(bp + 2);
 #pragma unroll
-        for (int e = 0; e < 2; e++) adx[n][e] = ACT_SMEM ? a_dx[n][e][s] : __ldg(a_dx[n][e] + s);
+        for (int e = 0; e < 2; e++) adx[n][e] = ACT_SMEM ? a_dx[n][e][sg] : __ldg(a_dx[n][e] + sg);
     }
     int sumi[NT][4], sumh[NT][4];
 #pragma unroll
@@ -448,13 +451,14 @@ gemv_q4k_direct_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K
     const int8_t * a_qs[NT];
     const int8_t * a_b8[NT];
     const float *  a_dx[NT][2];
+    int            gs[NT];                                      // tokens of the octet (pib_oct)
 #pragma unroll
     for (int n = 0; n < NT; n++) {
-        const int tok = min(n * 8 + g, b - 1);
-        a_qs[n] = aqs + (size_t) tok * K + t * 64;
-        a_b8[n] = abs8 + (size_t) tok * nsb * 16 + (t & 1) * 4;
+        gs[n] = min(8, b - 8 * n);
+        a_qs[n] = aqs + (size_t) n * 8 * K + min(g, gs[n] - 1) * 64 + t * 16;
+        a_b8[n] = abs8 + ((size_t) n * 8 * nsb + min(g, gs[n] - 1)) * 16 + (t & 1) * 4;
 #pragma unroll
-        for (int e = 0; e < 2; e++) a_dx[n][e] = ad + (size_t) min(n * 8 + 2 * t + e, b - 1) * nsb;
+        for (int e = 0; e < 2; e++) a_dx[n][e] = ad + (size_t) n * 8 * nsb + min(2 * t + e, gs[n] - 1);
     }
 
     int4 wq[4], hq[2];
@@ -484,7 +488,7 @@ gemv_q4k_direct_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K
             hn[0] = ld_stream_v4(hbase + (size_t) sn * MM_TILE_BYTES);
             hn[1] = ld_stream_v4(hbase + (size_t) sn * MM_TILE_BYTES + 128);
         }
-        q4k_record<NT>(wq, hq, s, t, a_qs, a_b8, a_dx, acc);
+        q4k_record<NT>(wq, hq, s, t, a_qs, a_b8, a_dx, gs, acc);
         if (sn < sb1) {
 #pragma unroll
             for (int c = 0; c < 4; c++) wq[c] = wn[c];
@@ -578,13 +582,14 @@ gemv_q4k_ring_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, 
     const int8_t * a_qs[NT];
     const int8_t * a_b8[NT];
     const float *  a_dx[NT][2];
+    int            gs[NT];                                      // tokens of the octet (pib_oct)
 #pragma unroll
     for (int n = 0; n < NT; n++) {
-        const int tok = min(n * 8 + g, b - 1);
-        a_qs[n] = aqs + (size_t) tok * K + t * 64;
-        a_b8[n] = abs8 + (size_t) tok * nsb * 16 + (t & 1) * 4;
+        gs[n] = min(8, b - 8 * n);
+        a_qs[n] = aqs + (size_t) n * 8 * K + min(g, gs[n] - 1) * 64 + t * 16;
+        a_b8[n] = abs8 + ((size_t) n * 8 * nsb + min(g, gs[n] - 1)) * 16 + (t & 1) * 4;
 #pragma unroll
-        for (int e = 0; e < 2; e++) a_dx[n][e] = ad + (size_t) min(n * 8 + 2 * t + e, b - 1) * nsb;
+        for (int e = 0; e < 2; e++) a_dx[n][e] = ad + (size_t) n * 8 * nsb + min(2 * t + e, gs[n] - 1);
     }
     pib_pdl_wait();
     pib_pdl_trigger();
@@ -600,7 +605,7 @@ gemv_q4k_ring_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, 
         for (int c = 0; c < 4; c++) wq[c] = *reinterpret_cast<const int4 *>(rs + c * 512 + lane * 16);
         hq[0] = *reinterpret_cast<const int4 *>(rs + 2048 + g * 16);
         hq[1] = *reinterpret_cast<const int4 *>(rs + 2048 + (g + 8) * 16);
-        q4k_record<NT>(wq, hq, s, t, a_qs, a_b8, a_dx, acc);
+        q4k_record<NT>(wq, hq, s, t, a_qs, a_b8, a_dx, gs, acc);
         stage = stage + 1 == STAGES ? 0 : stage + 1;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -759,8 +764,8 @@ gemv_q4k_pro_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, i
 #pragma unroll
             for (int j = 0; j < 8; j++) v[j] = xv[j];
         }
-        q8k_quantise_sb(v, lane, nullptr, s_qsp + (size_t) tk * K + sb * 256, nullptr, s_bs8 + ((size_t) tk * nsb + sb) * 16, nullptr, nullptr,
-                        s_d + (size_t) tk * nsb + sb);
+        const int os = sb * b + tk;                             // the octet order of the planes in memory
+        q8k_quantise_sb(v, lane, nullptr, s_qsp + (size_t) sb * b * 256 + tk * 64, nullptr, s_bs8 + (size_t) os * 16, nullptr, nullptr, s_d + os, nullptr, nullptr, nullptr, 64 * b);
     }
     __syncthreads();
 
@@ -769,12 +774,13 @@ gemv_q4k_pro_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, i
     const int8_t * a_qs[1];
     const int8_t * a_b8[1];
     const float *  a_dx[1][2];
+    const int      gs[1] = { b };
     {
         const int tok = min(g, b - 1);
-        a_qs[0] = s_qsp + (size_t) tok * K + t * 64;
-        a_b8[0] = s_bs8 + (size_t) tok * nsb * 16 + (t & 1) * 4;
+        a_qs[0] = s_qsp + tok * 64 + t * 16;
+        a_b8[0] = s_bs8 + tok * 16 + (t & 1) * 4;
 #pragma unroll
-        for (int e = 0; e < 2; e++) a_dx[0][e] = s_d + (size_t) min(2 * t + e, b - 1) * nsb;
+        for (int e = 0; e < 2; e++) a_dx[0][e] = s_d + min(2 * t + e, b - 1);
     }
     int stage = 0;
     for (int s = warp; s < nsb; s += GP_WARPS) {
@@ -788,7 +794,7 @@ gemv_q4k_pro_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, i
         for (int c = 0; c < 4; c++) wq[c] = *reinterpret_cast<const int4 *>(rs + c * 512 + lane * 16);
         hq[0] = *reinterpret_cast<const int4 *>(rs + 2048 + g * 16);
         hq[1] = *reinterpret_cast<const int4 *>(rs + 2048 + (g + 8) * 16);
-        q4k_record<1, true>(wq, hq, s, t, a_qs, a_b8, a_dx, acc);
+        q4k_record<1, true>(wq, hq, s, t, a_qs, a_b8, a_dx, gs, acc);
         stage = stage + 1 == STAGES ? 0 : stage + 1;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -871,13 +877,14 @@ gemv_q4k_stream_kernel(const uint8_t * __restrict__ tiles, int nsb, int n_tiles,
     const int8_t * a_qs[NT];
     const int8_t * a_b8[NT];
     const float *  a_dx[NT][2];
+    int            gs[NT];                                      // tokens of the octet (pib_oct)
 #pragma unroll
     for (int n = 0; n < NT; n++) {
-        const int tok = min(n * 8 + g, b - 1);
-        a_qs[n] = aqs + (size_t) tok * K + t * 64;
-        a_b8[n] = abs8 + (size_t) tok * nsb * 16 + (t & 1) * 4;
+        gs[n] = min(8, b - 8 * n);
+        a_qs[n] = aqs + (size_t) n * 8 * K + min(g, gs[n] - 1) * 64 + t * 16;
+        a_b8[n] = abs8 + ((size_t) n * 8 * nsb + min(g, gs[n] - 1)) * 16 + (t & 1) * 4;
 #pragma unroll
-        for (int e = 0; e < 2; e++) a_dx[n][e] = ad + (size_t) min(n * 8 + 2 * t + e, b - 1) * nsb;
+        for (int e = 0; e < 2; e++) a_dx[n][e] = ad + (size_t) n * 8 * nsb + min(2 * t + e, gs[n] - 1);
     }
     pib_pdl_wait();
     pib_pdl_trigger();
@@ -893,7 +900,7 @@ gemv_q4k_stream_kernel(const uint8_t * __restrict__ tiles, int nsb, int n_tiles,
         for (int c = 0; c < 4; c++) wq[c] = *reinterpret_cast<const int4 *>(rs + c * 512 + lane * 16);
         hq[0] = *reinterpret_cast<const int4 *>(rs + 2048 + g * 16);
         hq[1] = *reinterpret_cast<const int4 *>(rs + 2048 + (g + 8) * 16);
-        q4k_record<NT>(wq, hq, sb, t, a_qs, a_b8, a_dx, acc);
+        q4k_record<NT>(wq, hq, sb, t, a_qs, a_b8, a_dx, gs, acc);
         stage = stage + 1 == RG_STAGES ? 0 : stage + 1;
         if (++sb < nsb && u + 1 < u1) continue;
 
@@ -1022,7 +1029,7 @@ int pib_gemv_direct_launch(const pib_weight * w, const void * act_dev, int b, fl
     const int            nsb = (int) (w->K / 256), n_tiles = (int) ((w->N + 15) / 16);
     const dim3           grid(n_tiles, split);
     const int8_t *       aqs = (const int8_t *) (act + L.qsp_off);
-    const float *        ad  = (const float *) (act + L.d_off);
+    const float *        ad  = (const float *) (act + L.dxo_off);
     const int8_t *       bs  = (const int8_t *) (act + L.bs8_off);
     if (b <= 8) pib_launch(gemv_q4k_direct_kernel<1>, grid, dim3(MM_THREADS), 0, st, w->tiles, nsb, (int) w->N, (int) w->K, aqs, ad, bs, b, y_dev, partial, counters, cancel);
     else        pib_launch(gemv_q4k_direct_kernel<2>, grid, dim3(MM_THREADS), 0, st, w->tiles, nsb, (int) w->N, (int) w->K, aqs, ad, bs, b, y_dev, partial, counters, cancel);
@@ -1036,7 +1043,7 @@ int pib_gemv_mma_launch(const pib_weight * w, const void * act_dev, int b, float
     const uint8_t *      act = (const uint8_t *) act_dev;
     const int            nsb = (int) (w->K / 256), n_tiles = (int) ((w->N + 15) / 16);
     const int8_t *       aqs = (const int8_t *) (act + L.qsp_off);      // fragment-order quants
-    const float *        ad  = (const float *) (act + L.d_off);
+    const float *        ad  = (const float *) (act + L.dxo_off);
     const int8_t *       bs  = (const int8_t *) (act + L.bs8_off);
     static bool configured = false;
     if (!configured) {
@@ -1092,7 +1099,7 @@ int pib_gemv_ring(const pib_weight * w, const void * act_dev, int b, float * y_d
     const pib_act_layout L   = pib_act_layout_of(w->type, w->K, b);
     const uint8_t *      act = (const uint8_t *) act_dev;
     const int8_t * aqs = (const int8_t *) (act + L.qsp_off);
-    const float *  ad  = (const float *) (act + L.d_off);
+    const float *  ad  = (const float *) (act + L.dxo_off);
     const int8_t * bs  = (const int8_t *) (act + L.bs8_off);
     float * pp = s ? s->partial : nullptr;
     unsigned int * cc = s ? s->counters : nullptr;
@@ -1135,7 +1142,7 @@ int pib_gemv_stream(const pib_weight * w, const void * act_dev, int b, float * y
     const pib_act_layout L   = pib_act_layout_of(w->type, w->K, b);
     const uint8_t *      act = (const uint8_t *) act_dev;
     const int8_t * aqs = (const int8_t *) (act + L.qsp_off);
-    const float *  ad  = (const float *) (act + L.d_off);
+    const float *  ad  = (const float *) (act + L.dxo_off);
     const int8_t * bs  = (const int8_t *) (act + L.bs8_off);
     return b <= 8 ? stream_launch<1>(w, aqs, ad, bs, b, y_dev, runs, pmax, s->partial, s->counters, cancel, st)
                   : stream_launch<2>(w, aqs, ad, bs, b, y_dev, runs, pmax, s->partial, s->counters, cancel, st);

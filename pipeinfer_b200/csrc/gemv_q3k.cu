@@ -132,13 +132,14 @@ gemv_q3k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, co
     const int8_t * a_q[NT];
     const int8_t * a_b[NT];
     const float *  a_dx[NT][2];
+    int            gs[NT];                                      // tokens of the octet (pib_oct)
 #pragma unroll
     for (int n = 0; n < NT; n++) {
-        const int tok = min(n * 8 + g, b - 1);
-        a_q[n] = aq6 + (size_t) tok * K + t * 64;
-        a_b[n] = ab16 + (size_t) tok * nsb * 32 + 4 * t;
+        gs[n] = min(8, b - 8 * n);
+        a_q[n] = aq6 + (size_t) n * 8 * K + min(g, gs[n] - 1) * 64 + t * 16;
+        a_b[n] = ab16 + ((size_t) n * 8 * nsb + min(g, gs[n] - 1)) * 32 + 4 * t;
 #pragma unroll
-        for (int e = 0; e < 2; e++) a_dx[n][e] = ad + (size_t) min(n * 8 + 2 * t + e, b - 1) * nsb;
+        for (int e = 0; e < 2; e++) a_dx[n][e] = ad + (size_t) n * 8 * nsb + min(2 * t + e, gs[n] - 1);
     }
     pib_pdl_wait();
     pib_pdl_trigger();
@@ -159,13 +160,14 @@ gemv_q3k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, co
         const uint32_t s0t = t == 0 ? sc0.x : t == 1 ? sc0.y : t == 2 ? sc0.z : sc0.w, s1t = t == 0 ? sc1.x : t == 1 ? sc1.y : t == 2 ? sc1.z : sc1.w;
 #pragma unroll
         for (int n = 0; n < NT; n++) {
-            const int4 * ap = reinterpret_cast<const int4 *>(a_q[n] + (size_t) s * 256);
+            const int sg = s * gs[n];
+            const int4 * ap = reinterpret_cast<const int4 *>(a_q[n] + (size_t) sg * 256);
             int4 bq[4];
 #pragma unroll
-            for (int c = 0; c < 4; c++) bq[c] = __ldg(ap + c);
+            for (int c = 0; c < 4; c++) bq[c] = __ldg(ap + c * 4 * gs[n]);
             const int bw[16] = { bq[0].x, bq[0].y, bq[0].z, bq[0].w, bq[1].x, bq[1].y, bq[1].z, bq[1].w, bq[2].x, bq[2].y, bq[2].z, bq[2].w, bq[3].x, bq[3].y, bq[3].z, bq[3].w };
-            const int bh = __ldg(reinterpret_cast<const int *>(a_b[n] + (size_t) s * 32)), bl = __ldg(reinterpret_cast<const int *>(a_b[n] + (size_t) s * 32 + 16));
-            const float dx0 = __ldg(a_dx[n][0] + s), dx1 = __ldg(a_dx[n][1] + s);
+            const int bh = __ldg(reinterpret_cast<const int *>(a_b[n] + (size_t) sg * 32)), bl = __ldg(reinterpret_cast<const int *>(a_b[n] + (size_t) sg * 32 + 16));
+            const float dx0 = __ldg(a_dx[n][0] + sg), dx1 = __ldg(a_dx[n][1] + sg);
             int sum[4] = { 0, 0, 0, 0 };
 #pragma unroll
             for (int j = 0; j < 16; j++) {
@@ -220,7 +222,7 @@ static int launch_q3_tc(const pib_weight * w, const uint8_t * act, const pib_act
     }
     const int nsb = (int) (w->K / 256), n_tiles = (int) ((w->N + 15) / 16);
     PIB_CHECK(pib_launch(gemv_q3k_tc_kernel<NT>, dim3(n_tiles), dim3(Q3T_WARPS * 32), smem, st, w->tiles, nsb, (int) w->N, (int) w->K,
-                         (const int8_t *) (act + L.q6p_off), (const float *) (act + L.d_off), (const int8_t *) (act + L.b16_off), b, y, cancel));
+                         (const int8_t *) (act + L.q6p_off), (const float *) (act + L.dxo_off), (const int8_t *) (act + L.b16_off), b, y, cancel));
     return PIB_OK;
 }
 

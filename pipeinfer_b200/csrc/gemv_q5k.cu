@@ -186,13 +186,14 @@ gemv_q5k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, co
     const int8_t * a_qs[NT];
     const int8_t * a_b8[NT];
     const float *  a_dx[NT][2];
+    int            gs[NT];                                      // tokens of the octet (pib_oct)
 #pragma unroll
     for (int n = 0; n < NT; n++) {
-        const int tok = min(n * 8 + g, b - 1);
-        a_qs[n] = aqs + (size_t) tok * K + t * 64;
-        a_b8[n] = abs8 + (size_t) tok * nsb * 16 + (t & 1) * 4;
+        gs[n] = min(8, b - 8 * n);
+        a_qs[n] = aqs + (size_t) n * 8 * K + min(g, gs[n] - 1) * 64 + t * 16;
+        a_b8[n] = abs8 + ((size_t) n * 8 * nsb + min(g, gs[n] - 1)) * 16 + (t & 1) * 4;
 #pragma unroll
-        for (int e = 0; e < 2; e++) a_dx[n][e] = ad + (size_t) min(n * 8 + 2 * t + e, b - 1) * nsb;
+        for (int e = 0; e < 2; e++) a_dx[n][e] = ad + (size_t) n * 8 * nsb + min(2 * t + e, gs[n] - 1);
     }
     pib_pdl_wait();
     pib_pdl_trigger();
@@ -218,14 +219,15 @@ gemv_q5k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, co
         const uint32_t hw[4]  = { hb.x, hb.y, hb.z, hb.w };
 #pragma unroll
         for (int n = 0; n < NT; n++) {
-            const int4 * ap = reinterpret_cast<const int4 *>(a_qs[n] + (size_t) s * 256);
-            const int *  bp = reinterpret_cast<const int *>(a_b8[n] + (size_t) s * 16);
+            const int    sg = s * gs[n];
+            const int4 * ap = reinterpret_cast<const int4 *>(a_qs[n] + (size_t) sg * 256);
+            const int *  bp = reinterpret_cast<const int *>(a_b8[n] + (size_t) sg * 16);
             const int    amh = __ldg(bp), aml = __ldg(bp + 2);
-            const float  dx0 = __ldg(a_dx[n][0] + s), dx1 = __ldg(a_dx[n][1] + s);
+            const float  dx0 = __ldg(a_dx[n][0] + sg), dx1 = __ldg(a_dx[n][1] + sg);
             int sum[4] = { 0, 0, 0, 0 };
 #pragma unroll
             for (int c = 0; c < 4; c++) {
-                const int4     aq = __ldg(ap + c);
+                const int4     aq = __ldg(ap + c * 4 * gs[n]);
                 const uint32_t wx = wq[c].x, wy = wq[c].y, wz = wq[c].z, ww = wq[c].w, H = hw[c];
                 int c_lo[4] = { 0, 0, 0, 0 }, c_hi[4] = { 0, 0, 0, 0 };
                 q5_mma_u8s8(c_lo, (int) ((wx & 0x0F0F0F0Fu) | ((H << 4) & 0x10101010u)), (int) ((wz & 0x0F0F0F0Fu) | ((H << 3) & 0x10101010u)),
@@ -284,7 +286,7 @@ static int launch_q5_tc(const pib_weight * w, const uint8_t * act, const pib_act
     }
     const int nsb = (int) (w->K / 256), n_tiles = (int) ((w->N + 15) / 16);
     PIB_CHECK(pib_launch(gemv_q5k_tc_kernel<NT>, dim3(n_tiles), dim3(Q5T_WARPS * 32), smem, st, w->tiles, nsb, (int) w->N, (int) w->K,
-                         (const int8_t *) (act + L.qsp_off), (const float *) (act + L.d_off), (const int8_t *) (act + L.bs8_off), b, y, cancel));
+                         (const int8_t *) (act + L.qsp_off), (const float *) (act + L.dxo_off), (const int8_t *) (act + L.bs8_off), b, y, cancel));
     return PIB_OK;
 }
 

@@ -148,19 +148,22 @@ struct pib_act_layout {
     size_t d_off;      // float [b][K/32] (Q8_0 family) or [b][K/256] (Q8_K family)
     size_t bs_off;     // Q8_0 family: int32 [b][K/32] block sums (unused by the reference, used for the -8 offset);
                        // Q8_K family: int16 [b][K/16] bsums exactly as block_q8_K
-    size_t bs8_off;    // Q8_K family: int8 [b][K/256][16] = {hi_0..hi_7, lo_0..lo_7}: sub-block sums bsums[2j] + bsums[2j+1]
+    // Planes that the tensor-core matmuls read (bs8, qsp, q6p, b16, dxo): tokens 8n .. 8n + gs - 1 (gs = 8, the last ones fewer) are interleaved per super-block, in the order of
+    // a warp's loads: lane (g, t) takes token 8n + g.  Octet n starts at 8n rows; inside it [super-block][piece][gs tokens][...] (pib_oct).  (A token's row on its own made each load
+    // touch 16 lines where it now touches 4; the activations of 8 tokens are as many bytes as the weights.)
+    size_t bs8_off;    // Q8_K family: int8 [super-block][gs][16] = {hi_0..hi_7, lo_0..lo_7}: sub-block sums bsums[2j] + bsums[2j+1]
                        //   split as 64 * hi + lo (hi in [-64, 63], lo in [0, 63]) so that the min term of Q4_K can be a
                        //   tensor-core dot product; redundant with bs_off (same numbers)
-    size_t qsp_off;    // Q8_K family: int8 [b][K], the same quants as qs_off in tensor-core fragment order: inside each
-                       //   super-block, element e = 64c + 32h + 8t + i (chunk c, low/high-nibble half h, lane quarter t) is
-                       //   stored at 64t + 16c + 8h + i, so a lane's B fragments for all four chunks are 64 contiguous bytes
+    size_t qsp_off;    // Q8_K family: int8 [super-block][4 chunks c][gs][4 quarters t][16], the same quants as qs_off in tensor-core fragment order: element
+                       //   e = 64c + 32h + 8t + i (low/high-nibble half h) is byte 8h + i of piece (c, t), a lane's B fragments of chunk c
     size_t qsl_off;    // Q8_K family: int2 [b][K/256][8 lane groups g][8 sub-blocks j]: {x if g even else 0, x if g odd else 0} with x =
                        //   the four quants 4g .. 4g+3 of sub-block j -- the two B registers of the lane-exact kernel (gemv_q4k_lane.cu)
     size_t sbs_off;    // Q8_K family: int16 [b][K/32] sub-block sums bsums[2j] + bsums[2j+1]
-    size_t q6p_off;    // Q8_K family: int8 [b][K], the quants in the B-fragment order of mma.m16n8k16 over the 16-element groups of
-                       //   Q6_K: inside each super-block element e = 16j + 4t + i (group j, lane quarter t) sits at 64t + 4j + i
-    size_t b16_off;    // Q8_K family: int8 [b][K/256][32] = {hi_0..hi_15, lo_0..lo_15}: the 16 bsums split as 64 * hi + lo, so that the
+    size_t q6p_off;    // Q8_K family: int8 [super-block][4 quads c][gs][4 quarters t][16], the quants in the B-fragment order of mma.m16n8k16 over the 16-element groups of
+                       //   Q6_K: element e = 16j + 4t + i (group j = 4c + jj) is byte 4jj + i of piece (c, t)
+    size_t b16_off;    // Q8_K family: int8 [super-block][gs][32] = {hi_0..hi_15, lo_0..lo_15}: the 16 bsums split as 64 * hi + lo, so that the
                        //   -32 offset of Q6_K (sum_j scale_j * bsum_j) is two more tensor-core dot products (gemv_q6k.cu)
+    size_t dxo_off;    // Q8_K family: float [super-block][gs], the numbers of d_off
     size_t total;
 };
 __host__ __device__ inline pib_act_layout pib_act_layout_of(int wtype, int64_t K, int b) {
@@ -172,8 +175,8 @@ __host__ __device__ inline pib_act_layout pib_act_layout_of(int wtype, int64_t K
     L.bs_off = (L.d_off + nd * 4 + 255) & ~(size_t) 255;
     size_t nbs = (wtype == PIB_TYPE_Q4_K) ? (size_t) b * (K / 16) * 2 : (size_t) b * (K / PIB_QK) * 4;
     L.bs8_off = (L.bs_off + nbs + 255) & ~(size_t) 255;
-    // 32-element block formats: bs8 holds the "dxp" plane (fp16 block scales [b][ngr * 8], ngr = groups of 8 blocks, zero
-    // padded) and qsp the fragment-order quants [b][ngr * 256] of gemv_blk32.cu
+    // 32-element block formats: bs8 holds the "dxp" plane (fp16 block scales [group][gs][8], ngr = groups of 8 blocks, zero
+    // padded) and qsp the fragment-order quants [group][4 pieces][gs][4 quarters][16] of gemv_blk32.cu, octets of tokens as above
     const size_t ngr = (size_t) ((K + 255) / 256);
     size_t nbs8 = (wtype == PIB_TYPE_Q4_K) ? (size_t) b * (K / PIB_QK_K) * 16 : (size_t) b * ngr * 8 * 2;
     L.qsp_off = (L.bs8_off + nbs8 + 255) & ~(size_t) 255;
@@ -181,6 +184,10 @@ __host__ __device__ inline pib_act_layout pib_act_layout_of(int wtype, int64_t K
     L.sbs_off = (L.qsl_off + ((wtype == PIB_TYPE_Q4_K) ? 2 * qs : 0) + 255) & ~(size_t) 255;
     L.q6p_off = (L.sbs_off + ((wtype == PIB_TYPE_Q4_K) ? (size_t) b * (K / 32) * 2 : 0) + 255) & ~(size_t) 255;
     L.b16_off = (L.q6p_off + ((wtype == PIB_TYPE_Q4_K) ? qs : 0) + 255) & ~(size_t) 255;
-    L.total   = (L.b16_off + ((wtype == PIB_TYPE_Q4_K) ? (size_t) b * (K / PIB_QK_K) * 32 : 0) + 255) & ~(size_t) 255;
+    L.dxo_off = (L.b16_off + ((wtype == PIB_TYPE_Q4_K) ? (size_t) b * (K / PIB_QK_K) * 32 : 0) + 255) & ~(size_t) 255;
+    L.total   = (L.dxo_off + ((wtype == PIB_TYPE_Q4_K) ? nd * 4 : 0) + 255) & ~(size_t) 255;
     return L;
 }
+// where row `row` of b lies in an octet plane: the rows in front of its octet, its number in the octet and the octet's rows
+struct pib_oct { int before, g, gs; };
+__host__ __device__ __forceinline__ pib_oct pib_oct_of(int row, int b) { const int n8 = row & ~7, left = b - n8; return { n8, row - n8, left < 8 ? left : 8 }; }

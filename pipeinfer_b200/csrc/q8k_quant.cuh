@@ -10,13 +10,13 @@
 __host__ __device__ __forceinline__ int tg_kpos(int e) { return (e & 32) + ((e >> 2) & 1) * 16 + ((e >> 3) & 3) * 4 + ((e & 1) << 1 | ((e >> 1) & 1)); }
 
 // Every pointer addresses this super-block's part of its plane (see pib_act_layout) and may be null:
-//   qs   [256] int8   quants in element order           qsp [256] int8   the same in B-fragment order of mma.m16n8k32
+//   qs   [256] int8   quants in element order           qsp  int8   the same in B-fragment order of mma.m16n8k32: four pieces of 64, `cs` bytes apart
 //   bs   [16]  int16  sums of 16                         bs8 [16]  int8   sub-block (32) sums split as 64 hi + lo: hi[8], lo[8]
 //   sbs  [8]   int16  sub-block sums                     qsl [64]  int2   B registers of the lane-exact kernel     d [1] float
 //   xh   [256] fp16   quants times d in the GEMM's order (tg_kpos)
-//   q6p  [256] int8   quants in the k16 B-fragment order of the Q6_K kernel      b16 [32] int8   sums of 16 split as 64 hi + lo: hi[16], lo[16]
+//   q6p  int8   quants in the k16 B-fragment order of the Q6_K kernel, pieces as qsp's      b16 [32] int8   sums of 16 split as 64 hi + lo: hi[16], lo[16]
 __device__ __forceinline__ void q8k_quantise_sb(const float (&v)[8], int lane, int8_t * qs, int8_t * qsp, int16_t * bs, int8_t * bs8,
-                                                int16_t * sbs, int2 * qsl, float * d, int8_t * q6p = nullptr, int8_t * b16 = nullptr, __half * xh = nullptr) {
+                                                int16_t * sbs, int2 * qsl, float * d, int8_t * q6p = nullptr, int8_t * b16 = nullptr, __half * xh = nullptr, int cs = 64, float * dxo = nullptr) {
     // first element (in index order) with the largest |x|: strict '>' scan, ties keep the lower index
     float amax = 0.0f, mx = 0.0f;
     int   idx  = 1 << 30;
@@ -57,12 +57,13 @@ __device__ __forceinline__ void q8k_quantise_sb(const float (&v)[8], int lane, i
     packed.x = (q[0] & 0xff) | ((q[1] & 0xff) << 8) | ((q[2] & 0xff) << 16) | ((q[3] & 0xff) << 24);
     packed.y = (q[4] & 0xff) | ((q[5] & 0xff) << 8) | ((q[6] & 0xff) << 16) | ((q[7] & 0xff) << 24);
     if (qs) *reinterpret_cast<int2 *>(qs + lane * 8) = packed;
-    // fragment-order copy for the tensor-core GEMV: lane = 8c + 4h + t  ->  offset 64t + 16c + 8h
-    if (qsp) *reinterpret_cast<int2 *>(qsp + (lane & 3) * 64 + (lane >> 3) * 16 + ((lane >> 2) & 1) * 8) = packed;
+    // fragment-order copy for the tensor-core GEMV: lane = 8c + 4h + t  ->  piece c, offset 16t + 8h
+    if (qsp) *reinterpret_cast<int2 *>(qsp + (lane >> 3) * cs + (lane & 3) * 16 + ((lane >> 2) & 1) * 8) = packed;
     // lane l holds elements 8l .. 8l+7 = group l / 2, offsets 8 (l & 1) ..: quarters t = 2 (l & 1) and 2 (l & 1) + 1
     if (q6p) {
-        *reinterpret_cast<int *>(q6p + (2 * (lane & 1)) * 64 + (lane >> 1) * 4)     = packed.x;
-        *reinterpret_cast<int *>(q6p + (2 * (lane & 1) + 1) * 64 + (lane >> 1) * 4) = packed.y;
+        int8_t * o = q6p + (lane >> 3) * cs + (2 * (lane & 1)) * 16 + ((lane >> 1) & 3) * 4;
+        *reinterpret_cast<int *>(o)      = packed.x;
+        *reinterpret_cast<int *>(o + 16) = packed.y;
     }
     const int s8  = q[0] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + q[7];
     const int s16 = s8 + __shfl_xor_sync(0xffffffffu, s8, 1);
@@ -80,4 +81,5 @@ __device__ __forceinline__ void q8k_quantise_sb(const float (&v)[8], int lane, i
         o[8] = make_int2(0, packed.y);
     }
     if (d && lane == 0) *d = dval;
+    if (dxo && lane == 0) *dxo = dval;
 }
