@@ -239,10 +239,11 @@ gemv_blk32_kernel(const uint8_t * __restrict__ tiles, int ngr, int N, const int8
 // The same without a K split, for row tiles that are there (nearly) all at once: WARPS warps per tile, every warp streams its records through a private ring in shared
 // memory filled by cp.async, STAGES - 1 of them in flight (as gemv_q4k_ring_kernel).
 // What bounds it: a warp's chain of memory latencies, which more warps and a deeper prefetch shorten.  4096 x 4096 Q4_0 at 8 / 16 tokens 6.2 / 12.0 -> 4.4 / 7.7 us,
-// 4096 x 11008 9.8 / 20.8 -> 8.5 / 15.5, 11264 x 2048 (four warps) 7.3 -> 5.3.  With more rounds of tiles new CTAs keep arriving with their first records in flight, the
+// 4096 x 11008 9.8 / 20.8 -> 8.5 / 15.5, 11264 x 2048 (four warps) 7.3 -> 5.3; two token groups with two CTAs per SM instead of one: 4096 x 4096 7.0 -> 4.3,
+// 4096 x 11008 12.7 -> 9.3, 8192 x 4096 13.0 -> 8.0.  With one token group and more rounds of tiles new CTAs keep arriving with their first records in flight, the
 // ring's extra pass through shared memory is what counts (22016 x 4096 at 7 tokens 16.0 -> 16.5, Q8_0 18.9 -> 24.5), and gemv_blk32_kernel stays: pib_gemv_blk32.
 template <int WT, int NT, int WARPS, int STAGES>
-__global__ void __launch_bounds__(WARPS * 32, NT == 1 ? (WARPS == 4 ? 5 : 2) : (WARPS == 4 ? 3 : 1))
+__global__ void __launch_bounds__(WARPS * 32, NT == 1 ? (WARPS == 4 ? 5 : 2) : (WARPS == 4 ? 3 : 2))
 gemv_blk32_ring_kernel(const uint8_t * __restrict__ tiles, int ngr, int N, const int8_t * __restrict__ aqs, const __half * __restrict__ adx, int b, float * __restrict__ y, const int * __restrict__ cancel) {
     if (PIB_CANCELLED(cancel)) { pib_pdl_wait(); return; }
     constexpr int REC = WT == PIB_TYPE_Q4_0 ? 2304 : 4352, PIECES = (REC + 511) / 512;        // 512 bytes per warp-wide copy, the last one half
@@ -393,10 +394,11 @@ bool pib_gemv_blk32_supported(const pib_weight * w, int b) {
 
 template <int WT, int NT, int WARPS, int STAGES>
 static int bk_ring_launch(const pib_weight * w, int ngr, const int8_t * aqs, const __half * adx, int b, float * y_dev, const int * cancel, cudaStream_t st) {
-    const size_t smem = (size_t) WARPS * STAGES * bk_rec_bytes(WT);
+    const int    n_tiles = (int) ((w->N + 15) / 16);
+    const size_t ring = (size_t) WARPS * STAGES * bk_rec_bytes(WT), smem = WARPS == 8 ? pib_gemv_smem_spread(ring, n_tiles) : ring;
     static bool configured = false;
-    if (!configured) { PIB_CHECK(cudaFuncSetAttribute(gemv_blk32_ring_kernel<WT, NT, WARPS, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)); configured = true; }
-    PIB_CHECK(pib_launch(gemv_blk32_ring_kernel<WT, NT, WARPS, STAGES>, dim3((unsigned) ((w->N + 15) / 16)), dim3(WARPS * 32), smem, st, w->tiles, ngr, (int) w->N, aqs, adx, b, y_dev, cancel));
+    if (!configured) { PIB_CHECK(cudaFuncSetAttribute(gemv_blk32_ring_kernel<WT, NT, WARPS, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (ring > PIB_GEMV_SPREAD ? ring : PIB_GEMV_SPREAD))); configured = true; }
+    PIB_CHECK(pib_launch(gemv_blk32_ring_kernel<WT, NT, WARPS, STAGES>, dim3((unsigned) n_tiles), dim3(WARPS * 32), smem, st, w->tiles, ngr, (int) w->N, aqs, adx, b, y_dev, cancel));
     return PIB_OK;
 }
 
@@ -407,22 +409,22 @@ int pib_gemv_blk32(const pib_weight * w, const void * act_dev, int b, float * y_
     const int            ngr = (int) ((w->K + 255) / 256), n_tiles = (int) ((w->N + 15) / 16);
     const int8_t *       aqs = (const int8_t *) (act + L.qsp_off);
     const __half *       adx = (const __half *) (act + L.bs8_off);    // dxp plane of the 32-element block formats
-    // The ring kernels or the K split below, by where each was faster (us, ring / K split).  What decides are rounds: of the ring's eight-warp CTAs an SM holds two (one for
-    // two token groups), of its four-warp CTAs five, of the K split's four.
+    // The ring kernels or the K split below, by where each was faster (us, ring / K split).  What decides are rounds: of the ring's eight-warp CTAs an SM holds two, of its
+    // four-warp CTAs five, of the K split's four.
     // One token group, eight warps: while the K split would split, since from 80 % of its slots on it runs unsplit in one round (4096 wide, 8 tokens: 444 tiles of Q4_0
     // 7.3 / 10.1, 512 tiles 7.3 / 6.7; Q8_0 8.6 / 10.6 and 8.9 / 7.2).
-    // Two token groups: up to four rounds (592 tiles of Q4_0, 13 tokens: 4096 wide 13.7 / 15.3, 28672 wide 58.7 / 82.7; 740 tiles 16.8 / 15.6), but no second round with
-    // little in it of long rows (28672 wide, 149 tiles 28.1 / 26.0, 222 28.8 / 27.4, 240 28.8 / 40.9; 14848 wide, 149 15.2 / 15.9).
+    // Two token groups (behind a quantiser, 13 tokens): any number of tiles of Q4_0 (4096 wide, 740 tiles 12.8 / 14.6, 1376 20.9 / 23.0, 2000 27.5 / 28.8); of Q8_0 up to four tiles
+    // per SM and rows from 6144 on (4096 wide, 592 tiles 13.1 / 15.8, 880 18.5 / 17.1, 1184 22.9 / 22.2; 8192 wide, 740 25.4 / 26.7, 1376 40.6 / 45.5).
     // Few tiles of long rows go to the K split, which divides a row over up to 64 warps (28672 wide, 32 tiles: 8.8 / 5.1 and, 13 tokens, 14.5 / 11.0; 64 tiles 9.2 / 6.9 and
     // 14.6 / 15.8; 80 tiles 9.3 / 9.9; 8192 wide, 16 tiles 3.3 / 3.2, 48 3.5 / 4.1).
     // Four warps (Q4_0, one token group): one round of them, where eight make a second round with little in it, where the K split would split, takes a second round, or has too few records per
     // warp (8 tokens: 28672 wide, 328 tiles 28.1, eight warps 33.5, K split 30.9, 740 tiles 43.8 / 58.6; 2048 wide, 444 tiles 4.3 / 7.3, 592 4.5 / 4.7; 3072 wide, 592 6.0 / 5.7).
     const int  sms = pib_num_sms(), fill = pib_split_fill_target();
-    const bool two = b > 8, thin = n_tiles > sms && 5 * n_tiles < 8 * sms && ngr > 72;
+    const bool two = b > 8;
     const bool four = w->type == PIB_TYPE_Q4_0 && !two && n_tiles > 2 * sms && n_tiles <= 5 * sms && (ngr <= 8 || 5 * n_tiles <= 12 * sms || n_tiles > 4 * sms || (ngr < 16 && n_tiles < fill));
     const bool wide = ngr == 16 || 2 * n_tiles >= 3 * ngr || (two ? 5 * n_tiles >= 2 * sms : 2 * n_tiles > sms);
     if (four) return bk_ring_launch<PIB_TYPE_Q4_0, 1, 4, 4>(w, ngr, aqs, adx, b, y_dev, cancel, st);
-    if (ngr >= 16 && wide && (two ? n_tiles <= 4 * sms && !thin : n_tiles < fill)) {
+    if (ngr >= 16 && wide && (two ? w->type == PIB_TYPE_Q4_0 || n_tiles <= 4 * sms || ngr >= 24 : n_tiles < fill)) {
         if (w->type == PIB_TYPE_Q4_0) return two ? bk_ring_launch<PIB_TYPE_Q4_0, 2, 8, 4>(w, ngr, aqs, adx, b, y_dev, cancel, st) : bk_ring_launch<PIB_TYPE_Q4_0, 1, 8, 4>(w, ngr, aqs, adx, b, y_dev, cancel, st);
         return two ? bk_ring_launch<PIB_TYPE_Q8_0, 2, 8, 3>(w, ngr, aqs, adx, b, y_dev, cancel, st) : bk_ring_launch<PIB_TYPE_Q8_0, 1, 8, 3>(w, ngr, aqs, adx, b, y_dev, cancel, st);
     }

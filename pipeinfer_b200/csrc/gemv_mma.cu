@@ -19,6 +19,7 @@
 // k-slot 16+4t+i <-> element 8t+4+i" (the activations use the same permutation, so every B fragment is one contiguous
 // 8-byte load).  Then the 16 row headers {fp16 d, fp16 dmin, scales[12]}.  2304 bytes per (T, S), consecutive S
 // contiguous: every warp-wide load instruction reads 512 contiguous bytes.
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -540,7 +541,7 @@ gemv_q4k_direct_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K
 // super-blocks of the tile): 8 for single-wave shapes, 4 otherwise.
 #define RG_STAGES 4
 template <int NT, int WARPS, int STAGES>
-__global__ void __launch_bounds__(WARPS * 32, NT == 1 ? (WARPS == 4 ? 5 : 2) : (WARPS == 4 ? 3 : 1))
+__global__ void __launch_bounds__(WARPS * 32, NT == 1 ? (WARPS == 4 ? 5 : 2) : (WARPS == 4 ? 3 : 2))
 gemv_q4k_ring_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, const int8_t * __restrict__ aqs,
                      const float * __restrict__ ad, const int8_t * __restrict__ abs8, int b, float * __restrict__ y,
                      float * __restrict__ partial, unsigned int * __restrict__ counters, const int * __restrict__ cancel) {
@@ -1063,30 +1064,27 @@ int pib_gemv_mma_launch(const pib_weight * w, const void * act_dev, int b, float
 template <int NT, int WARPS, int STAGES>
 static int ring_launch(const pib_weight * w, const int8_t * aqs, const float * ad, const int8_t * bs, int b, float * y_dev, int split, float * partial,
                        unsigned int * counters, const int * cancel, cudaStream_t st) {
-    const size_t smem = (size_t) WARPS * STAGES * MM_TILE_BYTES;
+    const int    nsb = (int) (w->K / 256), n_tiles = (int) ((w->N + 15) / 16);
+    const size_t ring = (size_t) WARPS * STAGES * MM_TILE_BYTES, smem = WARPS == 8 ? pib_gemv_smem_spread(ring, n_tiles * split) : ring;
     static bool configured = false;
-    if (!configured) { PIB_CHECK(cudaFuncSetAttribute(gemv_q4k_ring_kernel<NT, WARPS, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)); configured = true; }
-    const int nsb = (int) (w->K / 256), n_tiles = (int) ((w->N + 15) / 16);
+    if (!configured) { PIB_CHECK(cudaFuncSetAttribute(gemv_q4k_ring_kernel<NT, WARPS, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) std::max(ring, (size_t) PIB_GEMV_SPREAD))); configured = true; }
     pib_launch(gemv_q4k_ring_kernel<NT, WARPS, STAGES>, dim3(n_tiles, split), dim3(WARPS * 32), smem, st, w->tiles, nsb, (int) w->N, (int) w->K, aqs, ad, bs, b, y_dev,
                partial, counters, cancel);
     PIB_CHECK(cudaGetLastError());
     return PIB_OK;
 }
 
-// variant 0 / 2: the ring kernel (cp.async-staged); PIB_Q4K_FAST=direct selects the register-prefetched direct kernel instead
-int pib_gemv_stream(const pib_weight * w, const void * act_dev, int b, float * y_dev, const int * cancel, cudaStream_t st);
-static bool stream_plan(int n_tiles, int nsb, int b, int * runs, int * pmax);
+// Q3_K, Q5_K, Q6_K: eight warps per tile while two such CTAs per SM take all tiles at once; below 8 super-blocks a warp would go without a record (us behind a quantiser, four / eight
+// warps: Q6_K 4096 x 4096 at 4 tokens 6.3 / 5.9, at 12 8.8 / 7.7, 4096 x 11008 13.7 / 12.0 and 18.1 / 16.6; 8192 x 4096 9.6 / 10.3; Q3_K 4096 x 11008 12.8 / 10.2)
+bool pib_gemv_wide(const pib_weight * w) { return (w->N + 15) / 16 <= 2 * pib_num_sms() && w->K / 256 >= 8; }
 
+// variant 0 / 2: the ring kernel (cp.async-staged); PIB_Q4K_FAST=direct selects the register-prefetched direct kernel instead
 int pib_gemv_ring(const pib_weight * w, const void * act_dev, int b, float * y_dev, const int * cancel, cudaStream_t st) {
     if (!pib_gemv_mma_supported(w, b)) { pib_set_error("pib_gemv: variant 2 needs Q4_K weights with tiles"); return PIB_ERR_UNSUPP; }
     const int nsb = (int) (w->K / 256), n_tiles = (int) ((w->N + 15) / 16);
-    // 9 .. 16 tokens (two column blocks per record): a record costs twice the issue slots, the SM with the most records sets the
-    // time, and the balanced stream kernel wins on every 70B shape (gate|up 100 vs 108 us, down 53 vs 63, attn_out 21 vs 23);
-    // at <= 8 tokens the tile-per-CTA ring is ahead (42 vs 53, 28 vs 30, 10.4 vs 12.7)
-    {
-        int runs = 0, pmax = 0;
-        if (b > 8 && (long long) n_tiles * nsb >= 16384 && stream_plan(n_tiles, nsb, b, &runs, &pmax)) return pib_gemv_stream(w, act_dev, b, y_dev, cancel, st);
-    }
+    // Also at 9 .. 16 tokens (two column blocks per record): with the activation planes in load order and two CTAs of eight warps per SM the tile-per-CTA ring is ahead of the
+    // balanced stream kernel (variant 8) behind a quantiser, whose CTAs find no room beside the stream's (us: 8192 x 28672 at 9 / 16 tokens 51.7 65.9 / 40.2 41.3, 22016 x 4096 at 13
+    // 22.0 / 18.7, 4096 x 11008 14.3 / 12.6, 57344 x 8192 at 9 75.8 / 66.9, at 16 76.8 / 77.8)
     // one wave of CTAs or less (4 CTAs of 4 warps per SM): eight warps per tile halve every warp's chain of records.  With 8 to 15 super-blocks they take the place of
     // K shares, which meet through memory (K = 2048, shares / eight warps, us: 2560 rows at 1 token 3.5 / 2.0, at 12 5.2 / 4.1; 4096 at 1 4.0 / 2.2); tiles enough to go
     // without shares keep four warps (8192 rows: 3.1 / 4.2)
@@ -1107,7 +1105,7 @@ int pib_gemv_ring(const pib_weight * w, const void * act_dev, int b, float * y_d
     return b <= 8 ? ring_launch<1, 4, 4>(w, aqs, ad, bs, b, y_dev, split, pp, cc, cancel, st) : ring_launch<2, 4, 4>(w, aqs, ad, bs, b, y_dev, split, pp, cc, cancel, st);
 }
 
-// variant 8 (and the default for shapes whose row tiles do not fill the machine evenly): the balanced stream kernel
+// variant 8: the balanced stream kernel
 template <int NT>
 static int stream_launch(const pib_weight * w, const int8_t * aqs, const float * ad, const int8_t * bs, int b, float * y_dev, int W, int pmax,
                          float * partial, unsigned int * counters, const int * cancel, cudaStream_t st) {

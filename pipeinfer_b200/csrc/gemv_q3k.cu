@@ -19,10 +19,11 @@
 // the activations' 16-sums (b16 plane), as for Q6_K's - 32.
 #include "pib_common.cuh"
 
+bool pib_gemv_wide(const pib_weight * w);      // gemv_mma.cu
+
 #include <stdlib.h>
 
 #define Q3T_BYTES  1824
-#define Q3T_WARPS  4
 #define Q3T_STAGES 4
 
 __device__ __forceinline__ void q3_mma_u8s8_k16(int (&c)[4], int a0, int a1, int b0) {
@@ -100,8 +101,8 @@ int pib_weight_build_tiles_q3k(pib_weight * w) {
     return PIB_OK;
 }
 
-template <int NT>
-__global__ void __launch_bounds__(Q3T_WARPS * 32, NT == 1 ? 4 : 3)
+template <int NT, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : NT == 1 ? 4 : 3)
 gemv_q3k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, const int8_t * __restrict__ aq6, const float * __restrict__ ad,
                    const int8_t * __restrict__ ab16, int b, float * __restrict__ y, const int * __restrict__ cancel) {
     if (PIB_CANCELLED(cancel)) { pib_pdl_wait(); return; }
@@ -119,7 +120,7 @@ gemv_q3k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, co
 #pragma unroll
             for (int c = 0; c < 3; c++) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + c * 512), "l"(src + c * 512) : "memory");
             if (lane < 18) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 1536), "l"(src + 1536) : "memory");
-            ps += Q3T_WARPS;
+            ps += WARPS;
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -144,7 +145,7 @@ gemv_q3k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, co
     pib_pdl_wait();
     pib_pdl_trigger();
     int stage = 0;
-    for (int s = warp; s < nsb; s += Q3T_WARPS) {
+    for (int s = warp; s < nsb; s += WARPS) {
         __syncwarp();
         issue((stage + Q3T_STAGES - 1) % Q3T_STAGES);
         asm volatile("cp.async.wait_group %0;" ::"n"(Q3T_STAGES - 1) : "memory");
@@ -200,28 +201,34 @@ gemv_q3k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, co
             red[warp][n * 8 + 2 * t + e][g + 8] = acc[n][2 + e];
         }
     __syncthreads();
-    for (int i = threadIdx.x; i < NT * 8 * 16; i += Q3T_WARPS * 32) {
+    for (int i = threadIdx.x; i < NT * 8 * 16; i += WARPS * 32) {
         const int tok = i / 16, r = i % 16, row = T * 16 + r;
         if (tok < b && row < N) {
             float v = red[0][tok][r];
 #pragma unroll
-            for (int w2 = 1; w2 < Q3T_WARPS; w2++) v += red[w2][tok][r];
+            for (int w2 = 1; w2 < 4; w2++) v += red[w2][tok][r];
+            if (WARPS == 8) {
+                float u = red[4 % WARPS][tok][r];
+#pragma unroll
+                for (int w2 = 5; w2 < 8; w2++) u += red[w2 % WARPS][tok][r];
+                v += u;
+            }
             y[(size_t) tok * N + row] = v;
         }
     }
 }
 
-template <int NT>
+template <int NT, int WARPS>
 static int launch_q3_tc(const pib_weight * w, const uint8_t * act, const pib_act_layout & L, int b, float * y, const int * cancel, cudaStream_t st) {
-    const size_t smem = (size_t) Q3T_WARPS * Q3T_STAGES * Q3T_BYTES;
+    const int    nsb = (int) (w->K / 256), n_tiles = (int) ((w->N + 15) / 16);
+    const size_t ring = (size_t) WARPS * Q3T_STAGES * Q3T_BYTES, smem = WARPS == 8 ? pib_gemv_smem_spread(ring, n_tiles) : ring;
     static bool configured = false;
     if (!configured) {
-        PIB_CHECK(cudaFuncSetAttribute(gemv_q3k_tc_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-        PIB_CHECK(cudaFuncSetAttribute(gemv_q3k_tc_kernel<NT>, cudaFuncAttributePreferredSharedMemoryCarveout, (int) cudaSharedmemCarveoutMaxShared));
+        PIB_CHECK(cudaFuncSetAttribute(gemv_q3k_tc_kernel<NT, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (ring > PIB_GEMV_SPREAD ? ring : PIB_GEMV_SPREAD)));
+        PIB_CHECK(cudaFuncSetAttribute(gemv_q3k_tc_kernel<NT, WARPS>, cudaFuncAttributePreferredSharedMemoryCarveout, (int) cudaSharedmemCarveoutMaxShared));
         configured = true;
     }
-    const int nsb = (int) (w->K / 256), n_tiles = (int) ((w->N + 15) / 16);
-    PIB_CHECK(pib_launch(gemv_q3k_tc_kernel<NT>, dim3(n_tiles), dim3(Q3T_WARPS * 32), smem, st, w->tiles, nsb, (int) w->N, (int) w->K,
+    PIB_CHECK(pib_launch(gemv_q3k_tc_kernel<NT, WARPS>, dim3(n_tiles), dim3(WARPS * 32), smem, st, w->tiles, nsb, (int) w->N, (int) w->K,
                          (const int8_t *) (act + L.q6p_off), (const float *) (act + L.dxo_off), (const int8_t *) (act + L.b16_off), b, y, cancel));
     return PIB_OK;
 }
@@ -230,7 +237,8 @@ int pib_gemv_q3k(const pib_weight * w, const void * act_dev, int b, float * y_de
     if (!w || w->type != PIB_TYPE_Q3_K || !w->tiles || b < 1 || b > PIB_MAX_BATCH) { pib_set_error("pib_gemv: not a resident Q3_K matrix (or batch > %d)", PIB_MAX_BATCH); return PIB_ERR_UNSUPP; }
     const pib_act_layout L   = pib_act_layout_of(PIB_TYPE_Q4_K, w->K, b);          // Q8_K family activations
     const uint8_t *      act = (const uint8_t *) act_dev;
-    return b <= 8 ? launch_q3_tc<1>(w, act, L, b, y_dev, cancel, st) : launch_q3_tc<2>(w, act, L, b, y_dev, cancel, st);
+    if (pib_gemv_wide(w)) return b <= 8 ? launch_q3_tc<1, 8>(w, act, L, b, y_dev, cancel, st) : launch_q3_tc<2, 8>(w, act, L, b, y_dev, cancel, st);
+    return b <= 8 ? launch_q3_tc<1, 4>(w, act, L, b, y_dev, cancel, st) : launch_q3_tc<2, 4>(w, act, L, b, y_dev, cancel, st);
 }
 
 // embedding rows: dequantize_row_q3_K (ggml-quants.c:1711-1758), one thread per element, same float operations in the same order

@@ -11,6 +11,8 @@
 // PIB_Q5K_TC=0); the default is the tensor-core kernel on fragment-major records further down.
 #include "pib_common.cuh"
 
+bool pib_gemv_wide(const pib_weight * w);      // gemv_mma.cu
+
 #include <stdlib.h>
 
 #define Q5_WARPS 4
@@ -90,7 +92,6 @@ static cudaError_t launch_q5(const pib_weight * w, const uint8_t * act, const pi
 // s = 4 sub + 2 lhalf + rowsel (sub: low / high-nibble sub-block 2c / 2c+1; lhalf: chunk positions 8t.. / 8t+4..; rowsel: row g / g+8),
 // so every A register is (nibbles & 0x0f0f0f0f) | ((word >> s) & 0x01010101) << 4.  Integer sums exact, fp32 terms per super-block.
 #define Q5T_BYTES  2816
-#define Q5T_WARPS  4
 #define Q5T_STAGES 4
 
 __device__ __forceinline__ void q5_mma_u8s8(int (&c)[4], int a0, int a1, int a2, int a3, int b0, int b1) {
@@ -153,8 +154,8 @@ int pib_weight_build_tiles_q5k(pib_weight * w) {
     return PIB_OK;
 }
 
-template <int NT>
-__global__ void __launch_bounds__(Q5T_WARPS * 32, NT == 1 ? 4 : 3)
+template <int NT, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : NT == 1 ? 4 : 3)
 gemv_q5k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, const int8_t * __restrict__ aqs, const float * __restrict__ ad,
                    const int8_t * __restrict__ abs8, int b, float * __restrict__ y, const int * __restrict__ cancel) {
     if (PIB_CANCELLED(cancel)) { pib_pdl_wait(); return; }
@@ -173,7 +174,7 @@ gemv_q5k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, co
             for (int c = 0; c < 4; c++) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + c * 512), "l"(src + c * 512) : "memory");
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 2304), "l"(src + 2304) : "memory");
             if (lane < 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 2048), "l"(src + 2048) : "memory");
-            ps += Q5T_WARPS;
+            ps += WARPS;
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -198,7 +199,7 @@ gemv_q5k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, co
     pib_pdl_wait();
     pib_pdl_trigger();
     int stage = 0;
-    for (int s = warp; s < nsb; s += Q5T_WARPS) {
+    for (int s = warp; s < nsb; s += WARPS) {
         __syncwarp();
         issue((stage + Q5T_STAGES - 1) % Q5T_STAGES);
         asm volatile("cp.async.wait_group %0;" ::"n"(Q5T_STAGES - 1) : "memory");
@@ -264,28 +265,34 @@ gemv_q5k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, co
             red[warp][n * 8 + 2 * t + e][g + 8] = acc[n][2 + e];
         }
     __syncthreads();
-    for (int i = threadIdx.x; i < NT * 8 * 16; i += Q5T_WARPS * 32) {
+    for (int i = threadIdx.x; i < NT * 8 * 16; i += WARPS * 32) {
         const int tok = i / 16, r = i % 16, row = T * 16 + r;
         if (tok < b && row < N) {
             float v = red[0][tok][r];
 #pragma unroll
-            for (int w2 = 1; w2 < Q5T_WARPS; w2++) v += red[w2][tok][r];
+            for (int w2 = 1; w2 < 4; w2++) v += red[w2][tok][r];
+            if (WARPS == 8) {
+                float u = red[4 % WARPS][tok][r];
+#pragma unroll
+                for (int w2 = 5; w2 < 8; w2++) u += red[w2 % WARPS][tok][r];
+                v += u;
+            }
             y[(size_t) tok * N + row] = v;
         }
     }
 }
 
-template <int NT>
+template <int NT, int WARPS>
 static int launch_q5_tc(const pib_weight * w, const uint8_t * act, const pib_act_layout & L, int b, float * y, const int * cancel, cudaStream_t st) {
-    const size_t smem = (size_t) Q5T_WARPS * Q5T_STAGES * Q5T_BYTES;
+    const int    nsb = (int) (w->K / 256), n_tiles = (int) ((w->N + 15) / 16);
+    const size_t ring = (size_t) WARPS * Q5T_STAGES * Q5T_BYTES, smem = WARPS == 8 ? pib_gemv_smem_spread(ring, n_tiles) : ring;
     static bool configured = false;
     if (!configured) {
-        PIB_CHECK(cudaFuncSetAttribute(gemv_q5k_tc_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-        PIB_CHECK(cudaFuncSetAttribute(gemv_q5k_tc_kernel<NT>, cudaFuncAttributePreferredSharedMemoryCarveout, (int) cudaSharedmemCarveoutMaxShared));
+        PIB_CHECK(cudaFuncSetAttribute(gemv_q5k_tc_kernel<NT, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (ring > PIB_GEMV_SPREAD ? ring : PIB_GEMV_SPREAD)));
+        PIB_CHECK(cudaFuncSetAttribute(gemv_q5k_tc_kernel<NT, WARPS>, cudaFuncAttributePreferredSharedMemoryCarveout, (int) cudaSharedmemCarveoutMaxShared));
         configured = true;
     }
-    const int nsb = (int) (w->K / 256), n_tiles = (int) ((w->N + 15) / 16);
-    PIB_CHECK(pib_launch(gemv_q5k_tc_kernel<NT>, dim3(n_tiles), dim3(Q5T_WARPS * 32), smem, st, w->tiles, nsb, (int) w->N, (int) w->K,
+    PIB_CHECK(pib_launch(gemv_q5k_tc_kernel<NT, WARPS>, dim3(n_tiles), dim3(WARPS * 32), smem, st, w->tiles, nsb, (int) w->N, (int) w->K,
                          (const int8_t *) (act + L.qsp_off), (const float *) (act + L.dxo_off), (const int8_t *) (act + L.bs8_off), b, y, cancel));
     return PIB_OK;
 }
@@ -295,8 +302,12 @@ int pib_gemv_q5k(const pib_weight * w, const void * act_dev, int b, float * y_de
     const pib_act_layout L   = pib_act_layout_of(PIB_TYPE_Q4_K, w->K, b);          // Q8_K family activations
     const uint8_t *      act = (const uint8_t *) act_dev;
     static const int use_tc = getenv("PIB_Q5K_TC") ? atoi(getenv("PIB_Q5K_TC")) : 1;
-    if (w->tiles && (use_tc || !w->qs) && b <= PIB_MAX_BATCH)
-        return b <= 8 ? launch_q5_tc<1>(w, act, L, b, y_dev, cancel, st) : launch_q5_tc<2>(w, act, L, b, y_dev, cancel, st);
+    if (w->tiles && (use_tc || !w->qs) && b <= PIB_MAX_BATCH) {
+        if (pib_gemv_wide(w) && b <= 8) return launch_q5_tc<1, 8>(w, act, L, b, y_dev, cancel, st);
+        // two column blocks: while a CTA per SM serves (4096 x 11008 at 12 tokens, two per SM: four / eight warps 16.4 / 17.5 us)
+        if (pib_gemv_wide(w) && (w->N + 15) / 16 <= pib_num_sms()) return launch_q5_tc<2, 8>(w, act, L, b, y_dev, cancel, st);
+        return b <= 8 ? launch_q5_tc<1, 4>(w, act, L, b, y_dev, cancel, st) : launch_q5_tc<2, 4>(w, act, L, b, y_dev, cancel, st);
+    }
     for (int t0 = 0; t0 < b; t0 += 8) {
         const int   nb = b - t0 < 8 ? b - t0 : 8;
         cudaError_t e  = cudaSuccess;

@@ -138,6 +138,11 @@ struct pib_weight {
     int       owns;
 };
 
+// Dynamic shared memory of decode-matmul CTAs of which an SM takes two: where there is one per SM or fewer, so much that it takes one.  (Launched while the quantiser in front still
+// runs, two would share an SM and leave others idle: Q4_0 2368 x 28672 at 13 tokens 26.6 us, 17.5 with one per SM; Q6_K 54.7 -> 28.)
+#define PIB_GEMV_SPREAD (116 * 1024)
+static inline size_t pib_gemv_smem_spread(size_t smem, int n_ctas) { return n_ctas <= pib_num_sms() && smem < (size_t) PIB_GEMV_SPREAD ? (size_t) PIB_GEMV_SPREAD : smem; }
+
 // activation format a weight type multiplies with, named by the weight type that owns the layout below: the K-quants share
 // Q8_K (reference type_traits[].vec_dot_type, ggml.c:455-560)
 static inline int pib_act_family(int wtype) { return (wtype == PIB_TYPE_Q6_K || wtype == PIB_TYPE_Q5_K || wtype == PIB_TYPE_Q3_K) ? PIB_TYPE_Q4_K : wtype; }
