@@ -54,8 +54,9 @@ __device__ __forceinline__ void aq_value8(const float * xr, const float * __rest
     }
 }
 
-// XH: a prompt pass, the rows go to xh as the tensor-core GEMM's fp16 operand and nowhere else
-template <bool Q8K, int PRO, bool XH>
+// XH: 0 the planes of a decode batch; 1 a prompt pass, the rows go to xh as the tensor-core GEMM's fp16 operand and nowhere else; 2 more rows than a decode batch has: xh, quants, scales
+// and sums, but none of the planes that only decode matmuls read
+template <bool Q8K, int PRO, int XH>
 __global__ void __launch_bounds__(AQ_THREADS) act_quant_kernel(const float * x, const float * __restrict__ x2,
                                                                int x2_per_row, float eps, int64_t K,
                                                                int8_t * __restrict__ qs, float * __restrict__ dplane,
@@ -248,7 +249,9 @@ __global__ void __launch_bounds__(AQ_THREADS) act_quant_kernel(const float * x, 
                 vo[1] = make_float4(v[4], v[5], v[6], v[7]);
             }
             const size_t rs = (size_t) row * nsb + sb;
-            if (XH) q8k_quantise_sb(v, lane, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, xh + (size_t) row * K + sb * PIB_QK_K);
+            if (XH == 1) q8k_quantise_sb(v, lane, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, xh + (size_t) row * K + sb * PIB_QK_K);
+            else if (XH == 2) q8k_quantise_sb(v, lane, qs + (size_t) row * K + sb * PIB_QK_K, nullptr, (int16_t *) bsplane + rs * 16, nullptr, nullptr, nullptr, dplane + rs, nullptr, nullptr,
+                                              xh + (size_t) row * K + sb * PIB_QK_K);
             else {
                 const size_t os = (size_t) oct.before * nsb + (size_t) sb * oct.gs + oct.g, of = (size_t) oct.before * K + (size_t) sb * oct.gs * PIB_QK_K + oct.g * 64;
                 q8k_quantise_sb(v, lane, qs + (size_t) row * K + sb * PIB_QK_K, qsp + of, (int16_t *) bsplane + rs * 16, bs8plane + os * 16, sbs + rs * 8, qsl + rs * 64, dplane + rs,
@@ -285,11 +288,13 @@ static int launch_aq(int wtype, const float * x, const float * x2, int x2_per_ro
     parts = max((int64_t) 1, min((int64_t) 32, parts));
     const dim3    grid(b, (unsigned) parts);
 #define AQ_GO(Q8K, XH) pib_launch(act_quant_kernel<Q8K, PRO, XH>, grid, dim3(AQ_THREADS), 0, st, x, x2, x2_per_row, eps, K, qs, d, bs, b8, qp, ql, sb, q6, b6, vout, lut, addend, sum_out, cancel, \
-                               xstride, bias, addend2, (__half *) xhat, dx)
+                               xstride, bias, addend2, (__half *) (XH == 2 ? (void *) ql : xhat), dx)
     constexpr bool PROMPT = PRO == PRO_PLAIN || PRO == PRO_RMSNORM || PRO == PRO_SILU_MUL;
-    if (wtype != PIB_TYPE_Q4_K) AQ_GO(false, false);
-    else if (PROMPT && xhat)    AQ_GO(true, PROMPT);
-    else                        AQ_GO(true, false);
+    // more rows than a decode matmul takes: the GEMM's operand takes the place of the qsl plane (pib_act_layout) and of the GEMM's own conversion (4 us a launch)
+    if (wtype != PIB_TYPE_Q4_K)   AQ_GO(false, 0);
+    else if (PROMPT && xhat)      AQ_GO(true, (PROMPT ? 1 : 0));
+    else if (b > PIB_MAX_BATCH)   AQ_GO(true, 2);
+    else                          AQ_GO(true, 0);
 #undef AQ_GO
     PIB_CHECK(cudaGetLastError());
     return PIB_OK;

@@ -433,6 +433,7 @@ int pib_gemm_q4k_tc(const pib_weight * w, const void * act_dev, int b, float * y
     const uint8_t * act = (const uint8_t *) act_dev;
     __half * xh = (__half *) xhat_dev;
     const int64_t n16 = (int64_t) b * (w->K / 16);
+    if (act && b > PIB_MAX_BATCH) { xh = (__half *) (const_cast<uint8_t *>(act) + L.qsl_off); act = nullptr; }      // the quantiser has written the operand
     if (act) pib_launch(tg_xhat_kernel, dim3((unsigned) ((n16 + 255) / 256)), dim3(256), 0, st, (const int8_t *) (act + L.qs_off), (const float *) (act + L.d_off), n16, (int) (w->K / 16), xh);
     PIB_CHECK(cudaGetLastError());
     const int NB = tg_nb_of(b), nsb = (int) (w->K / 256), nx = (int) ((w->N + TG_BM - 1) / TG_BM), sms = pib_num_sms();

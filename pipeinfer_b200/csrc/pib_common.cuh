@@ -162,7 +162,9 @@ struct pib_act_layout {
     size_t qsp_off;    // Q8_K family: int8 [super-block][4 chunks c][gs][4 quarters t][16], the same quants as qs_off in tensor-core fragment order: element
                        //   e = 64c + 32h + 8t + i (low/high-nibble half h) is byte 8h + i of piece (c, t), a lane's B fragments of chunk c
     size_t qsl_off;    // Q8_K family: int2 [b][K/256][8 lane groups g][8 sub-blocks j]: {x if g even else 0, x if g odd else 0} with x =
-                       //   the four quants 4g .. 4g+3 of sub-block j -- the two B registers of the lane-exact kernel (gemv_q4k_lane.cu)
+                       //   the four quants 4g .. 4g+3 of sub-block j -- the two B registers of the lane-exact kernel (gemv_q4k_lane.cu).
+                       //   With b > PIB_MAX_BATCH, where only the GEMM and the exact host forms read the buffer: fp16 [b][K], the GEMM's operand (tg_kpos), and of the planes
+                       //   only qs, d and bs are written
     size_t sbs_off;    // Q8_K family: int16 [b][K/32] sub-block sums bsums[2j] + bsums[2j+1]
     size_t q6p_off;    // Q8_K family: int8 [super-block][4 quads c][gs][4 quarters t][16], the quants in the B-fragment order of mma.m16n8k16 over the 16-element groups of
                        //   Q6_K: element e = 16j + 4t + i (group j = 4c + jj) is byte 4jj + i of piece (c, t)
