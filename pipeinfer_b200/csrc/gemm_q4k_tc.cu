@@ -16,6 +16,9 @@
 //   warps 3..       G groups of 8: a warp owns one 16-row tile, turns its 16-byte fragment pieces into fp16 pairs in registers and stores them with
 //                   tcgen05.st.16x256b: the record layout (lane g, t holds rows g and g + 8, gemv_mma.cu) IS that instruction's register layout, only
 //                   the order of k inside a 64-wide chunk differs, and x^ is written in the same order (tg_kpos).  Afterwards the epilogue.
+// Weights run four k-steps ahead in tensor memory; the activations' places are a ring of their own where they come in pieces (256 tokens: with two weight steps the groups waited for
+// the MMAs of the step before last; with four, and the producer and the issuing warp counting their places along, 12288 x 4096 32.7 -> 27.6 us, 4096 x 4096 18.8 -> 16.4,
+// 57344 x 8192 204 -> 192).
 // What bounds it: up to about 100 tokens the dequantisation, 109 warp instructions per 16 rows x 64 k issued at 0.6 per clock and scheduler (57344 x 8192
 // at 40 tokens 96 us, where the weights' bytes take 40; with the operand written to and read from shared memory, the form this replaces, 173 us); with
 // 256 tokens the tensor cores and the activation tiles' way into shared memory (203 us, before 246; 151 at the dense peak).
@@ -34,9 +37,9 @@
 // G groups of 8 warps feed the accumulator (G = 2: the groups take the k-steps in turn); with G = 1 two CTAs share an SM
 template <int NB, int G> struct tg_cfg {
     static constexpr int CTAS    = 3 - G;                                // per SM
-    static constexpr int STAGES  = G == 2 ? (NB > 128 ? 2 : 4) : NB > 64 ? 2 : 3;   // k-steps of weights in tensor memory
+    static constexpr int STAGES  = G == 2 ? 4 : NB > 64 ? 2 : 3;   // k-steps of weights in tensor memory
     static constexpr int PIECES  = NB > 128 ? 2 : 1;                     // activations arrive in pieces of a k-step: with two stages only, whole ones are late (256 tokens:
-    static constexpr int BSTAGES = PIECES * STAGES;                      // 246 -> 193 us); with more stages a second barrier per step costs more (24 tokens: 31 -> 44)
+    static constexpr int BSTAGES = NB > 128 ? 4 : STAGES;                // 246 -> 193 us); with more stages a second barrier per step costs more (24 tokens: 31 -> 44)
     static constexpr int WSTAGES = NB == 128 && G == 1 ? 2 : 3;          // super-blocks of weight records in shared memory
     static constexpr int WARPS   = 8 * G, THREADS = 96 + 32 * WARPS;
     static constexpr int W_BYTES = 8 * TG_TILE_BYTES, B_BYTES = NB * 256 / PIECES;
@@ -71,17 +74,26 @@ __global__ void __launch_bounds__(256) tg_xhat_kernel(const int8_t * __restrict_
     }
 }
 
-__device__ __forceinline__ void tg_tma_2d(uint32_t dst, const CUtensorMap * map, uint32_t bar, int x, int y) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-                 ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
-}
 __device__ __forceinline__ void tg_bulk(uint32_t dst, const void * src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
-// A in tensor memory, B in shared memory; called by a converged warp
-__device__ __forceinline__ void tg_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+// N (1 or 2) boxes of 64 k and the announcement of their bytes; by a converged warp, one elected lane issues (a lane's own loop with its places formed by division took 600 clocks a round)
+template <int N> __device__ __forceinline__ void tg_load(uint32_t dst, uint32_t box, const CUtensorMap * map, uint32_t bar, uint32_t bytes, int k) {
+    if (N == 2) asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%3], %4;\n\t"
+                             "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%2, {%5, %7}], [%3];\n\t"
+                             "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%1], [%2, {%6, %7}], [%3];\n\t}"
+                             ::"r"(dst), "r"(dst + box), "l"(map), "r"(bar), "r"(bytes), "r"(k), "r"(k + 64), "r"(0) : "memory");
+    else asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%2], %3;\n\t"
+                      "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%4, %5}], [%2];\n\t}"
+                      ::"r"(dst), "l"(map), "r"(bar), "r"(bytes), "r"(k), "r"(0) : "memory");
+}
+// four MMAs of 16 k, A in tensor memory, B in shared memory; by a converged warp
+__device__ __forceinline__ void tg_mma4(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p, q;\n\t.reg .b32 a;\n\t.reg .b64 b;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t"
+                 "add.s32 a, %1, 8;\n\tadd.s64 b, %2, 2;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, {%5, %5, %5, %5}, 1;\n\t"
+                 "add.s32 a, %1, 16;\n\tadd.s64 b, %2, 4;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, {%5, %5, %5, %5}, 1;\n\t"
+                 "add.s32 a, %1, 24;\n\tadd.s64 b, %2, 6;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, {%5, %5, %5, %5}, 1;\n\t}"
                  ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
 }
 // 16 lanes x 64 columns: register 4a + j of lane (g, t) is column 8a + 2t + (j & 1) of lane g + 8 (j >> 1)
@@ -110,15 +122,6 @@ template <uint32_t NAP = 0> __device__ __forceinline__ bool tg_wait(uint32_t bar
     *abort_s = 1;
     return false;
 }
-__device__ __forceinline__ bool tg_wait1(uint32_t bar, uint32_t parity, volatile int * abort_s) {      // by one thread
-    for (int it = 0; it < TG_TRIES; it++) {
-        if (tg_try<0>(bar, parity)) return true;
-        if ((it & 15) == 15 && *abort_s) return false;
-    }
-    *abort_s = 1;
-    return false;
-}
-
 __device__ __forceinline__ __half2 tg_h2(uint32_t v) { return *reinterpret_cast<const __half2 *>(&v); }
 __device__ __forceinline__ uint32_t tg_u(__half2 v) { return *reinterpret_cast<const uint32_t *>(&v); }
 
@@ -196,34 +199,34 @@ gemm_q4k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int x0, c
     if (warp == 0) {
         pib_pdl_wait();
         pib_pdl_trigger();
-        if (lane == 0) {
-            for (int kp = 0; kp < C::PIECES * n_ksteps; kp++) {
-                const int s = kp % C::BSTAGES;
-                if (kp >= C::BSTAGES && !tg_wait1(bar_bf + s * 8, ((kp / C::BSTAGES) - 1) & 1, abort_s)) break;
-                dt_mbar_expect_tx(bar_b + s * 8, C::B_BYTES);
-                for (int j = 0; j < 2 / C::PIECES; j++)
-                    tg_tma_2d(dt_smem(sB + s * C::B_BYTES + j * NB * 128), &xmap, bar_b + s * 8, sb_lo * 256 + (kp * (2 / C::PIECES) + j) * 64, 0);
-            }
+        int  s = 0, k = sb_lo * 256;
+        uint32_t ph = 1;                                           // the first round finds its places free
+        for (int kp = 0; kp < C::PIECES * n_ksteps; kp++, k += 128 / C::PIECES) {
+            if (!tg_wait(bar_bf + s * 8, ph, abort_s)) break;
+            tg_load<2 / C::PIECES>(dt_smem(sB) + s * C::B_BYTES, NB * 128, &xmap, bar_b + s * 8, C::B_BYTES, k);
+            if (++s == C::BSTAGES) { s = 0; ph ^= 1; }
         }
     } else if (warp == 1) {
         // instruction descriptor: fp32 accumulate, fp16 x fp16, both K-major, N = NB, M = 128
         constexpr uint32_t idesc = (1u << 4) | ((uint32_t) (NB >> 3) << 17) | ((uint32_t) (TG_BM >> 4) << 24);
         const uint64_t bd0 = dt_desc(dt_smem(sB));
+        int  s = 0, sp = 0;
+        uint32_t ph = 0, php = 0;
         for (int kt = 0; kt < n_ksteps && ok; kt++) {
-            const int s = kt % C::STAGES;
-            ok = tg_wait(bar_a + s * 8, (kt / C::STAGES) & 1, abort_s);
+            ok = tg_wait(bar_a + s * 8, ph, abort_s);
             for (int j = 0; j < C::PIECES && ok; j++) {
-                const int kp = C::PIECES * kt + j, sp = kp % C::BSTAGES;
-                ok = tg_wait(bar_b + sp * 8, (kp / C::BSTAGES) & 1, abort_s);
+                ok = tg_wait(bar_b + sp * 8, php, abort_s);
                 if (!ok) break;
                 dt_fence_after();
                 const uint64_t bd = bd0 + (uint64_t) (sp * C::B_BYTES >> 4);
-#pragma unroll
-                for (int k = 0; k < 8 / C::PIECES; k++)         // 8 columns of weights and 32 bytes of activations further along K
-                    tg_mma_ts(tmem, tmem + NB + s * 64 + j * 32 + k * 8, bd + 2 * (k & 3) + (k >> 2) * (NB * 128 >> 4), idesc, (kp | k) != 0);
-                if (C::PIECES > 1) dt_commit(bar_be + sp * 8);  // the piece is free when these MMAs have read it
+                const uint32_t ta = tmem + NB + s * 64 + j * 32;
+                tg_mma4(tmem, ta, bd, idesc, (kt | j) != 0);      // 8 columns of weights and 32 bytes of activations further along K each
+                if (C::PIECES == 1) tg_mma4(tmem, ta + 32, bd + (NB * 128 >> 4), idesc, 1);
+                else dt_commit(bar_be + sp * 8);                  // the piece is free when these MMAs have read it
+                if (++sp == C::BSTAGES) { sp = 0; php ^= 1; }
             }
             if (ok) dt_commit(bar_e + s * 8);
+            if (++s == C::STAGES) { s = 0; ph ^= 1; }
         }
         if (ok) dt_commit(bar_t);
     } else if (warp == 2) {
