@@ -828,7 +828,8 @@ static int enqueue_decode(pib_context * c, pib_run * run, int n_tokens, int batc
 
 // ---- wide batches (prompt ingestion): the matmuls of up to PIB_PROMPT_MAX tokens at once on the tcgen05 GEMM -----------------------
 // The reference takes a prompt of up to n_batch = 512 tokens in one ggml_compute_forward_mul_mat per matrix (common.h:52, ggml.c:9388).
-// Here every launch of a layer takes the whole pass (prompt_attn.cu for RoPE, KV store and attention; the row kernels take any number of rows);
+// Here every launch of a layer takes the whole pass, a whole prompt of up to 1024 tokens where one stage has all layers (700 tokens in passes of 256 left 52 of 148 SMs idle in a
+// 12288-row matmul, paid every launch's start and end three times and re-read the weights: 2.49 ms through four 4096-wide layers, now 2.06) (prompt_attn.cu for RoPE, KV store and attention; the row kernels take any number of rows);
 // the chunks' 16-token descriptors are spread into one array per field first.  Used for llama-architecture models whose matrices are all Q4_K, for decodes of more than two
 // chunks, outside exact mode (the GEMM is tolerance-checked, not bit-exact: gemm_q4k_tc.cu).
 static bool prompt_gemm_ok(const pib_context * c, int n_tokens) {
@@ -843,21 +844,33 @@ static bool prompt_gemm_ok(const pib_context * c, int n_tokens) {
     return pib_prompt_attention_supported(m->head_dim(), (int) c->n_ctx);
 }
 
-static int prompt_bufs(pib_context * c) {
-    if (c->pb.ready) return PIB_OK;
-    const pib_model * m = c->model;
-    const size_t P = PIB_PROMPT_MAX, E = m->n_embd, GQA = m->n_embd_gqa(), FF = m->n_ff, KM = std::max(E, FF);
+static void prompt_bufs_free(pib_context * c) {
     auto & b = c->pb;
-    if (cudaMalloc(&b.x, P * E * 4) != cudaSuccess || cudaMalloc(&b.x2, P * E * 4) != cudaSuccess || cudaMalloc(&b.qkv, P * (E + 2 * GQA) * 4) != cudaSuccess ||
-        cudaMalloc(&b.att, P * E * 4) != cudaSuccess || cudaMalloc(&b.proj, P * E * 4) != cudaSuccess || cudaMalloc(&b.gu, P * 2 * FF * 4) != cudaSuccess ||
-        cudaMalloc(&b.mask, P * c->n_ctx) != cudaSuccess || cudaMalloc(&b.ids, P * (3 + (size_t) c->n_words) * 4) != cudaSuccess ||
-        cudaMalloc(&b.xhat, pib_gemm_xhat_bytes((int64_t) KM, (int) P)) != cudaSuccess) {
+    for (void * p : { (void *) b.x, (void *) b.x2, (void *) b.qkv, (void *) b.att, (void *) b.proj, (void *) b.gu, (void *) b.mask, b.xhat, (void *) b.ids }) if (p) cudaFree(p);
+    b = pib_context::PromptBufs();
+}
+// buffers for passes of a prompt of n_tokens: all of it up to PIB_PROMPT_MAX (one stage; passes of 256 where stages overlap, or where memory holds no more)
+static int prompt_bufs(pib_context * c, int n_tokens) {
+    const int want = c->stage.size > 1 ? PIB_PROMPT_STAGE : std::min(PIB_PROMPT_MAX, (n_tokens + 255) / 256 * 256);
+    if (c->pb.cap >= want) return PIB_OK;
+    const pib_model * m = c->model;
+    const size_t E = m->n_embd, GQA = m->n_embd_gqa(), FF = m->n_ff, KM = std::max(E, FF);
+    auto & b = c->pb;
+    if (b.cap) cudaStreamSynchronize(c->stream);
+    for (size_t P = (size_t) want; P >= 256; P = P > 256 ? 256 : 0) {
+        prompt_bufs_free(c);
+        if (cudaMalloc(&b.x, P * E * 4) == cudaSuccess && cudaMalloc(&b.x2, P * E * 4) == cudaSuccess && cudaMalloc(&b.qkv, P * (E + 2 * GQA) * 4) == cudaSuccess &&
+            cudaMalloc(&b.att, P * E * 4) == cudaSuccess && cudaMalloc(&b.proj, P * E * 4) == cudaSuccess && cudaMalloc(&b.gu, P * 2 * FF * 4) == cudaSuccess &&
+            cudaMalloc(&b.mask, P * c->n_ctx) == cudaSuccess && cudaMalloc(&b.ids, PIB_PROMPT_MAX * (3 + (size_t) c->n_words) * 4) == cudaSuccess &&
+            cudaMalloc(&b.xhat, pib_gemm_xhat_bytes((int64_t) KM, (int) P)) == cudaSuccess) {
+            b.cap = (int) P;
+            return PIB_OK;
+        }
         cudaGetLastError();
-        pib_set_error("decode: out of memory for the prompt path's work buffers");
-        return PIB_ERR_NOMEM;
     }
-    b.ready = true;
-    return PIB_OK;
+    prompt_bufs_free(c);
+    pib_set_error("decode: out of memory for the prompt path's work buffers");
+    return PIB_ERR_NOMEM;
 }
 
 // one pass of `ntok` tokens = chunks [ch0, ch0 + nch) of the run
@@ -1030,8 +1043,13 @@ int pib_decode_start(pib_context * c, int n_tokens, const int32_t * token, const
             memcpy(tl + PIB_TREE_NP + PIB_TREE_NP * PIB_TREE_DEPTH, T.toks, sizeof(T.toks));
         }
         dq.push_back({ KVOP_ALLOC, (int32_t) (head + t0), nt, (int32_t) c->kv.n, s, 0 });
-        cudaMemcpyAsync(c->desc_dev + (size_t) dev_slot(c, s) * c->desc_stride, d, c->desc_stride, cudaMemcpyHostToDevice, c->stream);
-        c->h2d_bytes += c->desc_stride;
+    }
+    // neighbouring slots cross in one copy (a prompt's chunks take them in turn: 44 copies of a 700-token prompt)
+    for (int ch = 0, end; ch < n_chunks; ch = end) {
+        const int s0 = slots[ch], d0 = dev_slot(c, s0);
+        for (end = ch + 1; end < n_chunks && slots[end] == s0 + (end - ch) && dev_slot(c, slots[end]) == d0 + (end - ch); end++) {}
+        cudaMemcpyAsync(c->desc_dev + (size_t) d0 * c->desc_stride, c->desc_host + (size_t) s0 * c->desc_stride, c->desc_stride * (size_t) (end - ch), cudaMemcpyHostToDevice, c->stream);
+        c->h2d_bytes += c->desc_stride * (size_t) (end - ch);
     }
     dq.push_back({ KVOP_ADVANCE, n_tokens, (int32_t) head, 0, 0, 0 });
     kvlog_decode_end(c->kv, n_tokens);                                    // llama.cpp:5708-5713
@@ -1087,10 +1105,10 @@ static int enqueue_decode(pib_context * c, pib_run * run, int n_tokens, int batc
     SLOW_MARK("  apply ops");
     run->in_use = true; run->batch_id = batch_id; run->n_tokens = n_tokens; run->failed = false; run->tc_used = false;
     cudaMemcpyAsync(c->cancel_table, c->run_id_host + run->id, sizeof(int), cudaMemcpyHostToDevice, c->stream);   // "this run executes now"
-    if (prompt_gemm_ok(c, n_tokens) && prompt_bufs(c) == PIB_OK) {
-        const int per = PIB_PROMPT_MAX / PIB_CHUNK;
+    if (prompt_gemm_ok(c, n_tokens) && prompt_bufs(c, n_tokens) == PIB_OK) {
+        const int pass = c->stage.size > 1 ? PIB_PROMPT_STAGE : c->pb.cap, per = pass / PIB_CHUNK;
         for (int ch0 = 0; ch0 < n_chunks && !run->failed; ch0 += per) {
-            const int nch = std::min(per, n_chunks - ch0), ntok = std::min(PIB_PROMPT_MAX, n_tokens - ch0 * PIB_CHUNK);
+            const int nch = std::min(per, n_chunks - ch0), ntok = std::min(pass, n_tokens - ch0 * PIB_CHUNK);
             if (run_prompt_pass(c, *run, ch0, nch, ntok, slots) != PIB_OK) run->failed = true;
         }
         for (int ch = 0; ch < n_chunks; ch++) if (c->desc_ev[slots[ch]]) cudaEventRecord(c->desc_ev[slots[ch]], c->stream);

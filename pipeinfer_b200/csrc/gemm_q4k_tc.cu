@@ -1,4 +1,4 @@
-// gemm_q4k_tc.cu -- the quantised matmul (K1) for WIDE batches (prompt ingestion, 17 .. 256 tokens at once): Q4_K weights are dequantised to fp16
+// gemm_q4k_tc.cu -- the quantised matmul (K1) for WIDE batches (prompt ingestion, up to PIB_PROMPT_MAX tokens at once): Q4_K weights are dequantised to fp16
 // straight into tensor memory and multiplied there on the 5th-generation tensor cores (tcgen05.mma with A in tensor memory, fp32 accumulators), the
 // activation tile arriving by TMA.  Replaces, for these batch sizes, the reference's ggml_compute_forward_mul_mat at large ne11 (ggml.c:9388) /
 // ggml_cuda_op_mul_mat_cublas (ggml-cuda.cu:6562: dequantise + cuBLAS).
@@ -9,7 +9,7 @@
 // order and not bit-exact; it is checked against the oracle to a tolerance (tests/test_gpu_gemm.py) and used for prompt chunks only
 // -- verification batches (<= 16 tokens) keep the GEMV kernels.
 //
-// A CTA owns 128 output rows and up to 256 tokens, and one share of K when a cluster splits it:
+// A CTA owns 128 output rows and a tile of up to 256 tokens, and one share of K when a cluster splits it:
 //   warp 0          TMA: the activation tile [NB tokens x 128 k] fp16 of every k-step (cp.async.bulk.tensor.2d, 128-byte swizzle)
 //   warp 1          allocates tensor memory, issues the MMAs (8 x K=16 per k-step) and commits them to the mbarriers
 //   warp 2          weight records: one bulk copy per 16-row tile and super-block into a ring, started before the launch wait
@@ -78,14 +78,14 @@ __device__ __forceinline__ void tg_bulk(uint32_t dst, const void * src, uint32_t
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 // N (1 or 2) boxes of 64 k and the announcement of their bytes; by a converged warp, one elected lane issues (a lane's own loop with its places formed by division took 600 clocks a round)
-template <int N> __device__ __forceinline__ void tg_load(uint32_t dst, uint32_t box, const CUtensorMap * map, uint32_t bar, uint32_t bytes, int k) {
+template <int N> __device__ __forceinline__ void tg_load(uint32_t dst, uint32_t box, const CUtensorMap * map, uint32_t bar, uint32_t bytes, int k, int row) {
     if (N == 2) asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%3], %4;\n\t"
                              "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%2, {%5, %7}], [%3];\n\t"
                              "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%1], [%2, {%6, %7}], [%3];\n\t}"
-                             ::"r"(dst), "r"(dst + box), "l"(map), "r"(bar), "r"(bytes), "r"(k), "r"(k + 64), "r"(0) : "memory");
+                             ::"r"(dst), "r"(dst + box), "l"(map), "r"(bar), "r"(bytes), "r"(k), "r"(k + 64), "r"(row) : "memory");
     else asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%2], %3;\n\t"
                       "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%4, %5}], [%2];\n\t}"
-                      ::"r"(dst), "l"(map), "r"(bar), "r"(bytes), "r"(k), "r"(0) : "memory");
+                      ::"r"(dst), "l"(map), "r"(bar), "r"(bytes), "r"(k), "r"(row) : "memory");
 }
 // four MMAs of 16 k, A in tensor memory, B in shared memory; by a converged warp
 __device__ __forceinline__ void tg_mma4(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -158,10 +158,10 @@ template <int C, int J0> __device__ __forceinline__ void tg_chunk_row(uint32_t w
 }
 
 // ---- the GEMM ------------------------------------------------------------------------------------------------------------------
-// grid (row blocks, token blocks, K shares); the K shares of a tile are one cluster
+// grid (blocks, 1, K shares); the K shares of a block are one cluster
 template <int NB, int G>
 __global__ void __launch_bounds__(tg_cfg<NB, G>::THREADS, tg_cfg<NB, G>::CTAS)
-gemm_q4k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int x0, const __grid_constant__ CUtensorMap xmap, int b, float * __restrict__ y, int * __restrict__ err) {
+gemm_q4k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int x0, int ny, const __grid_constant__ CUtensorMap xmap, int b_all, float * __restrict__ y_all, int * __restrict__ err) {
     using C = tg_cfg<NB, G>;
     extern __shared__ __align__(1024) uint8_t tg_dsm[];
     uint8_t *  sB  = tg_dsm + ((1024u - (dt_smem(tg_dsm) & 1023u)) & 1023u);      // [BSTAGES][64 k][NB rows][128 B], 1024-byte aligned (swizzle atom)
@@ -175,7 +175,9 @@ gemm_q4k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int x0, c
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int S = gridDim.z, sb_lo = (int) ((long long) nsb * blockIdx.z / S), sb_hi = (int) ((long long) nsb * (blockIdx.z + 1) / S);
     const int n_sb = sb_hi - sb_lo, n_ksteps = n_sb * 2;
-    const int row0 = (x0 + blockIdx.x) * TG_BM;
+    // block x0 + blockIdx.x: row block and token tile, the ny tiles of a row block next to each other
+    const int row0 = (x0 + (int) blockIdx.x) / ny * TG_BM, tok0 = (x0 + (int) blockIdx.x) % ny * NB, b = min(NB, b_all - tok0);
+    float *   y = y_all + (size_t) tok0 * N;
     const int n_tiles = min(8, (N + 15) / 16 - row0 / 16);                   // 16-row tiles this block has
 
     if (threadIdx.x == 0) {
@@ -203,7 +205,7 @@ gemm_q4k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int x0, c
         uint32_t ph = 1;                                           // the first round finds its places free
         for (int kp = 0; kp < C::PIECES * n_ksteps; kp++, k += 128 / C::PIECES) {
             if (!tg_wait(bar_bf + s * 8, ph, abort_s)) break;
-            tg_load<2 / C::PIECES>(dt_smem(sB) + s * C::B_BYTES, NB * 128, &xmap, bar_b + s * 8, C::B_BYTES, k);
+            tg_load<2 / C::PIECES>(dt_smem(sB) + s * C::B_BYTES, NB * 128, &xmap, bar_b + s * 8, C::B_BYTES, k, tok0);
             if (++s == C::BSTAGES) { s = 0; ph ^= 1; }
         }
     } else if (warp == 1) {
@@ -366,9 +368,10 @@ static tg_encode_fn tg_encode() {
     return fn;
 }
 
-// tokens per CTA
-static int tg_nb_of(int b) { return b <= 32 ? 32 : b <= 64 ? 64 : b <= 96 ? 96 : b <= 128 ? 128 : b <= 192 ? 192 : 256; }
-size_t pib_gemm_xhat_bytes(int64_t K, int b) { return (size_t) (b <= 32 ? 32 : b <= 64 ? 64 : b <= 128 ? 128 : 256) * K * sizeof(__half); }
+// token tiles and tokens per CTA
+static int tg_tiles_of(int b) { return (b + 255) / 256; }
+static int tg_nb_of(int b_all) { const int ny = tg_tiles_of(b_all), b = (b_all + ny - 1) / ny; return b <= 32 ? 32 : b <= 64 ? 64 : b <= 96 ? 96 : b <= 128 ? 128 : b <= 192 ? 192 : 256; }
+size_t pib_gemm_xhat_bytes(int64_t K, int b) { return (size_t) (b <= 32 ? 32 : b <= 64 ? 64 : b <= 128 ? 128 : b <= 256 ? 256 : b) * K * sizeof(__half); }
 
 // Clusters of S CTAs, one CTA per SM, that the machine holds at once: not every GPC's SMs divide by S, so it is fewer than the SMs do (148 SMs: 148, 74, 33, 15 of
 // 1, 2, 4, 8 CTAs, which the launches bear out: 34 clusters of 4 take two rounds).
@@ -403,7 +406,7 @@ static int tg_fit_nb(int NB, int S) {
     }
 }
 
-// row blocks [x0, x0 + nx), K in S shares
+// blocks [x0, x0 + nx), K in S shares
 template <int NB, int G>
 static int tg_launch(const pib_weight * w, const __half * xh, int b, int x0, int nx, int S, float * y, cudaStream_t st) {
     using C = tg_cfg<NB, G>;
@@ -422,8 +425,8 @@ static int tg_launch(const pib_weight * w, const __half * xh, int b, int x0, int
     const dim3 grid((unsigned) nx, 1, (unsigned) S);
     int * err = pib_tc_error_word(st);
     if (!err) { pib_set_error("pib_gemm: no memory for the stream's error word"); return PIB_ERR_NOMEM; }
-    if (S > 1) pib_launch_cluster(gemm_q4k_tc_kernel<NB, G>, grid, dim3(C::THREADS), dim3(1, 1, (unsigned) S), C::SMEM, st, w->tiles, (int) (w->K / 256), (int) w->N, x0, map, b, y, err);
-    else       pib_launch(gemm_q4k_tc_kernel<NB, G>, grid, dim3(C::THREADS), C::SMEM, st, w->tiles, (int) (w->K / 256), (int) w->N, x0, map, b, y, err);
+    if (S > 1) pib_launch_cluster(gemm_q4k_tc_kernel<NB, G>, grid, dim3(C::THREADS), dim3(1, 1, (unsigned) S), C::SMEM, st, w->tiles, (int) (w->K / 256), (int) w->N, x0, tg_tiles_of(b), map, b, y, err);
+    else       pib_launch(gemm_q4k_tc_kernel<NB, G>, grid, dim3(C::THREADS), C::SMEM, st, w->tiles, (int) (w->K / 256), (int) w->N, x0, tg_tiles_of(b), map, b, y, err);
     PIB_CHECK(cudaGetLastError());
     return PIB_OK;
 }
@@ -431,7 +434,7 @@ static int tg_launch(const pib_weight * w, const __half * xh, int b, int x0, int
 // y[b][N] = W x^; act_dev = the Q8_K activation planes of `b` tokens (act_quant.cu), xhat_dev = scratch of pib_gemm_xhat_bytes; or act_dev = null and xhat_dev already
 // written by the quantiser (51 launches of 4 us in a 700-token prompt through four layers)
 int pib_gemm_q4k_tc(const pib_weight * w, const void * act_dev, int b, float * y_dev, void * xhat_dev, cudaStream_t st) {
-    if (!w || w->type != PIB_TYPE_Q4_K || !w->tiles || b < 1 || b > 256) { pib_set_error("pib_gemm: needs Q4_K tiles and 1 <= b <= 256"); return PIB_ERR_ARG; }
+    if (!w || w->type != PIB_TYPE_Q4_K || !w->tiles || b < 1 || b > PIB_PROMPT_MAX) { pib_set_error("pib_gemm: needs Q4_K tiles and 1 <= b <= %d", PIB_PROMPT_MAX); return PIB_ERR_ARG; }
     const pib_act_layout L = pib_act_layout_of(PIB_TYPE_Q4_K, w->K, b);
     const uint8_t * act = (const uint8_t *) act_dev;
     __half * xh = (__half *) xhat_dev;
@@ -439,8 +442,8 @@ int pib_gemm_q4k_tc(const pib_weight * w, const void * act_dev, int b, float * y
     if (act && b > PIB_MAX_BATCH) { xh = (__half *) (const_cast<uint8_t *>(act) + L.qsl_off); act = nullptr; }      // the quantiser has written the operand
     if (act) pib_launch(tg_xhat_kernel, dim3((unsigned) ((n16 + 255) / 256)), dim3(256), 0, st, (const int8_t *) (act + L.qs_off), (const float *) (act + L.d_off), n16, (int) (w->K / 16), xh);
     PIB_CHECK(cudaGetLastError());
-    const int NB = tg_nb_of(b), nsb = (int) (w->K / 256), nx = (int) ((w->N + TG_BM - 1) / TG_BM), sms = pib_num_sms();
-    // K shares of n row blocks, with G groups, whose clusters all find room at once; every share keeps at least two super-blocks.  With two CTAs per SM, S of them need
+    const int NB = tg_nb_of(b), nsb = (int) (w->K / 256), nx = (int) ((w->N + TG_BM - 1) / TG_BM) * tg_tiles_of(b), sms = pib_num_sms();
+    // K shares of n blocks, with G groups, whose clusters all find room at once; every share keeps at least two super-blocks.  With two CTAs per SM, S of them need
     // the room of S / 2, less a sixteenth that packing loses (occupancy queries count one CTA of this kernel per SM; of 4 CTAs 70 clusters ran at once, 72 did not).
     // us at 34 and 37 blocks of K = 4096 / 100 tokens and 17 of 8192 / 256, shares by room / by SMs alone: 16.9 / 22.5, 16.8 / 22.8, 22.6 / 31.6.
     auto shares = [&](int n, int G) {
@@ -483,7 +486,7 @@ int pib_gemm_q4k_tc(const pib_weight * w, const void * act_dev, int b, float * y
 
 extern "C" size_t pib_gemm_scratch_bytes(int64_t K, int b) { return pib_gemm_xhat_bytes(K, b); }
 extern "C" int pib_gemm(const pib_weight * w, const void * act_dev, int b, float * y_dev, void * scratch_dev, pib_stream s) {
-    if (!act_dev || !y_dev || !scratch_dev) { pib_set_error("pib_gemm: bad arguments"); return PIB_ERR_ARG; }
+    if (!act_dev || !y_dev || !scratch_dev || b > 256) { pib_set_error("pib_gemm: bad arguments"); return PIB_ERR_ARG; }
     return pib_gemm_q4k_tc(w, act_dev, b, y_dev, scratch_dev, (cudaStream_t) s);
 }
 extern "C" int pib_gemm_check(pib_stream s) { return pib_tc_check((cudaStream_t) s); }
