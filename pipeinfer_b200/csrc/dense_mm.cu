@@ -16,6 +16,7 @@
 
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #define MM_BM 64
@@ -265,9 +266,12 @@ __global__ void __launch_bounds__(256) mv_pair_kernel(mm_dev a, mm_dev b, bool x
 // before the launch wait where W is a weight, which nothing writes (not for the key and value rows that an attention gathers and passes as W: pib_mm.w_made).
 // The tensor core cuts what falls off its accumulator, always towards zero, so every product of 16 k starts from none and is added up here, rounded to nearest: one
 // accumulator for all of a warp's k drifted (error against 64 bits 2.4e-7 at K = 2048, 2.1e-6 at 16384; now 8.5e-8 and 1.7e-7, fused multiply-adds 8.0e-8 and 1.7e-7).
-// What bounds it: the weights' way from memory.  The form it replaces (a warp per weight row, mv_rows_kernel) rounded every activation for every weight row: at
+// What bounds it: the weights' way from memory.  The form it replaced (a warp per weight row, mv_rows_kernel) rounded every activation for every weight row: at
 // four tokens 32 conversions per 16 bytes of weights (5632 x 2048, 1 / 4 / 16 tokens: 5.8 / 6.1 / 9.1 us, at four 21.7 before).
-#define MVM_U 4                      // 32-k chunks a warp has in flight
+// Weights wait in shared memory: a warp asks for MVM_U chunks of 32 k at a time and DEPTH such groups at once (a lane copies what it reads back itself).  In registers one group was in
+// flight, and each trip paid memory's latency and then the activations'.  How deep: as many bytes as an SM's CTAs can hold (launch_mm).
+#define MVM_U 4                      // 32-k chunks of a group
+#define MVM_GROUP (MVM_U * 1024)     // bytes of a group and warp: 16 rows x 64 bytes a chunk
 __device__ __forceinline__ void mvm_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
@@ -277,24 +281,45 @@ __device__ __forceinline__ uint32_t mvm_pack(float lo, float hi) {
     return *reinterpret_cast<const uint32_t *>(&v);
 }
 // weight rows 16 tile .. + 15 of problem z against its rows [row0, row1) (at most 8 NT).  WAIT: the launch wait comes here, behind the first loads of immutable weights
-template <int EPI, int NT, bool WAIT>
+template <int EPI, int NT, int DEPTH, bool WAIT>
 __device__ __forceinline__ void mvm_body(const mm_dev & a, int z, int tile, int row0, int row1) {
     __shared__ float red[8][8 * NT][16];
+    extern __shared__ __align__(16) uint8_t mvm_ring[];
+    constexpr int D = DEPTH ? DEPTH : 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int nch = (a.K + 31) / 32, c0 = nch * warp / 8, c1 = nch * (warp + 1) / 8, n0 = tile * 16;
+    const int nch = (a.K + 31) / 32, c0 = nch * warp / 8, c1 = nch * (warp + 1) / 8, n0 = tile * 16, groups = (c1 - c0 + MVM_U - 1) / MVM_U;
     const __nv_bfloat16 * W = reinterpret_cast<const __nv_bfloat16 *>(a.W) + (size_t) z * a.wz + 8 * t;
     const __nv_bfloat16 * wa = W + (size_t) min(n0 + g, a.N - 1) * a.ldw, * wb = W + (size_t) min(n0 + g + 8, a.N - 1) * a.ldw;
-    int4 ra[MVM_U], rb[MVM_U];
-    auto load = [&](int c) {
+    const uint8_t * own  = mvm_ring + warp * (D * MVM_GROUP) + lane * 16;
+    const uint32_t  ring = (uint32_t) __cvta_generic_to_shared(own);
+    auto issue = [&](int q) {                                               // group q of this warp into place q mod DEPTH; pieces past the end become zeros and are not read
+        if (q < groups) {
+#pragma unroll
+            for (int u = 0; u < MVM_U; u++) {
+                const int  c  = c0 + q * MVM_U + u;
+                const bool in = c < c1 && c * 32 + 8 * t < a.K;
+                const uint32_t dst = ring + (uint32_t) (q % D) * MVM_GROUP + u * 1024, bytes = in ? 16u : 0u;
+                const __nv_bfloat16 * pa = in ? wa + c * 32 : reinterpret_cast<const __nv_bfloat16 *>(a.W), * pb = in ? wb + c * 32 : pa;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(pa), "r"(bytes) : "memory");
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + 512), "l"(pb), "r"(bytes) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int4 ra[MVM_U], rb[MVM_U];                                              // DEPTH 0: one group, in registers
+    auto load = [&](int q) {
 #pragma unroll
         for (int u = 0; u < MVM_U; u++) {
-            const bool in = c + u < c1 && (c + u) * 32 + 8 * t < a.K;
-            ra[u] = in ? ld_stream_v4(wa + (c + u) * 32) : make_int4(0, 0, 0, 0);
-            rb[u] = in ? ld_stream_v4(wb + (c + u) * 32) : make_int4(0, 0, 0, 0);
+            const int  c  = c0 + q * MVM_U + u;
+            const bool in = c < c1 && c * 32 + 8 * t < a.K;
+            ra[u] = in ? ld_stream_v4(wa + c * 32) : make_int4(0, 0, 0, 0);
+            rb[u] = in ? ld_stream_v4(wb + c * 32) : make_int4(0, 0, 0, 0);
         }
     };
     if (WAIT && a.w_made) pib_pdl_wait();
-    load(c0);
+    if (DEPTH == 0) load(0);
+#pragma unroll
+    for (int q = 0; q < DEPTH; q++) issue(q);
     if (WAIT) { pib_pdl_wait(); pib_pdl_trigger(); }      // a second wait returns at once
     const float * x[NT];
     bool          has[NT];
@@ -307,23 +332,45 @@ __device__ __forceinline__ void mvm_body(const mm_dev & a, int z, int tile, int 
     float acc[NT][4];
 #pragma unroll
     for (int j = 0; j < NT; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-    for (int c = c0; c < c1; c += MVM_U) {
-        if (c > c0) load(c);
-#pragma unroll
-        for (int u = 0; u < MVM_U; u++) {
+    for (int q = 0; q < groups; q++) {
+        const int c = c0 + q * MVM_U;
+        constexpr int XU = DEPTH ? MVM_U : 1;                               // DEPTH: the group's activations in flight together, in front of the wait for its weights
+        float4 xa[NT][XU], xb[NT][XU];
+        auto load_x = [&](int u, int k) {
             const bool in = c + u < c1 && (c + u) * 32 + 8 * t < a.K;
 #pragma unroll
             for (int j = 0; j < NT; j++) {
-                float4 p = make_float4(0.f, 0.f, 0.f, 0.f), q = p;
-                if (in && has[j]) { p = *reinterpret_cast<const float4 *>(x[j] + (c + u) * 32); q = *reinterpret_cast<const float4 *>(x[j] + (c + u) * 32 + 4); }
+                xa[j][k] = xb[j][k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (in && has[j]) { xa[j][k] = *reinterpret_cast<const float4 *>(x[j] + (c + u) * 32); xb[j][k] = *reinterpret_cast<const float4 *>(x[j] + (c + u) * 32 + 4); }
+            }
+        };
+        if (DEPTH) {
+#pragma unroll
+            for (int u = 0; u < MVM_U; u++) load_x(u, u % XU);
+        }
+        if (DEPTH == 0) { if (q) load(q); }
+        else asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");
+        const uint8_t * place = own + (q % D) * MVM_GROUP;
+#pragma unroll
+        for (int u = 0; u < MVM_U; u++) {
+            if (DEPTH == 0) load_x(u, 0);
+            if (DEPTH) { ra[u] = *reinterpret_cast<const int4 *>(place + u * 1024); rb[u] = *reinterpret_cast<const int4 *>(place + u * 1024 + 512); }
+#pragma unroll
+            for (int j = 0; j < NT; j++) {
+                const float4 p = xa[j][u % XU], r = xb[j][u % XU];
                 float c4[4] = { 0.f, 0.f, 0.f, 0.f }, d4[4] = { 0.f, 0.f, 0.f, 0.f };
                 mvm_mma(c4, (uint32_t) ra[u].x, (uint32_t) rb[u].x, (uint32_t) ra[u].y, (uint32_t) rb[u].y, mvm_pack(p.x, p.y), mvm_pack(p.z, p.w));
-                mvm_mma(d4, (uint32_t) ra[u].z, (uint32_t) rb[u].z, (uint32_t) ra[u].w, (uint32_t) rb[u].w, mvm_pack(q.x, q.y), mvm_pack(q.z, q.w));
+                mvm_mma(d4, (uint32_t) ra[u].z, (uint32_t) rb[u].z, (uint32_t) ra[u].w, (uint32_t) rb[u].w, mvm_pack(r.x, r.y), mvm_pack(r.z, r.w));
 #pragma unroll
                 for (int e = 0; e < 4; e++) acc[j][e] += c4[e] + d4[e];
             }
         }
+        if (DEPTH) {
+            __syncwarp();                                                   // the place has been read (by the lanes that fill it)
+            issue(q + DEPTH);
+        }
     }
+    if (DEPTH) asm volatile("cp.async.wait_all;" ::: "memory");
 #pragma unroll
     for (int j = 0; j < NT; j++) {
         red[warp][8 * j + 2 * t][g]     = acc[j][0]; red[warp][8 * j + 2 * t + 1][g]     = acc[j][1];
@@ -341,28 +388,28 @@ __device__ __forceinline__ void mvm_body(const mm_dev & a, int z, int tile, int 
     if (pib_epi_pairs(EPI)) { if (!(r & 1) && n + 1 < a.N) *mm_out(a, Y, row0 + m, n >> 1) = pib_glu_pair<EPI, true>(v, o, a.e0); }
     else if (n < a.N) *mm_out(a, Y, row0 + m, n) = pib_epilogue<EPI, true>(v, a.e0, a.e1);
 }
-template <int EPI, int NT>
-__global__ void __launch_bounds__(256, 3) mv_mma_kernel(mm_dev a) {
-    if (!a.zrange && !a.zlist) { mvm_body<EPI, NT, true>(a, blockIdx.z, blockIdx.x, 0, a.M); return; }
+template <int EPI, int NT, int DEPTH>
+__global__ void __launch_bounds__(256, DEPTH >= 5 ? 1 : (NT == 2 && DEPTH) || DEPTH >= 3 ? 2 : 3) mv_mma_kernel(mm_dev a) {
+    if (!a.zrange && !a.zlist) { mvm_body<EPI, NT, DEPTH, true>(a, blockIdx.z, blockIdx.x, 0, a.M); return; }
     pib_pdl_wait();
     pib_pdl_trigger();
     int z, row0, row1;
-    if (mv_problem(a, blockIdx.z, 8 * NT, z, row0, row1)) mvm_body<EPI, NT, false>(a, z, blockIdx.x, row0, row1);
+    if (mv_problem(a, blockIdx.z, 8 * NT, z, row0, row1)) mvm_body<EPI, NT, DEPTH, false>(a, z, blockIdx.x, row0, row1);
 }
 // mv_experts_kernel's and mv_pair_kernel's work in this form
 template <int EPI, int NT>
-__global__ void __launch_bounds__(256, 3) mv_mma_experts_kernel(mm_dev a, mm_dev b, int tiles_a, int za) {
+__global__ void __launch_bounds__(256, NT == 2 ? 2 : 3) mv_mma_experts_kernel(mm_dev a, mm_dev b, int tiles_a, int za) {
     const int blk = blockIdx.x - tiles_a * za;
-    if (blk >= 0) { mvm_body<EPI, NT, true>(b, 0, blk, 0, b.M); return; }
+    if (blk >= 0) { mvm_body<EPI, NT, 2, true>(b, 0, blk, 0, b.M); return; }
     pib_pdl_wait();
     pib_pdl_trigger();
     int z, row0, row1;
-    if (mv_problem(a, blockIdx.x / tiles_a, 8 * NT, z, row0, row1)) mvm_body<EPI, NT, false>(a, z, (int) blockIdx.x % tiles_a, row0, row1);
+    if (mv_problem(a, blockIdx.x / tiles_a, 8 * NT, z, row0, row1)) mvm_body<EPI, NT, 2, false>(a, z, (int) blockIdx.x % tiles_a, row0, row1);
 }
 template <int EPI_B, int NT>
-__global__ void __launch_bounds__(256, 3) mv_mma_pair_kernel(mm_dev a, mm_dev b, int tiles_a) {
-    if ((int) blockIdx.x < tiles_a) mvm_body<PIB_EPI_NONE, NT, true>(a, 0, blockIdx.x, 0, a.M);
-    else                            mvm_body<EPI_B, NT, true>(b, 0, blockIdx.x - tiles_a, 0, b.M);
+__global__ void __launch_bounds__(256, NT == 2 ? 2 : 3) mv_mma_pair_kernel(mm_dev a, mm_dev b, int tiles_a) {
+    if ((int) blockIdx.x < tiles_a) mvm_body<PIB_EPI_NONE, NT, 2, true>(a, 0, blockIdx.x, 0, a.M);
+    else                            mvm_body<EPI_B, NT, 2, true>(b, 0, blockIdx.x - tiles_a, 0, b.M);
 }
 // bfloat16 weights whose 16-byte pieces and the activations' lie on 16-byte boundaries (the caller has looked at the weights)
 template <typename WT, bool ROUND> static bool mvm_fits(const mm_dev & a, bool xvec) { return std::is_same<WT, __nv_bfloat16>::value && ROUND && xvec && a.K % 8 == 0; }
@@ -421,6 +468,17 @@ __global__ void __launch_bounds__(128) mm_few_cols_kernel(mm_dev a) {
         }
 }
 
+template <typename K> static void mvm_smem(K kernel, size_t smem) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int) cudaSharedmemCarveoutMaxShared);
+}
+#define MVM_SMEM(DEPTH) ((size_t) 8 * (DEPTH) * MVM_GROUP)          // none: the group sits in registers
+template <int EPI, int NT, int DEPTH> static void mvm_launch(dim3 grid, cudaStream_t st, const mm_dev & d) {
+    static bool configured = false;
+    if (DEPTH && !configured) { mvm_smem(mv_mma_kernel<EPI, NT, DEPTH>, MVM_SMEM(DEPTH)); configured = true; }
+    pib_launch(mv_mma_kernel<EPI, NT, DEPTH>, grid, dim3(256), MVM_SMEM(DEPTH), st, d);
+}
+
 template <typename WT, bool ROUND, int EPI>
 static int launch_mm(const pib_mm & a, const mm_dev & d, cudaStream_t st) {
     const int  V = wvec<WT>::N;
@@ -432,8 +490,16 @@ static int launch_mm(const pib_mm & a, const mm_dev & d, cudaStream_t st) {
         const bool xvec = a.ldx % 4 == 0 && a.xz % 4 == 0 && ((uintptr_t) a.X & 15) == 0;
         if (mvm_fits<WT, ROUND>(d, xvec)) {
             grid.x = (unsigned) ((a.N + 15) / 16);
-            if (a.M <= 8) pib_launch(mv_mma_kernel<EPI, 1>, grid, dim3(256), (size_t) 0, st, d);
-            else          pib_launch(mv_mma_kernel<EPI, 2>, grid, dim3(256), (size_t) 0, st, d);
+            // groups that a warp has at most, as far as the shared memory of one, two or more CTAs per SM holds them: what is not needed keeps the next launch's CTAs out
+            // (us a launch, one group in registers / this: 2048 x 5632 at 1 / 4 / 16 tokens 10.0 10.5 19.9 / 6.2 6.4 8.8, 2048 x 2048 4.2 4.3 7.3 / 3.0 3.0 4.2, 8000 x 2048 9.8 10.4 17.6 /
+            // 8.3 9.3 11.7).  Registers alone where a group is all and CTAs are many (32000 x 1024 at 8 tokens 15.8 / 18.2), and for 9 to 16 tokens where a round of three CTAs per SM, the
+            // registers' number, is enough and one of two is not (5120 x 2048 at 16 9.0 / 9.9)
+            const long long ctas = (long long) grid.x * grid.z, sms = pib_num_sms();
+            const int need = ((a.K + 31) / 32 + 8 * MVM_U - 1) / (8 * MVM_U), depth = std::min(need, ctas <= sms ? 5 : ctas <= 2 * sms ? 3 : 2);
+#define MVM_GO(DEPTH) do { if (a.M <= 8) mvm_launch<EPI, 1, DEPTH>(grid, st, d); else mvm_launch<EPI, 2, DEPTH>(grid, st, d); } while (0)
+            if (ctas > 2 * sms && (need == 1 || (a.M > 8 && ctas <= 3 * sms))) MVM_GO(0);
+            else if (depth <= 1) MVM_GO(1); else if (depth == 2) MVM_GO(2); else if (depth == 3) MVM_GO(3); else MVM_GO(5);
+#undef MVM_GO
         } else
         if (a.M == 1)      pib_launch(mv_rows_kernel<WT, ROUND, EPI, 1>, dim3(grid), dim3(256), (size_t) (0), st, d, xvec);
         else if (a.M == 2) pib_launch(mv_rows_kernel<WT, ROUND, EPI, 2>, dim3(grid), dim3(256), (size_t) (0), st, d, xvec);
@@ -490,8 +556,10 @@ static void launch_pair(const mm_dev & a, const mm_dev & b, bool xva, bool xvb, 
     const dim3 grid((unsigned) (ba + bb));
     if (mvm_fits<WT, ROUND>(a, xva) && mvm_fits<WT, ROUND>(b, xvb)) {
         const int ta = (a.N + 15) / 16, tb = (b.N + 15) / 16;
-        if (a.M <= 8) pib_launch(mv_mma_pair_kernel<EPI_B, 1>, dim3((unsigned) (ta + tb)), dim3(256), (size_t) 0, st, a, b, ta);
-        else          pib_launch(mv_mma_pair_kernel<EPI_B, 2>, dim3((unsigned) (ta + tb)), dim3(256), (size_t) 0, st, a, b, ta);
+        static bool configured = false;
+        if (!configured) { mvm_smem(mv_mma_pair_kernel<EPI_B, 1>, MVM_SMEM(2)); mvm_smem(mv_mma_pair_kernel<EPI_B, 2>, MVM_SMEM(2)); configured = true; }
+        if (a.M <= 8) pib_launch(mv_mma_pair_kernel<EPI_B, 1>, dim3((unsigned) (ta + tb)), dim3(256), MVM_SMEM(2), st, a, b, ta);
+        else          pib_launch(mv_mma_pair_kernel<EPI_B, 2>, dim3((unsigned) (ta + tb)), dim3(256), MVM_SMEM(2), st, a, b, ta);
     } else
     if (a.M == 1)      pib_launch(mv_pair_kernel<WT, ROUND, EPI_B, 1>, grid, dim3(256), (size_t) 0, st, a, b, xva, xvb, ba);
     else if (a.M == 2) pib_launch(mv_pair_kernel<WT, ROUND, EPI_B, 2>, grid, dim3(256), (size_t) 0, st, a, b, xva, xvb, ba);
@@ -525,8 +593,10 @@ static void launch_experts(const mm_dev & a, const mm_dev & b, bool xva, bool xv
     const dim3 grid((unsigned) (ba * za + bb));
     if (mvm_fits<WT, ROUND>(a, xva && a.xz % 4 == 0) && mvm_fits<WT, ROUND>(b, xvb)) {
         const int ta = (a.N + 15) / 16, tb = (b.N + 15) / 16;
-        if (rows <= 8) pib_launch(mv_mma_experts_kernel<EPI, 1>, dim3((unsigned) (ta * za + tb)), dim3(256), (size_t) 0, st, a, b, ta, za);
-        else           pib_launch(mv_mma_experts_kernel<EPI, 2>, dim3((unsigned) (ta * za + tb)), dim3(256), (size_t) 0, st, a, b, ta, za);
+        static bool configured = false;
+        if (!configured) { mvm_smem(mv_mma_experts_kernel<EPI, 1>, MVM_SMEM(2)); mvm_smem(mv_mma_experts_kernel<EPI, 2>, MVM_SMEM(2)); configured = true; }
+        if (rows <= 8) pib_launch(mv_mma_experts_kernel<EPI, 1>, dim3((unsigned) (ta * za + tb)), dim3(256), MVM_SMEM(2), st, a, b, ta, za);
+        else           pib_launch(mv_mma_experts_kernel<EPI, 2>, dim3((unsigned) (ta * za + tb)), dim3(256), MVM_SMEM(2), st, a, b, ta, za);
     } else
     if (rows == 1)      pib_launch(mv_experts_kernel<WT, ROUND, EPI, 1>, grid, dim3(256), (size_t) 0, st, a, b, xva, xvb, ba, za);
     else if (rows == 2) pib_launch(mv_experts_kernel<WT, ROUND, EPI, 2>, grid, dim3(256), (size_t) 0, st, a, b, xva, xvb, ba, za);
