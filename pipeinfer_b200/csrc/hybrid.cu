@@ -28,6 +28,7 @@ struct pib_hybrid_ctx {
     float * x = nullptr, * h = nullptr, * y = nullptr, * proj = nullptr, * cq = nullptr, * q = nullptr, * qlat = nullptr, * lat = nullptr, * att = nullptr;
     float * rlog = nullptr, * wts = nullptr, * eup = nullptr, * edn = nullptr, * ysh = nullptr;
     float * h2 = nullptr, * cv = nullptr, * vfirst = nullptr, * mixes = nullptr;   // parallel layers: second norm (pre-norm layers: the stream's second buffer); convolved q | k | v; first mixing layer's values; token-shift mixes
+    float * h16 = nullptr;                             // sandwich frame: the norm's rows as the bfloat16 operand of the matmul that alone reads them (W / 2 floats a row)
     float * rg = nullptr, * y2 = nullptr;       // gated frame: the residual gate's logits; the second branch's output
     float * cat = nullptr;                      // [stream ; embedding] rows of models whose layers are walked again
     int32_t * ids = nullptr, * perm = nullptr, * inv = nullptr, * counts = nullptr, * offs = nullptr, * act = nullptr, * done = nullptr;   // act: the experts with rows of a small batch; done: 0 between launches
@@ -180,9 +181,9 @@ static int grow_chunk(pib_context * c, size_t need) {
 static void free_scratch(pib_hybrid_ctx * x) {
     for (void * b : { (void *) x->x, (void *) x->h, (void *) x->y, (void *) x->proj, (void *) x->cq, (void *) x->q, (void *) x->qlat, (void *) x->lat, (void *) x->att,
                       (void *) x->rlog, (void *) x->wts, (void *) x->eup, (void *) x->edn, (void *) x->ysh, (void *) x->ids, (void *) x->perm, (void *) x->inv,
-                      (void *) x->counts, (void *) x->offs, (void *) x->act, (void *) x->done, (void *) x->h2, (void *) x->cv, (void *) x->vfirst, (void *) x->mixes, (void *) x->cat, (void *) x->rg, (void *) x->y2 }) if (b) cudaFree(b);
+                      (void *) x->counts, (void *) x->offs, (void *) x->act, (void *) x->done, (void *) x->h2, (void *) x->cv, (void *) x->vfirst, (void *) x->mixes, (void *) x->cat, (void *) x->rg, (void *) x->y2, (void *) x->h16 }) if (b) cudaFree(b);
     x->x = x->h = x->y = x->proj = x->cq = x->q = x->qlat = x->lat = x->att = x->rlog = x->wts = x->eup = x->edn = x->ysh = nullptr;
-    x->h2 = x->cv = x->vfirst = x->mixes = x->cat = x->rg = x->y2 = nullptr;
+    x->h2 = x->cv = x->vfirst = x->mixes = x->cat = x->rg = x->y2 = x->h16 = nullptr;
     x->ids = x->perm = x->inv = x->counts = x->offs = x->act = x->done = nullptr;
     x->cap = 0;
 }
@@ -225,7 +226,7 @@ static int grow_scratch(pib_context * c, int T) {
                     in(&x->ids, n * hy->w_pairs) && in(&x->perm, n * hy->w_pairs) && in(&x->inv, n * hy->w_pairs) && in(&x->counts, (size_t) hy->w_router + 1) &&
                     in(&x->offs, (size_t) hy->w_router + 2) && in(&x->act, (size_t) hy->w_router + 2) && in(&x->done, hy->w_router ? 4 : 0) && (!x->done || cudaMemset(x->done, 0, 16) == cudaSuccess) && fl(&x->h2, hy->form == PIB_FORM_PARALLEL || hy->form == PIB_FORM_PRENORM || hy->form == PIB_FORM_GATED ? W : 0) && fl(&x->cv, (size_t) hy->w_conv) &&
                     fl(&x->vfirst, (size_t) hy->w_vfirst) && fl(&x->mixes, (size_t) hy->w_shift) && fl(&x->cat, (size_t) hy->w_cat) &&
-                    fl(&x->rg, (size_t) hy->w_gate) && fl(&x->y2, (size_t) hy->w_y2);
+                    fl(&x->rg, (size_t) hy->w_gate) && fl(&x->y2, (size_t) hy->w_y2) && fl(&x->h16, hy->form == PIB_FORM_SANDWICH && hy->dtype != PIB_TYPE_F32 ? (W + 1) / 2 : 0);
     if (!ok) { cudaGetLastError(); free_scratch(x); pib_set_error("decode: out of memory for the work buffers of %d tokens", T); return PIB_ERR_NOMEM; }
     x->cap = (int) n;
     return PIB_OK;
@@ -288,7 +289,7 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
     // rows that only a tensor-core matmul reads are written as its bfloat16 operand by the kernel that makes them (the values that the matmul's own rounding would give)
     const bool dump = getenv("PIB_HYBRID_DUMP") != nullptr;
     auto takes = [&](const pib_weight * w) { return !exact && !dump && pib_dense_takes_rows(w, T); };
-    bool h_bf16 = false;                              // x->h holds such rows
+    bool h_bf16 = false;                              // the rows the last norm left are such rows, in x->h16 (x->h keeps what the mixture before reads: its identity outputs)
     auto mm16 = [&](const pib_weight * w, const float * X, float * Y, int ldy, int epi, float e0, float e1, bool x16, bool y16) {
         pib_mm a = mm_of(w, X, (int) w->K, Y, ldy, epi, e0, e1);
         a.x_bf16 = x16; a.y_bf16 = y16;
@@ -711,7 +712,7 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
         h_bf16 = w && h16;
         pib_norm_route nr;
         if (moe) { nr.rows = (const float *) moe->router->base; nr.R = router_of(*moe); nr.ids = x->ids; nr.wts = x->wts; nr.offs = x->offs; nr.perm = x->perm; nr.inv = x->inv; nr.act = x->act; nr.done = x->done; }
-        RC(moe ? HK_NORM_ROUTE : HK_SANDWICH, moe ? mmfl(moe->router) : 0, (moe ? wbytes(moe->router) : 0.0) + 4.0 * Td * Wd * ((leftn.y ? 3.0 : leftn.top ? 2.0 : 1.0) + leftn.top + (w ? 1.0 : 0.0)), pib_sandwich_norm(x->x, leftn, w, b, eps, T, W, w ? x->h : nullptr, st, moe ? &nr : nullptr, h_bf16));
+        RC(moe ? HK_NORM_ROUTE : HK_SANDWICH, moe ? mmfl(moe->router) : 0, (moe ? wbytes(moe->router) : 0.0) + 4.0 * Td * Wd * ((leftn.y ? 3.0 : leftn.top ? 2.0 : 1.0) + leftn.top + (w ? 1.0 : 0.0)), pib_sandwich_norm(x->x, leftn, w, b, eps, T, W, w ? (h_bf16 ? x->h16 : x->h) : nullptr, st, moe ? &nr : nullptr, h_bf16));
         leftn = pib_sublayer_y();
         return PIB_OK;
     };
@@ -720,13 +721,13 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
         int lds = 0;
         if (hy->form == PIB_FORM_SANDWICH) {
             if ((rc = sandwich(L.norm1, L.norm1_b, nullptr, L.mixer == PIB_MIXER_KV && takes(L.qkv))) != PIB_OK) return rc;
-            if ((rc = run_mixer(L, x->h)) != PIB_OK) return rc;
+            if ((rc = run_mixer(L, h_bf16 ? x->h16 : x->h)) != PIB_OK) return rc;
             leftn.y = x->y; leftn.w = L.post1; leftn.b = L.post1_b;
             const bool routed = L.mlp == PIB_MLP_MOE && pib_norm_route_fits(T, W, router_of(L));      // small batches: the router rides on the norm
             if (L.mlp != PIB_MLP_NONE && (rc = sandwich(L.norm2, L.norm2_b, routed ? &L : nullptr, L.mlp == PIB_MLP_RELU2 && takes(L.up))) != PIB_OK) return rc;
             if (L.mlp == PIB_MLP_RELU2) {
                 const bool z16 = takes(L.up) && takes(L.down);
-                RC(HK_UP, mmfl(L.up), mmby(L.up), mm16(L.up, x->h, x->proj, L.ff, PIB_EPI_RELU2, 0.f, 0.f, h_bf16, z16));
+                RC(HK_UP, mmfl(L.up), mmby(L.up), mm16(L.up, h_bf16 ? x->h16 : x->h, x->proj, L.ff, PIB_EPI_RELU2, 0.f, 0.f, h_bf16, z16));
                 RC(HK_DOWN, mmfl(L.down), mmby(L.down), mm16(L.down, x->proj, x->y, W, PIB_EPI_NONE, 0.f, 0.f, z16, false));
                 leftn.y = x->y;
             } else if (L.mlp == PIB_MLP_MOE && L.expert == PIB_EXPERT_SWIGLU) {
@@ -836,7 +837,7 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
     else if (hy->form == PIB_FORM_PRENORM)  { if ((rc = prenorm(hy->final_g, nullptr, 0, false)) != PIB_OK) return rc; }
     else if (hy->form == PIB_FORM_PARALLEL) RC(HK_FINAL, 0, 8.0 * Td * Wd, pib_rms_norm2(x->x, m->output_norm, nullptr, eps, hy->logit_scale, T, W, x->h, nullptr, st));
     else                                    RC(HK_FINAL, 0, 8.0 * Td * Wd, pib_layer_norm(x->x, m->output_norm, eps, T, W, x->h, 0, st));
-    RC(HK_HEAD, mmfl(m->output), mmby(m->output), mm16(m->output, x->h, run.logits, m->n_vocab, PIB_EPI_NONE, 0.f, 0.f, h_bf16, false));
+    RC(HK_HEAD, mmfl(m->output), mmby(m->output), mm16(m->output, h_bf16 ? x->h16 : x->h, run.logits, m->n_vocab, PIB_EPI_NONE, 0.f, 0.f, h_bf16, false));
     RC(HK_SAMPLE, 0, 4.0 * Td * m->n_vocab, pib_sample_topk(run.logits, T, m->n_vocab, c->bias_ids_dev, c->bias_val_dev, c->n_bias, run.res_dev, c->desc_dev, c->cancel_table, st));
 #undef RC
     return PIB_OK;

@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(NV >= 4 ? 512 : 1024) sandwich_norm_kernel(sw_
 #pragma unroll
             for (int i = 0; i < VEC; i++) h.v[i] = fmaf((x[n].v[i] - mx.x) * mx.y, w.v[i], b.v[i]);
             if (A.h_bf16) sw_store16<VEC>(reinterpret_cast<__nv_bfloat16 *>(A.h) + row + c, h);
-            else          sw_store<VEC>(A.h + row + c, h);             // a thread wrote and read only its own channels of this token: hin may be h
+            else          sw_store<VEC>(A.h + row + c, h);             // a thread wrote and read only its own channels of this token: hin may be h (float rows)
             if (ROUTE) sw_store<VEC>(sw_dyn + c, h);
         }
     }
@@ -182,6 +182,11 @@ bool pib_norm_route_fits(int T, int W, const pib_router & R) {
 // o empty: only the norm of x; h null: only the sum; h_bf16: h gets bfloat16 rows (what the tensor-core matmul behind it reads); route: see pib_norm_route (the caller has asked pib_norm_route_fits)
 int pib_sandwich_norm(float * x, const pib_sublayer_y & o, const float * w, const float * b, float eps, int T, int W, float * h, cudaStream_t st, const pib_norm_route * route, bool h_bf16) {
     sw_args A = { x, o, w, b, eps, W, h, h_bf16 ? 1 : 0, pib_norm_route() };
+    // bfloat16 rows are half as long as the rows they would lie over: a block's row would cover rows that other blocks have yet to read
+    if (h_bf16 && o.top > 0 && (const char *) h < (const char *) (o.hin + (size_t) T * W) && (const char *) o.hin < (const char *) h + (size_t) T * W * 2) {
+        pib_set_error("sandwich norm: bfloat16 rows over the mixture's input rows");
+        return PIB_ERR_ARG;
+    }
     if (route && h_bf16) { pib_set_error("sandwich norm: the router reads float rows"); return PIB_ERR_ARG; }
     if (route) {
         const int rc = pib_moe_router_check(route->R);

@@ -16,7 +16,7 @@ import numpy as np
 import pytest
 
 from tests import gusedra_oracle as O
-from tests.gusedra_configs import CONFIGS, drawn
+from tests.gusedra_configs import CONFIGS, drawn, model, moe, slopes
 from tests.test_gpu_rapisun import Served, row_err, spread, TOL32, TOL16
 
 pytestmark = pytest.mark.gpu
@@ -436,6 +436,22 @@ def test_portions_of_many_lengths_in_one_batch(tmp_path, name):
     s.close()
     for i, t in enumerate(many):
         assert close16(row_err(got[i], oracle_logits(cfg, W, t))), i
+
+
+@pytest.mark.parametrize("n", [17, 300, 2500])
+def test_identity_outputs_in_front_of_a_matmul_that_takes_bfloat16_rows(tmp_path, n):
+    """served mode: every token's choice falls on the identity outputs only, so what a norm reads is the rows that the norm before left, while it writes the bfloat16 rows of the
+    matmul behind it (an attention's, the output's); every row has to come out right, over many rounds of blocks.  No choice can turn, so no row may be far off"""
+    cfg = model(64, 140, [(slopes(2, 1, 8, 8, 3), moe(2, 4, 16, identity=4, scale=1.5, shared=24)), (slopes(1, 1, 8, 16, 2), moe(3, 2, 8, identity=2, scale=2.0))], mult=1.0)
+    W = O.random_weights(cfg, 51)
+    for i, identity in enumerate([4, 2]):
+        W["l%d.mlp.correction" % i][-identity:] = 64.0
+    toks = tokens(cfg, n, 52)
+    s = Served(tmp_path, cfg, W, float32=False, n_ctx=2600)
+    e = row_err(s.feed(0, toks, []), oracle_logits(cfg, W, toks))
+    s.close()
+    print("largest row error %.3g, median %.3g" % (e.max(), np.median(e)))
+    assert e.max() < TOL16
 
 
 @pytest.mark.parametrize("float32", [True, False])

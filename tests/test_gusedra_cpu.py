@@ -123,3 +123,23 @@ def test_a_later_layer_reads_an_earlier_layers_cells():
 def test_dense_feed_forward_squares_what_is_positive():
     W = {"up": np.array([[1.0], [-1.0]]), "down": np.array([[1.0, 100.0]])}
     assert np.allclose(O.dense_ff(np.array([[3.0], [-2.0]]), W, ""), [[9.0], [400.0]])
+
+
+def test_bfloat16_rows_never_lie_over_the_mixture_rows():
+    """the norm behind a mixture reads the mixture's float rows for identity outputs; a bfloat16 row of one token would cover rows that other tokens' blocks have yet to
+    read, so such a call is refused before anything is launched"""
+    import ctypes as C
+    import os
+    lib = C.CDLL(os.path.join(os.path.dirname(__file__), "..", "pipeinfer_b200", "libpipeinfer_b200.so"))
+    norm = lib._Z17pib_sandwich_normPfRK14pib_sublayer_yPKfS4_fiiS_P11CUstream_stPK14pib_norm_routeb
+    norm.argtypes = [C.c_void_p] * 4 + [C.c_float, C.c_int, C.c_int] + [C.c_void_p] * 3 + [C.c_bool]
+
+    class Y(C.Structure):
+        _fields_ = [(n, C.c_void_p) for n in ("y", "edn", "wts", "hin", "ids", "inv")] + [("top", C.c_int), ("n_real", C.c_int)] + [("w", C.c_void_p), ("b", C.c_void_p)]
+    T, W, hin = 40, 64, 1 << 20
+    ARG = -2
+    lib.pib_last_error.restype = C.c_char_p
+    o = Y(hin=hin, top=2, n_real=1)
+    for h in (hin, hin + T * W * 4 - 16, hin - T * W * 2 + 16):
+        assert norm(1 << 24, C.addressof(o), 1 << 25, 1 << 25, 1e-5, T, W, h, None, None, True) == ARG
+        assert b"mixture" in lib.pib_last_error()
