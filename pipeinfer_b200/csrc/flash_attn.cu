@@ -267,8 +267,8 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap qh, const __grid_constant_
             if (j > 1) {                                             // the group's product before has read its weights and left the accumulator
                 ok = dt_mbar_wait(bar_o + 8 * w, ((j >> 1) - 1) & 1, abort_s);
                 if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+                dt_fence_after();                                    // also without a rescale: the weights' stores below come behind that product's reads of them
                 if (rescale) {
-                    dt_fence_after();
                     for (int c = 0; c < A.VN; c += 32) {
                         uint32_t v[32];
                         dt_ld32(tm_w + c, v);
