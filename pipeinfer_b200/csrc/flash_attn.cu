@@ -9,14 +9,13 @@
 //                mask, running maximum, weights as two bfloat16 parts back into tensor memory (the first operand of the second product).  Each group has its own accumulator,
 //                rescaled only when a maximum has grown by more than 2^FA_LAZY; both are merged on the way out
 // Scores keep fp32 accuracy on bfloat16 operands: queries and keys enter as their bfloat16 part and the remainder of that rounding, three products are summed
-// (hi.hi + lo.hi + hi.lo); weights enter as two parts against the bfloat16 values, in short portions against the values' remainders too (hi.lo): those would otherwise go to
-// the per-token kernel, which keeps values in fp32.  The sink is the running state's start (maximum = sink, denominator = 1).
+// (hi.hi + lo.hi + hi.lo); weights enter as two parts against the bfloat16 values.  The sink is the running state's start (maximum = sink, denominator = 1).
 // The result leaves in token order, divided by the denominator and (optionally) gated.
 // Operands: fa_gather_kernel lays out, for every portion, key columns [kept first positions (n_front) | positions j0, j0 + 1, ... | zeros up to 64], values transposed, query rows;
 // tiles nobody in the block sees are not visited.  Every wait is bounded (tc_common.cuh).
 // What bounds it: the score products (24 MMAs of 64 keys a tile, 57 clocks each: a tile takes 2650 clocks), and with few tiles a block's start and end: code that runs once comes from far
 // away, 9 clocks an instruction.  Three portions of 517, 504 and 491 tokens, 16 heads of 128 over 4: one launch 34 us with slopes, 48 with a bias table and a gate (a launch per
-// portion, weights through shared memory, the table read from memory, a lane's own row written by it: 88 and 153); four of 51 to 90 tokens: 19 and 24 (per token 75 and 91).
+// portion, weights through shared memory, the table read from memory, a lane's own row written by it: 88 and 153).
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -48,7 +47,7 @@ __device__ __forceinline__ int fa_low(const fa_args & A, int p) { return A.mask 
 
 template <int NC> struct fa_cfg {                    // NC: 64-wide column chunks of a head (1 or 2)
     static constexpr int Q_TILE = FA_ROWS * 128, K_TILE = FA_KEYS * 128, V_TILE = 128 * 128;
-    static constexpr int Q_BYTES = 2 * NC * Q_TILE, K_BYTES = 2 * NC * K_TILE, STAGE = K_BYTES + 2 * V_TILE;
+    static constexpr int Q_BYTES = 2 * NC * Q_TILE, K_BYTES = 2 * NC * K_TILE, STAGE = K_BYTES + V_TILE;
     static constexpr size_t SMEM = (size_t) Q_BYTES + 2 * STAGE + 2 * FA_ROWS * 8 + 16 * 8 + 32 + 1024;    // behind the stages: the groups' maxima and denominators; then the bias table
 };
 
@@ -68,7 +67,7 @@ __device__ __forceinline__ void fa_st16(uint32_t taddr, const uint32_t * v) {
 template <int NC>
 __global__ void __launch_bounds__(FA_THREADS)
 flash_attn_kernel(const __grid_constant__ CUtensorMap qh, const __grid_constant__ CUtensorMap ql, const __grid_constant__ CUtensorMap kh, const __grid_constant__ CUtensorMap kl,
-                  const __grid_constant__ CUtensorMap vh, const __grid_constant__ CUtensorMap vl, const __grid_constant__ fa_args A) {
+                  const __grid_constant__ CUtensorMap vm, const __grid_constant__ fa_args A) {
     pib_pdl_wait();
     pib_pdl_trigger();
     using C = fa_cfg<NC>;
@@ -141,9 +140,8 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap qh, const __grid_constant_
                 const int k = 8 * (j & 1);
                 if (j + 1 < n_tiles && !(ok = keys(j + 1))) break;
                 if (j >= 2 && !dt_mbar_wait(bar_vf + k, ((j >> 1) - 1) & 1, abort_s)) break;
-                dt_mbar_expect_tx(bar_v + k, A.VN * 128 * (G.v_parts));
-                dt_tma_3d(dt_smem(sKV + (j & 1) * C::STAGE + C::K_BYTES), &vh, bar_v + k, G.col0 + tile_of(j) * FA_KEYS, 0, z);
-                if (G.v_parts > 1) dt_tma_3d(dt_smem(sKV + (j & 1) * C::STAGE + C::K_BYTES + C::V_TILE), &vl, bar_v + k, G.col0 + tile_of(j) * FA_KEYS, 0, z);
+                dt_mbar_expect_tx(bar_v + k, A.VN * 128);
+                dt_tma_3d(dt_smem(sKV + (j & 1) * C::STAGE + C::K_BYTES), &vm, bar_v + k, G.col0 + tile_of(j) * FA_KEYS, 0, z);
             }
         }
     } else if (warp == 1) {
@@ -177,9 +175,10 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap qh, const __grid_constant_
             dt_fence_after();
             const uint64_t dv = dt_desc(dt_smem(sKV + (j & 1) * C::STAGE + C::K_BYTES));
             const uint32_t tp = tm_p + 64 * (j & 1);
-            for (int part = 0; part < 1 + G.v_parts; part++)       // hi.hi, lo.hi, hi.lo
 #pragma unroll
-                for (int k = 0; k < 4; k++) fa_mma_ts(tm_o + 128 * (j & 1), tp + (part == 1 ? 32 : 0) + 8 * k, dv + (part == 2 ? (uint64_t) (C::V_TILE >> 4) : 0) + 2 * k, id_o, (j > 1) | ((part | k) != 0));
+            for (int part = 0; part < 2; part++)                   // the weights' parts
+#pragma unroll
+                for (int k = 0; k < 4; k++) fa_mma_ts(tm_o + 128 * (j & 1), tp + 32 * part + 8 * k, dv + 2 * k, id_o, (j > 1) | ((part | k) != 0));
             dt_commit(bar_o + 8 * (j & 1));
             dt_commit(bar_vf + 8 * (j & 1));
         }
@@ -314,7 +313,8 @@ flash_attn_kernel(const __grid_constant__ CUtensorMap qh, const __grid_constant_
             const float  f0 = (w == 0 ? fm : fo) * inv, f1 = (w == 0 ? fo : fm) * inv;
             // a chunk of 32 columns turns through shared memory (the operands' place: every product is done), so that a row's values leave and its gate's arrive in one piece (a
             // lane per row took 20 us of a gated block's time)
-            float * buf = reinterpret_cast<float *>(sKV) + (warp - 2) * 2 * 32 * 36, * gbuf = buf + 32 * 36;
+            static_assert(8 * 2 * 32 * 36 * 4 <= C::Q_BYTES + 2 * C::STAGE, "chunks of values and gates of eight warps");
+            float * buf = reinterpret_cast<float *>(sQ) + (warp - 2) * 2 * 32 * 36, * gbuf = buf + 32 * 36;
             const uint32_t gate_at = (uint32_t) (((size_t) (G.t0 + Rc / A.rep) * A.ldg + (size_t) h * A.V) / 4);
             const int row = (int) ((size_t) (G.t0 + Rc / A.rep) * A.H + h), rows = min(32, n_rows - row0 - q4 * 32);
 #pragma unroll 1
@@ -393,7 +393,7 @@ bool pib_flash_attention_fits(const pib_hlayer & L) {
 }
 
 // ---- operands ---------------------------------------------------------------------------------------------------------------------
-// keys Kb [GK][C][2 D] = [hi | lo], values Vt [2][GK][V][C] (hi, lo), queries Qc [GK][R][2 D], bfloat16; C columns and R rows of all portions (pib_attn_block: col0, row0)
+// keys Kb [GK][C][2 D] = [hi | lo], values Vt [GK][V][C], queries Qc [GK][R][2 D], bfloat16; C columns and R rows of all portions (pib_attn_block: col0, row0)
 struct fa_gather_args {
     const float * cache; int cache_row; const int32_t * cellmap; int n_ctx;
     const float * q; int ldq, vec_k, vec_q;                      // vec: four floats at a time
@@ -478,7 +478,7 @@ __global__ void __launch_bounds__(256) fa_gather_kernel(const __grid_constant__ 
         }
         return;
     }
-    const size_t vo = (size_t) A.GK * A.D + (size_t) (z / A.maps) * A.V, plane = (size_t) A.GK * A.V * A.C;
+    const size_t vo = (size_t) A.GK * A.D + (size_t) (z / A.maps) * A.V;
     const int v0 = (what - 2) * 32;
 #pragma unroll
     for (int i = 0; i < 8; i++) tile[warp + 8 * i][lane] = rows[i] && v0 + lane < A.V ? rows[i][vo + v0 + lane] : 0.f;
@@ -486,21 +486,14 @@ __global__ void __launch_bounds__(256) fa_gather_kernel(const __grid_constant__ 
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int c = warp + 8 * i;
-        if (v0 + c < A.V) {
-            const float a = tile[2 * lane][c], b = tile[2 * lane + 1][c];
-            const __nv_bfloat162 hi = __floats2bfloat162_rn(a, b);
-            const float2 f = __bfloat1622float2(hi);
-            __nv_bfloat16 * p = A.Vt + ((size_t) z * A.V + v0 + c) * A.C + c0 + 2 * lane;
-            *reinterpret_cast<__nv_bfloat162 *>(p)         = hi;
-            *reinterpret_cast<__nv_bfloat162 *>(p + plane) = __floats2bfloat162_rn(a - f.x, b - f.y);
-        }
+        if (v0 + c < A.V) *reinterpret_cast<__nv_bfloat162 *>(A.Vt + ((size_t) z * A.V + v0 + c) * A.C + c0 + 2 * lane) = __floats2bfloat162_rn(tile[2 * lane][c], tile[2 * lane + 1][c]);
     }
 }
 
 size_t pib_flash_attention_bytes(const pib_hlayer & L, long long cols, long long rows, size_t * k_bytes, size_t * v_bytes) {
     const size_t GK = (size_t) L.kv_heads * L.maps;
     *k_bytes = GK * cols * 2 * L.dim * 2;
-    *v_bytes = 2 * GK * L.vdim * cols * 2;
+    *v_bytes = GK * L.vdim * cols * 2;
     return GK * rows * 2 * L.dim * 2;
 }
 void pib_flash_attention_place(std::vector<pib_attn_block> & blocks, int rep, long long * cols, long long * rows) {
@@ -525,14 +518,13 @@ int pib_flash_attention(const pib_kv_query & q, const pib_hlayer & L, const std:
     pib_launch(fa_gather_kernel, dim3((unsigned) std::max(C / 64, R / 32), (unsigned) Z, (unsigned) (2 + (V + 31) / 32)), dim3(256), (size_t) 0, st, g);
     PIB_CHECK(cudaGetLastError());
     const __nv_bfloat16 * kb = (const __nv_bfloat16 *) Kb, * qc = (const __nv_bfloat16 *) Qc, * vt = (const __nv_bfloat16 *) Vt;
-    CUtensorMap qh, ql, kh, kl, vh, vl;
+    CUtensorMap qh, ql, kh, kl, vm;
     const int VN = (V + 15) & ~15;
     int rc = pib_tma_map3(&qh, qc, D, R, Z, 4 * (uint64_t) D, 4 * (uint64_t) D * R, FA_ROWS);
     if (rc == PIB_OK) rc = pib_tma_map3(&ql, qc + D, D, R, Z, 4 * (uint64_t) D, 4 * (uint64_t) D * R, FA_ROWS);
     if (rc == PIB_OK) rc = pib_tma_map3(&kh, kb, D, C, Z, 4 * (uint64_t) D, 4 * (uint64_t) D * C, FA_KEYS);
     if (rc == PIB_OK) rc = pib_tma_map3(&kl, kb + D, D, C, Z, 4 * (uint64_t) D, 4 * (uint64_t) D * C, FA_KEYS);
-    if (rc == PIB_OK) rc = pib_tma_map3(&vh, vt, C, V, Z, 2 * (uint64_t) C, 2 * (uint64_t) C * V, (uint32_t) VN);
-    if (rc == PIB_OK) rc = pib_tma_map3(&vl, vt + (size_t) Z * V * C, C, V, Z, 2 * (uint64_t) C, 2 * (uint64_t) C * V, (uint32_t) VN);
+    if (rc == PIB_OK) rc = pib_tma_map3(&vm, vt, C, V, Z, 2 * (uint64_t) C, 2 * (uint64_t) C * V, (uint32_t) VN);
     if (rc != PIB_OK) return rc;
     int * err = pib_tc_error_word(st);
     if (!err) { pib_set_error("attention: no error word"); return PIB_ERR_NOMEM; }
@@ -549,7 +541,7 @@ int pib_flash_attention(const pib_kv_query & q, const pib_hlayer & L, const std:
 #define FA_GO(NC) do {                                                                                                                             \
         static bool configured = false;                                                                                                            \
         if (!configured) { PIB_CHECK(cudaFuncSetAttribute(flash_attn_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (fa_cfg<NC>::SMEM + FA_REL_MAX))); configured = true; } \
-        pib_launch(flash_attn_kernel<NC>, dim3((unsigned) (row_blocks * Z)), dim3(FA_THREADS), fa_cfg<NC>::SMEM + extra, st, qh, ql, kh, kl, vh, vl, A); \
+        pib_launch(flash_attn_kernel<NC>, dim3((unsigned) (row_blocks * Z)), dim3(FA_THREADS), fa_cfg<NC>::SMEM + extra, st, qh, ql, kh, kl, vm, A); \
     } while (0)
     if (D <= 64) FA_GO(1); else FA_GO(2);
 #undef FA_GO

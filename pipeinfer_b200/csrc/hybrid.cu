@@ -235,16 +235,14 @@ static int grow_scratch(pib_context * c, int T) {
 // ---- the layers -----------------------------------------------------------------------------------------------------------------------
 // Attention of a segment of at least MM_ATTN_MIN_LEN tokens runs as matmuls on the tensor cores in served mode, in blocks of at most
 // MM_ATTN_BLOCK tokens: latent attention when its rows have at least MM_ATTN_MIN_ROW floats (a multiple of 8), key / value-head
-// attention when the head size is a multiple of 8.  Everything else (decoded tokens, short portions, float32 contexts) stays with the
+// attention when the head size is a multiple of 8.  (Shorter portions would be faster there -- four of 51 to 90 tokens 19 and 24 us a launch, per token 75 and 91 -- but the per-token
+// kernel holds queries, keys, weights and values in fp32, those forms in two bfloat16 parts at most.)  Everything else (decoded tokens, short portions, float32 contexts) stays with the
 // per-token kernels.
 #define MM_ATTN_MIN_LEN 128
 #define MM_ATTN_MIN_ROW 192
 #define MM_ATTN_BLOCK   512
 #define FLASH_ATTN_BLOCK 4096     // the form that keeps its scores on chip
 #define FLASH_ATTN_COLS  16384    // key columns laid out for one launch of it
-// Shorter portions go to the per-token kernel (two 2048-wide layers, us a prompt call, this form / per token: one sequence of 32 tokens 260 / 251, 48 274 / 282, 100 299 / 325;
-// three 340 / 325, 359 / 375, 406 / 542; eight 506 / 540, 540 / 630, 696 / 1075).  More than the 16 tokens of a captured step, whose portions may change.
-#define FLASH_ATTN_MIN_LEN 48
 // a recurrence's matmul form works through a segment in blocks of at most MM_SCAN_BLOCK tokens (its operands take a few hundred MB per block)
 #define MM_SCAN_BLOCK   2048
 struct pib_hseg { int start, len, seq, slot; bool fresh; };
@@ -364,15 +362,14 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
         const int H = L.heads * L.maps, G = L.kv_heads * L.maps, D = L.dim, V = L.vdim;      // query rows and key heads: one per map
         const double keys = key_pairs(L.window, L.mask, L.keep);
         const bool mm_ok = !exact && D % 8 == 0 && D >= 16 && V >= 16 && attn_mm_enabled();
-        const bool flash = mm_ok && pib_flash_attention_fits(L);                                           // no score rows in memory: shorter portions, longer blocks
-        const int  min_len = flash ? FLASH_ATTN_MIN_LEN : MM_ATTN_MIN_LEN;
+        const bool flash = mm_ok && pib_flash_attention_fits(L);                                           // no score rows in memory: longer blocks
         bool any_mm = false, any_simt = false;
-        for (const pib_hseg & g : segs) { if (mm_ok && g.len >= min_len) any_mm = true; else any_simt = true; }
+        for (const pib_hseg & g : segs) { if (mm_ok && g.len >= MM_ATTN_MIN_LEN) any_mm = true; else any_simt = true; }
         const bool o16 = out16 && flash && any_mm && !any_simt;          // bfloat16 rows out, where the caller asks and one form makes them all
         if (out16) *out16 = o16;
         if (any_simt)
             RC(HK_KVATTN, 2.0 * keys * H * (D + V), 4.0 * keys * G * (D + V) + 4.0 * Td * H * (D + V),
-               pib_kv_attention(q, L, B, cache, row, x->cellmap, (int) c->n_ctx, out, any_mm ? (flash ? B.faflag : B.mmflag) : nullptr, st));
+               pib_kv_attention(q, L, B, cache, row, x->cellmap, (int) c->n_ctx, out, any_mm ? B.mmflag : nullptr, st));
         // portions of all segments gathered into launches of up to FLASH_ATTN_COLS key columns
         std::vector<pib_attn_block> blocks;
         double bl_pairs = 0, bl_keys = 0, bl_tok = 0;
@@ -391,7 +388,7 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
             return PIB_OK;
         };
         for (const pib_hseg & g : segs) {
-            if (!mm_ok || g.len < min_len) continue;
+            if (!mm_ok || g.len < MM_ATTN_MIN_LEN) continue;
             const int block = flash ? FLASH_ATTN_BLOCK : MM_ATTN_BLOCK, nb = (g.len + block - 1) / block, per = (g.len + nb - 1) / nb;      // blocks of equal size: none is left with a handful of rows
             for (int o = 0; o < g.len; o += per) {
                 const int nq = std::min(per, g.len - o), p0 = B_pos_host[g.start + o];
@@ -402,7 +399,7 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
                 for (int i = 0; i < nq; i++) pairs += L.mask == PIB_MASK_CHUNK ? (p0 + i) % L.window + 1 : std::min<int64_t>(p0 + i + 1, (int64_t) L.window + L.keep);
                 if (flash) {
                     if (!blocks.empty() && ((int) blocks.size() == pib_flash_attention_max() || bl_keys + NK > FLASH_ATTN_COLS) && (rc = launch()) != PIB_OK) return rc;
-                    blocks.push_back({ nq, g.start + o, p0, j0, n_front, NK, g.slot, g.len < MM_ATTN_MIN_LEN ? 2 : 1, 0, 0, 0, 0 });
+                    blocks.push_back({ nq, g.start + o, p0, j0, n_front, NK, g.slot, 0, 0, 0, 0 });
                     bl_pairs += pairs; bl_keys += NK; bl_tok += nq;
                     continue;
                 }
@@ -898,8 +895,8 @@ int pib_hybrid_decode_start(pib_context * c, int n_tokens, const int32_t * token
         }
         x->slots.len[(size_t) g.slot] += g.len;
     }
-    // bookkeeping: [tok | pos | cell | slot | seg | mmflag | faflag] x T, then [seg_start | seg_len | seg_slot] x S
-    const int S = (int) segs.size(), words = 7 * T + 3 * S;
+    // bookkeeping: [tok | pos | cell | slot | seg | mmflag] x T, then [seg_start | seg_len | seg_slot] x S
+    const int S = (int) segs.size(), words = 6 * T + 3 * S;
     if (words > x->meta_cap) {
         cudaStreamSynchronize(st);
         for (auto & g : c->graphs) if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
@@ -920,8 +917,8 @@ int pib_hybrid_decode_start(pib_context * c, int n_tokens, const int32_t * token
     int32_t * mh = x->meta_host[ring];
     for (int sgi = 0; sgi < S; sgi++) {
         const pib_hseg & g = segs[(size_t) sgi];
-        for (int i = g.start; i < g.start + g.len; i++) { mh[3 * T + i] = g.slot; mh[4 * T + i] = sgi; mh[5 * T + i] = g.len >= MM_ATTN_MIN_LEN ? 1 : 0; mh[6 * T + i] = g.len >= FLASH_ATTN_MIN_LEN ? 1 : 0; }
-        mh[7 * T + sgi] = g.start; mh[7 * T + S + sgi] = g.len; mh[7 * T + 2 * S + sgi] = g.slot;
+        for (int i = g.start; i < g.start + g.len; i++) { mh[3 * T + i] = g.slot; mh[4 * T + i] = sgi; mh[5 * T + i] = g.len >= MM_ATTN_MIN_LEN ? 1 : 0; }
+        mh[6 * T + sgi] = g.start; mh[6 * T + S + sgi] = g.len; mh[6 * T + 2 * S + sgi] = g.slot;
     }
     memcpy(mh, token, (size_t) T * 4);
     memcpy(mh + T, pos, (size_t) T * 4);
@@ -930,7 +927,7 @@ int pib_hybrid_decode_start(pib_context * c, int n_tokens, const int32_t * token
     cudaEventRecord(x->meta_ev[ring], st);
     c->h2d_bytes += (size_t) words * 4;
     const int32_t * md = x->meta_dev;
-    pib_hbatch B = { md, md + T, md + 2 * T, md + 3 * T, md + 4 * T, md + 5 * T, md + 6 * T, md + 7 * T, md + 7 * T + S, md + 7 * T + 2 * S, T, S };
+    pib_hbatch B = { md, md + T, md + 2 * T, md + 3 * T, md + 4 * T, md + 5 * T, md + 6 * T, md + 6 * T + S, md + 6 * T + 2 * S, T, S };
     run->in_use = true; run->batch_id = batch_id; run->n_tokens = T; run->failed = false; run->has_walk = false;
     c->tree_pending.n_branches = 0;
     cudaMemcpyAsync(c->cancel_table, c->run_id_host + run->id, sizeof(int), cudaMemcpyHostToDevice, st);

@@ -284,7 +284,6 @@ pib_weight * pib_dense_upload(int type, const void * host, int64_t N, int64_t K)
 struct pib_hbatch {                  // device view of one batch's bookkeeping
     const int32_t * tok, * pos, * cell, * slot, * seg;       // [T]
     const int32_t * mmflag;                                   // [T] 1: the token's attention runs in the matmul form (long portions, served mode)
-    const int32_t * faflag;                                   // [T] 1: ... on the form that keeps its scores on chip (flash_attn.cu), where the layer has heads for it
     const int32_t * seg_start, * seg_len, * seg_slot;         // [S]
     int T, S;
 };
@@ -334,7 +333,7 @@ int pib_kv_attention_mm(const pib_kv_query & q, const pib_hlayer & L, const pib_
 // flash_attn.cu: the same for heads of up to 128 coordinates, scores and weights in tensor memory
 bool pib_flash_attention_fits(const pib_hlayer & L);
 struct pib_attn_block {              // consecutive tokens of one segment: batch rows t0 .., positions p0 ..; NK key columns: n_front kept first positions, then j0, j0 + 1, ...
-    int nq, t0, p0, j0, n_front, NK, slot, v_parts;           // v_parts 2: values enter with the remainder of their rounding
+    int nq, t0, p0, j0, n_front, NK, slot;
     int cols, row_blocks, col0, row0;                         // where its operands lie (pib_flash_attention_place)
 };
 void pib_flash_attention_place(std::vector<pib_attn_block> & blocks, int rep, long long * cols, long long * rows);

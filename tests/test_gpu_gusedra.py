@@ -16,7 +16,7 @@ import numpy as np
 import pytest
 
 from tests import gusedra_oracle as O
-from tests.gusedra_configs import CONFIGS, drawn, model, moe, slopes
+from tests.gusedra_configs import CONFIGS, buckets, dense, drawn, model, moe, slopes
 from tests.test_gpu_rapisun import Served, row_err, spread, TOL32, TOL16
 
 pytestmark = pytest.mark.gpu
@@ -417,25 +417,42 @@ def test_long_portions_take_the_matmul_forms(tmp_path, name):
 
 @pytest.mark.parametrize("name", ["wide_heads", "far_keys"])
 def test_portions_of_many_lengths_in_one_batch(tmp_path, name):
-    """served mode: one launch takes the portions of all sequences, around the shortest it takes, where values stop entering in two parts, at the edges of its key tiles and of its
-    row blocks; continued portions (keys of earlier batches in front), beside decoded tokens; and as many portions as fit a launch"""
+    """served mode: one launch takes the portions of all sequences, around the shortest it takes, at the edges of its key tiles and of its row blocks; continued portions (keys of
+    earlier batches in front), beside shorter ones and decoded tokens; and as many portions as fit a launch"""
     cfg = CONFIGS[name]()
     W = O.random_weights(cfg, 29)
-    lens = [47, 48, 49, 63, 64, 65, 127, 128, 129, 1, 200]
+    lens = [47, 64, 127, 128, 129, 1, 191, 192, 193, 200]
     seqs = [tokens(cfg, 2 * n + 2, 40 + i) for i, n in enumerate(lens)]
     refs = [oracle_logits(cfg, W, t) for t in seqs]
-    s = Served(tmp_path, cfg, W, float32=False, n_ctx=2048, slots=16)
+    s = Served(tmp_path, cfg, W, float32=False, n_ctx=2600, slots=16)
     a = s.step([(i, t[:n]) for i, (t, n) in enumerate(zip(seqs, lens))])
     b = s.step([(i, t[n:]) for i, (t, n) in reversed(list(enumerate(zip(seqs, lens))))])
     s.close()
     for i, ref in enumerate(refs):
         assert close16(row_err(np.concatenate([a[i], b[i]]), ref)), lens[i]
-    many = [tokens(cfg, 47 + i % 3, 80 + i) for i in range(32)]
-    s = Served(tmp_path, cfg, W, float32=False, n_ctx=1792, slots=32)
+    many = [tokens(cfg, 128 + i % 3, 80 + i) for i in range(32)]
+    s = Served(tmp_path, cfg, W, float32=False, n_ctx=4224, slots=32)
     got = s.step(list(enumerate(many)))
     s.close()
     for i, t in enumerate(many):
         assert close16(row_err(got[i], oracle_logits(cfg, W, t))), i
+
+
+@pytest.mark.parametrize("n", [48, 100, 127])
+def test_short_portions_keep_fp32_attention(tmp_path, n):
+    """served mode: a portion of up to 127 tokens goes through the kernel that holds queries, keys, weights and values in fp32, whatever its length.  A token's attention does not
+    depend on how its sequence is cut there, so with equally many tokens in every batch (which the other launches' shapes follow) whole and cut portions agree bit for bit"""
+    cfg = model(64, 160, [(slopes(8, 2, 32, 16, 70), None), (buckets(8, 2, 16, 24, 300, 12, n=20, reach=150), dense(96)), (slopes(4, 4, 128, 64), None)])
+    W = O.random_weights(cfg, 61)
+    toks, fill = tokens(cfg, n, 62), tokens(cfg, n, 63)
+    cut = 40
+    s = Served(tmp_path, cfg, W, float32=False, n_ctx=512)
+    whole = s.step([(0, toks)])[0]
+    a = s.step([(1, toks[:cut]), (2, fill[cut:])])
+    b = s.step([(1, toks[cut:]), (3, fill[:cut])])
+    s.close()
+    assert close16(row_err(whole, oracle_logits(cfg, W, toks)))
+    assert np.array_equal(whole, np.concatenate([a[1], b[1]]))
 
 
 @pytest.mark.parametrize("n", [17, 300, 2500])
