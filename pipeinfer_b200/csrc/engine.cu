@@ -844,33 +844,32 @@ static bool prompt_gemm_ok(const pib_context * c, int n_tokens) {
     return pib_prompt_attention_supported(m->head_dim(), (int) c->n_ctx);
 }
 
-static void prompt_bufs_free(pib_context * c) {
-    auto & b = c->pb;
+static void prompt_bufs_free(pib_context::PromptBufs & b) {
     for (void * p : { (void *) b.x, (void *) b.x2, (void *) b.qkv, (void *) b.att, (void *) b.proj, (void *) b.gu, (void *) b.mask, b.xhat, (void *) b.ids }) if (p) cudaFree(p);
     b = pib_context::PromptBufs();
 }
-// buffers for passes of a prompt of n_tokens: all of it up to PIB_PROMPT_MAX (one stage; passes of 256 where stages overlap, or where memory holds no more)
+// buffers for passes of a prompt of n_tokens: all of it up to PIB_PROMPT_MAX (one stage; passes of 256 where stages overlap, shorter ones than the prompt where memory holds no more)
 static int prompt_bufs(pib_context * c, int n_tokens) {
-    const int want = c->stage.size > 1 ? PIB_PROMPT_STAGE : std::min(PIB_PROMPT_MAX, (n_tokens + 255) / 256 * 256);
-    if (c->pb.cap >= want) return PIB_OK;
     const pib_model * m = c->model;
     const size_t E = m->n_embd, GQA = m->n_embd_gqa(), FF = m->n_ff, KM = std::max(E, FF);
-    auto & b = c->pb;
-    if (b.cap) cudaStreamSynchronize(c->stream);
-    for (size_t P = (size_t) want; P >= 256; P = P > 256 ? 256 : 0) {
-        prompt_bufs_free(c);
-        if (cudaMalloc(&b.x, P * E * 4) == cudaSuccess && cudaMalloc(&b.x2, P * E * 4) == cudaSuccess && cudaMalloc(&b.qkv, P * (E + 2 * GQA) * 4) == cudaSuccess &&
-            cudaMalloc(&b.att, P * E * 4) == cudaSuccess && cudaMalloc(&b.proj, P * E * 4) == cudaSuccess && cudaMalloc(&b.gu, P * 2 * FF * 4) == cudaSuccess &&
-            cudaMalloc(&b.mask, P * c->n_ctx) == cudaSuccess && cudaMalloc(&b.ids, PIB_PROMPT_MAX * (3 + (size_t) c->n_words) * 4) == cudaSuccess &&
-            cudaMalloc(&b.xhat, pib_gemm_xhat_bytes((int64_t) KM, (int) P)) == cudaSuccess) {
-            b.cap = (int) P;
-            return PIB_OK;
+    const bool ok = c->prompt_plan.grow(n_tokens, (int) c->n_ctx, c->stage.size, [&](int n) {
+        const size_t P = (size_t) n;
+        pib_context::PromptBufs b;
+        if (cudaMalloc(&b.x, P * E * 4) != cudaSuccess || cudaMalloc(&b.x2, P * E * 4) != cudaSuccess || cudaMalloc(&b.qkv, P * (E + 2 * GQA) * 4) != cudaSuccess ||
+            cudaMalloc(&b.att, P * E * 4) != cudaSuccess || cudaMalloc(&b.proj, P * E * 4) != cudaSuccess || cudaMalloc(&b.gu, P * 2 * FF * 4) != cudaSuccess ||
+            cudaMalloc(&b.mask, P * c->n_ctx) != cudaSuccess || cudaMalloc(&b.ids, PIB_PROMPT_MAX * (3 + (size_t) c->n_words) * 4) != cudaSuccess ||
+            cudaMalloc(&b.xhat, pib_gemm_xhat_bytes((int64_t) KM, n)) != cudaSuccess) {
+            cudaGetLastError();
+            prompt_bufs_free(b);
+            return false;
         }
-        cudaGetLastError();
-    }
-    prompt_bufs_free(c);
-    pib_set_error("decode: out of memory for the prompt path's work buffers");
-    return PIB_ERR_NOMEM;
+        if (c->prompt_plan.cap) cudaStreamSynchronize(c->stream);        // a pass on the old ones may be under way
+        std::swap(b, c->pb);
+        prompt_bufs_free(b);
+        return true;
+    });
+    if (!ok) { pib_set_error("decode: out of memory for the prompt path's work buffers"); return PIB_ERR_NOMEM; }
+    return PIB_OK;
 }
 
 // one pass of `ntok` tokens = chunks [ch0, ch0 + nch) of the run
@@ -1106,7 +1105,7 @@ static int enqueue_decode(pib_context * c, pib_run * run, int n_tokens, int batc
     run->in_use = true; run->batch_id = batch_id; run->n_tokens = n_tokens; run->failed = false; run->tc_used = false;
     cudaMemcpyAsync(c->cancel_table, c->run_id_host + run->id, sizeof(int), cudaMemcpyHostToDevice, c->stream);   // "this run executes now"
     if (prompt_gemm_ok(c, n_tokens) && prompt_bufs(c, n_tokens) == PIB_OK) {
-        const int pass = c->stage.size > 1 ? PIB_PROMPT_STAGE : c->pb.cap, per = pass / PIB_CHUNK;
+        const int pass = c->stage.size > 1 ? PIB_PROMPT_STAGE : c->prompt_plan.cap, per = pass / PIB_CHUNK;
         for (int ch0 = 0; ch0 < n_chunks && !run->failed; ch0 += per) {
             const int nch = std::min(per, n_chunks - ch0), ntok = std::min(pass, n_tokens - ch0 * PIB_CHUNK);
             if (run_prompt_pass(c, *run, ch0, nch, ntok, slots) != PIB_OK) run->failed = true;

@@ -5,6 +5,7 @@
 #include "pib_common.cuh"
 #include "desc.cuh"
 #include "kv_meta.cuh"
+#include "prompt_plan.cuh"
 
 #include <deque>
 #include <map>
@@ -12,8 +13,6 @@
 #include <vector>
 
 #define PIB_TOPK 8
-#define PIB_PROMPT_MAX 1024          // tokens per pass of the tensor-core prompt path (gemm_q4k_tc.cu)
-#define PIB_PROMPT_STAGE 256         // ... where several stages work on one prompt: passes of the stages overlap
 struct pib_prompt_slots { int32_t slot[PIB_PROMPT_MAX / PIB_CHUNK]; };      // device descriptor slots of a prompt pass's chunks (prompt_attn.cu)
 struct pib_row_result {            // per logits row: sorted top-8 {id, logit, p}; entry 0 is the greedy token
     int32_t id[PIB_TOPK];
@@ -132,11 +131,12 @@ struct pib_context {
     cudaEvent_t cancel_ev = nullptr;       // recorded on `ctrl` after every cancel write: the clearing memset on `stream` waits for it
     bool     cancel_ev_pending = false;
 
-    // wide-batch (prompt) path: work buffers for passes of up to `cap` tokens, allocated on the first prompt that needs them
+    // wide-batch (prompt) path: work buffers for passes of up to prompt_plan.cap tokens, allocated on the first prompt that needs them
     struct PromptBufs { float * x = nullptr, * x2 = nullptr, * qkv = nullptr, * att = nullptr, * proj = nullptr, * gu = nullptr;
                         uint8_t * mask = nullptr; void * xhat = nullptr;      // xhat: the matmuls' fp16 operand rows
                         int32_t * ids = nullptr;      // a pass's token ids | positions | cells [3][PIB_PROMPT_MAX], then sequence bitsets [PIB_PROMPT_MAX][n_words]
-                        int cap = 0; } pb;
+                      } pb;
+    pib_prompt_plan prompt_plan;
     int      fuse_pro = 0;                 // 1: small llama-arch Q4_K models run norm / quantise / silu inside the consuming GEMV (PIB_FUSE_PRO, engine.cu)
     int      prompt_gemm = 1;              // 0: prompts go through the GEMV kernels in chunks of 16 (PIB_PROMPT_GEMM=0, and always in exact mode)
 
