@@ -272,21 +272,26 @@ def test_cancel_mid_flight_on_k_split_shapes_leaves_the_next_decode_intact(llama
 
 
 def test_prompt_through_the_tensor_core_gemm_matches_the_chunked_path(llama):
-    """Prompts (> 32 tokens) run their matmuls on the tcgen05 GEMM, 256 tokens per pass; verification batches keep the
-    GEMV.  Same model, same 300-token prompt, both ways: logits within 2e-2 of each other (fp16 operands against int8 x int4 integer
+    """Prompts (> 32 tokens) run their matmuls on the tcgen05 GEMM, up to 1024 tokens per pass; verification batches keep the
+    GEMV.  Same model, same prompts, both ways: logits within 2e-2 of each other (fp16 operands against int8 x int4 integer
     arithmetic, on a model whose top logits are ~10), same argmax on every row that is not a near tie; and the KV cache the GEMM pass
-    leaves behind serves a following single-token decode equally well."""
+    leaves behind serves a following single-token decode equally well.  In one context: prompts on the shorter buffers, on the longer ones, with two, three and four
+    token tiles in a pass (the last one of a single token at 769), with a second pass (1100 tokens), and behind the end of the descriptor ring, whose 256 slots the
+    prompts before have used up."""
     shape = (4, 2048, 16, 2, 5632 // 256 * 256, 4096, 12, 1, 1, 1.0)
-    toks = [3 + (i * 7919) % 4093 for i in range(301)]
+    toks = [3 + (i * 7919) % 4093 for i in range(1101)]
     out = {}
     for mode in ("1", "0"):
         os.environ["PIB_PROMPT_GEMM"] = mode
-        ctx = llama.Context(None, n_ctx=512, max_seq=4, synthetic=shape)
-        rc, lg = ctx.decode(toks[:300], list(range(300)), [[0]] * 300)
-        assert rc == 0
-        rc, nxt = ctx.decode(toks[300:], [300], [[0]])
-        assert rc == 0
-        out[mode] = (lg, nxt)
+        ctx = llama.Context(None, n_ctx=1280, max_seq=4, synthetic=shape)
+        out[mode] = []
+        for n in (40, 256, 300, 257, 513, 769, 1024, 1100, 256):
+            rc, lg = ctx.decode(toks[:n], list(range(n)), [[0]] * n)
+            assert rc == 0
+            rc, nxt = ctx.decode([toks[n]], [n], [[0]])
+            assert rc == 0
+            out[mode] += [lg, nxt]
+            ctx.seq_rm(0, -1, -1)
         ctx.close()
     os.environ.pop("PIB_PROMPT_GEMM")
     for a, b in zip(out["1"], out["0"]):
