@@ -313,13 +313,12 @@ static int launch_att_qh(const float * qkv, const float * vsep, const uint8_t * 
                          const int * cancel, cudaStream_t st) {
     const int    vcap = std::min(n_ctx, ATQ_THREADS == 512 && att_smem(HD, n_ctx, ATQ_VCAP) <= ATQ_SMEM_MAX ? ATQ_VCAP : ATQ_VCAP_MIN);
     const size_t smem = att_smem(HD, n_ctx, vcap);   // scores + 32 x HD partial sums + staged V rows
-    static size_t configured = 0;
-    if (smem > configured) {
-        // several CTAs per SM (a verification batch of 3+ tokens is more CTAs than SMs): ask for the large shared-memory carve-out
-        PIB_CHECK(cudaFuncSetAttribute(attention_qh_kernel<HD, ATQ_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) std::max(smem, (size_t) 32 * 1024)));
-        PIB_CHECK(cudaFuncSetAttribute(attention_qh_kernel<HD, ATQ_THREADS>, cudaFuncAttributePreferredSharedMemoryCarveout, (int) cudaSharedmemCarveoutMaxShared));
-        configured = smem;
-    }
+    static pib_per_device attrs;
+    // several CTAs per SM (a verification batch of 3+ tokens is more CTAs than SMs): ask for the large shared-memory carve-out
+    PIB_CHECK(attrs.once(smem, [&] {
+        const cudaError_t e = cudaFuncSetAttribute(attention_qh_kernel<HD, ATQ_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) std::max(smem, (size_t) 32 * 1024));
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(attention_qh_kernel<HD, ATQ_THREADS>, cudaFuncAttributePreferredSharedMemoryCarveout, (int) cudaSharedmemCarveoutMaxShared);
+    }));
     pib_launch(attention_qh_kernel<HD, ATQ_THREADS>, dim3(n_head, n_tokens), dim3(ATQ_THREADS), smem, st, qkv, vsep, desc, rope, rope_n_pos, mode, kc, vc, mask, scalars,
                pib_get_luts().exp_f16, E, GQA, n_ctx, 1.0f / sqrtf((float) HD), out, cancel, gdiv, vcap);
     PIB_CHECK(cudaGetLastError());

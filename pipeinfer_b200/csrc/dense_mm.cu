@@ -468,15 +468,18 @@ __global__ void __launch_bounds__(128) mm_few_cols_kernel(mm_dev a) {
         }
 }
 
-template <typename K> static void mvm_smem(K kernel, size_t smem) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
-    cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int) cudaSharedmemCarveoutMaxShared);
+template <typename K> static cudaError_t mvm_smem(pib_per_device & attrs, K kernel, size_t smem) {
+    return attrs.once([&] {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int) cudaSharedmemCarveoutMaxShared);
+    });
 }
 #define MVM_SMEM(DEPTH) ((size_t) 8 * (DEPTH) * MVM_GROUP)          // none: the group sits in registers
-template <int EPI, int NT, int DEPTH> static void mvm_launch(dim3 grid, cudaStream_t st, const mm_dev & d) {
-    static bool configured = false;
-    if (DEPTH && !configured) { mvm_smem(mv_mma_kernel<EPI, NT, DEPTH>, MVM_SMEM(DEPTH)); configured = true; }
+template <int EPI, int NT, int DEPTH> static int mvm_launch(dim3 grid, cudaStream_t st, const mm_dev & d) {
+    static pib_per_device attrs;
+    if (DEPTH) PIB_CHECK(mvm_smem(attrs, mv_mma_kernel<EPI, NT, DEPTH>, MVM_SMEM(DEPTH)));
     pib_launch(mv_mma_kernel<EPI, NT, DEPTH>, grid, dim3(256), MVM_SMEM(DEPTH), st, d);
+    return PIB_OK;
 }
 
 template <typename WT, bool ROUND, int EPI>
@@ -496,10 +499,12 @@ static int launch_mm(const pib_mm & a, const mm_dev & d, cudaStream_t st) {
             // registers' number, is enough and one of two is not (5120 x 2048 at 16 9.0 / 9.9)
             const long long ctas = (long long) grid.x * grid.z, sms = pib_num_sms();
             const int need = ((a.K + 31) / 32 + 8 * MVM_U - 1) / (8 * MVM_U), depth = std::min(need, ctas <= sms ? 5 : ctas <= 2 * sms ? 3 : 2);
-#define MVM_GO(DEPTH) do { if (a.M <= 8) mvm_launch<EPI, 1, DEPTH>(grid, st, d); else mvm_launch<EPI, 2, DEPTH>(grid, st, d); } while (0)
+#define MVM_GO(DEPTH) rc = a.M <= 8 ? mvm_launch<EPI, 1, DEPTH>(grid, st, d) : mvm_launch<EPI, 2, DEPTH>(grid, st, d)
+            int rc;
             if (ctas > 2 * sms && (need == 1 || (a.M > 8 && ctas <= 3 * sms))) MVM_GO(0);
             else if (depth <= 1) MVM_GO(1); else if (depth == 2) MVM_GO(2); else if (depth == 3) MVM_GO(3); else MVM_GO(5);
 #undef MVM_GO
+            if (rc != PIB_OK) return rc;
         } else
         if (a.M == 1)      pib_launch(mv_rows_kernel<WT, ROUND, EPI, 1>, dim3(grid), dim3(256), (size_t) (0), st, d, xvec);
         else if (a.M == 2) pib_launch(mv_rows_kernel<WT, ROUND, EPI, 2>, dim3(grid), dim3(256), (size_t) (0), st, d, xvec);
@@ -551,13 +556,13 @@ int pib_dense_mm(const pib_mm & a, cudaStream_t st) {
 
 // a (no epilogue) and b (none or PIB_EPI_GEGLU_PAIR) do not depend on each other; up to MV_MAXB rows they share a launch, else they follow one another
 template <typename WT, bool ROUND, int EPI_B>
-static void launch_pair(const mm_dev & a, const mm_dev & b, bool xva, bool xvb, cudaStream_t st) {
+static int launch_pair(const mm_dev & a, const mm_dev & b, bool xva, bool xvb, cudaStream_t st) {
     const int ba = (a.N + 7) / 8, bb = ((pib_epi_pairs(EPI_B) ? b.N / 2 : b.N) + 7) / 8;
     const dim3 grid((unsigned) (ba + bb));
     if (mvm_fits<WT, ROUND>(a, xva) && mvm_fits<WT, ROUND>(b, xvb)) {
         const int ta = (a.N + 15) / 16, tb = (b.N + 15) / 16;
-        static bool configured = false;
-        if (!configured) { mvm_smem(mv_mma_pair_kernel<EPI_B, 1>, MVM_SMEM(2)); mvm_smem(mv_mma_pair_kernel<EPI_B, 2>, MVM_SMEM(2)); configured = true; }
+        static pib_per_device one, two;
+        PIB_CHECK(a.M <= 8 ? mvm_smem(one, mv_mma_pair_kernel<EPI_B, 1>, MVM_SMEM(2)) : mvm_smem(two, mv_mma_pair_kernel<EPI_B, 2>, MVM_SMEM(2)));
         if (a.M <= 8) pib_launch(mv_mma_pair_kernel<EPI_B, 1>, dim3((unsigned) (ta + tb)), dim3(256), MVM_SMEM(2), st, a, b, ta);
         else          pib_launch(mv_mma_pair_kernel<EPI_B, 2>, dim3((unsigned) (ta + tb)), dim3(256), MVM_SMEM(2), st, a, b, ta);
     } else
@@ -566,6 +571,8 @@ static void launch_pair(const mm_dev & a, const mm_dev & b, bool xva, bool xvb, 
     else if (a.M <= 4) pib_launch(mv_pair_kernel<WT, ROUND, EPI_B, 4>, grid, dim3(256), (size_t) 0, st, a, b, xva, xvb, ba);
     else if (a.M <= 8) pib_launch(mv_pair_kernel<WT, ROUND, EPI_B, 8>, grid, dim3(256), (size_t) 0, st, a, b, xva, xvb, ba);
     else               pib_launch(mv_pair_kernel<WT, ROUND, EPI_B, MV_MAXB>, grid, dim3(256), (size_t) 0, st, a, b, xva, xvb, ba);
+    PIB_CHECK(cudaGetLastError());
+    return PIB_OK;
 }
 int pib_dense_mm_pair(const pib_mm & a, const pib_mm & b, cudaStream_t st) {
     const int V = a.wtype == PIB_TYPE_BF16 ? 8 : 4;
@@ -577,24 +584,21 @@ int pib_dense_mm_pair(const pib_mm & a, const pib_mm & b, cudaStream_t st) {
     }
     auto dev = [](const pib_mm & m) { return mm_dev{ m.W, m.ldw, m.wz, m.X, m.ldx, m.xz, nullptr, 1, m.Y, m.ldy, m.yz, m.M, m.N, m.K, nullptr, m.e0, m.e1, nullptr, nullptr, 0, 0x7fffffff, nullptr, m.w_made }; };
     auto xvec = [](const pib_mm & m) { return m.ldx % 4 == 0 && ((uintptr_t) m.X & 15) == 0; };
-#define PAIR_GO(WT, ROUND) do { if (b.epi == PIB_EPI_NONE) launch_pair<WT, ROUND, PIB_EPI_NONE>(dev(a), dev(b), xvec(a), xvec(b), st); \
-                                else launch_pair<WT, ROUND, PIB_EPI_GEGLU_PAIR>(dev(a), dev(b), xvec(a), xvec(b), st); } while (0)
-    if (a.wtype == PIB_TYPE_BF16) PAIR_GO(__nv_bfloat16, true);
-    else if (a.exact) PAIR_GO(float, false);
-    else PAIR_GO(float, true);
+#define PAIR_GO(WT, ROUND) (b.epi == PIB_EPI_NONE ? launch_pair<WT, ROUND, PIB_EPI_NONE>(dev(a), dev(b), xvec(a), xvec(b), st) \
+                                                  : launch_pair<WT, ROUND, PIB_EPI_GEGLU_PAIR>(dev(a), dev(b), xvec(a), xvec(b), st))
+    if (a.wtype == PIB_TYPE_BF16) return PAIR_GO(__nv_bfloat16, true);
+    return a.exact ? PAIR_GO(float, false) : PAIR_GO(float, true);
 #undef PAIR_GO
-    PIB_CHECK(cudaGetLastError());
-    return PIB_OK;
 }
 
 template <typename WT, bool ROUND, int EPI>
-static void launch_experts(const mm_dev & a, const mm_dev & b, bool xva, bool xvb, int za, cudaStream_t st) {
+static int launch_experts(const mm_dev & a, const mm_dev & b, bool xva, bool xvb, int za, cudaStream_t st) {
     const int ba = ((pib_epi_pairs(EPI) ? a.N / 2 : a.N) + 7) / 8, bb = ((pib_epi_pairs(EPI) ? b.N / 2 : b.N) + 7) / 8, rows = a.M > b.M ? a.M : b.M;
     const dim3 grid((unsigned) (ba * za + bb));
     if (mvm_fits<WT, ROUND>(a, xva && a.xz % 4 == 0) && mvm_fits<WT, ROUND>(b, xvb)) {
         const int ta = (a.N + 15) / 16, tb = (b.N + 15) / 16;
-        static bool configured = false;
-        if (!configured) { mvm_smem(mv_mma_experts_kernel<EPI, 1>, MVM_SMEM(2)); mvm_smem(mv_mma_experts_kernel<EPI, 2>, MVM_SMEM(2)); configured = true; }
+        static pib_per_device one, two;
+        PIB_CHECK(rows <= 8 ? mvm_smem(one, mv_mma_experts_kernel<EPI, 1>, MVM_SMEM(2)) : mvm_smem(two, mv_mma_experts_kernel<EPI, 2>, MVM_SMEM(2)));
         if (rows <= 8) pib_launch(mv_mma_experts_kernel<EPI, 1>, dim3((unsigned) (ta * za + tb)), dim3(256), MVM_SMEM(2), st, a, b, ta, za);
         else           pib_launch(mv_mma_experts_kernel<EPI, 2>, dim3((unsigned) (ta * za + tb)), dim3(256), MVM_SMEM(2), st, a, b, ta, za);
     } else
@@ -603,6 +607,8 @@ static void launch_experts(const mm_dev & a, const mm_dev & b, bool xva, bool xv
     else if (rows <= 4) pib_launch(mv_experts_kernel<WT, ROUND, EPI, 4>, grid, dim3(256), (size_t) 0, st, a, b, xva, xvb, ba, za);
     else if (rows <= 8) pib_launch(mv_experts_kernel<WT, ROUND, EPI, 8>, grid, dim3(256), (size_t) 0, st, a, b, xva, xvb, ba, za);
     else                pib_launch(mv_experts_kernel<WT, ROUND, EPI, MV_MAXB>, grid, dim3(256), (size_t) 0, st, a, b, xva, xvb, ba, za);
+    PIB_CHECK(cudaGetLastError());
+    return PIB_OK;
 }
 int pib_dense_mm_experts(const pib_mm & a, const pib_mm & b, cudaStream_t st) {
     const int V = a.wtype == PIB_TYPE_BF16 ? 8 : 4;
@@ -617,14 +623,11 @@ int pib_dense_mm_experts(const pib_mm & a, const pib_mm & b, cudaStream_t st) {
     };
     auto xvec = [](const pib_mm & m) { return m.ldx % 4 == 0 && ((uintptr_t) m.X & 15) == 0; };
     const int za = a.zlist && a.M < a.Z ? a.M : a.Z;
-#define EXPERTS_GO(WT, ROUND) do { if (a.epi == PIB_EPI_NONE) launch_experts<WT, ROUND, PIB_EPI_NONE>(dev(a), dev(b), xvec(a), xvec(b), za, st); \
-                                   else launch_experts<WT, ROUND, PIB_EPI_SWIGLU_PAIR>(dev(a), dev(b), xvec(a), xvec(b), za, st); } while (0)
-    if (a.wtype == PIB_TYPE_BF16) EXPERTS_GO(__nv_bfloat16, true);
-    else if (a.exact) EXPERTS_GO(float, false);
-    else EXPERTS_GO(float, true);
+#define EXPERTS_GO(WT, ROUND) (a.epi == PIB_EPI_NONE ? launch_experts<WT, ROUND, PIB_EPI_NONE>(dev(a), dev(b), xvec(a), xvec(b), za, st) \
+                                                     : launch_experts<WT, ROUND, PIB_EPI_SWIGLU_PAIR>(dev(a), dev(b), xvec(a), xvec(b), za, st))
+    if (a.wtype == PIB_TYPE_BF16) return EXPERTS_GO(__nv_bfloat16, true);
+    return a.exact ? EXPERTS_GO(float, false) : EXPERTS_GO(float, true);
 #undef EXPERTS_GO
-    PIB_CHECK(cudaGetLastError());
-    return PIB_OK;
 }
 
 pib_weight * pib_dense_upload(int type, const void * host, int64_t N, int64_t K) {

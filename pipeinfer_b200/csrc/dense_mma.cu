@@ -215,16 +215,14 @@ int * pib_tc_error_word(cudaStream_t st) { dt_scratch * sc = dt_scratch_of(st, 0
 template <int NB>
 static int dt_launch(const pib_mm & a, const CUtensorMap & wmap, const CUtensorMap & xmap, int x_has_z, int * err, cudaStream_t st) {
     using C = dt_cfg<NB>;
-    static bool configured = false;
-    if (!configured) {
-        PIB_CHECK(cudaFuncSetAttribute(dense_tc_kernel<NB, PIB_EPI_NONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) C::SMEM));
-        PIB_CHECK(cudaFuncSetAttribute(dense_tc_kernel<NB, PIB_EPI_RELU2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) C::SMEM));
-        PIB_CHECK(cudaFuncSetAttribute(dense_tc_kernel<NB, PIB_EPI_XIELU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) C::SMEM));
-        PIB_CHECK(cudaFuncSetAttribute(dense_tc_kernel<NB, PIB_EPI_GLU_PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) C::SMEM));
-        PIB_CHECK(cudaFuncSetAttribute(dense_tc_kernel<NB, PIB_EPI_GEGLU_PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) C::SMEM));
-        PIB_CHECK(cudaFuncSetAttribute(dense_tc_kernel<NB, PIB_EPI_SWIGLU_PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) C::SMEM));
-        configured = true;
-    }
+    static pib_per_device attrs;
+    PIB_CHECK(attrs.once([&] {
+        cudaError_t e = cudaSuccess;
+        for (auto kernel : { dense_tc_kernel<NB, PIB_EPI_NONE>, dense_tc_kernel<NB, PIB_EPI_RELU2>, dense_tc_kernel<NB, PIB_EPI_XIELU>, dense_tc_kernel<NB, PIB_EPI_GLU_PAIR>,
+                             dense_tc_kernel<NB, PIB_EPI_GEGLU_PAIR>, dense_tc_kernel<NB, PIB_EPI_SWIGLU_PAIR> })
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) C::SMEM);
+        return e;
+    }));
     dim3 grid((unsigned) ((a.N + DT_BM - 1) / DT_BM), (unsigned) ((a.M + NB - 1) / NB), (unsigned) a.Z);
 #define DT_GO(EPI) pib_launch(dense_tc_kernel<NB, EPI>, dim3(grid), dim3(DT_THREADS), (size_t) (C::SMEM), st, wmap, xmap, a.M, a.N, a.K, a.zrange, x_has_z, a.Y, a.ldy, a.yz, err, a.e0, a.e1, \
                               a.Y2, a.ld2, a.Y2 ? a.n2 : 0x7fffffff, a.rows2)

@@ -274,8 +274,8 @@ int pib_dense_pair(const pib_mm & a, const CUtensorMap & wmap, const CUtensorMap
     const dp_args A = { a.M, a.N, a.K, NB, tiles_m, tiles, shares, a.w_made, a.Y, a.ldy, a.y_bf16, a.e0, a.e1, a.Y2, a.ld2, a.Y2 ? a.n2 : 0x7fffffff, a.rows2, err };
     const dim3 grid((unsigned) (2 * shares * (shares > 1 || tiles < pairs ? tiles : pairs)));
 #define DP_GO(EPI) do {                                                                                                                            \
-        static bool configured = false;                                                                                                            \
-        if (!configured) { PIB_CHECK(cudaFuncSetAttribute(dense_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) DP_SMEM)); configured = true; } \
+        static pib_per_device attrs;                                                                                                                \
+        PIB_CHECK(attrs.once([&] { return cudaFuncSetAttribute(dense_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) DP_SMEM); })); \
         pib_launch_cluster(dense_pair_kernel<EPI>, grid, dim3(DP_THREADS), dim3((unsigned) (2 * shares), 1, 1), DP_SMEM, st, wmap, xmap, A);         \
     } while (0)
     switch (a.epi) {

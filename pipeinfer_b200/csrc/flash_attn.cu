@@ -539,8 +539,8 @@ int pib_flash_attention(const pib_kv_query & q, const pib_hlayer & L, const std:
     for (const pib_attn_block & b : blocks) row_blocks += b.row_blocks;
     const size_t extra = (size_t) rel_smem * rep * 4;
 #define FA_GO(NC) do {                                                                                                                             \
-        static bool configured = false;                                                                                                            \
-        if (!configured) { PIB_CHECK(cudaFuncSetAttribute(flash_attn_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (fa_cfg<NC>::SMEM + FA_REL_MAX))); configured = true; } \
+        static pib_per_device attrs;                                                                                                                \
+        PIB_CHECK(attrs.once([&] { return cudaFuncSetAttribute(flash_attn_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (fa_cfg<NC>::SMEM + FA_REL_MAX)); })); \
         pib_launch(flash_attn_kernel<NC>, dim3((unsigned) (row_blocks * Z)), dim3(FA_THREADS), fa_cfg<NC>::SMEM + extra, st, qh, ql, kh, kl, vm, A); \
     } while (0)
     if (D <= 64) FA_GO(1); else FA_GO(2);

@@ -420,8 +420,8 @@ static int tg_launch(const pib_weight * w, const __half * xh, int b, int x0, int
     const CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void *) xh, gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { pib_set_error("pib_gemm: cuTensorMapEncodeTiled failed (%d)", (int) r); return PIB_ERR_CUDA; }
-    static bool configured = false;
-    if (!configured) { PIB_CHECK(cudaFuncSetAttribute(gemm_q4k_tc_kernel<NB, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) C::SMEM)); configured = true; }
+    static pib_per_device attrs;
+    PIB_CHECK(attrs.once([&] { return cudaFuncSetAttribute(gemm_q4k_tc_kernel<NB, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) C::SMEM); }));
     const dim3 grid((unsigned) nx, 1, (unsigned) S);
     int * err = pib_tc_error_word(st);
     if (!err) { pib_set_error("pib_gemm: no memory for the stream's error word"); return PIB_ERR_NOMEM; }

@@ -396,8 +396,8 @@ template <int WT, int NT, int WARPS, int STAGES>
 static int bk_ring_launch(const pib_weight * w, int ngr, const int8_t * aqs, const __half * adx, int b, float * y_dev, const int * cancel, cudaStream_t st) {
     const int    n_tiles = (int) ((w->N + 15) / 16);
     const size_t ring = (size_t) WARPS * STAGES * bk_rec_bytes(WT), smem = WARPS == 8 ? pib_gemv_smem_spread(ring, n_tiles) : ring;
-    static bool configured = false;
-    if (!configured) { PIB_CHECK(cudaFuncSetAttribute(gemv_blk32_ring_kernel<WT, NT, WARPS, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (ring > PIB_GEMV_SPREAD ? ring : PIB_GEMV_SPREAD))); configured = true; }
+    static pib_per_device attrs;
+    PIB_CHECK(attrs.once([&] { return cudaFuncSetAttribute(gemv_blk32_ring_kernel<WT, NT, WARPS, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (ring > PIB_GEMV_SPREAD ? ring : PIB_GEMV_SPREAD)); }));
     PIB_CHECK(pib_launch(gemv_blk32_ring_kernel<WT, NT, WARPS, STAGES>, dim3((unsigned) n_tiles), dim3(WARPS * 32), smem, st, w->tiles, ngr, (int) w->N, aqs, adx, b, y_dev, cancel));
     return PIB_OK;
 }

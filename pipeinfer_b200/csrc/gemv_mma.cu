@@ -1046,12 +1046,11 @@ int pib_gemv_mma_launch(const pib_weight * w, const void * act_dev, int b, float
     const int8_t *       aqs = (const int8_t *) (act + L.qsp_off);      // fragment-order quants
     const float *        ad  = (const float *) (act + L.dxo_off);
     const int8_t *       bs  = (const int8_t *) (act + L.bs8_off);
-    static bool configured = false;
-    if (!configured) {
-        PIB_CHECK(cudaFuncSetAttribute(gemv_q4k_mma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) mm_smem_bytes()));
-        PIB_CHECK(cudaFuncSetAttribute(gemv_q4k_mma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) mm_smem_bytes()));
-        configured = true;
-    }
+    static pib_per_device attrs;
+    PIB_CHECK(attrs.once([&] {
+        const cudaError_t e = cudaFuncSetAttribute(gemv_q4k_mma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) mm_smem_bytes());
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(gemv_q4k_mma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) mm_smem_bytes());
+    }));
     const int items = n_tiles << split;                                            // `split` is log2 of the split count here
     const int ctas  = (items + MM_WARPS - 1) / MM_WARPS;
     const int grid  = ctas < 4 * pib_num_sms() ? ctas : 4 * pib_num_sms();         // persistent: 4 CTAs per SM
@@ -1066,8 +1065,8 @@ static int ring_launch(const pib_weight * w, const int8_t * aqs, const float * a
                        unsigned int * counters, const int * cancel, cudaStream_t st) {
     const int    nsb = (int) (w->K / 256), n_tiles = (int) ((w->N + 15) / 16);
     const size_t ring = (size_t) WARPS * STAGES * MM_TILE_BYTES, smem = WARPS == 8 ? pib_gemv_smem_spread(ring, n_tiles * split) : ring;
-    static bool configured = false;
-    if (!configured) { PIB_CHECK(cudaFuncSetAttribute(gemv_q4k_ring_kernel<NT, WARPS, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) std::max(ring, (size_t) PIB_GEMV_SPREAD))); configured = true; }
+    static pib_per_device attrs;
+    PIB_CHECK(attrs.once([&] { return cudaFuncSetAttribute(gemv_q4k_ring_kernel<NT, WARPS, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) std::max(ring, (size_t) PIB_GEMV_SPREAD)); }));
     pib_launch(gemv_q4k_ring_kernel<NT, WARPS, STAGES>, dim3(n_tiles, split), dim3(WARPS * 32), smem, st, w->tiles, nsb, (int) w->N, (int) w->K, aqs, ad, bs, b, y_dev,
                partial, counters, cancel);
     PIB_CHECK(cudaGetLastError());
@@ -1110,8 +1109,8 @@ template <int NT>
 static int stream_launch(const pib_weight * w, const int8_t * aqs, const float * ad, const int8_t * bs, int b, float * y_dev, int W, int pmax,
                          float * partial, unsigned int * counters, const int * cancel, cudaStream_t st) {
     const size_t smem = (size_t) SK_WARPS * RG_STAGES * MM_TILE_BYTES;
-    static bool configured = false;
-    if (!configured) { PIB_CHECK(cudaFuncSetAttribute(gemv_q4k_stream_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)); configured = true; }
+    static pib_per_device attrs;
+    PIB_CHECK(attrs.once([&] { return cudaFuncSetAttribute(gemv_q4k_stream_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem); }));
     const int nsb = (int) (w->K / 256), n_tiles = (int) ((w->N + 15) / 16);
     pib_launch(gemv_q4k_stream_kernel<NT>, dim3((W + SK_WARPS - 1) / SK_WARPS), dim3(SK_WARPS * 32), smem, st, w->tiles, nsb, n_tiles, (int) w->N, (int) w->K, aqs,
                ad, bs, b, y_dev, partial, counters, pmax, W, cancel);
@@ -1158,12 +1157,11 @@ static int pro_launch(const pib_weight * w, int b, float * y, const float * x, c
                       float eps, const uint16_t * lut, const int * cancel, cudaStream_t st) {
     const int    nsb = (int) (w->K / 256), n_tiles = (int) ((w->N + 15) / 16);
     const size_t smem = (size_t) GP_WARPS * RG_STAGES * MM_TILE_BYTES + (size_t) b * (w->K + nsb * 20);
-    static size_t configured = 0;
-    if (smem > configured) {
-        PIB_CHECK(cudaFuncSetAttribute(gemv_q4k_pro_kernel<PRO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (100 * 1024)));
-        PIB_CHECK(cudaFuncSetAttribute(gemv_q4k_pro_kernel<PRO>, cudaFuncAttributePreferredSharedMemoryCarveout, (int) cudaSharedmemCarveoutMaxShared));
-        configured = 100 * 1024;
-    }
+    static pib_per_device attrs;
+    PIB_CHECK(attrs.once([&] {
+        const cudaError_t e = cudaFuncSetAttribute(gemv_q4k_pro_kernel<PRO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (100 * 1024));
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(gemv_q4k_pro_kernel<PRO>, cudaFuncAttributePreferredSharedMemoryCarveout, (int) cudaSharedmemCarveoutMaxShared);
+    }));
     pib_launch(gemv_q4k_pro_kernel<PRO>, dim3(n_tiles), dim3(GP_WARPS * 32), smem, st, w->tiles, nsb, (int) w->N, (int) w->K, b, y, x, x2, addend, sum_out,
                xstride, eps, lut, cancel);
     PIB_CHECK(cudaGetLastError());

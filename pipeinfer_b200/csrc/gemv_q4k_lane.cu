@@ -583,13 +583,9 @@ static int lx_get_scratch(cudaStream_t st, lx_scratch ** out) {
 template <int BMAX, int TB>
 static int lx_launch(const pib_weight * w, const void * act_dev, int b, float * y_dev, const int * cancel, cudaStream_t st, lx_scratch * s) {
     const size_t smem = lx_smem_bytes(b);
-    static bool configured = false;
+    static pib_per_device attrs;
     static int  per_sm_of[PIB_MAX_BATCH + 1];                            // CTAs per SM for each batch size (shared memory grows with b)
-    if (!configured) {
-        PIB_CHECK(cudaFuncSetAttribute(gemv_q4k_lane_kernel<BMAX, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) lx_smem_bytes(PIB_MAX_BATCH)));
-        for (int i = 0; i <= PIB_MAX_BATCH; i++) per_sm_of[i] = 0;
-        configured = true;
-    }
+    PIB_CHECK(attrs.once([&] { return cudaFuncSetAttribute(gemv_q4k_lane_kernel<BMAX, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) lx_smem_bytes(PIB_MAX_BATCH)); }));
     if (!per_sm_of[b]) PIB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_of[b], gemv_q4k_lane_kernel<BMAX, TB>, LX_THREADS, smem));
     int per_sm = per_sm_of[b];
     if (per_sm < 1) { pib_set_error("pib_gemv: lane kernel does not fit (b = %d)", b); return PIB_ERR_UNSUPP; }
@@ -613,13 +609,9 @@ static size_t lxw_smem_bytes(int b) { return (size_t) LX_WARPS * (LX_STAGES * LX
 template <int BMAX>
 static int lxw_launch(const pib_weight * w, const void * act_dev, int b, float * y_dev, const int * cancel, cudaStream_t st, lx_scratch * s) {
     const size_t smem = lxw_smem_bytes(b);
-    static bool configured = false;
+    static pib_per_device attrs;
     static int  per_sm_of[PIB_MAX_BATCH + 1];
-    if (!configured) {
-        PIB_CHECK(cudaFuncSetAttribute(gemv_q4k_lanew_kernel<BMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) lxw_smem_bytes(LX_MAXB_W)));
-        for (int i = 0; i <= PIB_MAX_BATCH; i++) per_sm_of[i] = 0;
-        configured = true;
-    }
+    PIB_CHECK(attrs.once([&] { return cudaFuncSetAttribute(gemv_q4k_lanew_kernel<BMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) lxw_smem_bytes(LX_MAXB_W)); }));
     if (!per_sm_of[b]) PIB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_of[b], gemv_q4k_lanew_kernel<BMAX>, LX_THREADS, smem));
     int per_sm = per_sm_of[b];
     if (per_sm < 1) { pib_set_error("pib_gemv: warp-per-tile kernel does not fit (b = %d)", b); return PIB_ERR_UNSUPP; }

@@ -286,12 +286,11 @@ template <int NT, int WARPS>
 static int launch_q5_tc(const pib_weight * w, const uint8_t * act, const pib_act_layout & L, int b, float * y, const int * cancel, cudaStream_t st) {
     const int    nsb = (int) (w->K / 256), n_tiles = (int) ((w->N + 15) / 16);
     const size_t ring = (size_t) WARPS * Q5T_STAGES * Q5T_BYTES, smem = WARPS == 8 ? pib_gemv_smem_spread(ring, n_tiles) : ring;
-    static bool configured = false;
-    if (!configured) {
-        PIB_CHECK(cudaFuncSetAttribute(gemv_q5k_tc_kernel<NT, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (ring > PIB_GEMV_SPREAD ? ring : PIB_GEMV_SPREAD)));
-        PIB_CHECK(cudaFuncSetAttribute(gemv_q5k_tc_kernel<NT, WARPS>, cudaFuncAttributePreferredSharedMemoryCarveout, (int) cudaSharedmemCarveoutMaxShared));
-        configured = true;
-    }
+    static pib_per_device attrs;
+    PIB_CHECK(attrs.once([&] {
+        const cudaError_t e = cudaFuncSetAttribute(gemv_q5k_tc_kernel<NT, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (ring > PIB_GEMV_SPREAD ? ring : PIB_GEMV_SPREAD));
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(gemv_q5k_tc_kernel<NT, WARPS>, cudaFuncAttributePreferredSharedMemoryCarveout, (int) cudaSharedmemCarveoutMaxShared);
+    }));
     PIB_CHECK(pib_launch(gemv_q5k_tc_kernel<NT, WARPS>, dim3(n_tiles), dim3(WARPS * 32), smem, st, w->tiles, nsb, (int) w->N, (int) w->K,
                          (const int8_t *) (act + L.qsp_off), (const float *) (act + L.dxo_off), (const int8_t *) (act + L.bs8_off), b, y, cancel));
     return PIB_OK;

@@ -9,6 +9,7 @@
 #include <string.h>
 
 #include "../../include/pipeinfer_b200.h"
+#include "per_device.cuh"
 
 #define PIB_CHECK(expr)                                                                                      \
     do {                                                                                                     \
