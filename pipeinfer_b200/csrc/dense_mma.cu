@@ -1,7 +1,7 @@
 // dense_mma.cu -- the dense matmul on the tensor cores: Y[m][n] = sum_k bf16(X[m][k]) * W[n][k], W bfloat16 rows, fp32 accumulation.
 //
-// More than DT_ROWS_MAX rows (prompt portions), tcgen05.  One problem: pairs of SMs (dense_pair.cu).  Several problems or rows grouped by expert: dense_tc_kernel, whose CTA owns
-// 128 weight rows x NB tokens of one problem z:
+// More than DT_ROWS_MAX rows (prompt portions), tcgen05.  One problem: pairs of SMs (dense_pair.cu), except where dt_one_cta says.  There, and for several problems or rows grouped
+// by expert: dense_tc_kernel, whose CTA owns 128 weight rows x NB tokens of one problem z:
 //   warp 0       one lane streams both operands by TMA (cp.async.bulk.tensor.3d, 128-byte swizzle): the weight tile [128 n][64 k] and
 //                the activation tile [NB m][64 k] of every k-step land in one stage and complete one mbarrier
 //   warp 1       allocates tensor memory; an elected lane issues tcgen05.mma.cta_group::1.kind::f16 (bf16 x bf16 -> fp32, M 128, N NB, 4 x K 16 per
@@ -241,6 +241,20 @@ static int dt_launch(const pib_mm & a, const CUtensorMap & wmap, const CUtensorM
 
 static bool dt_enabled() { static const int on = getenv("PIB_DENSE_TC") ? atoi(getenv("PIB_DENSE_TC")) : 1; return on != 0; }
 
+// One problem of up to 64 rows on this file's tiles instead of pairs.  Both read every weight once, what differs are the ends of a launch (us, one CTA / pairs, float rows given):
+//   a last round of pairs with few tiles in it, where the tiles of one CTA do not end in a nearly empty round of theirs (two per SM) -- 75 to 88 pair tiles: 19200 x 4096 at
+//   17 / 64 rows 40.7 45.5 / 43.5 47.7, 19200 x 8192 74.1 78.9 / 81.3 89.2, 22016 x 8192 78.1 83.5 / 83.3 90.5, 20480 x 1024 at 17 13.6 / 14.8, at 64 17.8 / 16.1, 92 tiles: 23552 x 4096
+//   46.3 51.0 / 46.2 49.9; more rounds only with long rows: 57344 x 8192 160.6 170.5 / 168.5 178.8, 58880 x 8192 167.7 176.6 / 176.3 183.2, 57344 x 4096 88.7 98.4 / 88.3 95.5,
+//   40960 x 8192 (one CTA: two rounds of 296 for 320 tiles) 140.6 150.2 / 129.0 136.4;
+//   up to 32 rows whose k is over before a pair has started, or lies across 128-byte lines: 1024 x 128 at 17 / 32 rows 4.7 5.2 / 5.4 5.8, x 384 5.8 6.3 / 6.0 6.2, x 512 6.3 6.8 / 6.4 6.5,
+//   x 520 7.0 7.5 / 7.9 8.1, x 640 6.9 7.5 / 6.8 6.9, x 776 7.8 8.6 / 8.8 8.8, 300 x 1040 8.6 9.2 / 8.3 8.5; 32768 x 512 10.2 10.6 / 10.7 10.8.
+static bool dt_one_cta(int M, int N, int K) {
+    const int sms = pib_num_sms(), pairs = sms / 2, tiles = (N + 255) / 256, ctas = (N + DT_BM - 1) / DT_BM, rem = tiles % pairs;
+    if (M > 64) return false;
+    if (M <= 32 && (K <= 384 || (K <= 896 && K % 64) || (K <= 512 && tiles > pairs))) return true;
+    return tiles > pairs && rem > 0 && rem <= pairs / 5 && ctas % (2 * sms) > sms / 4 && (K >= 8192 || (tiles < 2 * pairs && (K >= 4096 || M <= 32)));
+}
+
 bool pib_dense_takes_rows(const pib_weight * w, int M) {
     return dt_enabled() && w && w->type == PIB_TYPE_BF16 && M > DT_ROWS_MAX && !((uintptr_t) w->base & 15) && w->K % 8 == 0 && w->K >= 16;
 }
@@ -263,7 +277,7 @@ int pib_dense_mm_tc(const pib_mm & a, cudaStream_t st) {
     const int per = grouped ? (a.M + a.Z - 1) / a.Z : a.M;
     const int NB = per <= 32 ? 32 : per <= 64 ? 64 : 128;
     int pair = 0, shares = 1;
-    if (!grouped && a.Z == 1) pib_dense_pair_plan(a.M, a.N, a.K, &pair, &shares);
+    if (!grouped && a.Z == 1 && (a.y_bf16 || !dt_one_cta(a.M, a.N, a.K))) pib_dense_pair_plan(a.M, a.N, a.K, &pair, &shares);      // the pairs write bfloat16 rows
     CUtensorMap wmap, xmap;
     const uint32_t xbox = (uint32_t) (pair ? pair / 2 : NB);
     int rc = pib_tma_map3(&wmap, a.W, (uint64_t) a.K, (uint64_t) a.N, (uint64_t) a.Z, (uint64_t) a.ldw * 2, (uint64_t) (a.Z > 1 ? a.wz : (int64_t) a.N * a.ldw) * 2, DT_BM);

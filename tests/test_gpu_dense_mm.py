@@ -52,7 +52,7 @@ def test_plain(M, N, K):
 
 
 @pytest.mark.parametrize("M,N,K,epi", [(17, 1, 16, 0), (31, 255, 128, 0), (32, 257, 136, 1), (33, 256, 1024, 0), (65, 300, 2056, 1), (255, 256, 120, 0), (257, 512, 5632, 0), (700, 255, 264, 1),
-                                       (40, 5000, 512, 0), (1000, 8448, 256, 0), (2050, 4100, 64, 0), (4096, 5121, 40, 1)])
+                                       (40, 5000, 512, 0), (1000, 8448, 256, 0), (2050, 4100, 64, 0), (4096, 5121, 40, 1), (17, 1, 904, 0), (31, 255, 1024, 0), (32, 257, 1032, 1), (65, 18945, 128, 0)])
 def test_tiles_of_sm_pairs(M, N, K, epi):
     """edges of the pairs' tiles (256 weight rows, 32 .. 256 tokens, k-steps of 128), K in shares, and more tiles than two per pair (accumulators in turn);
     fp32 accumulation of bfloat16 products: |error| <= K * 2^-23 * sum |x w|, here against the largest row"""
@@ -67,6 +67,24 @@ def test_tiles_of_sm_pairs(M, N, K, epi):
         ref = z * z
     got = mm(W, X, M, N, K, epi=epi).reshape(M, N)
     assert (np.abs(got - ref) <= bound).all()
+
+
+@pytest.mark.parametrize("M,N,K,epi", [(17, 1, 16, 1), (32, 257, 384, 0), (32, 130, 392, 0), (32, 300, 512, 1), (20, 300, 640, 0), (17, 513, 776, 1), (32, 256, 888, 0), (31, 200, 896, 0), (33, 257, 264, 0),
+                                       (32, 18944, 512, 0), (32, 18945, 512, 0), (17, 18945, 640, 1), (32, 22529, 640, 0), (33, 18945, 520, 0), (64, 18945, 4096, 1), (64, 22529, 4096, 0), (64, 57000, 1024, 0)])
+def test_sides_of_the_line_between_pairs_and_one_cta(M, N, K, epi):
+    """up to 64 rows of one problem, on both sides of each line at which the one-CTA tiles take over from the pairs (dt_one_cta): few k, k across 128-byte lines, a last round of pairs
+    with few tiles in it (75 and 88 tiles against 74 and 89 on 148 SMs); the bound as above"""
+    rng = np.random.default_rng(M + N + K)
+    W = bf16_round(rng.standard_normal((N, K), dtype=np.float32))
+    X = bf16_round(rng.standard_normal((M, K)))
+    got = mm(W, X, M, N, K, epi=epi).reshape(M, N)
+    rows = np.unique(np.concatenate([np.arange(min(N, 300)), np.arange(max(0, N - 300), N), rng.integers(0, N, 300)]))
+    ref, bound = X @ W[rows].T.astype(np.float64), np.abs(X) @ np.abs(W[rows]).T.astype(np.float64) * 2.0 ** -23 * K + 1e-30
+    if epi:
+        z = np.maximum(ref, 0.0)
+        bound = (2 * z + bound) * bound + 2.0 ** -23 * z * z
+        ref = z * z
+    assert np.isfinite(got).all() and (np.abs(got[:, rows] - ref) <= bound).all()
 
 
 @pytest.mark.parametrize("M,F,K", [(1, 225, 200), (2, 65, 72), (7, 128, 1024), (16, 100, 104), (17, 196, 184), (100, 65, 200), (300, 500, 520), (1100, 228, 200)])
