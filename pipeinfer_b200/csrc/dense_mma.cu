@@ -255,9 +255,12 @@ static bool dt_one_cta(int M, int N, int K) {
     return tiles > pairs && rem > 0 && rem <= pairs / 5 && ctas % (2 * sms) > sms / 4 && (K >= 8192 || (tiles < 2 * pairs && (K >= 4096 || M <= 32)));
 }
 
-bool pib_dense_takes_rows(const pib_weight * w, int M) {
-    return dt_enabled() && w && w->type == PIB_TYPE_BF16 && M > DT_ROWS_MAX && !((uintptr_t) w->base & 15) && w->K % 8 == 0 && w->K >= 16;
+bool pib_dense_takes_rows(const pib_weight * w, int M, cudaStream_t st) {
+    return dt_enabled() && w && w->type == PIB_TYPE_BF16 && M > DT_ROWS_MAX && !((uintptr_t) w->base & 15) && w->K % 8 == 0 && w->K >= 16 && dt_scratch_of(st, 0);
 }
+static size_t dt_stage_bytes(int64_t Zs, int64_t M, int64_t K) { return (size_t) Zs * M * ((K + 7) & ~(int64_t) 7) * 2 + 256; }
+bool pib_dense_stages_rows(int64_t M, int64_t K, cudaStream_t st) { const dt_scratch * sc = dt_scratch_of(st, dt_stage_bytes(1, M, K)); return sc && sc->xs; }
+extern "C" int pib_dense_stages_rows_host(int64_t M, int64_t K) { return pib_dense_stages_rows(M, K, nullptr) ? 1 : 0; }
 
 int pib_dense_mm_tc(const pib_mm & a, cudaStream_t st) {
     if (a.y_bf16 && (a.Z != 1 || a.zrange || a.Y2)) return PIB_ERR_UNSUPP;
@@ -269,7 +272,7 @@ int pib_dense_mm_tc(const pib_mm & a, cudaStream_t st) {
     const bool grouped = a.zrange != nullptr;
     const int  Zs = grouped ? 1 : a.Z;
     if (a.x_bf16 && (grouped || a.xrows || a.ldx % 8 || ((uintptr_t) a.X & 15) || (a.Z > 1 && a.xz % 8))) return PIB_ERR_UNSUPP;
-    dt_scratch * sc = dt_scratch_of(st, a.x_bf16 ? 0 : (size_t) Zs * a.M * Kp * 2 + 256);
+    dt_scratch * sc = dt_scratch_of(st, a.x_bf16 ? 0 : dt_stage_bytes(Zs, a.M, a.K));
     if (!sc || (!a.x_bf16 && !sc->xs)) return PIB_ERR_UNSUPP;
     if (!a.x_bf16) pib_launch(dense_cast_kernel, dim3(dim3((unsigned) a.M, (unsigned) Zs)), dim3(128), (size_t) (0), st, a.X, a.ldx, a.xz, a.xrows, a.xdiv < 1 ? 1 : a.xdiv, a.M, a.K, Kp, sc->xs);
     PIB_CHECK(cudaGetLastError());

@@ -286,7 +286,7 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
     auto mm = [&](const pib_weight * w, const float * X, int ldx, float * Y, int ldy, int epi, float e0 = 0.f, float e1 = 0.f) { return pib_dense_mm(mm_of(w, X, ldx, Y, ldy, epi, e0, e1), st); };
     // rows that only a tensor-core matmul reads are written as its bfloat16 operand by the kernel that makes them (the values that the matmul's own rounding would give)
     const bool dump = getenv("PIB_HYBRID_DUMP") != nullptr;
-    auto takes = [&](const pib_weight * w) { return !exact && !dump && pib_dense_takes_rows(w, T); };
+    auto takes = [&](const pib_weight * w) { return !exact && !dump && pib_dense_takes_rows(w, T, st); };
     bool h_bf16 = false;                              // the rows the last norm left are such rows, in x->h16 (x->h keeps what the mixture before reads: its identity outputs)
     auto mm16 = [&](const pib_weight * w, const float * X, float * Y, int ldy, int epi, float e0, float e1, bool x16, bool y16) {
         pib_mm a = mm_of(w, X, (int) w->K, Y, ldy, epi, e0, e1);
@@ -723,7 +723,7 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
             const bool routed = L.mlp == PIB_MLP_MOE && pib_norm_route_fits(T, W, router_of(L));      // small batches: the router rides on the norm
             if (L.mlp != PIB_MLP_NONE && (rc = sandwich(L.norm2, L.norm2_b, routed ? &L : nullptr, L.mlp == PIB_MLP_RELU2 && takes(L.up))) != PIB_OK) return rc;
             if (L.mlp == PIB_MLP_RELU2) {
-                const bool z16 = takes(L.up) && takes(L.down);
+                const bool z16 = takes(L.up) && takes(L.down) && (h_bf16 || pib_dense_stages_rows(T, W, st));
                 RC(HK_UP, mmfl(L.up), mmby(L.up), mm16(L.up, h_bf16 ? x->h16 : x->h, x->proj, L.ff, PIB_EPI_RELU2, 0.f, 0.f, h_bf16, z16));
                 RC(HK_DOWN, mmfl(L.down), mmby(L.down), mm16(L.down, x->proj, x->y, W, PIB_EPI_NONE, 0.f, 0.f, z16, false));
                 leftn.y = x->y;
@@ -756,7 +756,7 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
             if (L.mlp == PIB_MLP_GLU) {
                 RC(HK_HYPER, 0, hby, pib_hyper_norm(x->x, Sn, pend_y, pend_b, L.hc2, L.norm2, L.norm2_b, eps, T, W, x->h, st));
                 // gate and up rows are interleaved: the clamps, the gate's sigmoid and the product ride on the matmul's way out
-                const bool z16 = takes(L.up) && takes(L.down);
+                const bool z16 = takes(L.up) && takes(L.down) && pib_dense_stages_rows(T, W, st);
                 RC(HK_GATEUP, mmfl(L.up), wbytes(L.up) + 4.0 * Td * (Wd + L.ff), mm16(L.up, x->h, x->proj, L.ff, PIB_EPI_GLU_PAIR, L.limit_s, 0.f, false, z16));
                 RC(HK_DOWN, mmfl(L.down), mmby(L.down), mm16(L.down, x->proj, x->y, W, PIB_EPI_NONE, 0.f, 0.f, z16, false));
                 pend_y = x->y; pend_b = L.hc2;
@@ -772,7 +772,7 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
             pend_y = x->y; pend_b = L.o_bias;
             if (L.mlp == PIB_MLP_XIELU) {
                 if ((rc = prenorm(L.g2, nullptr, 0, true)) != PIB_OK) return rc;
-                const bool z16 = takes(L.up) && takes(L.down);
+                const bool z16 = takes(L.up) && takes(L.down) && pib_dense_stages_rows(T, W, st);
                 RC(HK_UP, mmfl(L.up), mmby(L.up), mm16(L.up, x->h, x->proj, L.ff, PIB_EPI_XIELU, L.act[2], L.act[3], false, z16));      // the activation rides on the matmul's way out
                 RC(HK_DOWN, mmfl(L.down), mmby(L.down), mm16(L.down, x->proj, x->y, W, PIB_EPI_NONE, 0.f, 0.f, z16, false));
                 pend_y = x->y; pend_b = nullptr;

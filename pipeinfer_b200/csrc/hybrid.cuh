@@ -270,7 +270,8 @@ template <int EPI, bool FAST> __device__ __forceinline__ float pib_glu_pair(floa
 }
 #endif
 int pib_dense_mm(const pib_mm & a, cudaStream_t st);
-bool pib_dense_takes_rows(const pib_weight * w, int M);   // a matmul of M rows with w alone runs on the tensor cores of SM pairs: bfloat16 rows in (x_bf16) and out (y_bf16)
+bool pib_dense_takes_rows(const pib_weight * w, int M, cudaStream_t st);   // a matmul of M rows with w alone runs on the tensor cores: bfloat16 rows in (x_bf16), and out (y_bf16) where its input rows are bfloat16 or ...
+bool pib_dense_stages_rows(int64_t M, int64_t K, cudaStream_t st);         // ... there is memory for the bfloat16 copy of M float rows of K (without it a matmul falls back to kernels that read and write float rows)
 int pib_dense_mm_pair(const pib_mm & a, const pib_mm & b, cudaStream_t st);   // two independent matmuls; in decode steps one launch
 int pib_dense_mm_experts(const pib_mm & routed, const pib_mm & shared, cudaStream_t st);   // a grouped matmul and a plain one with the same epilogue; in decode steps one launch
 // dense_mma.cu: the error word of a stream, which a tensor-core kernel sets when one of its bounded waits runs out

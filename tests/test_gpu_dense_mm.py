@@ -186,3 +186,17 @@ def test_grouped_by_expert_with_gather(T, E, top, K, N):
         ref[i] = np.maximum(v, 0) ** 2
     got = mm(W, X, T * top, N, K, Z=E, ldw=K, wz=N * K, xrows=perm, xdiv=top, zrange=offs, epi=1).reshape(T * top, N)
     np.testing.assert_allclose(got, ref, rtol=2e-5, atol=1e-3 * np.sqrt(K))
+
+
+def test_staging_that_memory_does_not_hold():
+    """a caller that wants bfloat16 rows out of a matmul asks first whether its float input rows can be staged (without the staging the matmul falls back to kernels that read and
+    write float rows): what no memory holds is answered, not tried later, and a staging of ordinary size is there again behind it"""
+    from pipeinfer_b200 import load
+    lib = load()
+    lib.init(0)
+    ask = lib.L.pib_dense_stages_rows_host
+    ask.argtypes = [C.c_int64, C.c_int64]
+    assert ask(300, 2048) == 1
+    assert ask(1 << 30, 1 << 20) == 0
+    assert ask(300, 2048) == 1
+    test_plain(17, 392, 184)
