@@ -12,6 +12,7 @@
 #include "hybrid.cuh"
 
 #include <algorithm>
+#include <functional>
 
 int  pib_sample_topk(float * logits_dev, int n_rows, int n_vocab, const int32_t * bias_ids_dev, const float * bias_val_dev, int n_bias,
                      void * out_dev, const uint8_t * desc, const int * cancel, cudaStream_t st);
@@ -370,21 +371,31 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
         if (any_simt)
             RC(HK_KVATTN, 2.0 * keys * H * (D + V), 4.0 * keys * G * (D + V) + 4.0 * Td * H * (D + V),
                pib_kv_attention(q, L, B, cache, row, x->cellmap, (int) c->n_ctx, out, any_mm ? B.mmflag : nullptr, st));
-        // portions of all segments gathered into launches of up to FLASH_ATTN_COLS key columns
+        auto pairs_of = [&](int p0, int nq) {                                // (token, key) pairs of a block, for the profile: the two products the attention is
+            double n = 0;
+            for (int i = 0; i < nq; i++) n += L.mask == PIB_MASK_CHUNK ? (p0 + i) % L.window + 1 : std::min<int64_t>(p0 + i + 1, (int64_t) L.window + L.keep);
+            return n;
+        };
+        // portions of all segments gathered into launches of up to FLASH_ATTN_COLS key columns; where memory does not hold the operands of them all, half of them at a time
         std::vector<pib_attn_block> blocks;
-        double bl_pairs = 0, bl_keys = 0, bl_tok = 0;
-        auto launch = [&]() -> int {
-            if (blocks.empty()) return PIB_OK;
+        int64_t bl_keys = 0;
+        std::function<int(std::vector<pib_attn_block>)> launch = [&](std::vector<pib_attn_block> some) -> int {
+            if (some.empty()) return PIB_OK;
             long long cols = 0, rows = 0;
             size_t kb = 0, vb = 0;
-            pib_flash_attention_place(blocks, L.heads / L.kv_heads, &cols, &rows);
+            pib_flash_attention_place(some, L.heads / L.kv_heads, &cols, &rows);
             const size_t qb = pib_flash_attention_bytes(L, cols, rows, &kb, &vb);
-            if ((rc = grow_flash(c, kb, vb, qb)) != PIB_OK) return rc;
-            RC(HK_FLASH, 2.0 * H * bl_pairs * (D + V), 4.0 * bl_keys * G * (D + V) + 4.0 * bl_tok * H * (D + V),
-               pib_flash_attention(q, L, blocks, (int) cols, (int) rows, cache, row, x->cellmap, (int) c->n_ctx, x->am_kb, x->am_vt, x->am_q, out, st, o16));
+            if ((rc = grow_flash(c, kb, vb, qb)) != PIB_OK) {
+                if (some.size() == 1) return rc;
+                const auto mid = some.begin() + some.size() / 2;
+                rc = launch(std::vector<pib_attn_block>(some.begin(), mid));
+                return rc != PIB_OK ? rc : launch(std::vector<pib_attn_block>(mid, some.end()));
+            }
+            double pairs = 0, keys_of = 0, tok = 0;
+            for (const pib_attn_block & g : some) { pairs += pairs_of(g.p0, g.nq); keys_of += g.NK; tok += g.nq; }
+            RC(HK_FLASH, 2.0 * H * pairs * (D + V), 4.0 * keys_of * G * (D + V) + 4.0 * tok * H * (D + V),
+               pib_flash_attention(q, L, some, (int) cols, (int) rows, cache, row, x->cellmap, (int) c->n_ctx, x->am_kb, x->am_vt, x->am_q, out, st, o16));
             nk++;
-            blocks.clear();
-            bl_pairs = bl_keys = bl_tok = 0;
             return PIB_OK;
         };
         for (const pib_hseg & g : segs) {
@@ -395,23 +406,24 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
                 int j0 = L.mask == PIB_MASK_CHUNK ? p0 - p0 % L.window : std::max(0, p0 - L.window + 1), n_front = 0;
                 if (L.keep > 0) { if (j0 <= L.keep) j0 = 0; else n_front = L.keep; }        // kept first positions: columns of their own in front of the window's
                 const int NK = n_front + p0 + nq - j0;
-                double pairs = 0;                                            // (token, key) pairs of the block, for the profile: the two products the attention is
-                for (int i = 0; i < nq; i++) pairs += L.mask == PIB_MASK_CHUNK ? (p0 + i) % L.window + 1 : std::min<int64_t>(p0 + i + 1, (int64_t) L.window + L.keep);
                 if (flash) {
-                    if (!blocks.empty() && ((int) blocks.size() == pib_flash_attention_max() || bl_keys + NK > FLASH_ATTN_COLS) && (rc = launch()) != PIB_OK) return rc;
+                    if (!blocks.empty() && ((int) blocks.size() == pib_flash_attention_max() || bl_keys + NK > FLASH_ATTN_COLS)) {
+                        if ((rc = launch(blocks)) != PIB_OK) return rc;
+                        blocks.clear();
+                        bl_keys = 0;
+                    }
                     blocks.push_back({ nq, g.start + o, p0, j0, n_front, NK, g.slot, 0, 0, 0, 0 });
-                    bl_pairs += pairs; bl_keys += NK; bl_tok += nq;
+                    bl_keys += NK;
                     continue;
                 }
                 if ((rc = grow_attn_mm(c, (size_t) G * std::max(D, V), (size_t) 3 * G * D, nq * H, nq * H, NK, (size_t) std::max(6 * D, 4 * V))) != PIB_OK) return rc;
-                RC(HK_KVATTN_MM, 2.0 * H * pairs * (D + V), 4.0 * NK * G * (D + V) + 4.0 * nq * H * (D + V),
+                RC(HK_KVATTN_MM, 2.0 * H * pairs_of(p0, nq) * (D + V), 4.0 * NK * G * (D + V) + 4.0 * nq * H * (D + V),
                    pib_kv_attention_mm(q, L, B, cache, row, x->cellmap + (size_t) g.slot * c->n_ctx, g.start + o, nq, p0, j0, n_front, NK, x->am_kb, x->am_vt, x->am_q, x->am_s,
                                        x->am_p, out, st));
                 nk += 5;
             }
         }
-        if ((rc = launch()) != PIB_OK) return rc;
-        return PIB_OK;
+        return launch(blocks);
     };
     // windowed attention over cached key / value heads: projections, convolution, norms + value mixing + cache write, attention, output
     auto mixer_swa = [&](const pib_hlayer & L, const float * hin) -> int {
