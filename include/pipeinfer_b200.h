@@ -83,7 +83,7 @@ int pib_act_to_blocks(int wtype, const void * act_dev, int b, int64_t K, void * 
 /* y_dev float [b][N] = W[N][K] . act (b rows).  Integer block dot products, fp16 block scales, fp32 accumulation.
  * Replaces: ggml_compute_forward_mul_mat (ggml.c:9388) with ggml_vec_dot_q4_0_q8_0 / q8_0_q8_0 / q4_K_q8_K
  * (ggml-quants.c:2426, 3521, 5216).  `variant`: 0 = default (fastest available), 1 = warp-per-row dp4a kernel,
- * 2 = tensor-core kernel with register-prefetched weight tiles (Q4_K; the default there), 3 = persistent TMA-staged
+ * 2 = tensor-core kernel with weight records staged by cp.async (Q4_K; the default there), 3 = persistent TMA-staged
  * tensor-core kernel (Q4_K). */
 int pib_gemv(const pib_weight * w, const void * act_dev, int b, float * y_dev, int variant, pib_stream s);
 /* Same product as pib_gemv(variant 0) for Q4_K weights, for callers that must not allocate device memory while they
@@ -96,7 +96,8 @@ int pib_gemv(const pib_weight * w, const void * act_dev, int b, float * y_dev, i
  * used (true for every matrix the current split rule splits); otherwise PIB_ERR_ARG with the sizes in pib_last_error.
  * The first call on each device looks the array's address up (cudaGetSymbolAddress): issue it before any stream
  * capture.  All calls on a device share the array: calls that overlap in time (other streams, other threads) corrupt
- * each other's sums -- serialise them.  Results are bit-identical to pib_gemv's. */
+ * each other's sums -- serialise them.  Results are pib_gemv's up to the order of the fp32 additions: pib_gemv gives
+ * narrow matrices more warps per row where this kernel splits K. */
 #define PIB_GEMV_NOALLOC_SCRATCH_BYTES (2u * 1024u * 1024u)
 #define PIB_MAX_DEV_NOALLOC 64
 int pib_gemv_q4k_noalloc(const pib_weight * w, const void * act_dev, int b, float * y_dev, pib_stream s);
@@ -123,7 +124,9 @@ int pib_mul_mat_host(const pib_weight * w, const float * x_host, int b, float * 
  * against the oracle (fp16 operand rounding, another summation order), not bit-exact.  Host buffers in and out. */
 int pib_gemm_host(const pib_weight * w, const float * x_host, int b, float * y_host);
 /* Device-buffer form: act_dev = activation planes of b rows (pib_quantize_act_rows), scratch_dev = pib_gemm_scratch_bytes(K, b) bytes
- * (the fp16 copy of the activations the TMA loads from). */
+ * for the fp16 copy of the activations that the TMA loads from.  With b > 16 that copy is part of act_dev, written by the quantiser, so
+ * act_dev has to come from a quantiser of this library called with the same b rows; scratch_dev is then not touched (but still asked
+ * for).  With b <= 16 it is made in scratch_dev from the quants. */
 size_t pib_gemm_scratch_bytes(int64_t K, int b);
 int    pib_gemm(const pib_weight * w, const void * act_dev, int b, float * y_dev, void * scratch_dev, pib_stream s);
 /* pib_gemm returns when the launch is made.  Every wait inside the kernel is bounded; one that runs out leaves y_dev unwritten in places and the stream's error

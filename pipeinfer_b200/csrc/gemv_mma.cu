@@ -629,7 +629,7 @@ gemv_q4k_ring_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, 
             float v = red[0][tok][r];
 #pragma unroll
             for (int w2 = 1; w2 < 4; w2++) v += red[w2][tok][r];
-            if (WARPS == 8) {                                   // two halves, as two K shares would add up
+            if (WARPS == 8) {                                   // two halves: with 8 super-blocks as two K shares would add up
                 float u = red[4 % WARPS][tok][r];
 #pragma unroll
                 for (int w2 = 5; w2 < 8; w2++) u += red[w2 % WARPS][tok][r];

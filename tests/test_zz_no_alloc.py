@@ -10,7 +10,7 @@ import pytest
 from oracle import oracle_py as op
 
 pytestmark = pytest.mark.gpu
-REL_TOL = 3e-5          # same envelope as tests/test_gpu_kernels.py (in practice the two entry points agree bit for bit)
+REL_TOL = 3e-5          # same envelope as tests/test_gpu_kernels.py (they may add up in another order)
 
 
 @pytest.fixture(scope="module")
