@@ -495,8 +495,9 @@ static int launch_mm(const pib_mm & a, const mm_dev & d, cudaStream_t st) {
             grid.x = (unsigned) ((a.N + 15) / 16);
             // groups that a warp has at most, as far as the shared memory of one, two or more CTAs per SM holds them: what is not needed keeps the next launch's CTAs out
             // (us a launch, one group in registers / this: 2048 x 5632 at 1 / 4 / 16 tokens 10.0 10.5 19.9 / 6.2 6.4 8.8, 2048 x 2048 4.2 4.3 7.3 / 3.0 3.0 4.2, 8000 x 2048 9.8 10.4 17.6 /
-            // 8.3 9.3 11.7).  Registers alone where a group is all and CTAs are many (32000 x 1024 at 8 tokens 15.8 / 18.2), and for 9 to 16 tokens where a round of three CTAs per SM, the
-            // registers' number, is enough and one of two is not (5120 x 2048 at 16 9.0 / 9.9)
+            // 8.3 9.3 11.7; one group alone, at 4 / 9 / 16: 2048 x 1024 2.5 3.6 3.8 / 1.9 2.3 2.5, 3072 x 1024 3.0 4.2 4.5 / 2.4 2.9 3.6).  Registers where a group is all and two CTAs per
+            // SM do not take all rows at once (32000 x 1024 at 8 tokens 15.8 / 18.2), and for 9 to 16 tokens where a round of three CTAs per SM, the registers' number, is enough and one
+            // of two is not (5120 x 2048 at 16 9.0 / 9.9)
             const long long ctas = (long long) grid.x * grid.z, sms = pib_num_sms();
             const int need = ((a.K + 31) / 32 + 8 * MVM_U - 1) / (8 * MVM_U), depth = std::min(need, ctas <= sms ? 5 : ctas <= 2 * sms ? 3 : 2);
 #define MVM_GO(DEPTH) rc = a.M <= 8 ? mvm_launch<EPI, 1, DEPTH>(grid, st, d) : mvm_launch<EPI, 2, DEPTH>(grid, st, d)

@@ -24,6 +24,33 @@ def test_few_rows(M, N, K, ldx):
     assert np.array_equal(one, got[M - 1])
 
 
+# (148 SMs) CTAs of 16 rows: one per SM up to 2368 rows, two up to 4736, three up to 7104; groups of weights that a warp has: K / 1024
+@pytest.mark.parametrize("N,K", [(2368, 1024), (2369, 1000), (4736, 1024), (4737, 1024), (4737, 520),                    # one group: in shared memory, in registers
+                                 (4737, 2048), (7104, 1032), (7105, 2048), (7105, 4104),                                # two places, used once and in turn; registers for 9 to 16 tokens
+                                 (2369, 2056), (4736, 3080), (4720, 7168),                                              # three places
+                                 (2368, 4096), (2368, 5128), (40, 11272)])                                             # five places
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+def test_weights_in_flight(M, N, K):
+    """both sides of each line at which the groups of weights that a warp has in flight change (launch_mm), with more groups than places and fewer; the bound as above"""
+    rng = np.random.default_rng(M + 10 * N + K)
+    W, X = bf16_round(rng.standard_normal((N, K), dtype=np.float32)), bf16_round(rng.standard_normal((M, K)))
+    got, again = mm(W, X, M, N, K).reshape(M, N), mm(W, X, M, N, K).reshape(M, N)
+    assert np.array_equal(got, again)
+    assert (np.abs(got - X @ W.T) <= (K + 8) * 2.0 ** -23 * (np.abs(X) @ np.abs(W).T)).all()
+
+
+def test_weights_in_flight_of_grouped_rows():
+    """rows divided over problems, each launch of a problem behind the launch wait, with places used in turn"""
+    rng = np.random.default_rng(5)
+    Z, N, K, M = 6, 1000, 4104, 14
+    zr = [0, 3, 3, 4, 12, 12, 14]
+    W, X = bf16_round(rng.standard_normal((Z, N, K), dtype=np.float32)), bf16_round(rng.standard_normal((M, K)))
+    got = mm(W, X, M, N, K, Z=Z, wz=N * K, zrange=zr).reshape(M, N)
+    for z in range(Z):
+        r = slice(zr[z], zr[z + 1])
+        assert (np.abs(got[r] - X[r] @ W[z].T) <= (K + 8) * 2.0 ** -23 * (np.abs(X[r]) @ np.abs(W[z]).T)).all()
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 24, 64), (16, 40, 2048)])
 def test_weight_rows_of_the_launch_in_front(M, N, K):
     """W that an earlier launch makes (an attention's gathered keys): none of it is read before that launch is through, however late it is"""
