@@ -154,8 +154,10 @@ int pib_weight_build_tiles_q5k(pib_weight * w) {
     return PIB_OK;
 }
 
+// Eight warps with two column blocks are launched a CTA per SM: with the registers of two per SM their loads were not far enough in front (us behind a quantiser at 9 tokens, 128 / 164
+// registers, four warps before them: 1024 x 2816 6.6 / 4.4, 5.1; 2048 x 2048 4.9 / 3.8, 4.5; 1024 x 8192 9.9 / 6.4, 8.9; 2368 x 28672 29.5 / 18.0, 38.5).
 template <int NT, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : NT == 1 ? 4 : 3)
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? (NT == 1 ? 2 : 1) : NT == 1 ? 4 : 3)
 gemv_q5k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, const int8_t * __restrict__ aqs, const float * __restrict__ ad,
                    const int8_t * __restrict__ abs8, int b, float * __restrict__ y, const int * __restrict__ cancel) {
     if (PIB_CANCELLED(cancel)) { pib_pdl_wait(); return; }
