@@ -101,7 +101,7 @@ int pib_weight_build_tiles_q3k(pib_weight * w) {
     return PIB_OK;
 }
 
-template <int NT, int WARPS>
+template <int NT, int WARPS, bool ONE>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : NT == 1 ? 4 : 3)
 gemv_q3k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, const int8_t * __restrict__ aq6, const float * __restrict__ ad,
                    const int8_t * __restrict__ ab16, int b, float * __restrict__ y, const int * __restrict__ cancel) {
@@ -136,7 +136,7 @@ gemv_q3k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, co
     int            gs[NT];                                      // tokens of the octet (pib_oct)
 #pragma unroll
     for (int n = 0; n < NT; n++) {
-        gs[n] = min(8, b - 8 * n);
+        gs[n] = ONE ? 1 : min(8, b - 8 * n);                      // one token: distances known beforehand (gemv_blk32.cu)
         a_q[n] = aq6 + (size_t) n * 8 * K + min(g, gs[n] - 1) * 64 + t * 16;
         a_b[n] = ab16 + ((size_t) n * 8 * nsb + min(g, gs[n] - 1)) * 32 + 4 * t;
 #pragma unroll
@@ -218,16 +218,16 @@ gemv_q3k_tc_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, co
     }
 }
 
-template <int NT, int WARPS>
+template <int NT, int WARPS, bool ONE = false>
 static int launch_q3_tc(const pib_weight * w, const uint8_t * act, const pib_act_layout & L, int b, float * y, const int * cancel, cudaStream_t st) {
     const int    nsb = (int) (w->K / 256), n_tiles = (int) ((w->N + 15) / 16);
     const size_t ring = (size_t) WARPS * Q3T_STAGES * Q3T_BYTES, smem = WARPS == 8 ? pib_gemv_smem_spread(ring, n_tiles) : ring;
     static pib_per_device attrs;
     PIB_CHECK(attrs.once([&] {
-        const cudaError_t e = cudaFuncSetAttribute(gemv_q3k_tc_kernel<NT, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (ring > PIB_GEMV_SPREAD ? ring : PIB_GEMV_SPREAD));
-        return e != cudaSuccess ? e : cudaFuncSetAttribute(gemv_q3k_tc_kernel<NT, WARPS>, cudaFuncAttributePreferredSharedMemoryCarveout, (int) cudaSharedmemCarveoutMaxShared);
+        const cudaError_t e = cudaFuncSetAttribute(gemv_q3k_tc_kernel<NT, WARPS, ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (ring > PIB_GEMV_SPREAD ? ring : PIB_GEMV_SPREAD));
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(gemv_q3k_tc_kernel<NT, WARPS, ONE>, cudaFuncAttributePreferredSharedMemoryCarveout, (int) cudaSharedmemCarveoutMaxShared);
     }));
-    PIB_CHECK(pib_launch(gemv_q3k_tc_kernel<NT, WARPS>, dim3(n_tiles), dim3(WARPS * 32), smem, st, w->tiles, nsb, (int) w->N, (int) w->K,
+    PIB_CHECK(pib_launch(gemv_q3k_tc_kernel<NT, WARPS, ONE>, dim3(n_tiles), dim3(WARPS * 32), smem, st, w->tiles, nsb, (int) w->N, (int) w->K,
                          (const int8_t *) (act + L.q6p_off), (const float *) (act + L.dxo_off), (const int8_t *) (act + L.b16_off), b, y, cancel));
     return PIB_OK;
 }
@@ -236,8 +236,8 @@ int pib_gemv_q3k(const pib_weight * w, const void * act_dev, int b, float * y_de
     if (!w || w->type != PIB_TYPE_Q3_K || !w->tiles || b < 1 || b > PIB_MAX_BATCH) { pib_set_error("pib_gemv: not a resident Q3_K matrix (or batch > %d)", PIB_MAX_BATCH); return PIB_ERR_UNSUPP; }
     const pib_act_layout L   = pib_act_layout_of(PIB_TYPE_Q4_K, w->K, b);          // Q8_K family activations
     const uint8_t *      act = (const uint8_t *) act_dev;
-    if (pib_gemv_wide(w)) return b <= 8 ? launch_q3_tc<1, 8>(w, act, L, b, y_dev, cancel, st) : launch_q3_tc<2, 8>(w, act, L, b, y_dev, cancel, st);
-    return b <= 8 ? launch_q3_tc<1, 4>(w, act, L, b, y_dev, cancel, st) : launch_q3_tc<2, 4>(w, act, L, b, y_dev, cancel, st);
+    if (pib_gemv_wide(w)) return b == 1 ? launch_q3_tc<1, 8, true>(w, act, L, b, y_dev, cancel, st) : b <= 8 ? launch_q3_tc<1, 8>(w, act, L, b, y_dev, cancel, st) : launch_q3_tc<2, 8>(w, act, L, b, y_dev, cancel, st);
+    return b == 1 ? launch_q3_tc<1, 4, true>(w, act, L, b, y_dev, cancel, st) : b <= 8 ? launch_q3_tc<1, 4>(w, act, L, b, y_dev, cancel, st) : launch_q3_tc<2, 4>(w, act, L, b, y_dev, cancel, st);
 }
 
 // embedding rows: dequantize_row_q3_K (ggml-quants.c:1711-1758), one thread per element, same float operations in the same order

@@ -23,7 +23,8 @@ def blocks(rng, wt, N, K):
     (Q4, 9471, 4096, 15), (Q4, 9485, 4096, 9), (Q4, 2361, 8448, 16), (Q4, 40, 6400, 13),                          # 592 / 593 tiles; one CTA per SM
     (Q6, 2353, 1792, 3), (Q6, 2353, 2048, 8), (Q6, 2371, 2304, 9), (Q6, 4735, 4096, 15), (Q6, 4743, 4096, 16), (Q6, 19, 4352, 1),      # 148 / 149 and 296 / 297 tiles
     (Q5, 2353, 1792, 3), (Q5, 2353, 2048, 8), (Q5, 2353, 2304, 9), (Q5, 2371, 2304, 9), (Q5, 4735, 4096, 7), (Q5, 4743, 4096, 1),
-    (Q3, 2353, 1792, 3), (Q3, 2353, 2048, 8), (Q3, 2371, 2304, 9), (Q3, 4735, 4096, 15), (Q3, 4743, 4096, 16)])
+    (Q3, 2353, 1792, 3), (Q3, 2353, 2048, 8), (Q3, 2371, 2304, 9), (Q3, 4735, 4096, 15), (Q3, 4743, 4096, 16),
+    (Q3, 2353, 2048, 1), (Q3, 4743, 4096, 1), (Q5, 2353, 2048, 1), (Q6, 4743, 4096, 1), (Q5, 1031, 2816, 12), (Q5, 1031, 8192, 9)])      # one token; two octets, a CTA per SM
 def test_both_sides(oracle, wt, N, K, b):
     from pipeinfer_b200 import load
     lib = load()
