@@ -406,11 +406,14 @@ __global__ void __launch_bounds__(256, NT == 2 ? 2 : 3) mv_mma_experts_kernel(mm
     int z, row0, row1;
     if (mv_problem(a, blockIdx.x / tiles_a, 8 * NT, z, row0, row1)) mvm_body<EPI, NT, 2, false>(a, z, (int) blockIdx.x % tiles_a, row0, row1);
 }
-template <int EPI_B, int NT>
-__global__ void __launch_bounds__(256, NT == 2 ? 2 : 3) mv_mma_pair_kernel(mm_dev a, mm_dev b, int tiles_a) {
-    if ((int) blockIdx.x < tiles_a) mvm_body<PIB_EPI_NONE, NT, 2, true>(a, 0, blockIdx.x, 0, a.M);
-    else                            mvm_body<EPI_B, NT, 2, true>(b, 0, blockIdx.x - tiles_a, 0, b.M);
+template <int EPI_B, int NT, int DEPTH>
+__global__ void __launch_bounds__(256, NT == 2 && DEPTH ? 2 : 3) mv_mma_pair_kernel(mm_dev a, mm_dev b, int tiles_a) {
+    if ((int) blockIdx.x < tiles_a) mvm_body<PIB_EPI_NONE, NT, DEPTH, true>(a, 0, blockIdx.x, 0, a.M);
+    else                            mvm_body<EPI_B, NT, DEPTH, true>(b, 0, blockIdx.x - tiles_a, 0, b.M);
 }
+// whether one group of weights in registers is the better form of a launch (the figures: launch_mm); a warp has `need` groups at most
+static int  mvm_groups(int K) { return ((K + 31) / 32 + 8 * MVM_U - 1) / (8 * MVM_U); }
+static bool mvm_registers(long long ctas, int need, int M) { const long long sms = pib_num_sms(); return ctas > 2 * sms && (need == 1 || (M > 8 && ctas <= 3 * sms)); }
 // bfloat16 weights whose 16-byte pieces and the activations' lie on 16-byte boundaries (the caller has looked at the weights)
 template <typename WT, bool ROUND> static bool mvm_fits(const mm_dev & a, bool xvec) { return std::is_same<WT, __nv_bfloat16>::value && ROUND && xvec && a.K % 8 == 0; }
 
@@ -499,10 +502,10 @@ static int launch_mm(const pib_mm & a, const mm_dev & d, cudaStream_t st) {
             // SM do not take all rows at once (32000 x 1024 at 8 tokens 15.8 / 18.2), and for 9 to 16 tokens where a round of three CTAs per SM, the registers' number, is enough and one
             // of two is not (5120 x 2048 at 16 9.0 / 9.9)
             const long long ctas = (long long) grid.x * grid.z, sms = pib_num_sms();
-            const int need = ((a.K + 31) / 32 + 8 * MVM_U - 1) / (8 * MVM_U), depth = std::min(need, ctas <= sms ? 5 : ctas <= 2 * sms ? 3 : 2);
+            const int need = mvm_groups(a.K), depth = std::min(need, ctas <= sms ? 5 : ctas <= 2 * sms ? 3 : 2);
 #define MVM_GO(DEPTH) rc = a.M <= 8 ? mvm_launch<EPI, 1, DEPTH>(grid, st, d) : mvm_launch<EPI, 2, DEPTH>(grid, st, d)
             int rc;
-            if (ctas > 2 * sms && (need == 1 || (a.M > 8 && ctas <= 3 * sms))) MVM_GO(0);
+            if (mvm_registers(ctas, need, a.M)) MVM_GO(0);
             else if (depth <= 1) MVM_GO(1); else if (depth == 2) MVM_GO(2); else if (depth == 3) MVM_GO(3); else MVM_GO(5);
 #undef MVM_GO
             if (rc != PIB_OK) return rc;
@@ -563,9 +566,15 @@ static int launch_pair(const mm_dev & a, const mm_dev & b, bool xva, bool xvb, c
     if (mvm_fits<WT, ROUND>(a, xva) && mvm_fits<WT, ROUND>(b, xvb)) {
         const int ta = (a.N + 15) / 16, tb = (b.N + 15) / 16;
         static pib_per_device one, two;
-        PIB_CHECK(a.M <= 8 ? mvm_smem(one, mv_mma_pair_kernel<EPI_B, 1>, MVM_SMEM(2)) : mvm_smem(two, mv_mma_pair_kernel<EPI_B, 2>, MVM_SMEM(2)));
-        if (a.M <= 8) pib_launch(mv_mma_pair_kernel<EPI_B, 1>, dim3((unsigned) (ta + tb)), dim3(256), MVM_SMEM(2), st, a, b, ta);
-        else          pib_launch(mv_mma_pair_kernel<EPI_B, 2>, dim3((unsigned) (ta + tb)), dim3(256), MVM_SMEM(2), st, a, b, ta);
+        // (one group, 1024 + 5632 rows x 1024 at 8 / 9 / 16 tokens: registers 4.0 5.2 5.4 us, shared memory 4.3 6.3 7.3)
+        if (mvm_registers(ta + tb, mvm_groups(std::max(a.K, b.K)), a.M)) {
+            if (a.M <= 8) pib_launch(mv_mma_pair_kernel<EPI_B, 1, 0>, dim3((unsigned) (ta + tb)), dim3(256), MVM_SMEM(0), st, a, b, ta);
+            else          pib_launch(mv_mma_pair_kernel<EPI_B, 2, 0>, dim3((unsigned) (ta + tb)), dim3(256), MVM_SMEM(0), st, a, b, ta);
+        } else {
+            PIB_CHECK(a.M <= 8 ? mvm_smem(one, mv_mma_pair_kernel<EPI_B, 1, 2>, MVM_SMEM(2)) : mvm_smem(two, mv_mma_pair_kernel<EPI_B, 2, 2>, MVM_SMEM(2)));
+            if (a.M <= 8) pib_launch(mv_mma_pair_kernel<EPI_B, 1, 2>, dim3((unsigned) (ta + tb)), dim3(256), MVM_SMEM(2), st, a, b, ta);
+            else          pib_launch(mv_mma_pair_kernel<EPI_B, 2, 2>, dim3((unsigned) (ta + tb)), dim3(256), MVM_SMEM(2), st, a, b, ta);
+        }
     } else
     if (a.M == 1)      pib_launch(mv_pair_kernel<WT, ROUND, EPI_B, 1>, grid, dim3(256), (size_t) 0, st, a, b, xva, xvb, ba);
     else if (a.M == 2) pib_launch(mv_pair_kernel<WT, ROUND, EPI_B, 2>, grid, dim3(256), (size_t) 0, st, a, b, xva, xvb, ba);

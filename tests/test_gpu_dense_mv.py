@@ -76,3 +76,37 @@ def test_sums_do_not_drift(M, N, K):
     rel = got / (X.astype(np.float64) @ W.astype(np.float64).T) - 1
     print("K %d: mean relative error %.2g, mean size %.2g" % (K, rel.mean(), np.abs(rel).mean()))
     assert abs(rel.mean()) < 2.0 ** -23
+
+
+class MM(C.Structure):
+    """pib_mm (csrc/hybrid.cuh)"""
+    _fields_ = [("W", C.c_void_p), ("wtype", C.c_int), ("ldw", C.c_int64), ("wz", C.c_int64), ("X", C.c_void_p), ("ldx", C.c_int64), ("xz", C.c_int64), ("xrows", C.c_void_p), ("xdiv", C.c_int),
+                ("Y", C.c_void_p), ("ldy", C.c_int64), ("yz", C.c_int64), ("M", C.c_int), ("N", C.c_int), ("K", C.c_int), ("Z", C.c_int), ("zlist", C.c_void_p), ("zrange", C.c_void_p),
+                ("epi", C.c_int), ("e0", C.c_float), ("e1", C.c_float), ("exact", C.c_int), ("Y2", C.c_void_p), ("ld2", C.c_int64), ("n2", C.c_int), ("rows2", C.c_void_p),
+                ("x_bf16", C.c_int), ("y_bf16", C.c_int), ("w_made", C.c_int)]
+
+
+@pytest.mark.parametrize("N1,N2,K", [(1024, 3712, 1000), (1024, 3744, 1024), (1024, 3744, 2048), (1024, 6080, 2056), (1024, 6096, 2048)])      # 296 / 298 and 444 / 445 CTAs, one group and more
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+def test_two_matmuls_in_a_launch(N1, N2, K, M):
+    """both sides of the lines at which the pair's weights wait in registers or in shared memory; the bound as above"""
+    lib = load()
+    lib.init(0)
+    f = lib.L._Z17pib_dense_mm_pairRK6pib_mmS1_P11CUstream_st
+    f.argtypes = [C.c_void_p] * 3
+    rng = np.random.default_rng(M + N1 + N2 + K)
+    X = bf16_round(rng.standard_normal((M, K)))
+    Ws = [bf16_round(rng.standard_normal((n, K), dtype=np.float32)) for n in (N1, N2)]
+    x = lib.to_device(X.astype(np.float32))
+    mms, dev = [], [x]
+    for w in Ws:
+        wd, y = lib.to_device((w.astype(np.float32).view(np.uint32) >> 16).astype(np.uint16)), lib.to_device(np.full((M, len(w)), np.nan, np.float32))
+        dev += [wd, y]
+        mms.append(MM(W=wd, wtype=30, ldw=K, X=x, ldx=K, xdiv=1, Y=y, ldy=len(w), M=M, N=len(w), K=K, Z=1, n2=0x7fffffff))
+    lib.check(f(C.byref(mms[0]), C.byref(mms[1]), None))
+    lib.check(lib.L.pib_stream_sync(None))
+    for w, m in zip(Ws, mms):
+        got = lib.to_host(m.Y, (M, len(w)), np.float32)
+        assert (np.abs(got - X @ w.T) <= (K + 8) * 2.0 ** -23 * (np.abs(X) @ np.abs(w).T)).all()
+    for d in dev:
+        lib.free(d)
