@@ -25,6 +25,7 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "q8k_quant.cuh"
@@ -420,13 +421,17 @@ static int tg_launch(const pib_weight * w, const __half * xh, int b, int x0, int
     const CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void *) xh, gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { pib_set_error("pib_gemm: cuTensorMapEncodeTiled failed (%d)", (int) r); return PIB_ERR_CUDA; }
+    // Two CTAs of one group share an SM where there are more of them than SMs.  Where there are not, and all clusters find room at one per SM, they ask for so much shared memory
+    // that they do not: launched while the quantiser in front still runs they would double up (us a call: 4096 x 14336 at 56 / 64 tokens 28.8 29.1 / 21.9 22.3, 4096 x 12288
+    // at 64 26.2 / 20.3)
+    const size_t smem = G == 1 && nx * S <= pib_num_sms() && nx <= tg_fit_nb(NB, S) ? std::max(C::SMEM, (size_t) PIB_GEMV_SPREAD) : C::SMEM;
     static pib_per_device attrs;
-    PIB_CHECK(attrs.once([&] { return cudaFuncSetAttribute(gemm_q4k_tc_kernel<NB, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) C::SMEM); }));
+    PIB_CHECK(attrs.once([&] { return cudaFuncSetAttribute(gemm_q4k_tc_kernel<NB, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) std::max(C::SMEM, (size_t) PIB_GEMV_SPREAD)); }));
     const dim3 grid((unsigned) nx, 1, (unsigned) S);
     int * err = pib_tc_error_word(st);
     if (!err) { pib_set_error("pib_gemm: no memory for the stream's error word"); return PIB_ERR_NOMEM; }
-    if (S > 1) pib_launch_cluster(gemm_q4k_tc_kernel<NB, G>, grid, dim3(C::THREADS), dim3(1, 1, (unsigned) S), C::SMEM, st, w->tiles, (int) (w->K / 256), (int) w->N, x0, tg_tiles_of(b), map, b, y, err);
-    else       pib_launch(gemm_q4k_tc_kernel<NB, G>, grid, dim3(C::THREADS), C::SMEM, st, w->tiles, (int) (w->K / 256), (int) w->N, x0, tg_tiles_of(b), map, b, y, err);
+    if (S > 1) pib_launch_cluster(gemm_q4k_tc_kernel<NB, G>, grid, dim3(C::THREADS), dim3(1, 1, (unsigned) S), smem, st, w->tiles, (int) (w->K / 256), (int) w->N, x0, tg_tiles_of(b), map, b, y, err);
+    else       pib_launch(gemm_q4k_tc_kernel<NB, G>, grid, dim3(C::THREADS), smem, st, w->tiles, (int) (w->K / 256), (int) w->N, x0, tg_tiles_of(b), map, b, y, err);
     PIB_CHECK(cudaGetLastError());
     return PIB_OK;
 }
