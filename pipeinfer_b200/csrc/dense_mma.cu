@@ -243,8 +243,8 @@ static bool dt_enabled() { static const int on = getenv("PIB_DENSE_TC") ? atoi(g
 
 // One problem of up to 64 rows on this file's tiles instead of pairs.  Both read every weight once, what differs are the ends of a launch (us, one CTA / pairs, float rows given):
 //   a last round of pairs with few tiles in it, where the tiles of one CTA do not end in a nearly empty round of theirs (two per SM) -- 75 to 88 pair tiles: 19200 x 4096 at
-//   17 / 64 rows 40.7 45.5 / 43.5 47.7, 19200 x 8192 74.1 78.9 / 81.3 89.2, 22016 x 8192 78.1 83.5 / 83.3 90.5, 20480 x 1024 at 17 13.6 / 14.8, at 64 17.8 / 16.1, 92 tiles: 23552 x 4096
-//   46.3 51.0 / 46.2 49.9; more rounds only with long rows: 57344 x 8192 160.6 170.5 / 168.5 178.8, 58880 x 8192 167.7 176.6 / 176.3 183.2, 57344 x 4096 88.7 98.4 / 88.3 95.5,
+//   17 / 64 rows 40.7 45.5 / 43.5 47.7, 19200 x 8192 74.1 78.9 / 81.3 89.2, 22016 x 8192 78.1 83.5 / 83.3 90.5, 20480 x 1024 at 17 13.6 / 14.8, at 64 17.8 / 16.1, 92 tiles (up to 32
+//   rows only): 23552 x 2048 24.5 29.1 / 25.6 27.9, 23552 x 4096 46.3 51.0 / 46.2 49.9; more rounds only with long rows: 57344 x 8192 160.6 170.5 / 168.5 178.8, 58880 x 8192 167.7 176.6 / 176.3 183.2, 57344 x 4096 88.7 98.4 / 88.3 95.5,
 //   40960 x 8192 (one CTA: two rounds of 296 for 320 tiles) 140.6 150.2 / 129.0 136.4;
 //   up to 32 rows whose k is over before a pair has started, or lies across 128-byte lines: 1024 x 128 at 17 / 32 rows 4.7 5.2 / 5.4 5.8, x 384 5.8 6.3 / 6.0 6.2, x 512 6.3 6.8 / 6.4 6.5,
 //   x 520 7.0 7.5 / 7.9 8.1, x 640 6.9 7.5 / 6.8 6.9, x 776 7.8 8.6 / 8.8 8.8, 300 x 1040 8.6 9.2 / 8.3 8.5; 32768 x 512 10.2 10.6 / 10.7 10.8.
@@ -252,7 +252,7 @@ static bool dt_one_cta(int M, int N, int K) {
     const int sms = pib_num_sms(), pairs = sms / 2, tiles = (N + 255) / 256, ctas = (N + DT_BM - 1) / DT_BM, rem = tiles % pairs;
     if (M > 64) return false;
     if (M <= 32 && (K <= 384 || (K <= 896 && K % 64) || (K <= 512 && tiles > pairs))) return true;
-    return tiles > pairs && rem > 0 && rem <= pairs / 5 && ctas % (2 * sms) > sms / 4 && (K >= 8192 || (tiles < 2 * pairs && (K >= 4096 || M <= 32)));
+    return tiles > pairs && rem > 0 && rem <= (M <= 32 ? pairs / 4 : pairs / 5) && ctas % (2 * sms) > sms / 4 && (K >= 8192 || (tiles < 2 * pairs && (K >= 4096 || M <= 32)));
 }
 
 bool pib_dense_takes_rows(const pib_weight * w, int M, cudaStream_t st) {

@@ -70,10 +70,10 @@ def test_tiles_of_sm_pairs(M, N, K, epi):
 
 
 @pytest.mark.parametrize("M,N,K,epi", [(17, 1, 16, 1), (32, 257, 384, 0), (32, 130, 392, 0), (32, 300, 512, 1), (20, 300, 640, 0), (17, 513, 776, 1), (32, 256, 888, 0), (31, 200, 896, 0), (33, 257, 264, 0),
-                                       (32, 18944, 512, 0), (32, 18945, 512, 0), (17, 18945, 640, 1), (32, 22529, 640, 0), (33, 18945, 520, 0), (64, 18945, 4096, 1), (64, 22529, 4096, 0), (64, 57000, 1024, 0)])
+                                       (32, 18944, 512, 0), (32, 18945, 512, 0), (17, 18945, 640, 1), (32, 23552, 640, 0), (32, 23553, 640, 0), (33, 18945, 520, 0), (64, 18945, 4096, 1), (64, 22529, 4096, 0), (64, 57000, 1024, 0)])
 def test_sides_of_the_line_between_pairs_and_one_cta(M, N, K, epi):
     """up to 64 rows of one problem, on both sides of each line at which the one-CTA tiles take over from the pairs (dt_one_cta): few k, k across 128-byte lines, a last round of pairs
-    with few tiles in it (75 and 88 tiles against 74 and 89 on 148 SMs); the bound as above"""
+    with few tiles in it (75 and 88, or up to 32 rows 92, tiles against 74 and 89, or 93, on 148 SMs); the bound as above"""
     rng = np.random.default_rng(M + N + K)
     W = bf16_round(rng.standard_normal((N, K), dtype=np.float32))
     X = bf16_round(rng.standard_normal((M, K)))
