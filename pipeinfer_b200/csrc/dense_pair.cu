@@ -253,7 +253,8 @@ dense_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constan
 // Tile width and shares of K: the least of what a launch takes by this model of its time in us, made from 700 points (N x K of 3072 x 2048, 2048 x 5632, 5632 x 2048, 8000 x 2048
 // and 1024 x 2816, 20 to 2500 tokens): a k-step costs more the wider the tile and the more pairs read at once, from 160 tokens on the ring holds three steps instead of
 // four or more; a round is as long as its tiles; shares cost the meeting of their sums.  Shares of S take clusters of 2 S CTAs, of which the machine holds fewer than its SMs allow
-// (33 of 4 CTAs, 15 of 8).  The choice was at most 1.5 us behind the best point measured.
+// (33 of 4 CTAs, 15 of 8).  The choice was at most 1.5 us behind the best of those points.  Beyond them it holds as far as the one-CTA tiles are no faster, which was looked at for
+// 48 matrices up to 128256 x 4096 and 8192 x 28672 and is left to dt_one_cta (dense_mma.cu) where they are.
 void pib_dense_pair_plan(int M, int N, int K, int * nb, int * shares) {
     const int pairs = pib_num_sms() / 2, tn = (N + 255) / 256, steps = (K + DP_BK - 1) / DP_BK;
     double best = 0;

@@ -20,8 +20,8 @@
 // the MMAs of the step before last; with four, and the producer and the issuing warp counting their places along, 12288 x 4096 32.7 -> 27.6 us, 4096 x 4096 18.8 -> 16.4,
 // 57344 x 8192 204 -> 192).
 // What bounds it: up to about 100 tokens the dequantisation, 109 warp instructions per 16 rows x 64 k issued at 0.6 per clock and scheduler (57344 x 8192
-// at 40 tokens 96 us, where the weights' bytes take 40; with the operand written to and read from shared memory, the form this replaces, 173 us); with
-// 256 tokens the tensor cores and the activation tiles' way into shared memory (203 us, before 246; 151 at the dense peak).
+// at 40 tokens 96 us, where the weights' bytes take 40; with the operand written to and read from shared memory, the form this replaced, 173 us); with
+// 256 tokens the tensor cores and the activation tiles' way into shared memory (192 us; 151 at the dense peak).
 #include <cuda.h>
 #include <cuda_fp16.h>
 
@@ -39,8 +39,8 @@
 template <int NB, int G> struct tg_cfg {
     static constexpr int CTAS    = 3 - G;                                // per SM
     static constexpr int STAGES  = G == 2 ? 4 : NB > 64 ? 2 : 3;   // k-steps of weights in tensor memory
-    static constexpr int PIECES  = NB > 128 ? 2 : 1;                     // activations arrive in pieces of a k-step: with two stages only, whole ones are late (256 tokens:
-    static constexpr int BSTAGES = NB > 128 ? 4 : STAGES;                // 246 -> 193 us); with more stages a second barrier per step costs more (24 tokens: 31 -> 44)
+    static constexpr int PIECES  = NB > 128 ? 2 : 1;                     // activations arrive in pieces of a k-step where shared memory holds two whole steps only, which are
+    static constexpr int BSTAGES = NB > 128 ? 4 : STAGES;                // late then (256 tokens: 246 -> 193 us); elsewhere a second barrier per step costs more (24 tokens: 31 -> 44)
     static constexpr int WSTAGES = NB == 128 && G == 1 ? 2 : 3;          // super-blocks of weight records in shared memory
     static constexpr int WARPS   = 8 * G, THREADS = 96 + 32 * WARPS;
     static constexpr int W_BYTES = 8 * TG_TILE_BYTES, B_BYTES = NB * 256 / PIECES;

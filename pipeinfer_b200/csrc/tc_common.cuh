@@ -1,4 +1,4 @@
-// tc_common.cuh -- what the tcgen05 kernels share (dense_mma.cu, flash_attn.cu): bounded mbarrier waits, TMA loads, matrix descriptors, MMA issue and commit.
+// tc_common.cuh -- what the tcgen05 kernels share (dense_mma.cu, dense_pair.cu, flash_attn.cu, gemm_q4k_tc.cu): bounded mbarrier waits, TMA loads, matrix descriptors, MMA issue and commit.
 //
 // Every mbarrier wait is bounded: a wait that runs out raises the block's abort flag, on which the other roles give up too.
 #pragma once

@@ -102,8 +102,7 @@ def test_get_rows_bit_exact(lib, kern, name, wt):
 def variants(wt):
     # 1 = dp4a (all types), 2 = the default tensor-core kernel (all types), 3 = TMA-staged persistent kernel (Q4_K only),
     # 4 = the reference's summation order restated literally, one thread per output (all types), 6 = the tensor-core kernel that
-    # keeps the reference's order (Q4_K only), 8 = the balanced stream kernel (Q4_K only; what variant 2 picks for row-tile counts that
-    # do not fill the machine evenly)
+    # keeps the reference's order (Q4_K only), 8 = the balanced stream kernel (Q4_K only)
     return [1, 2, 3, 4, 6, 8] if wt == op.TYPE_Q4_K else [1, 2, 4]
 
 
