@@ -29,7 +29,7 @@ struct pib_hybrid_ctx {
     float * x = nullptr, * h = nullptr, * y = nullptr, * proj = nullptr, * cq = nullptr, * q = nullptr, * qlat = nullptr, * lat = nullptr, * att = nullptr;
     float * rlog = nullptr, * wts = nullptr, * eup = nullptr, * edn = nullptr, * ysh = nullptr;
     float * h2 = nullptr, * cv = nullptr, * vfirst = nullptr, * mixes = nullptr;   // parallel layers: second norm (pre-norm layers: the stream's second buffer); convolved q | k | v; first mixing layer's values; token-shift mixes
-    float * h16 = nullptr;                             // sandwich frame: the norm's rows as the bfloat16 operand of the matmul that alone reads them (W / 2 floats a row)
+    float * h16 = nullptr;                             // sandwich frame: where the norm's rows go as the bfloat16 operand of the matmul that alone reads them: the attention's rows, which are not there yet (null: too short)
     float * rg = nullptr, * y2 = nullptr;       // gated frame: the residual gate's logits; the second branch's output
     float * cat = nullptr;                      // [stream ; embedding] rows of models whose layers are walked again
     int32_t * ids = nullptr, * perm = nullptr, * inv = nullptr, * counts = nullptr, * offs = nullptr, * act = nullptr, * done = nullptr;   // act: the experts with rows of a small batch; done: 0 between launches
@@ -182,7 +182,7 @@ static int grow_chunk(pib_context * c, size_t need) {
 static void free_scratch(pib_hybrid_ctx * x) {
     for (void * b : { (void *) x->x, (void *) x->h, (void *) x->y, (void *) x->proj, (void *) x->cq, (void *) x->q, (void *) x->qlat, (void *) x->lat, (void *) x->att,
                       (void *) x->rlog, (void *) x->wts, (void *) x->eup, (void *) x->edn, (void *) x->ysh, (void *) x->ids, (void *) x->perm, (void *) x->inv,
-                      (void *) x->counts, (void *) x->offs, (void *) x->act, (void *) x->done, (void *) x->h2, (void *) x->cv, (void *) x->vfirst, (void *) x->mixes, (void *) x->cat, (void *) x->rg, (void *) x->y2, (void *) x->h16 }) if (b) cudaFree(b);
+                      (void *) x->counts, (void *) x->offs, (void *) x->act, (void *) x->done, (void *) x->h2, (void *) x->cv, (void *) x->vfirst, (void *) x->mixes, (void *) x->cat, (void *) x->rg, (void *) x->y2 }) if (b) cudaFree(b);
     x->x = x->h = x->y = x->proj = x->cq = x->q = x->qlat = x->lat = x->att = x->rlog = x->wts = x->eup = x->edn = x->ysh = nullptr;
     x->h2 = x->cv = x->vfirst = x->mixes = x->cat = x->rg = x->y2 = x->h16 = nullptr;
     x->ids = x->perm = x->inv = x->counts = x->offs = x->act = x->done = nullptr;
@@ -227,8 +227,9 @@ static int grow_scratch(pib_context * c, int T) {
                     in(&x->ids, n * hy->w_pairs) && in(&x->perm, n * hy->w_pairs) && in(&x->inv, n * hy->w_pairs) && in(&x->counts, (size_t) hy->w_router + 1) &&
                     in(&x->offs, (size_t) hy->w_router + 2) && in(&x->act, (size_t) hy->w_router + 2) && in(&x->done, hy->w_router ? 4 : 0) && (!x->done || cudaMemset(x->done, 0, 16) == cudaSuccess) && fl(&x->h2, hy->form == PIB_FORM_PARALLEL || hy->form == PIB_FORM_PRENORM || hy->form == PIB_FORM_GATED ? W : 0) && fl(&x->cv, (size_t) hy->w_conv) &&
                     fl(&x->vfirst, (size_t) hy->w_vfirst) && fl(&x->mixes, (size_t) hy->w_shift) && fl(&x->cat, (size_t) hy->w_cat) &&
-                    fl(&x->rg, (size_t) hy->w_gate) && fl(&x->y2, (size_t) hy->w_y2) && fl(&x->h16, hy->form == PIB_FORM_SANDWICH && hy->dtype != PIB_TYPE_F32 ? (W + 1) / 2 : 0);
+                    fl(&x->rg, (size_t) hy->w_gate) && fl(&x->y2, (size_t) hy->w_y2);
     if (!ok) { cudaGetLastError(); free_scratch(x); pib_set_error("decode: out of memory for the work buffers of %d tokens", T); return PIB_ERR_NOMEM; }
+    x->h16 = 2 * (size_t) hy->w_att >= W ? x->att : nullptr;
     x->cap = (int) n;
     return PIB_OK;
 }
@@ -718,7 +719,7 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
     // sandwich frame: what the sublayer before left is normed, scaled and added by the kernel that norms the stream for the next one
     pib_sublayer_y leftn;
     auto sandwich = [&](const float * w, const float * b, const pib_hlayer * moe = nullptr, bool h16 = false) -> int {
-        h_bf16 = w && h16;
+        h_bf16 = w && h16 && x->h16;
         pib_norm_route nr;
         if (moe) { nr.rows = (const float *) moe->router->base; nr.R = router_of(*moe); nr.ids = x->ids; nr.wts = x->wts; nr.offs = x->offs; nr.perm = x->perm; nr.inv = x->inv; nr.act = x->act; nr.done = x->done; }
         RC(moe ? HK_NORM_ROUTE : HK_SANDWICH, moe ? mmfl(moe->router) : 0, (moe ? wbytes(moe->router) : 0.0) + 4.0 * Td * Wd * ((leftn.y ? 3.0 : leftn.top ? 2.0 : 1.0) + leftn.top + (w ? 1.0 : 0.0)), pib_sandwich_norm(x->x, leftn, w, b, eps, T, W, w ? (h_bf16 ? x->h16 : x->h) : nullptr, st, moe ? &nr : nullptr, h_bf16));

@@ -459,7 +459,7 @@ def test_short_portions_keep_fp32_attention(tmp_path, n):
 def test_identity_outputs_in_front_of_a_matmul_that_takes_bfloat16_rows(tmp_path, n):
     """served mode: every token's choice falls on the identity outputs only, so what a norm reads is the rows that the norm before left, while it writes the bfloat16 rows of the
     matmul behind it (an attention's, the output's); every row has to come out right, over many rounds of blocks.  No choice can turn, so no row may be far off"""
-    cfg = model(64, 140, [(slopes(2, 1, 8, 8, 3), moe(2, 4, 16, identity=4, scale=1.5, shared=24)), (slopes(1, 1, 8, 16, 2), moe(3, 2, 8, identity=2, scale=2.0))], mult=1.0)
+    cfg = model(64, 140, [(slopes(4, 1, 8, 8, 3), moe(2, 4, 16, identity=4, scale=1.5, shared=24)), (slopes(1, 1, 8, 16, 2), moe(3, 2, 8, identity=2, scale=2.0))], mult=1.0)
     W = O.random_weights(cfg, 51)
     for i, identity in enumerate([4, 2]):
         W["l%d.mlp.correction" % i][-identity:] = 64.0
