@@ -95,8 +95,7 @@ __device__ __forceinline__ int bk_sub8(uint32_t nib) { return (int) (((nib | 0x8
 // NT = token groups of 8 (1: b <= 8, 2: b <= 16).  The next record is prefetched into registers while the current one is
 // multiplied; partial sums of the warps are reduced through shared memory in warp order; with k splits the last CTA to
 // arrive adds the splits' partial sums in split order (deterministic), exactly as gemv_q4k_direct_kernel does.
-// ONE: one token, whose pieces lie at distances known beforehand (distances that follow from the number of tokens cost a record addresses of its own: Q4_0 57344 x 8192 52.0 / 49.4 us,
-// 12288 x 4096 9.2 / 9.0, Q8_0 57344 x 8192 73.7 / 72.3).
+// ONE: one token, whose pieces lie at distances known beforehand (Q4_0 57344 x 8192 52.9 / 50.9 us, 32000 x 4096 18.0 / 17.6; Q8_0 goes without: 32000 x 2048 11.8 / 13.7).
 template <int WT, int NT, bool ONE>
 __global__ void __launch_bounds__(BK_THREADS, NT == 1 ? 4 : 3)
 gemv_blk32_kernel(const uint8_t * __restrict__ tiles, int ngr, int N, const int8_t * __restrict__ aqs, const __half * __restrict__ adx,
@@ -130,7 +129,12 @@ gemv_blk32_kernel(const uint8_t * __restrict__ tiles, int ngr, int N, const int8
         gs[n] = ONE ? 1 : min(8, b - 8 * n);
         a_q[n] = aqs + (size_t) n * 8 * ngr * 256 + min(g, gs[n] - 1) * 64 + t * 16;
 #pragma unroll
-        for (int e = 0; e < 2; e++) a_d[n][e] = adx + ((size_t) n * 8 * ngr + min(2 * t + e, gs[n] - 1)) * 8;
+        for (int e = 0; e < 2; e++) {
+            a_d[n][e] = adx + ((size_t) n * 8 * ngr + min(2 * t + e, gs[n] - 1)) * 8;
+            // Two addresses of which nothing more is known: formed from one another, as neighbours allow, they cost up to 2.4 us a launch (at 2 tokens Q8_0 32000 x 2048 14.2 / 11.8,
+            // 32000 x 1536 12.1 / 9.9, Q4_0 57344 x 8192 54.3 / 52.9; found by trying, instructions and bytes are the same)
+            asm("" : "+l"(a_d[n][e]));
+        }
     }
 
     int4 wq[NQ], dq[2];
@@ -445,8 +449,7 @@ int pib_gemv_blk32(const pib_weight * w, const void * act_dev, int b, float * y_
         else if (b <= 8) e = pib_launch(gemv_blk32_kernel<PIB_TYPE_Q4_0, 1, false>, grid, dim3(BK_THREADS), 0, st, w->tiles, ngr, (int) w->N, aqs, adx, b, y_dev, pp, cc, cancel);
         else        e = pib_launch(gemv_blk32_kernel<PIB_TYPE_Q4_0, 2, false>, grid, dim3(BK_THREADS), 0, st, w->tiles, ngr, (int) w->N, aqs, adx, b, y_dev, pp, cc, cancel);
     } else {
-        if (b == 1) e = pib_launch(gemv_blk32_kernel<PIB_TYPE_Q8_0, 1, true>, grid, dim3(BK_THREADS), 0, st, w->tiles, ngr, (int) w->N, aqs, adx, b, y_dev, pp, cc, cancel);
-        else if (b <= 8) e = pib_launch(gemv_blk32_kernel<PIB_TYPE_Q8_0, 1, false>, grid, dim3(BK_THREADS), 0, st, w->tiles, ngr, (int) w->N, aqs, adx, b, y_dev, pp, cc, cancel);
+        if (b <= 8) e = pib_launch(gemv_blk32_kernel<PIB_TYPE_Q8_0, 1, false>, grid, dim3(BK_THREADS), 0, st, w->tiles, ngr, (int) w->N, aqs, adx, b, y_dev, pp, cc, cancel);
         else        e = pib_launch(gemv_blk32_kernel<PIB_TYPE_Q8_0, 2, false>, grid, dim3(BK_THREADS), 0, st, w->tiles, ngr, (int) w->N, aqs, adx, b, y_dev, pp, cc, cancel);
     }
     PIB_CHECK(e);
