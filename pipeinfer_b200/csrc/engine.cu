@@ -27,10 +27,10 @@ bool pib_gemv_pro_supported(const pib_weight * w, int b);
 int  pib_gemv_pro(const pib_weight * w, int pro, const float * x, const float * x2, const float * addend, float * sum_out, int64_t xstride, float eps,
                   int b, float * y, const int * cancel, cudaStream_t st);
 int  pib_silu_mul_quantize_act(int wtype, const float * gate_dev, const float * up_dev, int64_t row_stride, int b, int64_t K,
-                               void * act_dev, const int * cancel, cudaStream_t st, void * xhat = nullptr);
-int  pib_quantize_act_c(int wtype, const float * x_dev, int b, int64_t K, void * act_dev, const int * cancel, cudaStream_t st, void * xhat = nullptr);
+                               void * act_dev, const int * cancel, cudaStream_t st, void * xhat = nullptr, bool lean = false);
+int  pib_quantize_act_c(int wtype, const float * x_dev, int b, int64_t K, void * act_dev, const int * cancel, cudaStream_t st, void * xhat = nullptr, bool lean = false);
 int  pib_add_rmsnorm_quantize_act(int wtype, const float * x_dev, const float * addend_dev, float * sum_out_dev,
-                                  const float * norm_w_dev, float eps, int b, int64_t K, void * act_dev, const int * cancel, cudaStream_t st, void * xhat = nullptr);
+                                  const float * norm_w_dev, float eps, int b, int64_t K, void * act_dev, const int * cancel, cudaStream_t st, void * xhat = nullptr, bool lean = false);
 int  pib_add_layernorm_quantize_act(int wtype, const float * x_dev, const float * addend_dev, const float * addend2_dev,
                                     float * sum_out_dev, const float * norm_w_dev, const float * norm_b_dev, float eps, int b,
                                     int64_t K, void * act_dev, const int * cancel, cudaStream_t st);
@@ -471,6 +471,13 @@ pib_context * pib_context_new(pib_model * m, uint32_t n_ctx, int max_seq, pib_st
     c->runs.resize(64);
     for (int i = 0; i < (int) c->runs.size(); i++) c->runs[i].id = i;
     if (stage.size > 1 && pib_pipe_hop_setup(c) != PIB_OK) goto fail;
+    c->lean_act = m->arch == 0;
+    for (int il = m->layer_begin; il < m->layer_end; il++) {
+        const pib_layer & L = m->layers[il];
+        for (const pib_weight * w : { L.wqkv, L.wo, L.wgu, L.wdown }) c->lean_act = c->lean_act && w->type == m->wtype && w->tiles;
+        c->lean_act = c->lean_act && !L.wv;
+    }
+    if (m->output) c->lean_act = c->lean_act && m->output->type == m->wtype && m->output->tiles;
     return c;
 fail:
     pib_context_free(c);
@@ -691,6 +698,7 @@ static int run_chunk_body(pib_context * c, pib_run & run, int chunk, int ntok, i
         }
         return PIB_OK;
     }
+    const bool lean = c->lean_act && var == 0;
     // x holds layer_inp; `pending_add` = a down-projection result still to be added to x2 (ffn_inp) to form the next x
     bool pending_add = (part & 1) ? false : m->layer_end > m->layer_begin;
     for (int il = m->layer_begin; (part & 1) && il < m->layer_end; il++) {
@@ -714,16 +722,16 @@ static int run_chunk_body(pib_context * c, pib_run & run, int chunk, int ntok, i
             TL(7, il, pib_attention(c->qkv, nullptr, desc, c->rope, c->rope_n_pos, 0, c->kcache + lo, c->vcache + lo, c->mask, c->kvd.scalars, ntok,
                                     m->n_head, m->n_head_kv, hd, (int) c->n_ctx, c->att, cancel, st));
             GEMVP(1, L.wo, 0, c->att, nullptr, nullptr, nullptr, 0, 0.f, ntok, c->proj);
-            TL(9, il, pib_add_rmsnorm_quantize_act(wt, c->proj, c->x, c->x2, L.ffn_norm, m->rms_eps, ntok, E, c->act, cancel, st));   // x2 = ffn_inp
+            TL(9, il, pib_add_rmsnorm_quantize_act(wt, c->proj, c->x, c->x2, L.ffn_norm, m->rms_eps, ntok, E, c->act, cancel, st, nullptr, lean));   // x2 = ffn_inp
             GEMV(2, il, L.wgu, c->gu);
-            TL(10, il, pib_silu_mul_quantize_act(wt, c->gu, c->gu + FF, 2 * (int64_t) FF, ntok, FF, c->act, cancel, st));
+            TL(10, il, pib_silu_mul_quantize_act(wt, c->gu, c->gu + FF, 2 * (int64_t) FF, ntok, FF, c->act, cancel, st, nullptr, lean));
             GEMV(3, il, L.wdown, c->proj);
             pending_add = true;
             continue;
         }
 #undef GEMVP
-        if (pending_add) TL(5, il, pib_add_rmsnorm_quantize_act(wt, c->proj, c->x2, c->x, L.attn_norm, m->rms_eps, ntok, E, c->act, cancel, st));
-        else             TL(5, il, pib_add_rmsnorm_quantize_act(wt, c->x, nullptr, nullptr, L.attn_norm, m->rms_eps, ntok, E, c->act, cancel, st));
+        if (pending_add) TL(5, il, pib_add_rmsnorm_quantize_act(wt, c->proj, c->x2, c->x, L.attn_norm, m->rms_eps, ntok, E, c->act, cancel, st, nullptr, lean));
+        else             TL(5, il, pib_add_rmsnorm_quantize_act(wt, c->x, nullptr, nullptr, L.attn_norm, m->rms_eps, ntok, E, c->act, cancel, st, nullptr, lean));
         GEMV(0, il, L.wqkv, c->qkv);
         if (L.wv) GEMV(0, il, L.wv, c->vsep);
         dump_dev(c, "inp", il, c->x, ntok, E, E);
@@ -733,15 +741,15 @@ static int run_chunk_body(pib_context * c, pib_run & run, int chunk, int ntok, i
         TL(7, il, pib_attention(c->qkv, L.wv ? c->vsep : nullptr, desc, c->rope, c->rope_n_pos, 0, c->kcache + lo, c->vcache + lo, c->mask, c->kvd.scalars, ntok,
                                 m->n_head, m->n_head_kv, hd, (int) c->n_ctx, c->att, cancel, st));
         dump_dev(c, "att", il, c->att, ntok, E, E);
-        TL(8, il, pib_quantize_act_c(wt, c->att, ntok, E, c->act, cancel, st));
+        TL(8, il, pib_quantize_act_c(wt, c->att, ntok, E, c->act, cancel, st, nullptr, lean));
         GEMV(1, il, L.wo, c->proj);
         dump_dev(c, "o", il, c->proj, ntok, E, E);
-        TL(9, il, pib_add_rmsnorm_quantize_act(wt, c->proj, c->x, c->x2, L.ffn_norm, m->rms_eps, ntok, E, c->act, cancel, st));   // x2 = ffn_inp
+        TL(9, il, pib_add_rmsnorm_quantize_act(wt, c->proj, c->x, c->x2, L.ffn_norm, m->rms_eps, ntok, E, c->act, cancel, st, nullptr, lean));   // x2 = ffn_inp
         dump_dev(c, "ffi", il, c->x2, ntok, E, E);
         GEMV(2, il, L.wgu, c->gu);
         dump_dev(c, "gate", il, c->gu, ntok, FF, 2 * (size_t) FF);
         dump_dev(c, "up", il, c->gu + FF, ntok, FF, 2 * (size_t) FF);
-        TL(10, il, pib_silu_mul_quantize_act(wt, c->gu, c->gu + FF, 2 * (int64_t) FF, ntok, FF, c->act, cancel, st));
+        TL(10, il, pib_silu_mul_quantize_act(wt, c->gu, c->gu + FF, 2 * (int64_t) FF, ntok, FF, c->act, cancel, st, nullptr, lean));
         GEMV(3, il, L.wdown, c->proj);
         dump_dev(c, "down", il, c->proj, ntok, E, E);
         pending_add = true;
@@ -749,8 +757,8 @@ static int run_chunk_body(pib_context * c, pib_run & run, int chunk, int ntok, i
     if (c->stage.last() && !(part & 2)) return PIB_OK;
     if (!c->stage.last() && !(part & 1)) return PIB_OK;
     if (c->stage.last()) {
-        if (pending_add) RC(pib_add_rmsnorm_quantize_act(wt, c->proj, c->x2, c->x, m->output_norm, m->rms_eps, ntok, E, c->act, cancel, st));
-        else             RC(pib_add_rmsnorm_quantize_act(wt, c->x, nullptr, nullptr, m->output_norm, m->rms_eps, ntok, E, c->act, cancel, st));
+        if (pending_add) RC(pib_add_rmsnorm_quantize_act(wt, c->proj, c->x2, c->x, m->output_norm, m->rms_eps, ntok, E, c->act, cancel, st, nullptr, lean));
+        else             RC(pib_add_rmsnorm_quantize_act(wt, c->x, nullptr, nullptr, m->output_norm, m->rms_eps, ntok, E, c->act, cancel, st, nullptr, lean));
         float * lg = run.logits + (size_t) chunk * PIB_CHUNK * m->n_vocab;
         GEMV(4, c->prof_layer >= 0 ? c->prof_layer : -2, m->output, lg);
         RC(pib_sample_topk(lg, ntok, m->n_vocab, c->bias_ids_dev, c->bias_val_dev, c->n_bias, run.res_dev + (size_t) chunk * PIB_CHUNK,

@@ -137,6 +137,7 @@ struct pib_context {
                         int32_t * ids = nullptr;      // a pass's token ids | positions | cells [3][PIB_PROMPT_MAX], then sequence bitsets [PIB_PROMPT_MAX][n_words]
                       } pb;
     pib_prompt_plan prompt_plan;
+    bool     lean_act = false;             // all matrices are of one type and have tensor-core records: the quantiser writes only what their decode matmuls read
     int      fuse_pro = 0;                 // 1: small llama-arch Q4_K models run norm / quantise / silu inside the consuming GEMV (PIB_FUSE_PRO, engine.cu)
     int      prompt_gemm = 1;              // 0: prompts go through the GEMV kernels in chunks of 16 (PIB_PROMPT_GEMM=0, and always in exact mode)
 

@@ -498,7 +498,7 @@ extern "C" int pib_gemm_check(pib_stream s) { return pib_tc_check((cudaStream_t)
 // activation quantiser for any number of rows (pib_quantize_act is limited to verification batches)
 extern "C" int pib_quantize_act_rows(int wtype, const float * x_dev, int b, int64_t K, void * act_dev, pib_stream s);
 
-int pib_quantize_act_c(int wtype, const float * x_dev, int b, int64_t K, void * act_dev, const int * cancel, cudaStream_t st, void * xhat = nullptr);
+int pib_quantize_act_c(int wtype, const float * x_dev, int b, int64_t K, void * act_dev, const int * cancel, cudaStream_t st, void * xhat = nullptr, bool lean = false);
 
 // host-buffer convenience for the parity tests (like pib_mul_mat_host): x_host [b][K] fp32 -> y_host [b][N]
 extern "C" int pib_gemm_host(const pib_weight * w, const float * x_host, int b, float * y_host) {
