@@ -24,6 +24,8 @@
 // kernels implemented in the other translation units
 int  pib_gemv_internal(const pib_weight * w, const void * act_dev, int b, float * y_dev, int variant, const int * cancel, cudaStream_t st);
 bool pib_gemv_pro_supported(const pib_weight * w, int b);
+bool pib_gemv_gated_ok(const pib_weight * w, int b);
+int  pib_gemv_gated(const pib_weight * w, const void * act_dev, int b, float * y_dev, const int * cancel, cudaStream_t st);
 int  pib_gemv_pro(const pib_weight * w, int pro, const float * x, const float * x2, const float * addend, float * sum_out, int64_t xstride, float eps,
                   int b, float * y, const int * cancel, cudaStream_t st);
 int  pib_silu_mul_quantize_act(int wtype, const float * gate_dev, const float * up_dev, int64_t row_stride, int b, int64_t K,
@@ -601,9 +603,10 @@ int (*pib_hop_send)(pib_context * c, const float * x, int n_tokens, const int * 
 
 // debugging aid (PIB_DUMP_DIR=<dir>, graphs off): every intermediate of the llama graph goes to <dir>/<name>.<layer>.bin as float32,
 // under the names the oracle uses for the same tensors (PO_DUMP_DIR, oracle/pib_oracle.c), so the two can be compared step by step
+static const char * const dumps = getenv("PIB_DUMP_DIR");
 static void dump_dev(const pib_context * c, const char * name, int il, const float * dev, size_t rows, size_t cols, size_t ld) {
-    static const char * dir = getenv("PIB_DUMP_DIR");
-    if (!dir) return;
+    if (!dumps) return;
+    const char * dir = dumps;
     cudaStreamSynchronize(c->stream);
     std::vector<float> h(rows * cols);
     cudaMemcpy2D(h.data(), cols * 4, dev, ld * 4, cols * 4, rows, cudaMemcpyDeviceToHost);
@@ -746,10 +749,15 @@ static int run_chunk_body(pib_context * c, pib_run & run, int chunk, int ntok, i
         dump_dev(c, "o", il, c->proj, ntok, E, E);
         TL(9, il, pib_add_rmsnorm_quantize_act(wt, c->proj, c->x, c->x2, L.ffn_norm, m->rms_eps, ntok, E, c->act, cancel, st, nullptr, lean));   // x2 = ffn_inp
         dump_dev(c, "ffi", il, c->x2, ntok, E, E);
-        GEMV(2, il, L.wgu, c->gu);
-        dump_dev(c, "gate", il, c->gu, ntok, FF, 2 * (size_t) FF);
-        dump_dev(c, "up", il, c->gu + FF, ntok, FF, 2 * (size_t) FF);
-        TL(10, il, pib_silu_mul_quantize_act(wt, c->gu, c->gu + FF, 2 * (int64_t) FF, ntok, FF, c->act, cancel, st, nullptr, lean));
+        if (lean && !dumps && pib_gemv_gated_ok(L.wgu, ntok)) {
+            TL(2, il, pib_gemv_gated(L.wgu, c->act, ntok, c->gu, cancel, st));
+            TL(10, il, pib_quantize_act_c(wt, c->gu, ntok, FF, c->act, cancel, st, nullptr, lean));
+        } else {
+            GEMV(2, il, L.wgu, c->gu);
+            dump_dev(c, "gate", il, c->gu, ntok, FF, 2 * (size_t) FF);
+            dump_dev(c, "up", il, c->gu + FF, ntok, FF, 2 * (size_t) FF);
+            TL(10, il, pib_silu_mul_quantize_act(wt, c->gu, c->gu + FF, 2 * (int64_t) FF, ntok, FF, c->act, cancel, st, nullptr, lean));
+        }
         GEMV(3, il, L.wdown, c->proj);
         dump_dev(c, "down", il, c->proj, ntok, E, E);
         pending_add = true;

@@ -540,8 +540,11 @@ gemv_q4k_direct_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K
 // a chain of record latencies, and that chain is what the deeper prefetch shortens.  WARPS = warps per CTA (interleaving the
 // super-blocks of the tile): 8 for single-wave shapes, 4 otherwise.
 #define RG_STAGES 4
-template <int NT, int WARPS, int STAGES>
-__global__ void __launch_bounds__(WARPS * 32, NT == 1 ? (WARPS == 4 ? 5 : 2) : (WARPS == 4 ? 3 : 2))
+// GATED: rows of a gate and rows of its factor gridDim.x row tiles on, half of the warps each (in the order of the four-warp form); what is written is silu(gate) * factor, through
+// the reference's table (ggml.c:1490; in the place of the K shares' sums, of which there are none).  In the quantiser behind it the product's look-ups (32 places of the
+// table at once, while the next matmul's weights come) took 2 us of a draft step's layer: the step 681 -> 669 us.
+template <int NT, int WARPS, int STAGES, bool GATED = false>
+__global__ void __launch_bounds__(WARPS * 32, NT == 1 ? (WARPS == 4 ? 5 : GATED ? 3 : 2) : (WARPS == 4 ? 3 : 2))
 gemv_q4k_ring_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, const int8_t * __restrict__ aqs,
                      const float * __restrict__ ad, const int8_t * __restrict__ abs8, int b, float * __restrict__ y,
                      float * __restrict__ partial, unsigned int * __restrict__ counters, const int * __restrict__ cancel) {
@@ -556,12 +559,14 @@ gemv_q4k_ring_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, 
     const int nsplit = gridDim.y, split = blockIdx.y;
     const int sb_per = (nsb + nsplit - 1) / nsplit;
     const int sb0 = split * sb_per, sb1 = min(nsb, sb0 + sb_per);
-    const uint8_t * tbase = tiles + (size_t) T * nsb * MM_TILE_BYTES + lane * 16;
+    constexpr int SHARE = GATED ? WARPS / 2 : WARPS;            // warps that share a row tile
+    const int w1 = GATED ? warp % SHARE : warp;
+    const uint8_t * tbase = tiles + (size_t) (GATED && warp >= SHARE ? T + (int) gridDim.x : T) * nsb * MM_TILE_BYTES + lane * 16;
     uint8_t *       ring  = rg_smem + warp * (STAGES * MM_TILE_BYTES);
     const uint32_t  ring_a = smem_u32(ring) + lane * 16;
 
     // prefetch cursor: this warp's records sb0 + warp, + WARPS, ...
-    int ps = sb0 + warp;
+    int ps = sb0 + w1;
     auto issue = [&](int stage) {
         if (ps < sb1) {
             const uint8_t * src = tbase + (size_t) ps * MM_TILE_BYTES;
@@ -569,7 +574,7 @@ gemv_q4k_ring_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, 
 #pragma unroll
             for (int c = 0; c < 4; c++) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + c * 512), "l"(src + c * 512) : "memory");
             if (lane < 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 2048), "l"(src + 2048) : "memory");
-            ps += WARPS;
+            ps += SHARE;
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -595,7 +600,7 @@ gemv_q4k_ring_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, 
     pib_pdl_wait();
     pib_pdl_trigger();
     int stage = 0;
-    for (int s = sb0 + warp; s < sb1; s += WARPS) {
+    for (int s = sb0 + w1; s < sb1; s += SHARE) {
         __syncwarp();                                           // every lane has read the stage about to be refilled
         issue((stage + STAGES - 1) % STAGES);
         asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
@@ -633,7 +638,7 @@ gemv_q4k_ring_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, 
                 float u = red[4 % WARPS][tok][r];
 #pragma unroll
                 for (int w2 = 5; w2 < 8; w2++) u += red[w2 % WARPS][tok][r];
-                v += u;
+                v = GATED ? __fmul_rn(pib_h2f(reinterpret_cast<const uint16_t *>(partial)[pib_f2h(v)]), u) : v + u;
             }
             if (nsplit == 1) y[(size_t) tok * N + row] = v;
             else partial[((size_t) split * b + tok) * N + row] = v;
@@ -1060,22 +1065,27 @@ int pib_gemv_mma_launch(const pib_weight * w, const void * act_dev, int b, float
     return PIB_OK;
 }
 
-template <int NT, int WARPS, int STAGES>
+template <int NT, int WARPS, int STAGES, bool GATED = false>
 static int ring_launch(const pib_weight * w, const int8_t * aqs, const float * ad, const int8_t * bs, int b, float * y_dev, int split, float * partial,
                        unsigned int * counters, const int * cancel, cudaStream_t st) {
-    const int    nsb = (int) (w->K / 256), n_tiles = (int) ((w->N + 15) / 16);
+    const int    nsb = (int) (w->K / 256), N = (int) (GATED ? w->N / 2 : w->N), n_tiles = (N + 15) / 16;
     const size_t ring = (size_t) WARPS * STAGES * MM_TILE_BYTES, smem = WARPS == 8 ? pib_gemv_smem_spread(ring, n_tiles * split) : ring;
     static pib_per_device attrs;
-    PIB_CHECK(attrs.once([&] { return cudaFuncSetAttribute(gemv_q4k_ring_kernel<NT, WARPS, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) std::max(ring, (size_t) PIB_GEMV_SPREAD)); }));
-    pib_launch(gemv_q4k_ring_kernel<NT, WARPS, STAGES>, dim3(n_tiles, split), dim3(WARPS * 32), smem, st, w->tiles, nsb, (int) w->N, (int) w->K, aqs, ad, bs, b, y_dev,
-               partial, counters, cancel);
-    PIB_CHECK(cudaGetLastError());
+    PIB_CHECK(attrs.once([&] { return cudaFuncSetAttribute(gemv_q4k_ring_kernel<NT, WARPS, STAGES, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) std::max(ring, (size_t) PIB_GEMV_SPREAD)); }));
+    PIB_CHECK(pib_launch(gemv_q4k_ring_kernel<NT, WARPS, STAGES, GATED>, dim3(n_tiles, split), dim3(WARPS * 32), smem, st, w->tiles, nsb, N, (int) w->K, aqs, ad, bs, b, y_dev,
+                         partial, counters, cancel));
     return PIB_OK;
 }
 
 // Q3_K, Q5_K, Q6_K: eight warps per tile while two such CTAs per SM take all tiles at once; below 8 super-blocks a warp would go without a record (us behind a quantiser, four / eight
 // warps: Q6_K 4096 x 4096 at 4 tokens 6.3 / 5.9, at 12 8.8 / 7.7, 4096 x 11008 13.7 / 12.0 and 18.1 / 16.6; 8192 x 4096 9.6 / 10.3; Q3_K 4096 x 11008 12.8 / 10.2)
 bool pib_gemv_wide(const pib_weight * w) { return (w->N + 15) / 16 <= 2 * pib_num_sms() && w->K / 256 >= 8; }
+
+// eight warps per row tile: see pib_gemv_ring
+static bool ring_wide(int n_tiles, int nsb) {
+    static const int wide_on = getenv("PIB_RING_WIDE") ? atoi(getenv("PIB_RING_WIDE")) : 1;
+    return wide_on && n_tiles <= 2 * pib_num_sms() * 2 && (nsb >= 16 || (nsb >= 8 && n_tiles < pib_split_fill_target()));          // <= 2 CTAs of 8 warps per SM
+}
 
 // variant 0 / 2: the ring kernel (cp.async-staged); PIB_Q4K_FAST=direct selects the register-prefetched direct kernel instead
 int pib_gemv_ring(const pib_weight * w, const void * act_dev, int b, float * y_dev, const int * cancel, cudaStream_t st) {
@@ -1087,8 +1097,7 @@ int pib_gemv_ring(const pib_weight * w, const void * act_dev, int b, float * y_d
     // one wave of CTAs or less (4 CTAs of 4 warps per SM): eight warps per tile halve every warp's chain of records.  With 8 to 15 super-blocks they take the place of
     // K shares, which meet through memory (K = 2048, shares / eight warps, us: 2560 rows at 1 token 3.5 / 2.0, at 12 5.2 / 4.1; 4096 at 1 4.0 / 2.2); tiles enough to go
     // without shares keep four warps (8192 rows: 3.1 / 4.2)
-    static const int wide_on = getenv("PIB_RING_WIDE") ? atoi(getenv("PIB_RING_WIDE")) : 1;
-    const bool wide = wide_on && n_tiles <= 2 * pib_num_sms() * 2 && (nsb >= 16 || (nsb >= 8 && n_tiles < pib_split_fill_target()));          // <= 2 CTAs of 8 warps per SM
+    const bool wide = ring_wide(n_tiles, nsb);
     static const int split_env = getenv("PIB_RING_SPLIT") ? atoi(getenv("PIB_RING_SPLIT")) : 0;
     const int  split = fit_split(split_env > 0 ? split_env : wide ? 1 : choose_split_direct(n_tiles, nsb), b, w->N, n_tiles);
     mm_scratch * s = nullptr;
@@ -1102,6 +1111,22 @@ int pib_gemv_ring(const pib_weight * w, const void * act_dev, int b, float * y_d
     unsigned int * cc = s ? s->counters : nullptr;
     if (wide) return b <= 8 ? ring_launch<1, 8, 4>(w, aqs, ad, bs, b, y_dev, split, pp, cc, cancel, st) : ring_launch<2, 8, 4>(w, aqs, ad, bs, b, y_dev, split, pp, cc, cancel, st);
     return b <= 8 ? ring_launch<1, 4, 4>(w, aqs, ad, bs, b, y_dev, split, pp, cc, cancel, st) : ring_launch<2, 4, 4>(w, aqs, ad, bs, b, y_dev, split, pp, cc, cancel, st);
+}
+
+// gate and factor of a feed-forward (rows 0 .. N / 2 - 1 and N / 2 .. N - 1 of w) and their gated product [b][N / 2]: where the matmul has four warps per tile and no K shares
+bool pib_gemv_gated_ok(const pib_weight * w, int b) {
+    if (!pib_gemv_mma_supported(w, b) || w->N % 32) return false;
+    const int nsb = (int) (w->K / 256), n_tiles = (int) (w->N / 16);
+    return !ring_wide(n_tiles, nsb) && choose_split_direct(n_tiles, nsb) == 1;
+}
+int pib_gemv_gated(const pib_weight * w, const void * act_dev, int b, float * y_dev, const int * cancel, cudaStream_t st) {
+    if (!pib_gemv_gated_ok(w, b)) { pib_set_error("pib_gemv_gated: not for this matrix"); return PIB_ERR_UNSUPP; }
+    const pib_act_layout L   = pib_act_layout_of(w->type, w->K, b);
+    const uint8_t *      act = (const uint8_t *) act_dev;
+    const int8_t * aqs = (const int8_t *) (act + L.qsp_off), * bs = (const int8_t *) (act + L.bs8_off);
+    const float *  ad  = (const float *) (act + L.dxo_off);
+    float *        lut = (float *) const_cast<uint16_t *>(pib_get_luts().silu_f16);
+    return b <= 8 ? ring_launch<1, 8, 4, true>(w, aqs, ad, bs, b, y_dev, 1, lut, nullptr, cancel, st) : ring_launch<2, 8, 4, true>(w, aqs, ad, bs, b, y_dev, 1, lut, nullptr, cancel, st);
 }
 
 // variant 8: the balanced stream kernel

@@ -1,5 +1,5 @@
 """The activation quantiser's forms (csrc/act_quant.cu) at the edges of how rows are divided (a warp per 256 values, 32 warps per row, blocks of 8 that share a normed row), with operands
-on any address, bit for bit against the oracle's quantiser; the planes of the lean form against the general ones, bit for bit."""
+on any address, bit for bit against the oracle's quantiser; the planes of the lean form and the gated matmul (csrc/gemv_mma.cu) against the general ones, bit for bit."""
 import ctypes as C
 import ctypes.util
 import subprocess
@@ -14,7 +14,8 @@ pytestmark = pytest.mark.gpu
 Q4_0, Q8_0, Q4_K = op.TYPE_Q4_0, op.TYPE_Q8_0, op.TYPE_Q4_K
 V, I, F, L64 = C.c_void_p, C.c_int, C.c_float, C.c_int64
 ARGS = {"pib_quantize_act_c": [I, V, I, L64, V, V, V, V, C.c_bool], "pib_silu_mul_quantize_act": [I, V, V, L64, I, L64, V, V, V, V, C.c_bool], "pib_gelu_quantize_act": [I, V, I, L64, V, V, V],
-        "pib_add_rmsnorm_quantize_act": [I, V, V, V, V, F, I, L64, V, V, V, V, C.c_bool], "pib_add_layernorm_quantize_act": [I, V, V, V, V, V, V, F, I, L64, V, V, V]}
+        "pib_add_rmsnorm_quantize_act": [I, V, V, V, V, F, I, L64, V, V, V, V, C.c_bool], "pib_add_layernorm_quantize_act": [I, V, V, V, V, V, V, F, I, L64, V, V, V],
+        "pib_gemv_gated": [V, V, I, V, V, V], "pib_gemv_gated_ok": [V, I]}
 
 
 @pytest.fixture(scope="module")
@@ -27,6 +28,7 @@ def lib():
     for n, args in ARGS.items():
         L.f[n] = getattr(L.L, next(s for s in names if s.startswith("_Z%d%s" % (len(n), n))))
         L.f[n].argtypes = args
+    L.f["pib_gemv_gated_ok"].restype = C.c_bool
     return L
 
 
@@ -140,3 +142,21 @@ def test_lean_planes(lib, wt, b):
     lib.L.pib_weight_free(w)
     B.free()
     assert np.array_equal(*out) and np.abs(out[0]).sum() > 0
+
+
+@pytest.mark.parametrize("N,K", [(32, 256), (96, 1024), (7584, 2048), (9504, 4096)])
+@pytest.mark.parametrize("b", [1, 3, 8, 9, 16])
+def test_gated_matmul(lib, tables, N, K, b):
+    rng = np.random.default_rng(N + b)
+    B = Buffers(lib, 0)
+    w = lib.weight_upload(Q4_K, rand_q4k(rng, N, K), K)
+    x, act = B.put(rng.standard_normal((b, K)) * 0.3), B.act(Q4_K, b, K)
+    y, h = B.put(np.zeros((b, N))), B.put(np.full((b, N // 2), np.nan))
+    lib.check(lib.L.pib_quantize_act(Q4_K, x, b, K, act, None))
+    lib.check(lib.L.pib_gemv(w, act, b, y, 0, None))
+    assert lib.f["pib_gemv_gated_ok"](w, b)
+    lib.check(lib.f["pib_gemv_gated"](w, act, b, h, None, None))
+    gu, got = lib.to_host(y, (b, N), np.float32), lib.to_host(h, (b, N // 2), np.float32)
+    lib.L.pib_weight_free(w)
+    B.free()
+    assert np.array_equal(got, look(tables[0], gu[:, :N // 2]) * gu[:, N // 2:])
