@@ -176,7 +176,7 @@ static dt_encode_fn dt_encode() {
 }
 
 // per (device, stream): the bfloat16 staging of the activations and the error word of the kernels' bounded waits
-struct dt_scratch { __nv_bfloat16 * xs = nullptr; size_t cap = 0; int * err = nullptr; int * err_host = nullptr; };
+struct dt_scratch { __nv_bfloat16 * xs = nullptr; size_t cap = 0; int * err = nullptr; int * err_host = nullptr; uint64_t uses = 0; };     // uses: launches that got the error word
 static dt_scratch * dt_scratch_of(cudaStream_t st, size_t bytes) {
     static std::map<std::pair<int, cudaStream_t>, dt_scratch> all;
     static std::mutex mu;
@@ -210,7 +210,8 @@ int pib_tma_map3(CUtensorMap * map, const void * base, uint64_t d0, uint64_t d1,
     return PIB_OK;
 }
 
-int * pib_tc_error_word(cudaStream_t st) { dt_scratch * sc = dt_scratch_of(st, 0); return sc ? sc->err : nullptr; }
+int * pib_tc_error_word(cudaStream_t st) { dt_scratch * sc = dt_scratch_of(st, 0); if (sc) sc->uses++; return sc ? sc->err : nullptr; }
+uint64_t pib_tc_uses(cudaStream_t st) { dt_scratch * sc = dt_scratch_of(st, 0); return sc ? sc->uses : 0; }
 
 template <int NB>
 static int dt_launch(const pib_mm & a, const CUtensorMap & wmap, const CUtensorMap & xmap, int x_has_z, int * err, cudaStream_t st) {
@@ -287,6 +288,7 @@ int pib_dense_mm_tc(const pib_mm & a, cudaStream_t st) {
     if (rc == PIB_OK && a.x_bf16) rc = pib_tma_map3(&xmap, a.X, (uint64_t) a.K, (uint64_t) a.M, (uint64_t) a.Z, (uint64_t) a.ldx * 2, (uint64_t) (a.Z > 1 ? a.xz : (int64_t) a.M * a.ldx) * 2, xbox);
     else if (rc == PIB_OK) rc = pib_tma_map3(&xmap, sc->xs, (uint64_t) Kp, (uint64_t) a.M, (uint64_t) Zs, (uint64_t) Kp * 2, (uint64_t) a.M * Kp * 2, xbox);
     if (rc != PIB_OK) return rc;
+    sc->uses++;
     if (pair) return pib_dense_pair(a, wmap, xmap, pair, shares, sc->err, st);
     switch (NB) {
         case 32:  return dt_launch<32>(a, wmap, xmap, grouped ? 0 : 1, sc->err, st);

@@ -547,6 +547,7 @@ void pib_context_free(pib_context * c) {
         if (r.res_host) cudaFreeHost(r.res_host);
         if (r.acc_dev) cudaFree(r.acc_dev);
         if (r.acc_host) cudaFreeHost(r.acc_host);
+        if (r.pin) cudaFreeHost(r.pin);
     }
     for (auto e : c->desc_ev) if (e) cudaEventDestroy(e);
     if (c->cancel_ev) cudaEventDestroy(c->cancel_ev);
@@ -973,6 +974,9 @@ pib_run * pib_take_run(pib_context * c, int n_tokens) {
     for (auto & r : c->runs) {
         if (r.in_use || r.id == c->last_finished) continue;
         r.want_lo = r.want_hi = 0;
+        r.marks.swap(c->marks_next);
+        c->marks_next.clear();
+        r.pinned = false;
         if (!r.done) cudaEventCreateWithFlags(&r.done, cudaEventDisableTiming);
         if (!r.acc_host && ((!r.acc_dev && cudaMalloc(&r.acc_dev, sizeof(pib_accept_result)) != cudaSuccess) ||
                             cudaMallocHost(&r.acc_host, sizeof(pib_accept_result) + sizeof(int)) != cudaSuccess)) {
@@ -1083,7 +1087,7 @@ int pib_decode_start(pib_context * c, int n_tokens, const int32_t * token, const
 }
 
 // ship the queued device-level op-log to the GPU and replay it on the KV replica
-int pib_apply_devops(pib_context * c) {
+int pib_apply_devops(pib_context * c, int run_slot) {
     std::vector<KvOp> & dq = devq(c);
     const int n = (int) dq.size();
     if (n == 0) return PIB_OK;
@@ -1094,7 +1098,7 @@ int pib_apply_devops(pib_context * c) {
         if (c->ops_host[c->ops_next + i].op == KVOP_ALLOC) c->ops_host[c->ops_next + i].p1 = dev_slot(c, c->ops_host[c->ops_next + i].p1);
     cudaMemcpyAsync(c->ops_dev + c->ops_next, c->ops_host + c->ops_next, sizeof(KvOp) * n, cudaMemcpyHostToDevice, c->stream);
     c->h2d_bytes += sizeof(KvOp) * n;
-    if (kv_device_apply(&c->kvd, c->ops_dev + c->ops_next, n, c->desc_dev, c->desc_stride, c->stream) != PIB_OK) return PIB_ERR_CUDA;
+    if (kv_device_apply(&c->kvd, c->ops_dev + c->ops_next, n, c->desc_dev, c->desc_stride, run_slot >= 0 ? c->cancel_table : nullptr, run_slot, c->stream) != PIB_OK) return PIB_ERR_CUDA;
     c->n_kernels++;
     c->ops_next += n;
     dq.clear();
@@ -1116,10 +1120,11 @@ int pib_kv_sync_replicas(pib_context * c) {
 static int enqueue_decode(pib_context * c, pib_run * run, int n_tokens, int batch_id, const std::vector<int> & slots) {
     const int n_chunks = (int) slots.size();
     int64_t t_mark = slow_trace() ? now_us() : 0;
-    if (pib_apply_devops(c) != PIB_OK) return -1;
+    const bool ops = !devq(c).empty();
+    if (pib_apply_devops(c, run->id) != PIB_OK) return -1;
     SLOW_MARK("  apply ops");
     run->in_use = true; run->batch_id = batch_id; run->n_tokens = n_tokens; run->failed = false; run->tc_used = false;
-    cudaMemcpyAsync(c->cancel_table, c->run_id_host + run->id, sizeof(int), cudaMemcpyHostToDevice, c->stream);   // "this run executes now"
+    if (!ops) cudaMemcpyAsync(c->cancel_table, c->run_id_host + run->id, sizeof(int), cudaMemcpyHostToDevice, c->stream);   // "this run executes now": with ops their kernel has written it
     if (prompt_gemm_ok(c, n_tokens) && prompt_bufs(c, n_tokens) == PIB_OK) {
         const int pass = c->stage.size > 1 ? PIB_PROMPT_STAGE : c->prompt_plan.cap, per = pass / PIB_CHUNK;
         for (int ch0 = 0; ch0 < n_chunks && !run->failed; ch0 += per) {
@@ -1149,6 +1154,7 @@ static int enqueue_decode(pib_context * c, pib_run * run, int n_tokens, int batc
                 c->d2h_bytes += sizeof(pib_row_result) * (size_t) n_tokens;
                 run->rows_on_host = true;
             }
+            pib_logits_prefetch(c, *run);
         }
     }
     cudaEventRecord(run->done, c->stream);
@@ -1196,7 +1202,10 @@ int pib_decode_replay(pib_context * c, int batch_id, int n_tokens, int n_chunks,
 
 // Clear a run slot's cancel flag in stream order after the run's last kernel -- and after any cancel write still travelling on the
 // control stream: without the event a late cancel copy could land after the clear and poison the slot's next run.
+// A run that nobody cancelled has none (the memset is a command of the host and of the stream in every step).
 static void clear_cancel_flag(pib_context * c, int slot) {
+    if (!c->runs[slot].cancel_sent) return;
+    c->runs[slot].cancel_sent = false;
     if (c->cancel_ev_pending) { cudaStreamWaitEvent(c->stream, c->cancel_ev, 0); c->cancel_ev_pending = false; }
     cudaMemsetAsync(c->cancel_table + 1 + slot, 0, sizeof(int), c->stream);
 }
@@ -1230,7 +1239,12 @@ int pib_run_finish(pib_context * c, int run) {
     if (r.tc_used && pib_tc_error(*r.tc_err) != PIB_OK) r.failed = true;
     if (c->stage.size > 1 && c->stage.first() && pib_pipe_take_failure(r.batch_id)) { pib_set_error("finish: a kernel of another stage gave up on a barrier wait (batch %d)", r.batch_id); r.failed = true; }
     r.in_use         = false;
+    if (c->last_finished >= 0 && c->runs[c->last_finished].pinned && !c->runs[c->last_finished].pin_read) {           // rows that crossed and nobody read
+        c->d2h_bytes += c->runs[c->last_finished].marks.size() * c->model->n_vocab * 4;
+        c->runs[c->last_finished].pin_read = true;
+    }
     c->last_finished = run;     // its buffers stay reserved until the next finish (llama_get_logits_ith contract)
+    c->rows_asked    = false;
     c->logits_row_valid.assign((size_t) r.n_tokens, 0);
     return r.failed ? -1 : 0;
 }
@@ -1254,12 +1268,45 @@ const pib_accept_result * pib_last_accept(pib_context * c) {
     return c->runs[c->last_finished].acc_host;
 }
 
+// the marked rows' copies to the run's page-locked memory; false: no memory there (or more rows than a decode batch has)
+static bool pin_rows(pib_context * c, pib_run & r) {
+    if (r.marks.empty() || r.marks.back() >= r.n_tokens || !r.logits) return false;
+    const size_t V = (size_t) c->model->n_vocab, n = r.marks.size() * V;
+    if (r.pin_cap < n) {
+        if (!r.pin && c->n_pins >= PIB_PINS) return false;
+        if (r.pin) { cudaFreeHost(r.pin); c->n_pins--; }
+        r.pin = nullptr; r.pin_cap = 0;
+        if (cudaMallocHost(&r.pin, n * 4) != cudaSuccess) { cudaGetLastError(); r.pin = nullptr; return false; }
+        r.pin_cap = n;
+        c->n_pins++;
+    }
+    for (size_t a = 0, b; a < r.marks.size(); a = b) {                // neighbouring rows in one copy
+        for (b = a + 1; b < r.marks.size() && r.marks[b] == r.marks[b - 1] + 1; b++) {}
+        if (cudaMemcpyAsync(r.pin + a * V, r.logits + (size_t) r.marks[a] * V, (b - a) * V * 4, cudaMemcpyDeviceToHost, c->stream) != cudaSuccess) { cudaGetLastError(); return false; }
+    }
+    r.pin_read = false;
+    return r.pinned = true;
+}
+// A program that reads a run's rows of logits reads the next run's, too: they cross behind its kernels, and are there when it is finished (a copy asked for then takes 10 .. 25 us of
+// waiting).  A program that reads none pays for none.
+void pib_logits_prefetch(pib_context * c, pib_run & r) { if (c->rows_asked && c->stage.size == 1) pin_rows(c, r); }
+
 const float * pib_logits_row(pib_context * c, int i) {
     if (c->last_finished < 0) return nullptr;
     pib_run & r = c->runs[c->last_finished];
     const bool remote = !r.logits && c->stage.size > 1 && c->stage.first();       // the rows live on the last pipeline stage
     if (i < 0 || i >= r.n_tokens || (!r.logits && !remote)) return nullptr;
     const size_t V = (size_t) c->model->n_vocab;
+    c->rows_asked = true;
+    const auto mark = std::lower_bound(r.marks.begin(), r.marks.end(), i);
+    if (!remote && mark != r.marks.end() && *mark == i) {
+        if (!r.pinned && pin_rows(c, r)) cudaStreamSynchronize(c->stream);
+        if (r.pinned) {
+            if (!r.pin_read) c->d2h_bytes += r.marks.size() * V * 4;
+            r.pin_read = true;
+            return r.pin + (size_t) (mark - r.marks.begin()) * V;
+        }
+    }
     if (!remote && r.n_tokens <= PIB_CHUNK) {
         // A decode or verification batch: the rows marked in it cross together into page-locked memory on the first one asked for.  A copy of one row into pageable
         // memory takes 23 us at 8 000 values and 50 at 32 000, nearly all of it latency, and a sampler wants every row it marked.  Any other row crosses alone.
@@ -1306,6 +1353,7 @@ void pib_cancel(pib_context * c, const int32_t * batch_ids, int n) {
             pib_run & r = c->runs[id];
             if (r.in_use && r.batch_id == batch_ids[i]) {
                 cudaMemcpyAsync(c->cancel_table + 1 + r.id, c->cancel_one, sizeof(int), cudaMemcpyDeviceToDevice, c->ctrl);
+                r.cancel_sent = true;
                 wrote = true;
             }
         }

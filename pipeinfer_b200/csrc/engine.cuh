@@ -76,6 +76,7 @@ struct pib_model {
     int n_embd_gqa() const { return head_dim() * n_head_kv; }
 };
 
+#define PIB_PINS 4
 struct pib_run {                   // one (possibly still executing) decode: the opaque handle of the async API
     int          id        = -1;   // index in the context's run table
     bool         in_use    = false;
@@ -90,6 +91,11 @@ struct pib_run {                   // one (possibly still executing) decode: the
     bool         has_walk  = false;       // the batch came with an acceptance table: only the walk's result crosses to the host
     bool         rows_on_host = false;
     int          want_lo = 0, want_hi = 0;   // logits rows that the caller marked in its batch: [want_lo, want_hi) holds all of them
+    std::vector<int> marks;                  // rows that cross together, in order: of a batch of up to PIB_CHUNK tokens [want_lo, want_hi), of a longer one the marked rows while no more than PIB_CHUNK
+    float *      pin = nullptr;              // page-locked [marks][n_vocab], pin_cap floats: their copies once `pinned`
+    size_t       pin_cap = 0;
+    bool         pinned = false, pin_read = false;       // pin_read: some of them were asked for (their bytes are counted then, or when the run is let go)
+    bool         cancel_sent = false;        // a cancel flag was written for this run: to be cleared when it is finished
     pib_accept_result * acc_dev = nullptr, * acc_host = nullptr;
     int *        tc_err    = nullptr;     // pinned, behind acc_host: the stream's error word behind this run's kernels (pib_tc_error_take)
     bool         tc_used   = false;       // the run launched kernels that set it
@@ -168,6 +174,9 @@ struct pib_context {
     float *              logits_pin = nullptr;      // the same for runs of up to PIB_CHUNK tokens: page-locked, the marked rows in one copy
     size_t               logits_pin_cap = 0;        // floats
     std::vector<uint8_t> logits_row_valid;
+    std::vector<int>     marks_next;              // marked rows of the decode that is about to be started
+    bool                 rows_asked = false;      // the run finished last was asked for rows of logits: the next one's cross behind its kernels
+    int                  n_pins = 0;              // runs that have page-locked rows, PIB_PINS at most
     bool                 logits_all = true;
     uint64_t             n_kernels = 0;   // launches issued by this context (bench: gpu_launches)
     uint64_t             h2d_bytes = 0, d2h_bytes = 0;     // host<->device traffic issued by this context
@@ -178,7 +187,7 @@ struct pib_context {
     std::vector<ProfRec> prof;
     uint64_t             n_decode  = 0;
     // CUDA graphs of the layer part of single-chunk decodes, keyed by n_tokens (engine.cu: run_chunk)
-    struct GraphEntry { cudaGraphExec_t exec = nullptr; int uses = 0; int n_kernels = 0; bool failed = false; };
+    struct GraphEntry { cudaGraphExec_t exec = nullptr; int uses = 0; int n_kernels = 0; bool failed = false; bool tc = false; };     // tc: holds kernels with bounded waits
     std::map<int, GraphEntry> graphs;
     bool                 use_graphs = true;
     uint64_t             n_graph_launches = 0;
@@ -209,7 +218,8 @@ void pib_cancel(pib_context * c, const int32_t * batch_ids, int n);
 int  pib_decode_replay(pib_context * c, int batch_id, int n_tokens, int n_chunks, const uint8_t * descs, size_t desc_stride,
                        const KvOp * ops, int n_ops);
 void pib_stage_finish(pib_context * c, int batch_id);
-int  pib_apply_devops(pib_context * c);
+int  pib_apply_devops(pib_context * c, int run_slot = -1);      // run_slot >= 0: the run that follows (PIB_CANCELLED)
+void pib_logits_prefetch(pib_context * c, pib_run & r);          // in stream order behind a run's kernels
 int  pib_kv_sync_replicas(pib_context * c);
 
 // pipeline.cu

@@ -684,7 +684,7 @@ static int run_layers(pib_context * c, pib_run & run, const pib_hbatch & B, cons
         return PIB_OK;
     };
 
-    RC(HK_CELLMAP, 0, 16.0 * Td, pib_cellmap_set(x->cellmap, (int) c->n_ctx, B, st));
+    RC(HK_CELLMAP, 0, 16.0 * Td, pib_cellmap_set(x->cellmap, (int) c->n_ctx, B, c->cancel_table, run.id, st));
     if (hy->form == PIB_FORM_HYPER)        RC(HK_EMBSCALE, 0, (2.0 + 4.0 * hy->streams) * Td * Wd, pib_embed_scale(m->tok_embd, B.tok, hy->embd_scale, T, W, x->x, st, hy->streams));
     else if (hy->form == PIB_FORM_PARALLEL || hy->form == PIB_FORM_GATED || hy->form == PIB_FORM_SANDWICH) RC(HK_EMBSCALE, 0, 6.0 * Td * Wd, pib_embed_scale(m->tok_embd, B.tok, hy->embd_scale, T, W, x->x, st));
     else if (hy->form == PIB_FORM_PRENORM) RC(HK_EMBPAIR, 0, (hy->loops ? 10.0 : 6.0) * Td * Wd, pib_embed_pair(m->tok_embd, B.tok, T, W, x->x, hy->loops ? x->cat : nullptr, st));
@@ -941,9 +941,8 @@ int pib_hybrid_decode_start(pib_context * c, int n_tokens, const int32_t * token
     c->h2d_bytes += (size_t) words * 4;
     const int32_t * md = x->meta_dev;
     pib_hbatch B = { md, md + T, md + 2 * T, md + 3 * T, md + 4 * T, md + 5 * T, md + 6 * T, md + 6 * T + S, md + 6 * T + 2 * S, T, S };
-    run->in_use = true; run->batch_id = batch_id; run->n_tokens = T; run->failed = false; run->has_walk = false;
+    run->in_use = true; run->batch_id = batch_id; run->n_tokens = T; run->failed = false; run->has_walk = false; run->tc_used = false;
     c->tree_pending.n_branches = 0;
-    cudaMemcpyAsync(c->cancel_table, c->run_id_host + run->id, sizeof(int), cudaMemcpyHostToDevice, st);
     // decode steps (few tokens) are launch-bound: like the other architectures' single-chunk decodes they replay a CUDA graph, captured on
     // the second use of its shape.  Every address a kernel gets is fixed for a given (tokens, segments, run slot); what varies between
     // steps (tokens, positions, cells, slots) lives in the bookkeeping block on the device.
@@ -952,7 +951,7 @@ int pib_hybrid_decode_start(pib_context * c, int n_tokens, const int32_t * token
         pib_context::GraphEntry & g = c->graphs[(T << 16) | (S << 8) | run->id];
         g.uses++;
         if (!g.exec && !g.failed && g.uses >= 2) {
-            const uint64_t k0 = c->n_kernels;
+            const uint64_t k0 = c->n_kernels, tc0 = pib_tc_uses(st);
             cudaGraph_t graph = nullptr;
             bool ok = cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed) == cudaSuccess;
             if (ok) {
@@ -962,6 +961,7 @@ int pib_hybrid_decode_start(pib_context * c, int n_tokens, const int32_t * token
             if (ok) ok = cudaGraphInstantiate(&g.exec, graph, 0) == cudaSuccess;
             if (graph) cudaGraphDestroy(graph);
             g.n_kernels = (int) (c->n_kernels - k0);
+            g.tc        = pib_tc_uses(st) != tc0;
             c->n_kernels = k0;
             if (!ok) { cudaGetLastError(); g.exec = nullptr; g.failed = true; }
         }
@@ -969,21 +969,26 @@ int pib_hybrid_decode_start(pib_context * c, int n_tokens, const int32_t * token
             if (cudaGraphLaunch(g.exec, st) != cudaSuccess) { pib_set_error("decode: graph launch failed: %s", cudaGetErrorString(cudaGetLastError())); run->failed = true; }
             c->n_kernels += (uint64_t) g.n_kernels;
             c->n_graph_launches++;
+            run->tc_used = g.tc;
             done = true;
         }
     }
     if (!done) {
         // event-timed launches run in plain stream order: with programmatic dependent launch a kernel starts before the event in front of it fires
         if (c->prof_layer >= 0) pib_pdl_suspend(true);
+        const uint64_t tc0 = pib_tc_uses(st);
         if (run_layers(c, *run, B, pos, segs) != PIB_OK) run->failed = true;
+        run->tc_used = pib_tc_uses(st) != tc0;
         if (c->prof_layer >= 0) pib_pdl_suspend(false);
     }
     if (!run->failed) {
         cudaMemcpyAsync(run->res_host, run->res_dev, sizeof(pib_row_result) * (size_t) T, cudaMemcpyDeviceToHost, st);
         c->d2h_bytes += sizeof(pib_row_result) * (size_t) T;
         run->rows_on_host = true;
+        pib_logits_prefetch(c, *run);
     }
-    if ((run->tc_used = hy->dtype == PIB_TYPE_BF16) && pib_tc_error_take(st, run->tc_err, true) != PIB_OK) run->failed = true;
+    // the error word of bounded waits: where a kernel that has them was launched (not in a step of few tokens)
+    if (run->tc_used && pib_tc_error_take(st, run->tc_err, true) != PIB_OK) run->failed = true;
     cudaEventRecord(run->done, st);
     c->inflight.push_back(run->id);
     c->n_decode++;

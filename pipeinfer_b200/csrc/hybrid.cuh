@@ -276,6 +276,7 @@ int pib_dense_mm_pair(const pib_mm & a, const pib_mm & b, cudaStream_t st);   //
 int pib_dense_mm_experts(const pib_mm & routed, const pib_mm & shared, cudaStream_t st);   // a grouped matmul and a plain one with the same epilogue; in decode steps one launch
 // dense_mma.cu: the error word of a stream, which a tensor-core kernel sets when one of its bounded waits runs out
 int * pib_tc_error_word(cudaStream_t st);                 // device word; null: no memory for it
+uint64_t pib_tc_uses(cudaStream_t st);                    // launches of this stream so far that got it
 int pib_tc_error_take(cudaStream_t st, int * host, bool clear);      // copies it to page-locked memory, and clears it, in stream order
 int pib_tc_error(int word);                               // a copied word as a status
 int pib_tc_check(cudaStream_t st);                        // waits for the stream; the status since the last check
@@ -318,7 +319,7 @@ int pib_moe_route_sort(const float * logits, int T, const pib_router & r, int32_
                        cudaStream_t st);   // both steps of a small batch in one launch; act = [how many experts have pairs | which]
 int pib_moe_sort(const int32_t * ids, int n_pairs, int E, int32_t * counts, int32_t * offs, int32_t * perm, int32_t * inv, cudaStream_t st);
 int pib_moe_combine(const float * shared, const float * edn, const float * wts, const int32_t * inv, int T, int top, int W, float * y, cudaStream_t st);
-int pib_cellmap_set(int32_t * cellmap, int n_ctx, const pib_hbatch & b, cudaStream_t st);
+int pib_cellmap_set(int32_t * cellmap, int n_ctx, const pib_hbatch & b, int * current, int run_slot, cudaStream_t st);
 
 // mixer_kernels.cu
 int pib_embed_scale(const pib_weight * embd, const int32_t * tok, float scale, int T, int W, float * x, cudaStream_t st, int copies = 1);

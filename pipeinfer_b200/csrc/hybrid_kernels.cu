@@ -202,14 +202,15 @@ int pib_canon_conv(const float * x, const float * w, int taps, const pib_hbatch 
 
 // ---- position -> cell table of each state slot -----------------------------------------------------------------------------------
 __global__ void cellmap_kernel(int32_t * __restrict__ cellmap, int n_ctx, const int32_t * __restrict__ pos, const int32_t * __restrict__ cell,
-                               const int32_t * __restrict__ slot, int T) {
+                               const int32_t * __restrict__ slot, int T, int * __restrict__ current, int run_slot) {
     pib_pdl_wait();
     pib_pdl_trigger();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t == 0) *current = run_slot;                        // "this run executes now" (PIB_CANCELLED)
     if (t < T) cellmap[(size_t) slot[t] * n_ctx + pos[t]] = cell[t];
 }
-int pib_cellmap_set(int32_t * cellmap, int n_ctx, const pib_hbatch & b, cudaStream_t st) {
-    pib_launch(cellmap_kernel, dim3((b.T + 255) / 256), dim3(256), (size_t) (0), st, cellmap, n_ctx, b.pos, b.cell, b.slot, b.T);
+int pib_cellmap_set(int32_t * cellmap, int n_ctx, const pib_hbatch & b, int * current, int run_slot, cudaStream_t st) {
+    pib_launch(cellmap_kernel, dim3((b.T + 255) / 256), dim3(256), (size_t) (0), st, cellmap, n_ctx, b.pos, b.cell, b.slot, b.T, current, run_slot);
     CKL();
     return PIB_OK;
 }

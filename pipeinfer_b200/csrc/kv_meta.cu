@@ -260,12 +260,12 @@ __device__ __forceinline__ void dev_range(uint32_t * r, int W, int first, int la
 __global__ void __launch_bounds__(KVT) kv_apply_kernel(int32_t * __restrict__ pos, uint32_t * __restrict__ bits,
                                                        int32_t * __restrict__ scalars, int size, int W,
                                                        const KvOp * __restrict__ ops, int n_ops,
-                                                       const uint8_t * __restrict__ desc_base, size_t desc_stride) {
+                                                       const uint8_t * __restrict__ desc_base, size_t desc_stride, int * __restrict__ current, int run_slot) {
     __shared__ int s_min[KVT / 32];
     __shared__ int s_cnt[KVT / 32];
     __shared__ int s_head, s_used, s_n;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) { s_head = scalars[0]; s_used = scalars[1]; s_n = scalars[2]; }
+    if (tid == 0) { s_head = scalars[0]; s_used = scalars[1]; s_n = scalars[2]; if (current) *current = run_slot; }
     __syncthreads();
     for (int k = 0; k < n_ops; k++) {
         const KvOp op       = ops[k];
@@ -413,10 +413,10 @@ void kv_device_free(KvDevice * kv) {
 }
 
 int kv_device_apply(const KvDevice * kv, const KvOp * ops_dev, int n_ops, const uint8_t * desc_base, size_t desc_stride,
-                    cudaStream_t st) {
+                    int * current, int run_slot, cudaStream_t st) {
     if (n_ops <= 0) return PIB_OK;
     kv_apply_kernel<<<1, KVT, 0, st>>>(kv->pos, kv->bits, kv->scalars, (int) kv->size, kv->n_words, ops_dev, n_ops,
-                                       desc_base, desc_stride);
+                                       desc_base, desc_stride, current, run_slot);
     PIB_CHECK(cudaGetLastError());
     return PIB_OK;
 }

@@ -97,7 +97,8 @@ int kv_device_init(KvDevice * kv, uint32_t n_ctx, int32_t n_words);
 void kv_device_free(KvDevice * kv);
 // replay n_ops ops (device array) ; ALLOC ops read the batch descriptor at desc_base + slot * desc_stride:
 //   int32 pos[PIB_DESC_MAX_TOK] then uint32 tokbits[PIB_DESC_MAX_TOK][n_words]   (see context.cuh)
-int kv_device_apply(const KvDevice * kv, const KvOp * ops_dev, int n_ops, const uint8_t * desc_base, size_t desc_stride,
+// current (or null): gets run_slot, the run whose kernels follow
+int kv_device_apply(const KvDevice * kv, const KvOp * ops_dev, int n_ops, const uint8_t * desc_base, size_t desc_stride, int * current, int run_slot,
                     cudaStream_t st);
 // mask[t][i] = 1 when cell i is NOT visible to token t (reference llama.cpp:5200-5240), for i < n (read from scalars)
 int kv_device_mask(const KvDevice * kv, const int32_t * tpos_dev, const uint32_t * tokbits_dev, int n_tokens,

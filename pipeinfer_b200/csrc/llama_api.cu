@@ -383,16 +383,21 @@ static int start_from_batch(llama_context * ctx, const llama_batch & batch) {
         for (int i = 0; i < n; i++) seqp[i] = &seq1[i];
         ns = nseq.data(); sp = seqp.data();
     }
-    const int run = pib_decode_start(ctx->c, n, batch.token, p, ns, sp, batch.batch_id);
-    if (run < 0) return run;
     // rows that the caller will read (llama.cpp:5798): those it marked, else all or the last one
-    pib_run & r = ctx->c->runs[run];
-    r.want_lo = batch.logits || ctx->c->logits_all ? 0 : n - 1;
-    r.want_hi = n;
+    std::vector<int> & marks = ctx->c->marks_next;
+    marks.clear();
+    int lo = batch.logits || ctx->c->logits_all ? 0 : n - 1, hi = n;
     if (batch.logits) {
-        while (r.want_lo < n && !batch.logits[r.want_lo]) r.want_lo++;
-        while (r.want_hi > r.want_lo && !batch.logits[r.want_hi - 1]) r.want_hi--;
+        while (lo < n && !batch.logits[lo]) lo++;
+        while (hi > lo && !batch.logits[hi - 1]) hi--;
     }
+    for (int i = lo; i < hi && marks.size() <= PIB_CHUNK; i++) if (n <= PIB_CHUNK || !batch.logits || batch.logits[i]) marks.push_back(i);
+    if (marks.size() > PIB_CHUNK) marks.clear();
+    const int run = pib_decode_start(ctx->c, n, batch.token, p, ns, sp, batch.batch_id);
+    marks.clear();
+    if (run < 0) return run;
+    pib_run & r = ctx->c->runs[run];
+    r.want_lo = lo; r.want_hi = hi;
     return run;
 }
 
@@ -426,7 +431,9 @@ float * llama_get_logits(struct llama_context * ctx) {
     if (c->last_finished < 0) return nullptr;
     pib_run & r = c->runs[c->last_finished];
     const int n = r.n_tokens;
-    r.want_lo = 0; r.want_hi = n;                             // every row, marked or not
+    if (r.pinned && (int) r.marks.size() == n) return const_cast<float *>(pib_logits_row(c, 0));
+    r.want_lo = 0; r.want_hi = n;                             // every row, marked or not, next to each other
+    r.marks.clear();
     for (int i = 0; i < n; i++) pib_logits_row(c, i);
     return const_cast<float *>(pib_logits_row(c, 0));         // rows are contiguous
 }

@@ -61,3 +61,30 @@ def test_all_rows(ctx, marks):
     want, _ = read(ctx, 9, range(9), range(9))
     got, c = read(ctx, 9, marks, [], whole=True)
     assert np.array_equal(got, want) and c == 9
+
+
+def test_rows_that_cross_behind_the_kernels(ctx):
+    """a program that read the last run's rows gets the next one's without a copy of their own: the same values, of decode batches and of prompts with marks far apart, also when it
+    then reads other rows, all rows, or none"""
+    want = {n: read(ctx, n, range(n), range(n))[0] for n in (1, 5, 16, 40)}
+    for n, marks, rows in [(5, range(5), [0, 4]), (5, [1, 3], [3, 1, 2, 0]), (16, [15], [15]), (40, [3, 17, 39], [39, 3, 17, 20]), (40, range(16), [15, 0]), (40, range(17), [16, 2]), (1, [0], []), (1, [0], [0]),
+                           (16, range(16), [7]), (40, [39], [39, 39])]:
+        got, _ = read(ctx, n, marks, rows)
+        assert not len(rows) or np.array_equal(got, want[n][list(rows)])
+    for n, marks in [(16, range(16)), (16, [2]), (40, [39]), (5, [])]:
+        read(ctx, n, marks, [marks[0]] if len(marks) else [0])
+        assert np.array_equal(read(ctx, n, marks, [], whole=True)[0], want[n])
+
+
+def test_bytes_of_rows_nobody_reads(ctx):
+    sent = C.c_uint64()
+
+    def count():
+        ctx.L.llama_pib_io_bytes(ctx.ctx, C.byref(C.c_uint64()), C.byref(sent))
+        return sent.value
+    per = []
+    for rows in ([0], [], [], []):                                   # read once, then never: one run's rows cross in vain
+        before = count()
+        read(ctx, 4, range(4), rows)
+        per.append((count() - before) // (4 * V))
+    assert per == [4, 0, 4, 0]
