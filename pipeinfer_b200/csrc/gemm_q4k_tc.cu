@@ -379,8 +379,8 @@ size_t pib_gemm_xhat_bytes(int64_t K, int b) { return (size_t) (b <= 32 ? 32 : b
 template <int NB>
 static int tg_fit(int S) {
     using C = tg_cfg<NB, 2>;
-    static std::atomic<int> known[4];                                            // of 1, 2, 4, 8; + 1
-    std::atomic<int> & k = known[S == 1 ? 0 : S == 2 ? 1 : S == 4 ? 2 : 3];
+    static std::atomic<int> known[5];                                            // of 1, 2, 3, 4, 8; + 1
+    std::atomic<int> & k = known[S < 5 ? S - 1 : 4];
     if (const int v = k.load()) return v - 1;
     int n = 0;
     if (cudaFuncSetAttribute(gemm_q4k_tc_kernel<NB, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) C::SMEM) == cudaSuccess) {
@@ -454,14 +454,21 @@ int pib_gemm_q4k_tc(const pib_weight * w, const void * act_dev, int b, float * y
     auto shares = [&](int n, int G) {
         int S = 1;
         while (S < 8 && nsb / (S * 2) >= 2 && n <= (G == 2 ? tg_fit_nb(NB, S * 2) : tg_fit_nb(NB, S) * 15 / 16)) S *= 2;
+        // three where four do not fit (two / three, 34 .. 42 blocks: K = 4096 at 100 / 256 tokens 23.6 33.8 / 21.5 29.7 .. 31.7, K = 14336 44.0 62.2 / 35.8 50.2)
+        if (G == 2 && S == 2 && nsb >= 6 && n <= tg_fit_nb(NB, 3)) S = 3;
         return S;
     };
+    // More blocks than clusters of two find room for, and no more than three shares of each find at two CTAs per SM (of 90 blocks; of 92 they take two rounds): without them the
+    // blocks are fewer than the SMs.  From the K on where a share is worth its meeting (one / three shares, us, 40 64 100 128 tokens: 80 blocks of 8192 38.0 40.0 43.0 44.9 / 31.8 33.8
+    // 39.9 42.0, of 14336 59.1 60.7 66.1 67.7 / 44.0 46.1 54.2 56.9; of 6144 31.7 32.7 35.8 35.7 / 27.6 29.6 35.4 36.7; of 4096 25.5 25.6 27.7 27.9 / 24.9 25.6 30.2 31.7;
+    // 90 blocks of 8192 39.5 39.9 43.4 44.4 / 33.7 35.8 42.0 46.4: above 64 tokens 81 blocks at most).
+    const bool three = NB <= 128 && nx > tg_fit_nb(NB, 2) && (NB <= 64 ? 18 * nx <= 11 * sms && nsb >= 18 : 20 * nx <= 11 * sms && nsb >= 32);
     // One CTA with two groups, or two CTAs with one, per SM (us, one / two, 40 and 128 tokens): 12288 x 4096 (96 row blocks) 18.7 / 20.8 and 20.9 / 29.6,
     // 10240 x 8192 (80) 31.4 / 33.4 and 33.8 / 42.7, 22016 x 4096 (172) 35.5 / 29.4 and 39.5 / 34.7, 8192 x 28672 (64, in 2 / 4 shares) 54.2 / 49.1 and 68.5 / 67.7.
     // Above 128 tokens the accumulator takes half of the tensor memory: one.
     const bool two = NB <= 128 && (nx > sms || (NB <= 64 && shares(nx, 2) > 1));
-    if (two) {
-        const int S = shares(nx, 1);
+    if (two || three) {
+        const int S = three ? 3 : shares(nx, 1);
         switch (NB) {
             case 32: return tg_launch<32, 1>(w, xh, b, 0, nx, S, y_dev, st);
             case 64: return tg_launch<64, 1>(w, xh, b, 0, nx, S, y_dev, st);
