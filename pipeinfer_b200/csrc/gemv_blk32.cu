@@ -425,10 +425,22 @@ int pib_gemv_blk32(const pib_weight * w, const void * act_dev, int b, float * y_
     // 14.6 / 15.8; 80 tiles 9.3 / 9.9; 8192 wide, 16 tiles 3.3 / 3.2, 48 3.5 / 4.1).
     // Four warps (Q4_0, one token group): one round of them, where eight make a second round with little in it, where the K split would split, takes a second round, or has too few records per
     // warp (8 tokens: 28672 wide, 328 tiles 28.1, eight warps 33.5, K split 30.9, 740 tiles 43.8 / 58.6; 2048 wide, 444 tiles 4.3 / 7.3, 592 4.5 / 4.7; 3072 wide, 592 6.0 / 5.7).
+    // Four warps, two token groups (three CTAs per SM; us at 9 / 16 tokens, before / four-warp ring): up to a round of them (4096 wide, 444 tiles of Q4_0 9.8 9.8 / 8.7 8.9, of Q8_0 11.7
+    // 12.3 / 9.5 9.7; 2048 wide 10.6 10.7 / 7.6 7.8) but not few tiles of long rows (256 of 11008 12.8 / 15.1 at 16), and from two rounds on (4096 wide, 2000 tiles, 13 tokens: Q4_0 27.6 / 25.5,
+    // Q8_0 32.5 / 28.2; 57344 x 8192 76.1 80.7 / 72.4 75.6 and 88.7 88.6 / 82.3 89.8); between, eight warps have fuller rounds (Q4_0 512 tiles 10.5 10.6 / 11.4 11.4, 640 12.1 12.4 / 12.8
+    // 12.7; Q8_0 512 tiles of 8192 18.5 18.8 / 20.4 20.6), except of Q8_0 in rows up to 4096 (640 tiles 14.8 14.8 / 13.4 13.6) and of short rows (704 of 2048 at 13: 9.2 / 8.7, 10.2 / 9.7).
+    // One token group of Q4_0 from 2.4 rounds of them on (four or fewer tokens, or long rows): 57344 x 8192 at 1, 4, 7 tokens 52.3 55.2 56.5 / 50.2 51.4 55.0, 57344 x 4096 at 3 30.8 / 28.9, but
+    // 32000 x 4096 at 8 19.4 / 20.5.  The sums are those of the four-warp K split where it does not split.
     const int  sms = pib_num_sms(), fill = pib_split_fill_target();
-    const bool two = b > 8;
-    const bool four = w->type == PIB_TYPE_Q4_0 && !two && n_tiles > 2 * sms && n_tiles <= 5 * sms && (ngr <= 8 || 5 * n_tiles <= 12 * sms || n_tiles > 4 * sms || (ngr < 16 && n_tiles < fill));
+    const bool two = b > 8, q8 = w->type == PIB_TYPE_Q8_0;
+    const bool many = two ? (n_tiles > 2 * sms && ngr <= 16 && (n_tiles <= 3 * sms || (q8 ? ngr > 8 || n_tiles > 4 * sms : ngr <= 8 || n_tiles > 6 * sms))) || n_tiles > 8 * sms
+                          : !q8 && n_tiles > 12 * sms && (b <= 4 || ngr >= 32);
+    const bool four = !q8 && !two && n_tiles > 2 * sms && n_tiles <= 5 * sms && (ngr <= 8 || 5 * n_tiles <= 12 * sms || n_tiles > 4 * sms || (ngr < 16 && n_tiles < fill));
     const bool wide = ngr == 16 || 2 * n_tiles >= 3 * ngr || (two ? 5 * n_tiles >= 2 * sms : 2 * n_tiles > sms);
+    if (many) {
+        if (q8) return bk_ring_launch<PIB_TYPE_Q8_0, 2, 4, 3>(w, ngr, aqs, adx, b, y_dev, cancel, st);
+        return two ? bk_ring_launch<PIB_TYPE_Q4_0, 2, 4, 4>(w, ngr, aqs, adx, b, y_dev, cancel, st) : bk_ring_launch<PIB_TYPE_Q4_0, 1, 4, 4>(w, ngr, aqs, adx, b, y_dev, cancel, st);
+    }
     if (four) return bk_ring_launch<PIB_TYPE_Q4_0, 1, 4, 4>(w, ngr, aqs, adx, b, y_dev, cancel, st);
     if (ngr >= 16 && wide && (two ? w->type == PIB_TYPE_Q4_0 || n_tiles <= 4 * sms || ngr >= 24 : n_tiles < fill)) {
         if (w->type == PIB_TYPE_Q4_0) return two ? bk_ring_launch<PIB_TYPE_Q4_0, 2, 8, 4>(w, ngr, aqs, adx, b, y_dev, cancel, st) : bk_ring_launch<PIB_TYPE_Q4_0, 1, 8, 4>(w, ngr, aqs, adx, b, y_dev, cancel, st);
