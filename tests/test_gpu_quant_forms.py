@@ -160,3 +160,21 @@ def test_gated_matmul(lib, tables, N, K, b):
     lib.L.pib_weight_free(w)
     B.free()
     assert np.array_equal(got, look(tables[0], gu[:, :N // 2]) * gu[:, N // 2:])
+
+
+@pytest.mark.parametrize("b,K", [(300, 4096), (4800, 256), (151, 8448), (290, 4352)])        # from a super-block per warp of the machine on (32 x 148): the table in shared memory
+def test_gated_rows_of_prompts(lib, b, K):
+    """the fp16 rows of a long prompt's gated product are those of its parts, which are too short for that route"""
+    rng = np.random.default_rng(b)
+    B = Buffers(lib, 0)
+    g = rng.standard_normal((b, 2 * K)).astype(np.float32) * 3
+    g[0, :256], g[1, 5] = 0, 40000.0
+    gu, out, part = B.put(g), B.put(np.zeros((b, K // 2))), B.put(np.zeros((b, K // 2)))
+    f = lib.f["pib_silu_mul_quantize_act"]
+    lib.check(f(Q4_K, gu, gu + 4 * K, 2 * K, b, K, None, None, None, out, False))
+    for r in range(0, b, 40):
+        n = min(40, b - r)
+        lib.check(f(Q4_K, gu + 8 * K * r, gu + 8 * K * r + 4 * K, 2 * K, n, K, None, None, None, part + 2 * K * r, False))
+    got, want = lib.to_host(out, (b, K), np.float16), lib.to_host(part, (b, K), np.float16)
+    B.free()
+    assert np.array_equal(got.view(np.uint16), want.view(np.uint16)) and np.abs(want.astype(np.float32)).sum() > 0
