@@ -543,8 +543,8 @@ gemv_q4k_direct_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K
 // GATED: rows of a gate and rows of its factor gridDim.x row tiles on, half of the warps each (in the order of the four-warp form); what is written is silu(gate) * factor, through
 // the reference's table (ggml.c:1490; in the place of the K shares' sums, of which there are none).  In the quantiser behind it the product's look-ups (32 places of the
 // table at once, while the next matmul's weights come) took 2 us of a draft step's layer: the step 681 -> 669 us.
-template <int NT, int WARPS, int STAGES, bool GATED = false, int PER = NT == 1 ? (WARPS == 4 ? 5 : GATED ? 3 : 2) : (WARPS == 4 ? 3 : 2)>
-__global__ void __launch_bounds__(WARPS * 32, PER)
+template <int NT, int WARPS, int STAGES, bool GATED = false>
+__global__ void __launch_bounds__(WARPS * 32, NT == 1 ? (WARPS == 4 ? 5 : GATED ? 3 : 2) : (WARPS == 4 ? 3 : 2))
 gemv_q4k_ring_kernel(const uint8_t * __restrict__ tiles, int nsb, int N, int K, const int8_t * __restrict__ aqs,
                      const float * __restrict__ ad, const int8_t * __restrict__ abs8, int b, float * __restrict__ y,
                      float * __restrict__ partial, unsigned int * __restrict__ counters, const int * __restrict__ cancel) {
@@ -1065,14 +1065,14 @@ int pib_gemv_mma_launch(const pib_weight * w, const void * act_dev, int b, float
     return PIB_OK;
 }
 
-template <int NT, int WARPS, int STAGES, bool GATED = false, int PER = NT == 1 ? (WARPS == 4 ? 5 : GATED ? 3 : 2) : (WARPS == 4 ? 3 : 2)>
+template <int NT, int WARPS, int STAGES, bool GATED = false>
 static int ring_launch(const pib_weight * w, const int8_t * aqs, const float * ad, const int8_t * bs, int b, float * y_dev, int split, float * partial,
                        unsigned int * counters, const int * cancel, cudaStream_t st) {
     const int    nsb = (int) (w->K / 256), N = (int) (GATED ? w->N / 2 : w->N), n_tiles = (N + 15) / 16;
     const size_t ring = (size_t) WARPS * STAGES * MM_TILE_BYTES, smem = WARPS == 8 ? pib_gemv_smem_spread(ring, n_tiles * split) : ring;
     static pib_per_device attrs;
-    PIB_CHECK(attrs.once([&] { return cudaFuncSetAttribute(gemv_q4k_ring_kernel<NT, WARPS, STAGES, GATED, PER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) std::max(ring, (size_t) PIB_GEMV_SPREAD)); }));
-    PIB_CHECK(pib_launch(gemv_q4k_ring_kernel<NT, WARPS, STAGES, GATED, PER>, dim3(n_tiles, split), dim3(WARPS * 32), smem, st, w->tiles, nsb, N, (int) w->K, aqs, ad, bs, b, y_dev,
+    PIB_CHECK(attrs.once([&] { return cudaFuncSetAttribute(gemv_q4k_ring_kernel<NT, WARPS, STAGES, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) std::max(ring, (size_t) PIB_GEMV_SPREAD)); }));
+    PIB_CHECK(pib_launch(gemv_q4k_ring_kernel<NT, WARPS, STAGES, GATED>, dim3(n_tiles, split), dim3(WARPS * 32), smem, st, w->tiles, nsb, N, (int) w->K, aqs, ad, bs, b, y_dev,
                          partial, counters, cancel));
     return PIB_OK;
 }
@@ -1109,15 +1109,6 @@ int pib_gemv_ring(const pib_weight * w, const void * act_dev, int b, float * y_d
     const int8_t * bs  = (const int8_t *) (act + L.bs8_off);
     float * pp = s ? s->partial : nullptr;
     unsigned int * cc = s ? s->counters : nullptr;
-    // Eight warps per tile also where the tiles are a little more than a round of four-warp CTAs (5 per SM), for long rows up to nearly three rounds: half as long CTAs leave less of
-    // the last round empty.  One or two tokens at three CTAs per SM, more at two (more registers); by shape alone otherwise, so that sums are the same at any number of tokens.
-    // us behind a quantiser, four / eight warps, 1, 4, 8, 9 and 16 tokens: 12288 x 8192 18.1 18.4 18.7 21.6 21.7 / 16.5 16.3 16.5 21.2 22.9, 24576 x 8192 25.8 26.8 28.8 33.7 38.2 / 24.7
-    // 25.4 25.7 34.6 38.0, 32000 x 8192 29.7 31.7 33.5 40.9 46.9 / 29.7 30.9 31.2 42.7 46.5, 12288 x 4096 11.3 11.4 11.7 13.8 14.0 / 10.7 10.7 10.8 13.5 13.7, 16384 x 4096 12.7 12.9 13.1
-    // 15.9 16.1 / 12.1 12.4 12.6 16.1 16.6; beyond: 22016 x 4096 15.3 15.3 15.9 / 14.4 15.3 15.5 but 19.1 / 20.1 at 9, 57344 x 8192 45.6 48.7 54.1 / 47.7 49.8 51.7, 32000 x 2048 11.7 / 12.7.
-    const int  sms = pib_num_sms();
-    const bool eight = !wide && split == 1 && nsb >= 16 && n_tiles > 5 * sms && n_tiles <= (nsb >= 32 ? 14 : 7) * sms;
-    if (eight) return b <= 2 ? ring_launch<1, 8, 4, false, 3>(w, aqs, ad, bs, b, y_dev, split, pp, cc, cancel, st) : b <= 8 ? ring_launch<1, 8, 4>(w, aqs, ad, bs, b, y_dev, split, pp, cc, cancel, st)
-                             : ring_launch<2, 8, 4>(w, aqs, ad, bs, b, y_dev, split, pp, cc, cancel, st);
     if (wide) return b <= 8 ? ring_launch<1, 8, 4>(w, aqs, ad, bs, b, y_dev, split, pp, cc, cancel, st) : ring_launch<2, 8, 4>(w, aqs, ad, bs, b, y_dev, split, pp, cc, cancel, st);
     return b <= 8 ? ring_launch<1, 4, 4>(w, aqs, ad, bs, b, y_dev, split, pp, cc, cancel, st) : ring_launch<2, 4, 4>(w, aqs, ad, bs, b, y_dev, split, pp, cc, cancel, st);
 }
