@@ -91,7 +91,14 @@ template <int HD, int ATQ_THREADS>
 static int launch_att_qh(const float * qkv, const float * vsep, const uint8_t * desc, const float2 * rope, int rope_n_pos, int mode, __half * kc, __half * vc,
                          const uint8_t * mask, const int32_t * scalars, int E, int GQA, int n_ctx, int n_tokens, int n_head, int gdiv, float * out,
                          const int * cancel, cudaStream_t st) {
-    const int    vcap = std::min(n_ctx, ATQ_THREADS == 512 && att_core_smem(HD, n_ctx, ATQ_VCAP(HD)) <= ATQ_SMEM_MAX(HD) ? ATQ_VCAP(HD) : ATQ_VCAP_MIN);
+    // as many V rows as are worth it while two CTAs of heads of 64 share an SM (a long score row leaves room for fewer)
+    int vcap = ATQ_VCAP_MIN;
+    if (ATQ_THREADS == 512) {
+        vcap = ATQ_VCAP(HD);
+        if (HD == 64 && 2 * (att_core_smem(HD, n_ctx, vcap) + 1024) > 228 * 1024) vcap = 384;
+        if (att_core_smem(HD, n_ctx, vcap) > ATQ_SMEM_MAX(HD)) vcap = ATQ_VCAP_MIN;
+    }
+    vcap = std::min(n_ctx, vcap);
     const size_t smem = att_core_smem(HD, n_ctx, vcap);   // scores + 32 x HD partial sums + staged V rows
     static pib_per_device attrs;
     // several CTAs per SM (a verification batch of 3+ tokens is more CTAs than SMs): ask for the large shared-memory carve-out

@@ -419,7 +419,7 @@ int pib_gemv_blk32(const pib_weight * w, const void * act_dev, int b, float * y_
     // four-warp CTAs five, of the K split's four.
     // One token group, eight warps: while the K split would split, since from 80 % of its slots on it runs unsplit in one round (4096 wide, 8 tokens: 444 tiles of Q4_0
     // 7.3 / 10.1, 512 tiles 7.3 / 6.7; Q8_0 8.6 / 10.6 and 8.9 / 7.2).
-    // Two token groups (behind a quantiser, 13 tokens): any number of tiles of Q4_0 (4096 wide, 740 tiles 12.8 / 14.6, 1376 20.9 / 23.0, 2000 27.5 / 28.8); of Q8_0 up to four tiles
+    // Two token groups, eight warps (where four, below, are not faster; behind a quantiser, 13 tokens): any number of tiles of Q4_0 (4096 wide, 740 tiles 12.8 / 14.6, 1376 20.9 / 23.0, 2000 27.5 / 28.8); of Q8_0 up to four tiles
     // per SM and rows from 6144 on (4096 wide, 592 tiles 13.1 / 15.8, 880 18.5 / 17.1, 1184 22.9 / 22.2; 8192 wide, 740 25.4 / 26.7, 1376 40.6 / 45.5).
     // Few tiles of long rows go to the K split, which divides a row over up to 64 warps (28672 wide, 32 tiles: 8.8 / 5.1 and, 13 tokens, 14.5 / 11.0; 64 tiles 9.2 / 6.9 and
     // 14.6 / 15.8; 80 tiles 9.3 / 9.9; 8192 wide, 16 tiles 3.3 / 3.2, 48 3.5 / 4.1).
@@ -429,11 +429,14 @@ int pib_gemv_blk32(const pib_weight * w, const void * act_dev, int b, float * y_
     // 12.3 / 9.5 9.7; 2048 wide 10.6 10.7 / 7.6 7.8) but not few tiles of long rows (256 of 11008 12.8 / 15.1 at 16), and from two rounds on (4096 wide, 2000 tiles, 13 tokens: Q4_0 27.6 / 25.5,
     // Q8_0 32.5 / 28.2; 57344 x 8192 76.1 80.7 / 72.4 75.6 and 88.7 88.6 / 82.3 89.8); between, eight warps have fuller rounds (Q4_0 512 tiles 10.5 10.6 / 11.4 11.4, 640 12.1 12.4 / 12.8
     // 12.7; Q8_0 512 tiles of 8192 18.5 18.8 / 20.4 20.6), except of Q8_0 in rows up to 4096 (640 tiles 14.8 14.8 / 13.4 13.6) and of short rows (704 of 2048 at 13: 9.2 / 8.7, 10.2 / 9.7).
+    // Not for Q8_0 in rows of 1024 (one round, 310 tiles at 13: 4.4 / 4.7; 444 of 1536 7.0 / 6.1) or of many records (1800 tiles of 12288 at 9 and 13: 70.3 65.7 / 72.7 73.4, of 7168 45.1 47.5 /
+    // 39.7 45.2).
     // One token group of Q4_0 from 2.4 rounds of them on (four or fewer tokens, or long rows): 57344 x 8192 at 1, 4, 7 tokens 52.3 55.2 56.5 / 50.2 51.4 55.0, 57344 x 4096 at 3 30.8 / 28.9, but
     // 32000 x 4096 at 8 19.4 / 20.5.  The sums are those of the four-warp K split where it does not split.
     const int  sms = pib_num_sms(), fill = pib_split_fill_target();
     const bool two = b > 8, q8 = w->type == PIB_TYPE_Q8_0;
-    const bool many = two ? (n_tiles > 2 * sms && ngr <= 16 && (n_tiles <= 3 * sms || (q8 ? ngr > 8 || n_tiles > 4 * sms : ngr <= 8 || n_tiles > 6 * sms))) || n_tiles > 8 * sms
+    const bool many = two ? (n_tiles > 2 * sms && ngr <= 16 && (n_tiles <= 3 * sms ? !q8 || ngr > 4 : q8 ? ngr > 8 || n_tiles > 4 * sms : ngr <= 8 || n_tiles > 6 * sms)) ||
+                                (n_tiles > 8 * sms && (!q8 || ngr <= 28))
                           : !q8 && n_tiles > 12 * sms && (b <= 4 || ngr >= 32);
     const bool four = !q8 && !two && n_tiles > 2 * sms && n_tiles <= 5 * sms && (ngr <= 8 || 5 * n_tiles <= 12 * sms || n_tiles > 4 * sms || (ngr < 16 && n_tiles < fill));
     const bool wide = ngr == 16 || 2 * n_tiles >= 3 * ngr || (two ? 5 * n_tiles >= 2 * sms : 2 * n_tiles > sms);

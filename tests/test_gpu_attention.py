@@ -64,7 +64,7 @@ def one_head(q, K, V, seen, scale, exp16):
 
 @pytest.mark.parametrize("hd,H,G,n,b,cell0,n_ctx", [
     (64, 4, 2, 32, 1, 31, 64), (64, 4, 1, 33, 3, 20, 512), (64, 8, 2, 63, 16, 40, 512), (64, 4, 4, 257, 2, 255, 512), (64, 4, 1, 300, 1, 299, 512), (64, 4, 2, 511, 4, 100, 512),
-    (64, 4, 1, 513, 1, 512, 1024), (64, 2, 1, 705, 3, 702, 1024), (64, 2, 1, 736, 2, 734, 1024), (64, 2, 2, 930, 5, 700, 1000), (64, 2, 1, 1100, 2, 300, 1301),
+    (64, 4, 1, 513, 1, 512, 1024), (64, 2, 1, 705, 3, 702, 1024), (64, 2, 1, 736, 2, 734, 1024), (64, 2, 2, 930, 5, 700, 1000), (64, 2, 1, 1100, 2, 300, 1301), (64, 2, 2, 420, 2, 390, 3400),
     (128, 2, 1, 32, 1, 30, 64), (128, 4, 4, 129, 2, 127, 256), (128, 2, 1, 300, 1, 299, 512), (128, 2, 2, 385, 3, 382, 512), (128, 2, 1, 700, 2, 200, 1024),
     (128, 32, 4, 95, 16, 79, 256), (128, 32, 4, 290, 8, 250, 512), (128, 16, 4, 415, 16, 380, 640)])      # from 149 (head, token) pairs on 256 threads
 @pytest.mark.parametrize("mode,sep", [(0, False), (2, True)])

@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("wt", [Q4, Q8])
 @pytest.mark.parametrize("N,K,b", [(4731, 2048, 9), (4737, 2048, 16), (4739, 4096, 13), (7099, 4096, 9), (7105, 4096, 16), (7111, 1056, 11), (9466, 2048, 12), (9475, 2048, 9), (14208, 4096, 9),
-                                   (14211, 4096, 10), (7099, 4352, 9), (18939, 4352, 9), (18945, 4352, 16), (18946, 96, 15)])      # 296 / 297, 444 / 445, 592 / 593, 888 / 889, 1184 / 1185 tiles; 16 / 17 records
+                                   (14211, 4096, 10), (7099, 4352, 9), (18939, 4352, 9), (18945, 4352, 16), (18946, 96, 15), (4960, 1024, 13), (4961, 1056, 13), (18960, 7168, 10),
+                                   (18961, 7200, 16)])      # 296 / 297, 444 / 445, 592 / 593, 888 / 889, 1184 / 1185 tiles; 4 / 5, 16 / 17, 28 / 29 records
 def test_two_groups(oracle, wt, N, K, b):
     both_sides(oracle, wt, N, K, b)
 
