@@ -275,18 +275,17 @@ static int launch_aq(int wtype, const float * x, const float * x2, int x2_per_ro
     a.vec = (at & 15) == 0;
     constexpr bool NORM = PRO == PRO_RMSNORM || PRO == PRO_LAYERNORM, PROMPT = PRO == PRO_PLAIN || PRO == PRO_RMSNORM || PRO == PRO_SILU_MUL;
     const int units = (int) ((K + 255) / 256);
-    // With a norm: the row in one block, or a decode batch's row in several.  Without: a warp per block while that makes no more than eight blocks per SM (two of a prompt: 40 rows of
-    // 8192 1 % of the matmul), up to eight warps from there on.
+    // With a norm: the row in one block, or a decode batch's row in several.  Without: up to eight warps per block, as many as leave no more than 32 blocks.  The matmul behind is
+    // launched while these blocks run, and where it has a few CTAs per SM its placement follows the room that they leave: a warp on most SMs of the machine sends a third and fourth CTA to
+    // the others (us with the matmul, 1 / 2 / 4 / 8 warps per block: Q4_0 5024 x 16128, 2 tokens 21.8 18.3 15.4 15.4; 4992 x 14336, 4 tokens 19.5 18.6 16.9 14.2; Q5_K 5520 x 9984, 6 tokens
+    // 16.2 16.3 16.0 13.5; Q4_K 8192 x 28672, 64 rows 61.9 57.8 54.8 54.3), while eight warps of one block cost a small row more than eight blocks (2048, one token 3.85 / 4.05).
     int W = std::min(32, units), parts = 1;
     if (NORM) {
         a.per = b <= PIB_MAX_BATCH ? 8 : units;
         parts = (units + a.per - 1) / a.per;
     } else {
         W = 1;
-        if (b * units > 256) {
-            const int most = (b <= PIB_MAX_BATCH ? 8 : 2) * pib_num_sms();
-            while (W < 8 && b * ((units + W - 1) / W) > most) W *= 2;
-        }
+        while (W < 8 && W < units && b * ((units + W - 1) / W) > 32) W *= 2;
         parts = (units + W - 1) / W;
     }
     // a prompt's gated product: from a super-block per warp of the machine on
