@@ -60,6 +60,8 @@ __device__ __forceinline__ void aq_store8(float * p, int vec, const float (&v)[8
 // Grid: a row per blockIdx.x.  Without a norm the row's warps are spread over blockIdx.y.  With one, up to 32 warps of a block have the whole row in registers (longer rows take turns)
 // and nothing is read twice; of a decode batch, blocks of eight units each (blockIdx.y) form the row's sum for themselves and quantise and write their own units: what a unit stores
 // keeps an SM busy (4 rows of 8192: 3.4 us behind the wait with one block per row, 2.1 with four).
+// The unit that a warp quantises stays in its registers from the sum on also where it is the warp's second of the row (with a matmul of 1712 rows, one token of 10240 9.65 -> 8.86 us, of 14848
+// 12.0 -> 11.2; read again 0.6 us behind the sum otherwise).
 // What bounds it: a chain of round trips behind the launch in front (operands 0.35 .. 0.6 us, the sum's two reductions and its barrier 0.3, the quants 0.25, their stores 0.4) and
 // instructions that no earlier launch left in the cache (6 .. 9 clocks each).  Before (a warp's lanes on 32 neighbours for 32-element blocks, passes of up to four pieces per warp) / now,
 // us that a launch adds to its chain: Q8_0 blocks, norm, 4 rows of 4096 4.6 / 2.7; Q8_K, norm, one row of 2048 3.2 / 2.8, plain 1.9 / 1.5; prompts of 700 rows, norm 4096 14.1 / 10.2.
@@ -77,10 +79,11 @@ __global__ void __launch_bounds__(1024) act_quant_kernel(const aq_args a) {
     const int     i00  = u0 * 256 + lane * 8;
     const int     u_lo = NORM ? blockIdx.y * a.per : 0, u_hi = NORM ? min(units, u_lo + a.per) : units;      // the units that this block quantises
     float v[8] = { 0, 0, 0, 0, 0, 0, 0, 0 }, w[8] = { 0, 0, 0, 0, 0, 0, 0, 0 }, bi[8] = { 0, 0, 0, 0, 0, 0, 0, 0 };
-    // the first unit's norm weights are immutable: fetched before the wait on the producer of x
-    if (NORM && i00 < K) {
-        aq_load8(x2r + i00, a.vec, w);
-        if (PRO == PRO_LAYERNORM) aq_load8(a.bias + i00, a.vec, bi);
+    // the first unit that this warp quantises stays in registers; its norm weights are immutable: fetched before the wait on the producer of x
+    const int uo = NORM && u0 < u_lo ? u0 + (u_lo - u0 + step - 1) / step * step : u0, io = uo * 256 + lane * 8;
+    if (NORM && io < K) {
+        aq_load8(x2r + io, a.vec, w);
+        if (PRO == PRO_LAYERNORM) aq_load8(a.bias + io, a.vec, bi);
     }
     pib_pdl_wait();
     pib_pdl_trigger();
@@ -131,6 +134,10 @@ __global__ void __launch_bounds__(1024) act_quant_kernel(const aq_args a) {
             fetch(i, y);
 #pragma unroll
             for (int j = 0; j < 8; j++) s += term(y[j]);
+            if (i == io) {
+#pragma unroll
+                for (int j = 0; j < 8; j++) v[j] = y[j];
+            }
         }
         const float m = mean_of(total(s, red[0]));
         if (PRO == PRO_RMSNORM) scale = 1.0f / sqrtf(m + a.eps);
@@ -140,14 +147,14 @@ __global__ void __launch_bounds__(1024) act_quant_kernel(const aq_args a) {
             mean = m;
             s = 0.0;
             auto square = [&](float y) -> double { const float t = __fsub_rn(y, mean); return (double) __fmul_rn(t, t); };
-            if (i00 < K) {
-#pragma unroll
-                for (int j = 0; j < 8; j++) s += square(v[j]);
-            }
 #pragma unroll 1
-            for (int i = i00 + step * 256; i < K; i += step * 256) {
+            for (int i = i00; i < K; i += step * 256) {
                 float y[8];
-                fetch(i, y);
+                if (i != io) fetch(i, y);
+                else {
+#pragma unroll
+                    for (int j = 0; j < 8; j++) y[j] = v[j];
+                }
 #pragma unroll
                 for (int j = 0; j < 8; j++) s += square(y[j]);
             }
@@ -157,13 +164,12 @@ __global__ void __launch_bounds__(1024) act_quant_kernel(const aq_args a) {
     }
 
 #pragma unroll 1
-    for (int u = u0; u < u_hi; u += step) {
-        if (NORM && u < u_lo) continue;
+    for (int u = uo; u < u_hi; u += step) {
         const int  i  = u * 256 + lane * 8;
         const bool in = Q8K || i < K;                             // the last group of 32-element blocks may end before 256: zeros
-        if (!NORM || u != u0) {
+        if (!NORM || u != uo) {
             if (in) aq_load8(xr + i, a.vec, v);
-            if (PRO == PRO_SILU_MUL || (NORM && u != u0)) { if (in) aq_load8(x2r + i, a.vec, w); }
+            if (PRO == PRO_SILU_MUL || NORM) { if (in) aq_load8(x2r + i, a.vec, w); }
             if (PRO == PRO_LAYERNORM) { if (in) aq_load8(a.bias + i, a.vec, bi); }
         }
 #pragma unroll
