@@ -180,25 +180,25 @@ __global__ void __launch_bounds__(512) kv_attn_kernel(kva_args A) {
     const int32_t * map = nullptr;
     const float *   rel = A.rel && live ? A.rel + (size_t) h * A.n_rel : nullptr;
     const float     slope = A.slopes && live ? A.slopes[h] : 0.f;
-    float kk[UK][RPL], c[UK][RPL], bias[UK];
+    float kk[UK][RPL], c[UK][RPL], rv[UK];
     auto place = [&]() {
         p  = A.pos[t];
         lo = A.mask == PIB_MASK_CHUNK ? p - p % A.window : max(0, p - A.window + 1);
         nf = min(A.keep, lo); n_keys = nf + p - lo + 1;                  // kept positions in front of the window, then the window
         map = A.cellmap + (size_t) A.slot[t] * A.n_ctx;
     };
-    // rows of the trip's keys and their distance biases; a trip past the end reads the last key again, its score is dropped below.  own: the token's own row too
+    // position of the u-th key of the trip at e0; past the end the last key once more, its score is dropped below
+    auto key = [&](int e0, int u) { const int e = min(e0 + u * all, n_keys - 1); return e < nf ? e : lo + e - nf; };
+    // rows of the trip's keys and their table biases.  own: the token's own row too
     auto fetch = [&](int e0, bool own, bool others) {
 #pragma unroll
         for (int u = 0; u < UK; u++) {
-            const int e = min(e0 + u * all, n_keys - 1), j = e < nf ? e : lo + e - nf;
+            const int j = key(e0, u);
             if (j == p ? !own : !others) continue;
             const float * row = A.cache + (size_t) map[j] * A.cache_row;
 #pragma unroll
             for (int i = 0; i < RPL; i++) { const int r = i * 32 + lane; kk[u][i] = r < D ? row[ko + r] : 0.f; c[u][i] = r < V ? row[vo + r] : 0.f; }
-            bias[u] = 0.f;
-            if (A.slopes) bias[u] = -(slope * (float) (p - j));
-            if (rel) bias[u] += rel[min(p - j, A.n_rel - 1)];
+            rv[u] = rel ? rel[min(p - j, A.n_rel - 1)] : 0.f;
         }
     };
     if (EARLY && live) { place(); if (first < n_keys) fetch(first, false, true); }
@@ -226,25 +226,26 @@ __global__ void __launch_bounds__(512) kv_attn_kernel(kva_args A) {
             }
             float bs[UK];
 #pragma unroll
-            for (int u = 0; u < UK; u++) bs[u] = bias[u];
+            for (int u = 0; u < UK; u++) bs[u] = rv[u];
             if (EARLY && e0 + all * UK < n_keys) fetch(e0 + all * UK, true, true);
+            // Both forms round alike, whatever the compiler contracts: a sequence's bits do not depend on what else its batch holds.  The slope's term joins with one rounding.
             float mn = m;
 #pragma unroll
             for (int u = 0; u < UK; u++) {
                 s[u] = warp_sum(s[u]);
-                if (A.softcap > 0.f) s[u] = A.softcap * tanhf(s[u] / A.softcap);
-                s[u] += bs[u];
+                if (A.softcap > 0.f) s[u] = __fmul_rn(A.softcap, tanhf(__fdiv_rn(s[u], A.softcap)));
+                if (A.slopes) s[u] = __fmaf_rn(-slope, (float) (p - key(e0, u)), s[u]);
+                if (rel) s[u] = __fadd_rn(s[u], bs[u]);
                 if (UK > 1 && e0 + u * all >= n_keys) s[u] = -INFINITY;
                 mn = fmaxf(mn, s[u]);
             }
-            const float a = expf(m - mn);                                              // m == -inf only before the first key: a = 0
-            l *= a;
+            const float a = expf(__fsub_rn(m, mn));                                    // m == -inf only before the first key: a = 0
 #pragma unroll
-            for (int i = 0; i < RPL; i++) acc[i] *= a;
+            for (int i = 0; i < RPL; i++) acc[i] = __fmul_rn(acc[i], a);
 #pragma unroll
             for (int u = 0; u < UK; u++) {
-                const float w = expf(s[u] - mn);
-                l += w;
+                const float w = expf(__fsub_rn(s[u], mn));
+                l = u == 0 ? __fmaf_rn(l, a, w) : __fadd_rn(l, w);
 #pragma unroll
                 for (int i = 0; i < RPL; i++) acc[i] = fmaf(w, cv[u][i], acc[i]);
             }

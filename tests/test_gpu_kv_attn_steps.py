@@ -10,9 +10,9 @@ from tests.gusedra_configs import CONFIGS
 pytestmark = pytest.mark.gpu
 
 
-def run(cfg, prompts, steps, two):
+def run(cfg, prompts, steps, two, alone=False):
     from pipeinfer_b200 import llama
-    ctx = llama.Context(config=json.dumps(cfg), n_ctx=1024, max_seq=8, float32=True, seed=5, state_slots=6)
+    ctx = llama.Context(config=json.dumps(cfg), n_ctx=1024, max_seq=8, float32=True, seed=5, state_slots=8)
     L, S, out = ctx.L, len(prompts), []
 
     def decode(toks, pos, seqs):
@@ -25,6 +25,8 @@ def run(cfg, prompts, steps, two):
         toks, pos, seqs = list(row), [len(p) + k for p in prompts], list(range(S))
         if two:                                                      # another sequence's two tokens behind them
             toks, pos, seqs = toks + [3, 4], pos + [2 * k, 2 * k + 1], seqs + [S, S]
+        if alone:                                                    # two other sequences' one token each: as many rows, every one a sequence of its own
+            toks, pos, seqs = toks + [3, 4], pos + [k, k], seqs + [S, S + 1]
         out.append(decode(toks, pos, seqs)[:S])
     ctx.close()
     return np.stack(out)
@@ -39,3 +41,13 @@ def test_steps_both_ways(name):
     a, b = run(cfg, prompts, steps, False), run(cfg, prompts, steps, True)
     # fp32 throughout; matmuls of 5 and of 7 rows add in the same order, so what differs is at most the rounding of a fused multiply-add per score
     assert np.abs(a - b).max() <= 1e-4 * np.abs(b).max()
+
+
+@pytest.mark.parametrize("name", ["slope_only", "bucket_only", "shared_cells", "far_keys", "wide_heads", "big_heads", "mixed_small"])
+def test_same_bits_beside_other_sequences(name):
+    """as many rows in a batch, so that the same blocks share a head's keys: the two forms of the kernel round alike"""
+    cfg = CONFIGS[name]()
+    rng = np.random.default_rng(4)
+    prompts = [rng.integers(0, cfg["vocab"], n).tolist() for n in (2, 15, 64, 65, 301)]
+    steps = rng.integers(0, cfg["vocab"], (6, len(prompts))).tolist()
+    assert np.array_equal(run(cfg, prompts, steps, False, alone=True), run(cfg, prompts, steps, True))
