@@ -164,8 +164,9 @@ template <int RPL> __device__ __forceinline__ void kva_merge(const float * base,
     }
 }
 // EARLY: every segment of the batch is one token, so that all rows but the token's own were final before the launch in front started; the first trip's rows and biases are fetched
-// before the wait on it, and a trip's rows while the one before is worked on.  (Prompts go without: twice the registers leave an SM one block instead of two.)  (4 tokens, 16 heads of 128, about 100 keys: a chain of two trips' look-ups and rows
-// behind the projections, 10.4 us of a step's chain, now 7.7.)
+// before the wait on it, and a trip's rows while the one before is worked on (4 tokens, 16 heads of 128, about 100 keys: 10.4 us of a step's chain, now 7.7).  Prompts go without (with both
+// 155 us where 143 without, 4 prompts of 90 tokens): it costs registers (heads of up to 64 coordinates 80 instead of 64, one block of 512 threads per SM instead of two; of 128 127 instead of
+// 85, of 32 64 instead of 56: one block, and two, either way).
 template <int RPL, int UK, bool EARLY>
 __global__ void __launch_bounds__(512) kv_attn_kernel(kva_args A) {
     extern __shared__ float sm[];                 // [HPB * KS (+ 1 in a cluster: the block's own merged state)][V + 2] partial states
@@ -180,7 +181,8 @@ __global__ void __launch_bounds__(512) kv_attn_kernel(kva_args A) {
     const int32_t * map = nullptr;
     const float *   rel = A.rel && live ? A.rel + (size_t) h * A.n_rel : nullptr;
     const float     slope = A.slopes && live ? A.slopes[h] : 0.f;
-    float kk[UK][RPL], c[UK][RPL], rv[UK];
+    constexpr int NE = EARLY ? UK : 1;
+    float kk[NE][RPL], c[NE][RPL], rv[NE];                               // a trip's rows and table biases, EARLY only
     auto place = [&]() {
         p  = A.pos[t];
         lo = A.mask == PIB_MASK_CHUNK ? p - p % A.window : max(0, p - A.window + 1);
@@ -192,7 +194,7 @@ __global__ void __launch_bounds__(512) kv_attn_kernel(kva_args A) {
     // rows of the trip's keys and their table biases.  own: the token's own row too
     auto fetch = [&](int e0, bool own, bool others) {
 #pragma unroll
-        for (int u = 0; u < UK; u++) {
+        for (int u = 0; u < NE; u++) {
             const int j = key(e0, u);
             if (j == p ? !own : !others) continue;
             const float * row = A.cache + (size_t) map[j] * A.cache_row;
@@ -213,20 +215,23 @@ __global__ void __launch_bounds__(512) kv_attn_kernel(kva_args A) {
         for (int i = 0; i < RPL; i++) { const int r = i * 32 + lane; qv[i] = r < D ? qp[r] * A.scale : 0.f; acc[i] = 0.f; }
         if (ks == 0 && rank == 0 && A.sink) { m = A.sink[h]; l = 1.f; }
         if (!EARLY) place();
-        else if (first < n_keys) fetch(first, true, false);
+        if (EARLY && first < n_keys) fetch(first, true, false);
 #pragma unroll 1
         for (int e0 = first; e0 < n_keys; e0 += all * UK) {
-            if (!EARLY) fetch(e0, true, true);
-            float s[UK], cv[UK][RPL];
+            float s[UK], cv[UK][RPL], bs[UK];
 #pragma unroll
             for (int u = 0; u < UK; u++) {
                 s[u] = 0.f;
+                if (EARLY) {
+                    bs[u] = rv[u % NE];
 #pragma unroll
-                for (int i = 0; i < RPL; i++) { if (i * 32 + lane < D) s[u] = fmaf(qv[i], kk[u][i], s[u]); cv[u][i] = c[u][i]; }
+                    for (int i = 0; i < RPL; i++) { if (i * 32 + lane < D) s[u] = fmaf(qv[i], kk[u % NE][i], s[u]); cv[u][i] = c[u % NE][i]; }
+                } else {
+                    const float * row = A.cache + (size_t) map[key(e0, u)] * A.cache_row;
+#pragma unroll
+                    for (int i = 0; i < RPL; i++) { const int r = i * 32 + lane; if (r < D) s[u] = fmaf(qv[i], row[ko + r], s[u]); cv[u][i] = r < V ? row[vo + r] : 0.f; }
+                }
             }
-            float bs[UK];
-#pragma unroll
-            for (int u = 0; u < UK; u++) bs[u] = rv[u];
             if (EARLY && e0 + all * UK < n_keys) fetch(e0 + all * UK, true, true);
             // Both forms round alike, whatever the compiler contracts: a sequence's bits do not depend on what else its batch holds.  The slope's term joins with one rounding.
             float mn = m;
@@ -234,8 +239,9 @@ __global__ void __launch_bounds__(512) kv_attn_kernel(kva_args A) {
             for (int u = 0; u < UK; u++) {
                 s[u] = warp_sum(s[u]);
                 if (A.softcap > 0.f) s[u] = __fmul_rn(A.softcap, tanhf(__fdiv_rn(s[u], A.softcap)));
-                if (A.slopes) s[u] = __fmaf_rn(-slope, (float) (p - key(e0, u)), s[u]);
-                if (rel) s[u] = __fadd_rn(s[u], bs[u]);
+                const int dist = p - key(e0, u);
+                if (A.slopes) s[u] = __fmaf_rn(-slope, (float) dist, s[u]);
+                if (rel) s[u] = __fadd_rn(s[u], EARLY ? bs[u] : rel[min(dist, A.n_rel - 1)]);
                 if (UK > 1 && e0 + u * all >= n_keys) s[u] = -INFINITY;
                 mn = fmaxf(mn, s[u]);
             }
