@@ -1268,18 +1268,28 @@ const pib_accept_result * pib_last_accept(pib_context * c) {
     return c->runs[c->last_finished].acc_host;
 }
 
-// the marked rows' copies to the run's page-locked memory; false: no memory there (or more rows than a decode batch has)
-static bool pin_rows(pib_context * c, pib_run & r) {
-    if (r.marks.empty() || r.marks.back() >= r.n_tokens || !r.logits) return false;
-    const size_t V = (size_t) c->model->n_vocab, n = r.marks.size() * V;
-    if (r.pin_cap < n) {
-        if (!r.pin && c->n_pins >= PIB_PINS) return false;
-        if (r.pin) { cudaFreeHost(r.pin); c->n_pins--; }
-        r.pin = nullptr; r.pin_cap = 0;
-        if (cudaMallocHost(&r.pin, n * 4) != cudaSuccess) { cudaGetLastError(); r.pin = nullptr; return false; }
-        r.pin_cap = n;
-        c->n_pins++;
+// Page-locked memory for the marked rows of a finished run and of the one that the next decode takes, when rows are read: allocating it can wait for the device, which reading rows may and
+// starting a decode may not.  Without it (more rows than were read before, a fifth run in flight) rows are copied when they are read.  (The largest size at once, 8 MB of 32 000 values, costs
+// the first read 10 ms.)
+static void pin_grow(pib_context * c, pib_run & read) {
+    const int rows = (int) read.marks.size();
+    if (rows > PIB_CHUNK) return;
+    pib_run * next = nullptr;
+    for (auto & r : c->runs) if (!r.in_use && r.id != c->last_finished) { next = &r; break; }        // as pib_take_run
+    for (pib_run * r : { &read, next }) {
+        if (!r || r->pin_rows >= rows || (!r->pin && c->n_pins >= PIB_PINS)) continue;
+        if (r->pin) { cudaFreeHost(r->pin); c->n_pins--; }
+        r->pin = nullptr; r->pin_rows = 1;
+        while (r->pin_rows < rows) r->pin_rows *= 2;
+        if (cudaMallocHost(&r->pin, (size_t) r->pin_rows * c->model->n_vocab * 4) == cudaSuccess) { c->n_pins++; continue; }
+        cudaGetLastError();
+        r->pin = nullptr; r->pin_rows = 0;
     }
+}
+// the marked rows' copies to the run's page-locked memory; false: not enough of it there (or the batch has more rows than a decode batch)
+static bool pin_rows(pib_context * c, pib_run & r) {
+    if (r.marks.empty() || r.marks.back() >= r.n_tokens || !r.logits || r.pin_rows < (int) r.marks.size()) return false;
+    const size_t V = (size_t) c->model->n_vocab;
     for (size_t a = 0, b; a < r.marks.size(); a = b) {                // neighbouring rows in one copy
         for (b = a + 1; b < r.marks.size() && r.marks[b] == r.marks[b - 1] + 1; b++) {}
         if (cudaMemcpyAsync(r.pin + a * V, r.logits + (size_t) r.marks[a] * V, (b - a) * V * 4, cudaMemcpyDeviceToHost, c->stream) != cudaSuccess) { cudaGetLastError(); return false; }
@@ -1300,7 +1310,10 @@ const float * pib_logits_row(pib_context * c, int i) {
     c->rows_asked = true;
     const auto mark = std::lower_bound(r.marks.begin(), r.marks.end(), i);
     if (!remote && mark != r.marks.end() && *mark == i) {
-        if (!r.pinned && pin_rows(c, r)) cudaStreamSynchronize(c->stream);
+        if (!r.pinned) {
+            pin_grow(c, r);
+            if (pin_rows(c, r)) cudaStreamSynchronize(c->stream);
+        }
         if (r.pinned) {
             if (!r.pin_read) c->d2h_bytes += r.marks.size() * V * 4;
             r.pin_read = true;

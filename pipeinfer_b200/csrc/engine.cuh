@@ -92,8 +92,8 @@ struct pib_run {                   // one (possibly still executing) decode: the
     bool         rows_on_host = false;
     int          want_lo = 0, want_hi = 0;   // logits rows that the caller marked in its batch: [want_lo, want_hi) holds all of them
     std::vector<int> marks;                  // rows that cross together, in order: of a batch of up to PIB_CHUNK tokens [want_lo, want_hi), of a longer one the marked rows while no more than PIB_CHUNK
-    float *      pin = nullptr;              // page-locked [marks][n_vocab], pin_cap floats: their copies once `pinned`
-    size_t       pin_cap = 0;
+    float *      pin = nullptr;              // page-locked [pin_rows][n_vocab]: the marked rows' copies once `pinned`
+    int          pin_rows = 0;
     bool         pinned = false, pin_read = false;       // pin_read: some of them were asked for (their bytes are counted then, or when the run is let go)
     bool         cancel_sent = false;        // a cancel flag was written for this run: to be cleared when it is finished
     pib_accept_result * acc_dev = nullptr, * acc_host = nullptr;

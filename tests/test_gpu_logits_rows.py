@@ -88,3 +88,92 @@ def test_bytes_of_rows_nobody_reads(ctx):
         read(ctx, 4, range(4), rows)
         per.append((count() - before) // (4 * V))
     assert per == [4, 0, 4, 0]
+
+
+# rows that cross behind the kernels have memory of their run slot, of PIB_PINS slots
+PINS = 4
+
+
+def fresh():
+    from pipeinfer_b200 import llama
+    return llama.Context(None, n_ctx=256, max_seq=16, synthetic=(2, 256, 4, 2, 512, V, 12, 2, 1, 0.8))
+
+
+def row(ctx, i):
+    return np.ctypeslib.as_array(ctx.L.llama_get_logits_ith(ctx.ctx, i), shape=(V,)).copy()
+
+
+def check_rows(ctx, n):
+    """the finished run's rows are its own: they hold what its sampling kernel found"""
+    for i in reversed(range(n)):
+        r, top = row(ctx, i), ctx.top8(i)
+        assert [float(r[t[0]]) for t in top] == [t[1] for t in top] and r.max() == top[0][1]
+
+
+def test_nothing_is_allocated_while_a_decode_is_started():
+    """rows of a run with more marked rows than were ever read do not cross behind its kernels: only reading makes the memory larger, of the run read and of the next one"""
+    ctx, sent, per = fresh(), C.c_uint64(), []
+    ctx.L.llama_pib_io_bytes.argtypes = [C.c_void_p, C.POINTER(C.c_uint64), C.POINTER(C.c_uint64)]
+    try:
+        for n, rows in [(1, [0]), (16, []), (1, []), (16, [0]), (16, []), (16, [])]:
+            ctx.L.llama_pib_io_bytes(ctx.ctx, C.byref(C.c_uint64()), C.byref(sent))
+            before = sent.value
+            read(ctx, n, range(n), rows)
+            ctx.L.llama_pib_io_bytes(ctx.ctx, C.byref(C.c_uint64()), C.byref(sent))
+            per.append((sent.value - before) // (4 * V))             # rows nobody read count when the next run is finished
+        assert per == [1, 0, 0, 16, 0, 16]
+    finally:
+        ctx.close()
+
+
+def test_rows_with_runs_in_flight():
+    """more of them than there are places, with growing numbers of rows, each read after it is finished while others run"""
+    ctx = fresh()
+    try:
+        ctx.L.llama_kv_cache_clear(ctx.ctx)
+        h, b, keep = ctx.start([3], [0], [[15]])
+        assert ctx.finish(h, b) == 1
+        row(ctx, 0)
+        runs = []
+        for k in range(24):
+            n = 1 + (5 * k) % 9
+            ctx.seq_rm(k % 12, 0, 64)
+            runs.append((n, ctx.start([(31 * k + 7 * i) % V for i in range(n)], list(range(n)), [[k % 12]] * n)))
+            if len(runs) > PINS + 2:
+                n0, (h, b, keep) = runs.pop(0)
+                assert ctx.finish(h, b) == 1
+                check_rows(ctx, n0)
+        for n0, (h, b, keep) in runs:
+            assert ctx.finish(h, b) == 1
+            check_rows(ctx, n0)
+    finally:
+        ctx.close()
+
+
+def test_rows_behind_a_cancelled_run():
+    """runs behind a cancelled one, and the run that gets its slot, have their own rows: those of the same tokens without a cancellation"""
+    ctx = fresh()
+    try:
+        def go(cancel):
+            ctx.L.llama_kv_cache_clear(ctx.ctx)
+            out, runs = [], []
+            for k in range(3):
+                runs.append(ctx.start([40 + 10 * k + i for i in range(4)], list(range(4)), [[k]] * 4, batch_id=100 + k))
+                if k == 1 and cancel:
+                    ctx.L.llama_cancel_run(ctx.ctx, (C.c_int32 * 1)(101), 1)
+            for k, (h, b, keep) in enumerate(runs):
+                assert ctx.finish(h, b) == 1
+                if k != 1:
+                    check_rows(ctx, 4)
+                    out.append(np.stack([row(ctx, i) for i in range(4)]))
+            for k in range(4):                                       # the slots again
+                h, b, keep = ctx.start([70 + k], [0], [[4 + k]], batch_id=110 + k)
+                assert ctx.finish(h, b) == 1
+                check_rows(ctx, 1)
+                out.append(row(ctx, 0)[None])
+            return np.concatenate(out)
+        want = go(False)
+        for _ in range(3):
+            assert np.array_equal(go(True), want)
+    finally:
+        ctx.close()
