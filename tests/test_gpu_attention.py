@@ -1,4 +1,4 @@
-"""RoPE, KV store and attention of a decode batch (csrc/attention_core.cuh) against the reference's order of operations restated in numpy, bit for bit: cells left over behind
+"""RoPE, KV store and attention of a decode batch (csrc/attention.cu) against the reference's order of operations restated in numpy, bit for bit: cells left over behind
 the last multiple of 32, rounds of cells held in registers or not, value rows staged in shared memory or not, the batch's cells at the end of the range, inside it and on
 both sides of the staged rows, masked cells that hold anything."""
 import ctypes as C
