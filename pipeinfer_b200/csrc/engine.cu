@@ -604,10 +604,10 @@ int (*pib_hop_send)(pib_context * c, const float * x, int n_tokens, const int * 
 
 // debugging aid (PIB_DUMP_DIR=<dir>, graphs off): every intermediate of the llama graph goes to <dir>/<name>.<layer>.bin as float32,
 // under the names the oracle uses for the same tensors (PO_DUMP_DIR, oracle/pib_oracle.c), so the two can be compared step by step
-static const char * const dumps = getenv("PIB_DUMP_DIR");
+static const char * dump_dir() { static const char * dir = getenv("PIB_DUMP_DIR"); return dir; }       // as it is at the first decode
 static void dump_dev(const pib_context * c, const char * name, int il, const float * dev, size_t rows, size_t cols, size_t ld) {
-    if (!dumps) return;
-    const char * dir = dumps;
+    const char * dir = dump_dir();
+    if (!dir) return;
     cudaStreamSynchronize(c->stream);
     std::vector<float> h(rows * cols);
     cudaMemcpy2D(h.data(), cols * 4, dev, ld * 4, cols * 4, rows, cudaMemcpyDeviceToHost);
@@ -750,7 +750,7 @@ static int run_chunk_body(pib_context * c, pib_run & run, int chunk, int ntok, i
         dump_dev(c, "o", il, c->proj, ntok, E, E);
         TL(9, il, pib_add_rmsnorm_quantize_act(wt, c->proj, c->x, c->x2, L.ffn_norm, m->rms_eps, ntok, E, c->act, cancel, st, nullptr, lean));   // x2 = ffn_inp
         dump_dev(c, "ffi", il, c->x2, ntok, E, E);
-        if (lean && !dumps && pib_gemv_gated_ok(L.wgu, ntok)) {
+        if (lean && !dump_dir() && pib_gemv_gated_ok(L.wgu, ntok)) {
             TL(2, il, pib_gemv_gated(L.wgu, c->act, ntok, c->gu, cancel, st));
             TL(10, il, pib_quantize_act_c(wt, c->gu, ntok, FF, c->act, cancel, st, nullptr, lean));
         } else {
