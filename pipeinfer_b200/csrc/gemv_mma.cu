@@ -1087,7 +1087,13 @@ static bool ring_wide(int n_tiles, int nsb) {
     return wide_on && n_tiles <= 2 * pib_num_sms() * 2 && (nsb >= 16 || (nsb >= 8 && n_tiles < pib_split_fill_target()));          // <= 2 CTAs of 8 warps per SM
 }
 
-// variant 0 / 2: the ring kernel (cp.async-staged); PIB_Q4K_FAST=direct selects the register-prefetched direct kernel instead
+// K shares of a row tile (PIB_RING_SPLIT=n: n everywhere)
+static int ring_split(int n_tiles, int nsb) {
+    static const int split_env = getenv("PIB_RING_SPLIT") ? atoi(getenv("PIB_RING_SPLIT")) : 0;
+    return split_env > 0 ? split_env : ring_wide(n_tiles, nsb) ? 1 : choose_split_direct(n_tiles, nsb);
+}
+
+// variant 0 / 2: the ring kernel (cp.async-staged)
 int pib_gemv_ring(const pib_weight * w, const void * act_dev, int b, float * y_dev, const int * cancel, cudaStream_t st) {
     if (!pib_gemv_mma_supported(w, b)) { pib_set_error("pib_gemv: variant 2 needs Q4_K weights with tiles"); return PIB_ERR_UNSUPP; }
     const int nsb = (int) (w->K / 256), n_tiles = (int) ((w->N + 15) / 16);
@@ -1098,8 +1104,7 @@ int pib_gemv_ring(const pib_weight * w, const void * act_dev, int b, float * y_d
     // K shares, which meet through memory (K = 2048, shares / eight warps, us: 2560 rows at 1 token 3.5 / 2.0, at 12 5.2 / 4.1; 4096 at 1 4.0 / 2.2); tiles enough to go
     // without shares keep four warps (8192 rows: 3.1 / 4.2)
     const bool wide = ring_wide(n_tiles, nsb);
-    static const int split_env = getenv("PIB_RING_SPLIT") ? atoi(getenv("PIB_RING_SPLIT")) : 0;
-    const int  split = fit_split(split_env > 0 ? split_env : wide ? 1 : choose_split_direct(n_tiles, nsb), b, w->N, n_tiles);
+    const int  split = fit_split(ring_split(n_tiles, nsb), b, w->N, n_tiles);
     mm_scratch * s = nullptr;
     if (split > 1 && ensure_scratch((size_t) split * b * w->N, (size_t) n_tiles, st, &s) != PIB_OK) { pib_set_error("pib_gemv: scratch allocation failed"); return PIB_ERR_NOMEM; }
     const pib_act_layout L   = pib_act_layout_of(w->type, w->K, b);
@@ -1117,7 +1122,7 @@ int pib_gemv_ring(const pib_weight * w, const void * act_dev, int b, float * y_d
 bool pib_gemv_gated_ok(const pib_weight * w, int b) {
     if (!pib_gemv_mma_supported(w, b) || w->N % 32) return false;
     const int nsb = (int) (w->K / 256), n_tiles = (int) (w->N / 16);
-    return !ring_wide(n_tiles, nsb) && choose_split_direct(n_tiles, nsb) == 1;
+    return !ring_wide(n_tiles, nsb) && ring_split(n_tiles, nsb) == 1;
 }
 int pib_gemv_gated(const pib_weight * w, const void * act_dev, int b, float * y_dev, const int * cancel, cudaStream_t st) {
     if (!pib_gemv_gated_ok(w, b)) { pib_set_error("pib_gemv_gated: not for this matrix"); return PIB_ERR_UNSUPP; }

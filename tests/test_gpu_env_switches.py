@@ -24,3 +24,16 @@ def test_dumps_of_a_program_that_asks_for_them_before_its_first_decode(tmp_path)
     for il in range(2):
         gate, up = (np.fromfile(tmp_path / f"{n}.{il}.bin", np.float32) for n in ("gate", "up"))
         assert gate.shape == up.shape == (3 * 512,) and np.isfinite(gate).all() and gate.any() and up.any()
+
+
+@pytest.mark.gpu
+def test_k_shares_of_every_matmul(tmp_path):
+    """PIB_RING_SPLIT reaches the gate and up matmul of a decode batch also where its product would be formed behind it (with dumps it is not: the same bits with and without)"""
+    out = []
+    for k, env in enumerate([{}, {"PIB_DUMP_DIR": str(tmp_path)}]):
+        path = tmp_path / f"logits{k}.npy"
+        child("import numpy as np\nfrom pipeinfer_b200 import llama\n"
+              "c = llama.Context(None, n_ctx=64, max_seq=2, synthetic=(4, 2048, 32, 4, 5632, 512, 12, 2, 0, 0.0))\n"
+              f"np.save({str(path)!r}, c.decode([1, 2, 3], [0, 1, 2], [[0]] * 3)[1])\nc.close()\n", PIB_GRAPHS="0", PIB_RING_SPLIT="2", **env)
+        out.append(np.load(path))
+    assert np.array_equal(out[0], out[1])
