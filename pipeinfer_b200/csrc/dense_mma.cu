@@ -17,6 +17,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -176,7 +177,7 @@ static dt_encode_fn dt_encode() {
 }
 
 // per (device, stream): the bfloat16 staging of the activations and the error word of the kernels' bounded waits
-struct dt_scratch { __nv_bfloat16 * xs = nullptr; size_t cap = 0; int * err = nullptr; int * err_host = nullptr; uint64_t uses = 0; };     // uses: launches that got the error word
+struct dt_scratch { __nv_bfloat16 * xs = nullptr; size_t cap = 0; int * err = nullptr; int * err_host = nullptr; std::atomic<uint64_t> uses { 0 }; };     // uses: launches that got the error word (threads may share a stream)
 static dt_scratch * dt_scratch_of(cudaStream_t st, size_t bytes) {
     static std::map<std::pair<int, cudaStream_t>, dt_scratch> all;
     static std::mutex mu;
