@@ -212,7 +212,7 @@ int pib_tma_map3(CUtensorMap * map, const void * base, uint64_t d0, uint64_t d1,
 }
 
 int * pib_tc_error_word(cudaStream_t st) { dt_scratch * sc = dt_scratch_of(st, 0); if (sc) sc->uses++; return sc ? sc->err : nullptr; }
-uint64_t pib_tc_uses(cudaStream_t st) { dt_scratch * sc = dt_scratch_of(st, 0); return sc ? sc->uses : 0; }
+uint64_t pib_tc_uses(cudaStream_t st) { dt_scratch * sc = dt_scratch_of(st, 0); return sc ? sc->uses.load() : 0; }
 
 template <int NB>
 static int dt_launch(const pib_mm & a, const CUtensorMap & wmap, const CUtensorMap & xmap, int x_has_z, int * err, cudaStream_t st) {
