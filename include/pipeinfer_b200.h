@@ -132,6 +132,9 @@ int    pib_gemm(const pib_weight * w, const void * act_dev, int b, float * y_dev
 /* pib_gemm returns when the launch is made.  Every wait inside the kernel is bounded; one that runs out leaves y_dev unwritten in places and the stream's error
  * word set.  This call waits for the stream and returns 0, or PIB_ERR_CUDA when that has happened to any pib_gemm on it since the last check. */
 int    pib_gemm_check(pib_stream s);
+/* K shares of each row block in which pib_gemm forms a matmul of N x K and b tokens on the current device (of its last blocks where those in front are whole rounds of the
+ * GPU); groups (or null): 1 two CTAs per SM of one group of dequantising warps, 2 one CTA of two.  -1: not a shape of pib_gemm. */
+int    pib_gemm_shares(int64_t N, int64_t K, int b, int * groups);
 int    pib_quantize_act_rows(int wtype, const float * x_dev, int b, int64_t K, void * act_dev, pib_stream s);
 
 /* ---- K3: embedding rows ---------------------------------------------------------------------------------------- */

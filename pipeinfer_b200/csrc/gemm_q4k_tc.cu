@@ -436,18 +436,10 @@ static int tg_launch(const pib_weight * w, const __half * xh, int b, int x0, int
     return PIB_OK;
 }
 
-// y[b][N] = W x^; act_dev = the Q8_K activation planes of `b` tokens (act_quant.cu), xhat_dev = scratch of pib_gemm_xhat_bytes; or act_dev = null and xhat_dev already
-// written by the quantiser (51 launches of 4 us in a 700-token prompt through four layers)
-int pib_gemm_q4k_tc(const pib_weight * w, const void * act_dev, int b, float * y_dev, void * xhat_dev, cudaStream_t st) {
-    if (!w || w->type != PIB_TYPE_Q4_K || !w->tiles || b < 1 || b > PIB_PROMPT_MAX) { pib_set_error("pib_gemm: needs Q4_K tiles and 1 <= b <= %d", PIB_PROMPT_MAX); return PIB_ERR_ARG; }
-    const pib_act_layout L = pib_act_layout_of(PIB_TYPE_Q4_K, w->K, b);
-    const uint8_t * act = (const uint8_t *) act_dev;
-    __half * xh = (__half *) xhat_dev;
-    const int64_t n16 = (int64_t) b * (w->K / 16);
-    if (act && b > PIB_MAX_BATCH) { xh = (__half *) (const_cast<uint8_t *>(act) + L.qsl_off); act = nullptr; }      // the quantiser has written the operand
-    if (act) pib_launch(tg_xhat_kernel, dim3((unsigned) ((n16 + 255) / 256)), dim3(256), 0, st, (const int8_t *) (act + L.qs_off), (const float *) (act + L.d_off), n16, (int) (w->K / 16), xh);
-    PIB_CHECK(cudaGetLastError());
-    const int NB = tg_nb_of(b), nsb = (int) (w->K / 256), nx = (int) ((w->N + TG_BM - 1) / TG_BM) * tg_tiles_of(b), sms = pib_num_sms();
+// The launches of a matmul of N x K and b tokens: blocks [0, full) and behind them `rest`, each with its K shares; G groups of dequantising warps per CTA (1: two CTAs per SM).
+struct tg_plan { int G, full, s_full, rest, s_rest; };
+static tg_plan tg_plan_of(int64_t N, int64_t K, int b) {
+    const int NB = tg_nb_of(b), nsb = (int) (K / 256), nx = (int) ((N + TG_BM - 1) / TG_BM) * tg_tiles_of(b), sms = pib_num_sms();
     // K shares of n blocks, with G groups, whose clusters all find room at once; every share keeps at least two super-blocks.  With two CTAs per SM, S of them need
     // the room of S / 2, less a sixteenth that packing loses (occupancy queries count one CTA of this kernel per SM; of 4 CTAs 70 clusters ran at once, 72 did not).
     // us at 34 and 37 blocks of K = 4096 / 100 tokens and 17 of 8192 / 256, shares by room / by SMs alone: 16.9 / 22.5, 16.8 / 22.8, 22.6 / 31.6.
@@ -467,20 +459,40 @@ int pib_gemm_q4k_tc(const pib_weight * w, const void * act_dev, int b, float * y
     // 10240 x 8192 (80) 31.4 / 33.4 and 33.8 / 42.7, 22016 x 4096 (172) 35.5 / 29.4 and 39.5 / 34.7, 8192 x 28672 (64, in 2 / 4 shares) 54.2 / 49.1 and 68.5 / 67.7.
     // Above 128 tokens the accumulator takes half of the tensor memory: one.
     const bool two = NB <= 128 && (nx > sms || (NB <= 64 && shares(nx, 2) > 1));
-    if (two || three) {
-        const int S = three ? 3 : shares(nx, 1);
-        switch (NB) {
-            case 32: return tg_launch<32, 1>(w, xh, b, 0, nx, S, y_dev, st);
-            case 64: return tg_launch<64, 1>(w, xh, b, 0, nx, S, y_dev, st);
-            case 96: return tg_launch<96, 1>(w, xh, b, 0, nx, S, y_dev, st);
-            default: return tg_launch<128, 1>(w, xh, b, 0, nx, S, y_dev, st);
-        }
-    }
+    if (two || three) return { 1, nx, three ? 3 : shares(nx, 1), 0, 1 };
     // whole rounds of one CTA per SM, then what is left over in K shares (448 row blocks are three rounds and four blocks)
     int full = nx / sms * sms, rest = nx - full;
     if (full > 0 && shares(rest, 2) == 1) { full = nx; rest = 0; }
-    auto go = [&](int x0, int n) {
-        const int S = shares(n, 2);
+    return { 2, full, full > 0 ? shares(full, 2) : 1, rest, rest > 0 ? shares(rest, 2) : 1 };
+}
+extern "C" int pib_gemm_shares(int64_t N, int64_t K, int b, int * groups) {
+    if (N <= 0 || K <= 0 || K % 256 || b < 1 || b > PIB_PROMPT_MAX) return -1;
+    const tg_plan p = tg_plan_of(N, K, b);
+    if (groups) *groups = p.G;
+    return p.rest ? p.s_rest : p.s_full;
+}
+
+// y[b][N] = W x^; act_dev = the Q8_K activation planes of `b` tokens (act_quant.cu), xhat_dev = scratch of pib_gemm_xhat_bytes; or act_dev = null and xhat_dev already
+// written by the quantiser (51 launches of 4 us in a 700-token prompt through four layers)
+int pib_gemm_q4k_tc(const pib_weight * w, const void * act_dev, int b, float * y_dev, void * xhat_dev, cudaStream_t st) {
+    if (!w || w->type != PIB_TYPE_Q4_K || !w->tiles || b < 1 || b > PIB_PROMPT_MAX) { pib_set_error("pib_gemm: needs Q4_K tiles and 1 <= b <= %d", PIB_PROMPT_MAX); return PIB_ERR_ARG; }
+    const pib_act_layout L = pib_act_layout_of(PIB_TYPE_Q4_K, w->K, b);
+    const uint8_t * act = (const uint8_t *) act_dev;
+    __half * xh = (__half *) xhat_dev;
+    const int64_t n16 = (int64_t) b * (w->K / 16);
+    if (act && b > PIB_MAX_BATCH) { xh = (__half *) (const_cast<uint8_t *>(act) + L.qsl_off); act = nullptr; }      // the quantiser has written the operand
+    if (act) pib_launch(tg_xhat_kernel, dim3((unsigned) ((n16 + 255) / 256)), dim3(256), 0, st, (const int8_t *) (act + L.qs_off), (const float *) (act + L.d_off), n16, (int) (w->K / 16), xh);
+    PIB_CHECK(cudaGetLastError());
+    const tg_plan p = tg_plan_of(w->N, w->K, b);
+    const int NB = tg_nb_of(b);
+    auto go = [&](int x0, int n, int S) {
+        if (p.G == 1)
+            switch (NB) {
+                case 32: return tg_launch<32, 1>(w, xh, b, x0, n, S, y_dev, st);
+                case 64: return tg_launch<64, 1>(w, xh, b, x0, n, S, y_dev, st);
+                case 96: return tg_launch<96, 1>(w, xh, b, x0, n, S, y_dev, st);
+                default: return tg_launch<128, 1>(w, xh, b, x0, n, S, y_dev, st);
+            }
         switch (NB) {
             case 32:  return tg_launch<32, 2>(w, xh, b, x0, n, S, y_dev, st);
             case 64:  return tg_launch<64, 2>(w, xh, b, x0, n, S, y_dev, st);
@@ -491,8 +503,8 @@ int pib_gemm_q4k_tc(const pib_weight * w, const void * act_dev, int b, float * y
         }
     };
     int rc = PIB_OK;
-    if (full > 0) rc = go(0, full);
-    if (rc == PIB_OK && rest > 0) rc = go(full, rest);
+    if (p.full > 0) rc = go(0, p.full, p.s_full);
+    if (rc == PIB_OK && p.rest > 0) rc = go(p.full, p.rest, p.s_rest);
     return rc;
 }
 

@@ -32,3 +32,17 @@ def test_three_shares(N, K, b):
     for r in range(0, N, 1600):                                      # the reference in pieces of rows
         want, bound = shapes.reference(w[r:r + 1600], x)
         assert (np.abs(ys[0][:, r:r + 1600] - want) <= bound).all()
+
+
+@pytest.mark.parametrize("N,K,b,shares,groups", [
+    (9600, 4608, 24, 3, 1), (11520, 4608, 64, 3, 1), (11515, 4864, 33, 3, 1), (11528, 4608, 40, 1, 2), (9472, 4608, 40, 2, 1), (9601, 8192, 100, 3, 1), (10368, 8192, 128, 3, 1), (10496, 8192, 97, 1, 2),
+    (4352, 1536, 100, 3, 2), (4992, 1792, 180, 3, 2), (4355, 2048, 256, 3, 2), (5120, 1280, 97, 2, 2), (6000, 1536, 130, 2, 2)])
+def test_route(N, K, b, shares, groups):
+    """which of the shapes above take three shares"""
+    from pipeinfer_b200 import load
+    lib = load()
+    lib.init(0)
+    lib.L.pib_gemm_shares.argtypes = [C.c_int64, C.c_int64, C.c_int, C.POINTER(C.c_int)]
+    g = C.c_int()
+    assert (lib.L.pib_gemm_shares(N, K, b, C.byref(g)), g.value) == (shares, groups)
+    assert lib.L.pib_gemm_shares(N, K + 1, b, None) == lib.L.pib_gemm_shares(0, K, b, None) == lib.L.pib_gemm_shares(N, K, 0, None) == -1
