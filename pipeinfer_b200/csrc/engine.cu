@@ -505,8 +505,6 @@ static pib_context * hybrid_context_new(pib_model * m, uint32_t n_ctx, int max_s
     CK(cudaMemset(c->cancel_table, 0, 128 * sizeof(int)));
     c->cancel_one = c->cancel_table + 100;
     { int one = 1; CK(cudaMemcpy(c->cancel_one, &one, 4, cudaMemcpyHostToDevice)); }
-    CK(cudaMallocHost(&c->run_id_host, 64 * sizeof(int)));
-    for (int i = 0; i < 64; i++) c->run_id_host[i] = i;
     c->desc_stride = pib_desc_stride(c->n_words);
     c->desc_slots  = 1;                                   // one zeroed descriptor: the sampler's launch contract
     CK(cudaMalloc(&c->desc_dev, c->desc_stride * 2));
