@@ -205,7 +205,13 @@ __global__ void __launch_bounds__(1024) act_quant_kernel(const aq_args a) {
             for (int k = 0; k < 8; k++) amax = fmaxf(amax, fabsf(v[k]));
             amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
             amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-            const float d = amax / 127.f, id = amax != 0.0f ? 127.f / amax : 0.0f;
+            const float d = amax / 127.f;
+            float       id = amax != 0.0f ? 127.f / amax : 0.0f;
+            if (id > 3.4028235e38f) {                                 // overflow (scale 0): the reference's conversion gives the lowest whole number for every element
+                id = 128.f;
+#pragma unroll
+                for (int k = 0; k < 8; k++) v[k] = -1.f;
+            }
             int q[8];
 #pragma unroll
             for (int k = 0; k < 8; k++) q[k] = __float2int_rn(__fmul_rn(v[k], id));

@@ -38,9 +38,10 @@ __device__ __forceinline__ void q8k_quantise_sb(const float (&v)[8], int lane, i
     amax = wmax;
     int   q[8];
     float dval = 0.0f;
-    if (amax == 0.0f) {
+    if (amax <= 0x1p-121f) {                                               // zeros, or -128 / mx overflows: the reference's whole numbers are 0 then, its scale 1 / iscale
 #pragma unroll
         for (int j = 0; j < 8; j++) q[j] = 0;
+        if (amax != 0.0f) dval = copysignf(0.0f, -mx);
     } else {
         const float iscale = -128.f / mx;
 #pragma unroll

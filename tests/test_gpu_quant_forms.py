@@ -117,6 +117,21 @@ def test_forms(lib, oracle, tables, wt, K, b, off):
 
 
 @pytest.mark.parametrize("wt", [Q4_0, Q8_0, Q4_K])
+def test_tiny_maxima(lib, oracle, wt):
+    """blocks whose largest value is so small that the factor overflows, around that border and at the smallest numbers: the reference's bytes"""
+    K, edge = 256 * 12, np.float32(2.0 ** -121 if wt == Q4_K else 127.0 / float(np.finfo(np.float32).max))
+    tops = [0.0, edge, np.nextafter(edge, np.float32(1)), np.nextafter(edge, np.float32(0)), 1e-38, 1e-45, 3e-37, 4e-37, 1e-36, 1e-40, -1e-38, -edge]
+    x = np.random.default_rng(1).uniform(-1, 1, (12, 256)).astype(np.float32)
+    x[:, ::7] = 0
+    x /= np.abs(x).max(1, keepdims=True)
+    x = (x.astype(np.float64) * np.array(tops, np.float64)[:, None]).astype(np.float32)
+    x[:, 3] = tops
+    x = x.reshape(1, K)
+    with np.errstate(all="ignore"):
+        assert np.array_equal(lib.quantize_act(wt, x), oracle.quantize_act(wt, x))
+
+
+@pytest.mark.parametrize("wt", [Q4_0, Q8_0, Q4_K])
 @pytest.mark.parametrize("b", [1, 5, 8, 9, 16])
 def test_lean_planes(lib, wt, b):
     """a matmul behind the lean form reads the same planes as behind the general one"""
