@@ -164,8 +164,8 @@ template <int RPL> __device__ __forceinline__ void kva_merge(const float * base,
     }
 }
 // EARLY: every segment of the batch is one token, so that all rows but the token's own were final before the launch in front started; the first trip's rows and biases are fetched
-// before the wait on it, and a trip's rows while the one before is worked on (4 tokens, 16 heads of 128, about 100 keys: 10.4 us of a step's chain, now 7.7).  Prompts go without (with both
-// 155 us where 143 without, 4 prompts of 90 tokens): it costs registers (heads of up to 64 coordinates 80 instead of 64, one block of 512 threads per SM instead of two; of 128 127 instead of
+// before the wait on it, and a trip's rows while the one before is worked on (4 tokens, 16 heads of 128, about 100 keys: 10.4 us of a step's chain, now 7.7).  Prompts go without (their
+// launch takes 143 us without and 155 with a trip ahead): it costs registers (heads of up to 64 coordinates 80 instead of 64, one block of 512 threads per SM instead of two; of 128 127 instead of
 // 85, of 32 64 instead of 56: one block, and two, either way).
 template <int RPL, int UK, bool EARLY>
 __global__ void __launch_bounds__(512) kv_attn_kernel(kva_args A) {
